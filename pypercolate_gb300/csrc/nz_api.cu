@@ -151,7 +151,7 @@ int nz_microcanonical(const NzGraph *graph, int32_t spanning, int32_t n_runs, in
     micro_layout(c, g, n_runs, perm_mode, &nodes, &state, &flag, &mt_perms);
     if (!workspace || !c.ok()) return NZ_ERR_WORKSPACE;
     cudaStream_t s = as_stream(stream);
-    launch_init_runs(g, n_runs, nodes, state, flag, s);
+    const uint32_t *init_flag = launch_init_runs(g, n_runs, nodes, state, flag, s);
     const uint32_t *perm_src = perms;
     int mode = perm_mode;
     if (perm_mode == NZ_PERM_MT19937) {
@@ -171,6 +171,8 @@ int nz_microcanonical(const NzGraph *graph, int32_t spanning, int32_t n_runs, in
     p.perms = perm_src;
     p.rec = *out;
     p.errors = nullptr;
+    p.init_flag = init_flag;
+    p.tiled = false;
     {
         ProfScope prof(NZ_PROF_UNION_FIND, s);
         launch_uf_window(p, mode, spanning != 0, n_runs >= 128 ? 128 : 32, s);
@@ -302,6 +304,7 @@ int nz_canonical_statistics_records(const NzRecords *rec, uint32_t num_nodes, ui
     p.conv_tile = 8;
     p.acc = out;
     p.errors = nullptr;
+    p.tiled = false;
     launch_conv_window(p, 0, s);
     return check_launch();
 }
@@ -345,6 +348,7 @@ int nz_microcanonical_reduce(const NzRecords *rec, uint32_t num_nodes, uint32_t 
     if (!acc->count || !acc->span_count || !acc->sum_lo || !acc->sum_hi || !acc->m2) return NZ_ERR_INVALID;
     MicroParams mp;
     mp.rec = *rec;
+    mp.tiled = false;
     mp.n_begin = n_begin;
     mp.n_end = n_end;
     mp.N = num_nodes;
@@ -508,7 +512,9 @@ size_t ensemble_layout(Carver &c, const GraphDev &g, int32_t n_runs, int32_t P, 
     L.nodes = c.take<uint32_t>((size_t)n_runs * g.slots);
     L.state = c.take<RunState>((size_t)n_runs);
     L.flag = c.take<uint32_t>(4);
-    const size_t plane = (size_t)L.window * n_runs;
+    // bond ensembles write tiled records: whole tiles of 32 rows
+    const size_t rows = lattice_extension(g) ? (size_t)L.window : ((size_t)L.window + 31) / 32 * 32;
+    const size_t plane = rows * n_runs;
     for (int b = 0; b < 2; ++b) {
         NzRecords &r = L.rec[b];
         // up to N = 65,536 nodes m0 (< 2^16) and m2 (<= N^2/4) are stored in
@@ -634,8 +640,11 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
     up.key = key;
     up.run0 = run0;
     up.perms = nullptr;
+    up.init_flag = nullptr;
+    up.tiled = !lattice_extension(g);
     up.errors = L.flag + 1;  // zeroed in the set-up; read by nz_ensemble_errors
     ConvParams cp;
+    cp.tiled = up.tiled;
     cp.N = N;
     cp.n_runs = n_runs;
     cp.spanning = spanning;
@@ -654,6 +663,7 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
     cp.errors = L.flag + 1;  // with the union-find's corruption count
     MicroParams mp;
     if (micro) {
+        mp.tiled = up.tiled;
         mp.N = N;
         mp.n_runs = n_runs;
         mp.acc = *micro;

@@ -14,6 +14,7 @@
 #include "nz_internal.cuh"
 #include "nz_math.cuh"
 #include "nz_records.cuh"
+#include "nz_wide.cuh"
 
 namespace nz {
 
@@ -393,6 +394,126 @@ __device__ __forceinline__ void conv_rows_max(const ConvParams &p, uint32_t c0, 
     }
 }
 
+// ---- the same sums over tiled records.  A chunk's rows are read in groups of
+// 8 (16-byte loads of one run's consecutive rows, kTileAhead groups in flight)
+// from the group that holds its first row; s_w row 0 is that group's first row
+// and rows outside the chunk have zero weights, which leave every FP32 partial
+// sum as it is.  Rows are added in increasing order, chunk by chunk, as above.
+constexpr int kTileAhead = 3;
+
+template <int S>
+using tile_raw = typename std::conditional<S == 8, uint16_t,
+                                           typename std::conditional<S == 4 || S == 5 || S == 6 || S == 7, uint64_t,
+                                                                     uint32_t>::type>::type;
+template <int S>
+__device__ __forceinline__ const tile_raw<S> *tile_plane(const NzRecords &rec) {
+    if constexpr (S == 0 || S == 1 || S == 3) return rec.max_span;
+    else if constexpr (S == 2) return rec.m0;
+    else if constexpr (S == 4) return rec.m2;
+    else if constexpr (S == 5) return rec.m3;
+    else if constexpr (S == 8) return reinterpret_cast<const uint16_t *>(rec.m0);
+    else if constexpr (S == 9) return reinterpret_cast<const uint32_t *>(rec.m2);
+    else return rec.m4_lo;
+}
+template <int PRECISION, int S>
+__device__ __forceinline__ auto tile_value(tile_raw<S> q, uint32_t hi) {
+    if constexpr (PRECISION == 0) {
+        if constexpr (S == 6) return fma((double)hi, 18446744073709551616.0, (double)q);
+        else return (double)q;
+    } else {
+        if constexpr (S == 6) return fmaf((float)hi, 18446744073709551616.0f, u64_to_f32(q));
+        else if constexpr (sizeof(tile_raw<S>) == 8) return u64_to_f32(q);
+        else return (float)q;
+    }
+}
+
+// calls step(row group index k, loaded groups) for the 8-row groups of
+// [first, first + 8 * groups) of run r, kTileAhead of them in flight
+template <int AHEAD, typename Raw, typename Load, typename Step>
+__device__ __forceinline__ void for_groups(uint32_t groups, Load load, Step step) {
+    Raw q[AHEAD];
+#pragma unroll
+    for (int a = 0; a < AHEAD; ++a)
+        if ((uint32_t)a < groups) load(a, q[a]);
+    for (uint32_t k = 0; k < groups; k += AHEAD) {
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a) {
+            if (k + a >= groups) break;
+            const Raw cur = q[a];
+            if (k + a + AHEAD < groups) load(k + a + AHEAD, q[a]);
+            step(k + a, cur);
+        }
+    }
+}
+
+template <int PRECISION, int S, int kConvPT>
+__device__ __forceinline__ void conv_rows_tiled(const ConvParams &p, uint32_t first, uint32_t groups, int r,
+                                                const typename std::conditional<PRECISION == 0, double, float>::type (*s_w)[kConvPT],
+                                                ConvAcc<PRECISION> *acc) {
+    using wtype = typename std::conditional<PRECISION == 0, double, float>::type;
+    struct Raw {
+        tile_raw<S> q[8];
+        uint32_t hi[S == 6 ? 8 : 1];
+    };
+    wtype part[kConvPT];
+#pragma unroll
+    for (int j = 0; j < kConvPT; ++j) part[j] = 0;
+    for_groups<(sizeof(tile_raw<S>) == 8 ? 2 : kTileAhead), Raw>(
+        groups,
+        [&](uint32_t k, Raw &q) {
+            const size_t off = record_off(p.rec, true, first + 8 * k, r);
+            load_rows8(tile_plane<S>(p.rec), off, q.q);
+            if constexpr (S == 6) load_rows8(p.rec.m4_hi, off, q.hi);
+        },
+        [&](uint32_t k, const Raw &q) {
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const wtype v = tile_value<PRECISION, S>(q.q[b], S == 6 ? q.hi[S == 6 ? b : 0] : 0u);
+#pragma unroll
+                for (int j = 0; j < kConvPT; ++j) part[j] = fma(s_w[8 * k + b][j], v, part[j]);
+            }
+        });
+#pragma unroll
+    for (int j = 0; j < kConvPT; ++j) acc[j].add(part[j]);
+}
+
+template <int PRECISION, int kConvPT>
+__device__ __forceinline__ void conv_rows_max_tiled(const ConvParams &p, uint32_t first, uint32_t groups, int r,
+                                                    const typename std::conditional<PRECISION == 0, double, float>::type (*s_w)[kConvPT],
+                                                    ConvAcc<PRECISION> *acc0, ConvAcc<PRECISION> *acc1,
+                                                    ConvAcc<PRECISION> *acc3) {
+    using wtype = typename std::conditional<PRECISION == 0, double, float>::type;
+    struct Raw {
+        uint32_t q[8];
+    };
+    wtype p0[kConvPT], p1[kConvPT], p3[kConvPT];
+#pragma unroll
+    for (int j = 0; j < kConvPT; ++j) p0[j] = p1[j] = p3[j] = 0;
+    for_groups<kTileAhead, Raw>(
+        groups, [&](uint32_t k, Raw &q) { load_rows8(p.rec.max_span, record_off(p.rec, true, first + 8 * k, r), q.q); },
+        [&](uint32_t k, const Raw &q) {
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const uint32_t mx = q.q[b] & ~kSpanBit;
+                const wtype q0 = (q.q[b] & kSpanBit) ? (wtype)1 : (wtype)0;
+                const wtype q1 = (wtype)mx, q3 = (wtype)(p.N - mx);
+#pragma unroll
+                for (int j = 0; j < kConvPT; ++j) {
+                    const wtype w = s_w[8 * k + b][j];
+                    p0[j] = fma(w, q0, p0[j]);
+                    p1[j] = fma(w, q1, p1[j]);
+                    p3[j] = fma(w, q3, p3[j]);
+                }
+            }
+        });
+#pragma unroll
+    for (int j = 0; j < kConvPT; ++j) {
+        acc0[j].add(p0[j]);
+        acc1[j].add(p1[j]);
+        acc3[j].add(p3[j]);
+    }
+}
+
 // Each thread accumulates the kConvPT canonical values of its run over the
 // window's rows, with the tile's weights staged in shared memory (zero
 // outside each p's band).  PRECISION 0: FP64 products and sums.  PRECISION 1:
@@ -407,10 +528,13 @@ __device__ __forceinline__ void conv_rows_max(const ConvParams &p, uint32_t c0, 
 #else
 #define NZ_CONV_BOUNDS __launch_bounds__(kConvRuns)
 #endif
-template <int PRECISION, bool SITE, bool MAXSET, int kConvPT>
+enum class Layout { kBond, kSite, kTiled };  // n-major bond records, n-major site records, tiled bond records
+
+template <int PRECISION, Layout LAYOUT, bool MAXSET, int kConvPT>
 __global__ void NZ_CONV_BOUNDS conv_window_kernel(ConvParams p) {
     using wtype = typename std::conditional<PRECISION == 0, double, float>::type;
-    __shared__ wtype s_w[kConvChunk][kConvPT];
+    constexpr bool SITE = LAYOUT == Layout::kSite, TILED = LAYOUT == Layout::kTiled;
+    __shared__ wtype s_w[kConvChunk + (TILED ? 8 : 0)][kConvPT];
     __shared__ uint32_t s_lo[kConvPT], s_len[kConvPT];
     __shared__ uint32_t s_range[2];
     const int r = blockIdx.x * kConvRuns + threadIdx.x;
@@ -439,19 +563,39 @@ __global__ void NZ_CONV_BOUNDS conv_window_kernel(ConvParams p) {
     ConvAcc<PRECISION> acc[kConvPT], acc0[MAXSET ? kConvPT : 1], acc3[MAXSET ? kConvPT : 1];
     for (uint32_t c0 = nlo; c0 < nhi; c0 += kConvChunk) {
         const uint32_t cn = min((uint32_t)kConvChunk, nhi - c0);
+        // tiled: rows of the 8-row group that holds c0 come first
+        const uint32_t lead = TILED ? (c0 - p.n_begin) & 7u : 0u;
         __syncthreads();
-        for (int i = threadIdx.x; i < kConvChunk * kConvPT; i += kConvRuns) {
+        for (int i = threadIdx.x; i < (kConvChunk + (TILED ? 8 : 0)) * kConvPT; i += kConvRuns) {
             const int row = i / kConvPT, j = i % kConvPT;
-            const uint32_t n = c0 + row;
+            const uint32_t n = c0 + row - lead;
             wtype v = 0;
-            if (row < (int)cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
+            if ((uint32_t)row - lead < cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
                 const size_t widx = (size_t)(p0 + j) * p.cap + (n - s_lo[j]);
                 v = PRECISION == 0 ? (wtype)p.w64[widx] : (wtype)p.w32[widx];
             }
             s_w[row][j] = v;
         }
         __syncthreads();
-        if (r < p.n_runs) {
+        if constexpr (TILED) {
+            if (r < p.n_runs) {
+                const uint32_t first = c0 - p.n_begin - lead, groups = (lead + cn + 7u) / 8u;
+                if (MAXSET) {
+                    conv_rows_max_tiled<PRECISION, kConvPT>(p, first, groups, r, s_w, acc0, acc, acc3);
+                } else if (s == 2) {
+                    if (p.rec.narrow) conv_rows_tiled<PRECISION, 8, kConvPT>(p, first, groups, r, s_w, acc);
+                    else conv_rows_tiled<PRECISION, 2, kConvPT>(p, first, groups, r, s_w, acc);
+                } else if (s == 4) {
+                    if (p.rec.narrow) conv_rows_tiled<PRECISION, 9, kConvPT>(p, first, groups, r, s_w, acc);
+                    else conv_rows_tiled<PRECISION, 4, kConvPT>(p, first, groups, r, s_w, acc);
+                } else if (s == 5) {
+                    conv_rows_tiled<PRECISION, 5, kConvPT>(p, first, groups, r, s_w, acc);
+                } else {
+                    if (p.rec.m4_hi) conv_rows_tiled<PRECISION, 6, kConvPT>(p, first, groups, r, s_w, acc);
+                    else conv_rows_tiled<PRECISION, 7, kConvPT>(p, first, groups, r, s_w, acc);
+                }
+            }
+        } else if (r < p.n_runs) {
             if (MAXSET) {
                 conv_rows_max<PRECISION, SITE, kConvPT>(p, c0, cn, r, s_w, acc0, acc, acc3);
             } else {
@@ -568,9 +712,10 @@ constexpr int kM2Batch = NZ_M2_BATCH;
 // on the same box 8 gave 1085.8 and 1204.7 ms per 100,000-run L = 256 step
 // against 1108.8 and 1224.7 ms for 16 (two boxes); 32 measured 1285 against
 // 1128 ms for 16)
-template <bool NARROW, int kM2PT>
+template <bool NARROW, int kM2PT, bool TILED>
 __global__ void NZ_CONV_BOUNDS conv_m2_comp_kernel(ConvParams p) {
-    __shared__ float s_wh[kConvChunk][kM2PT], s_wl[kConvChunk][kM2PT];
+    constexpr int kRows = kConvChunk + (TILED ? 8 : 0);
+    __shared__ float s_wh[kRows][kM2PT], s_wl[kRows][kM2PT];
     __shared__ uint32_t s_lo[kM2PT], s_len[kM2PT], s_clo[kM2PT], s_clen[kM2PT];
     __shared__ uint32_t s_range[2];
     const int r = blockIdx.x * kConvRuns + threadIdx.x;
@@ -602,12 +747,13 @@ __global__ void NZ_CONV_BOUNDS conv_m2_comp_kernel(ConvParams p) {
 #pragma unroll
         for (int j = 0; j < kM2PT; ++j)
             core |= s_clen[j] && s_clo[j] < c0 + cn && c0 < s_clo[j] + s_clen[j];
+        const uint32_t lead = TILED ? (c0 - p.n_begin) & 7u : 0u;
         __syncthreads();
-        for (int i = threadIdx.x; i < kConvChunk * kM2PT; i += kConvRuns) {
+        for (int i = threadIdx.x; i < kRows * kM2PT; i += kConvRuns) {
             const int rw = i / kM2PT, j = i % kM2PT;
-            const uint32_t n = c0 + rw;
+            const uint32_t n = c0 + rw - lead;
             float vh = 0.0f, vl = 0.0f;
-            if (rw < (int)cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
+            if ((uint32_t)rw - lead < cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
                 const size_t widx = (size_t)(p0 + j) * p.cap + (n - s_lo[j]);
                 vh = p.w32[widx];
                 vl = p.w32lo[widx];
@@ -627,6 +773,40 @@ __global__ void NZ_CONV_BOUNDS conv_m2_comp_kernel(ConvParams p) {
             if constexpr (NARROW) split_u32(w, qh, ql);
             else split_u64(w, qh, ql);
         };
+        if constexpr (TILED) {
+            // a row outside the chunk has zero weights: a compensated term of
+            // zeros leaves (s, c) as they are
+            struct Raw {
+                raw_t q[8];
+            };
+            const uint32_t first = c0 - p.n_begin - lead, groups = (lead + cn + 7u) / 8u;
+            auto load = [&](uint32_t k, Raw &q) { load_rows8(plane, record_off(p.rec, true, first + 8 * k, r), q.q); };
+            if (core) {
+                for_groups<kTileAhead, Raw>(groups, load, [&](uint32_t k, const Raw &q) {
+#pragma unroll
+                    for (int b = 0; b < 8; ++b) {
+                        float qh, ql;
+                        split(q.q[b], qh, ql);
+#pragma unroll
+                        for (int j = 0; j < kM2PT; ++j) acc[j].add(s_wh[8 * k + b][j], s_wl[8 * k + b][j], qh, ql);
+                    }
+                });
+            } else {
+                for_groups<kTileAhead, Raw>(groups, load, [&](uint32_t k, const Raw &q) {
+#pragma unroll
+                    for (int b = 0; b < 8; ++b) {
+                        float qh, ql;
+                        split(q.q[b], qh, ql);
+                        const float v = __fadd_rn(qh, ql);
+#pragma unroll
+                        for (int j = 0; j < kM2PT; ++j) acc[j].add_tail(s_wh[8 * k + b][j], v);
+                    }
+                });
+#pragma unroll
+                for (int j = 0; j < kM2PT; ++j) acc[j].flush_tail();
+            }
+            continue;
+        }
         uint32_t i = 0;
         if (core) {
             for (; i + kM2Batch <= cn; i += kM2Batch) {
@@ -686,12 +866,19 @@ void launch_conv_m2_comp(const ConvParams &p, cudaStream_t s) {
     if (p.n_runs <= 0 || p.P <= 0) return;
     const int pt = p.m2_tile == 16 ? 16 : 8;
     dim3 g((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + pt - 1) / pt, 1);
+    auto launch = [&](auto narrow, auto tile) {
+        constexpr bool N = decltype(narrow)::value;
+        constexpr int PT = decltype(tile)::value;
+        if (p.tiled) conv_m2_comp_kernel<N, PT, true><<<g, kConvRuns, 0, s>>>(p);
+        else conv_m2_comp_kernel<N, PT, false><<<g, kConvRuns, 0, s>>>(p);
+    };
+    using std::integral_constant;
     if (pt == 8) {
-        if (p.rec.narrow) conv_m2_comp_kernel<true, 8><<<g, kConvRuns, 0, s>>>(p);
-        else conv_m2_comp_kernel<false, 8><<<g, kConvRuns, 0, s>>>(p);
+        if (p.rec.narrow) launch(integral_constant<bool, true>(), integral_constant<int, 8>());
+        else launch(integral_constant<bool, false>(), integral_constant<int, 8>());
     } else {
-        if (p.rec.narrow) conv_m2_comp_kernel<true, 16><<<g, kConvRuns, 0, s>>>(p);
-        else conv_m2_comp_kernel<false, 16><<<g, kConvRuns, 0, s>>>(p);
+        if (p.rec.narrow) launch(integral_constant<bool, true>(), integral_constant<int, 16>());
+        else launch(integral_constant<bool, false>(), integral_constant<int, 16>());
     }
 }
 
@@ -711,25 +898,20 @@ static void launch_conv_window_pt(const ConvParams &p, int precision, cudaStream
     dim3 gother(gmax.x, (p.P + PT_OTHER - 1) / PT_OTHER, precision == 0 ? 4 : 3);
     // the record model is a template parameter: a run-time test in the row
     // loop cost 17 % of the kernel's time
-    if (p.rec.site) {
+    auto launch = [&](auto layout) {
+        constexpr Layout LAYOUT = decltype(layout)::value;
         if (precision == 0) {
-            conv_window_kernel<0, true, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-            conv_window_kernel<0, true, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
+            conv_window_kernel<0, LAYOUT, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
+            conv_window_kernel<0, LAYOUT, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
         } else {
-            conv_window_kernel<1, true, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-            conv_window_kernel<1, true, false, PT_OTHER><<<gother, kConvRuns, 0, s>>>(p);
+            conv_window_kernel<1, LAYOUT, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
+            conv_window_kernel<1, LAYOUT, false, PT_OTHER><<<gother, kConvRuns, 0, s>>>(p);
             launch_conv_m2_comp(p, s);
         }
-    } else {
-        if (precision == 0) {
-            conv_window_kernel<0, false, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-            conv_window_kernel<0, false, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
-        } else {
-            conv_window_kernel<1, false, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-            conv_window_kernel<1, false, false, PT_OTHER><<<gother, kConvRuns, 0, s>>>(p);
-            launch_conv_m2_comp(p, s);
-        }
-    }
+    };
+    if (p.tiled) launch(std::integral_constant<Layout, Layout::kTiled>());
+    else if (p.rec.site) launch(std::integral_constant<Layout, Layout::kSite>());
+    else launch(std::integral_constant<Layout, Layout::kBond>());
 }
 
 void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
@@ -896,7 +1078,6 @@ void launch_reduce_runs(const double *stats, int32_t n_runs, int32_t P, uint64_t
 //     power-of-two scale 2^-e, e from N, keeps squares and sums inside FP32's
 //     range).  FP64 runs at 1/64 of the FP32 rate on this chip, and the FP64
 //     squares were most of this kernel's time.
-typedef unsigned __int128 u128;
 typedef __int128 i128;
 
 __device__ __forceinline__ u128 shfl_down_u128(u128 v, int off) {
@@ -1141,9 +1322,145 @@ __global__ void NZ_MICRO_BOUNDS micro_window_kernel(MicroParams p) {
     p.acc.span_count[n] += span;
 }
 
+// The same reductions over tiled records: a block takes 32 rows, lane = row,
+// and its warps share out the runs, so nothing is summed across lanes.  Sums
+// of x and of x^2 are exact integers (x^2 of up to 168 bits), and the
+// numerator R sum x^2 - (sum x)^2 of M2 is formed in 256 bits.
+//
+// What bounds it: reading the records once.
+constexpr int kMicroWarps = 16;
+
+template <bool NARROW>
+struct MicroSums {
+    uint32_t span;
+    uint64_t s_max, s_m0, s_m2;  // max, m0 < 2^21 and m2 < 2^42, of at most 2^24 runs
+    u128 s_m3, s_m4;
+    u128 q_max, q_m0, q_m2;
+    typename std::conditional<NARROW, u128, U192>::type q_m3;  // m3 < 2^48 (narrow) or 2^63
+    U192 q_m4;                                                 // m4 < 2^64 (narrow) or 2^84
+
+    static __device__ __forceinline__ void accumulate(u128 &a, u128 x) { a += x; }
+    static __device__ __forceinline__ void accumulate(U192 &a, u128 x) { a.add(x); }
+    __device__ __forceinline__ void add(const MicroSums &o) {
+        span += o.span;
+        s_max += o.s_max;
+        s_m0 += o.s_m0;
+        s_m2 += o.s_m2;
+        s_m3 += o.s_m3;
+        s_m4 += o.s_m4;
+        q_max += o.q_max;
+        q_m0 += o.q_m0;
+        q_m2 += o.q_m2;
+        if constexpr (NARROW) q_m3 += o.q_m3;
+        else q_m3.add(o.q_m3);
+        q_m4.add(o.q_m4);
+    }
+    __device__ __forceinline__ U256 wide_m3() const {
+        if constexpr (NARROW) return u256_from_u128(q_m3);
+        else return q_m3.wide();
+    }
+};
+
+template <bool NARROW>
+__global__ void __launch_bounds__(32 * kMicroWarps) micro_tiled_kernel(MicroParams p) {
+    __shared__ MicroSums<NARROW> s_sum[32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t i = blockIdx.x * 32u + lane, n = p.n_begin + i;
+    const NzRecords &rec = p.rec;
+    MicroSums<NARROW> a = {};
+    uint64_t q_max = 0, q_m0 = 0;  // per thread: at most 2^20 runs' squares < 2^42
+    struct Rec {
+        uint32_t ms, m0, m4_hi;
+        uint64_t m2, m3, m4;
+    };
+    auto load = [&](int r) -> Rec {
+        const size_t off = record_off(rec, true, i, r);
+        Rec q;
+        q.ms = rec.max_span[off];
+        q.m0 = NARROW ? (uint32_t)reinterpret_cast<const uint16_t *>(rec.m0)[off] : rec.m0[off];
+        q.m2 = NARROW ? (uint64_t)reinterpret_cast<const uint32_t *>(rec.m2)[off] : rec.m2[off];
+        q.m3 = rec.m3[off];
+        q.m4 = rec.m4_lo[off];
+        q.m4_hi = (!NARROW && rec.m4_hi) ? rec.m4_hi[off] : 0u;
+        return q;
+    };
+    auto add = [&](const Rec &q) {
+        const uint32_t mx = q.ms & ~kSpanBit;
+        a.span += q.ms >> 31;
+        a.s_max += mx;
+        a.s_m0 += q.m0;
+        a.s_m2 += q.m2;
+        a.s_m3 += q.m3;
+        a.s_m4 += ((u128)q.m4_hi << 64) | q.m4;
+        q_max += (uint64_t)mx * mx;
+        q_m0 += (uint64_t)q.m0 * q.m0;
+        a.q_m2 += NARROW ? (u128)(q.m2 * q.m2) : (u128)q.m2 * q.m2;
+        MicroSums<NARROW>::accumulate(a.q_m3, (u128)q.m3 * q.m3);
+        a.q_m4.add((u128)q.m4 * q.m4);
+        if (!NARROW) {  // (hi 2^64 + lo)^2 = lo^2 + 2 lo hi 2^64 + hi^2 2^128, hi < 2^20
+            const u128 mid = ((u128)q.m4 * q.m4_hi) << 1;  // < 2^85
+            a.q_m4.add(mid << 64);
+            a.q_m4.w2 += (uint64_t)(mid >> 64) + (uint64_t)q.m4_hi * q.m4_hi;
+        }
+    };
+    constexpr int kAhead = 4;  // runs whose records are in flight per thread
+    int r = (int)warp;
+    for (; r + (kAhead - 1) * kMicroWarps < p.n_runs; r += kAhead * kMicroWarps) {
+        Rec q[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) q[k] = load(r + k * kMicroWarps);
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) add(q[k]);
+    }
+    for (; r < p.n_runs; r += kMicroWarps) add(load(r));
+    a.q_max = q_max;
+    a.q_m0 = q_m0;
+    for (uint32_t w = 0; w < (uint32_t)kMicroWarps; ++w) {
+        if (warp == w) {
+            if (w == 0) s_sum[lane] = a;
+            else s_sum[lane].add(a);
+        }
+        __syncthreads();
+    }
+    // the six statistics of the rows are shared out over the warps
+    if (n >= p.n_end || warp >= 7) return;
+    const MicroSums<NARROW> &t = s_sum[lane];
+    if (warp == 6) {
+        p.acc.span_count[n] += t.span;
+        return;
+    }
+    const uint64_t R = (uint64_t)p.n_runs;
+    const u128 held = (u128)p.N * R;
+    u128 sum = 0;
+    U256 sq = {{0, 0, 0, 0}};
+    switch (warp) {  // 0 max, 1 m0, 2 m1 (= N - max: same M2 as max), 3 m2, 4 m3, 5 m4
+        case 1: sum = t.s_m0; sq = u256_from_u128(t.q_m0); break;
+        case 3: sum = t.s_m2; sq = u256_from_u128(t.q_m2); break;
+        case 4: sum = t.s_m3; sq = t.wide_m3(); break;
+        case 5: sum = t.s_m4; sq = t.q_m4.wide(); break;
+        default: sum = t.s_max; sq = u256_from_u128(t.q_max); break;
+    }
+    const double m2b = u256_to_f64(u256_sub(u256_mul64(sq, R), u128_sq(sum))) / (double)R;
+    if (warp == 2) sum = held - sum;
+    const double na = (double)*p.count_before;
+    const size_t idx = (size_t)warp * (p.M + 1) + n;
+    const u128 acc = ((u128)p.acc.sum_hi[idx] << 64) | p.acc.sum_lo[idx];
+    double nn = na, mm = na > 0 ? u128_to_f64(acc) / na : 0.0, ss = p.acc.m2[idx];
+    chan_merge(nn, mm, ss, (double)R, u128_to_f64(sum) / (double)R, m2b);
+    const u128 total = acc + sum;
+    p.acc.sum_lo[idx] = (uint64_t)total;
+    p.acc.sum_hi[idx] = (uint64_t)(total >> 64);
+    p.acc.m2[idx] = ss;
+}
+
 void launch_micro_window(const MicroParams &p, cudaStream_t s) {
     const uint32_t rows = p.n_end - p.n_begin;
     if (rows == 0 || p.n_runs <= 0) return;
+    if (p.tiled) {
+        if (p.rec.narrow) micro_tiled_kernel<true><<<(rows + 31) / 32, 32 * kMicroWarps, 0, s>>>(p);
+        else micro_tiled_kernel<false><<<(rows + 31) / 32, 32 * kMicroWarps, 0, s>>>(p);
+        return;
+    }
     micro_window_kernel<256><<<rows, 256, 0, s>>>(p);
 }
 

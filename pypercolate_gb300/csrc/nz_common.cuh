@@ -73,22 +73,9 @@ __host__ __device__ inline void philox4x32_10(uint32_t c[4], uint32_t k0, uint32
 constexpr int kFeistelRounds = 8;
 constexpr uint32_t kPermTag = 0x5045524Du;  // "PERM"
 
-__host__ __device__ __forceinline__ uint32_t lowbias32(uint32_t x) {
-    x ^= x >> 16;
-    x *= 0x7feb352du;
-    x ^= x >> 15;
-    x *= 0x846ca68bu;
-    x ^= x >> 16;
-    return x;
-}
-
-__host__ __device__ __forceinline__ uint32_t feistel_f(uint32_t v, uint32_t obits, uint32_t k) {
-    return obits ? (lowbias32(v ^ k) >> (32u - obits)) : 0u;
-}
-
 struct FeistelPerm {
-    uint32_t M, hl, hr, maskL, maskR;
-    uint32_t k[kFeistelRounds];
+    uint32_t M, hr, maskL, maskR, shL, shR;
+    uint32_t k[kFeistelRounds];  // round keys, each xored with its own upper half
 
     __host__ __device__ void init(uint64_t key, uint64_t run_id, uint32_t m) {
         uint32_t bits = 0;
@@ -96,26 +83,40 @@ struct FeistelPerm {
             uint32_t x = m - 1;
             while (x) { ++bits; x >>= 1; }
         }
+        const uint32_t hl = bits / 2;
         M = m;
-        hl = bits / 2;
         hr = bits - hl;
         maskL = (1u << hl) - 1u;
         maskR = (1u << hr) - 1u;
+        shL = hl ? 32u - hl : 31u;
+        shR = hr ? 32u - hr : 31u;
 #pragma unroll
         for (uint32_t half = 0; half < 2; ++half) {
             uint32_t c[4] = {(uint32_t)run_id, (uint32_t)(run_id >> 32), half, kPermTag};
             philox4x32_10(c, (uint32_t)key, (uint32_t)(key >> 32));
 #pragma unroll
-            for (int i = 0; i < 4; ++i) k[4 * half + i] = c[i];
+            for (int i = 0; i < 4; ++i) k[4 * half + i] = c[i] ^ (c[i] >> 16);
         }
+    }
+
+    // lowbias32(v ^ key) up to its last xorshift, for v < 2^16 (either part has
+    // at most 16 bits): x ^ (x >> 16) of x = v ^ key is v ^ (key ^ (key >> 16)),
+    // the stored key; and the last x ^= x >> 16 leaves the top 16 bits alone,
+    // of which the caller takes at most 16.  7 instead of 11 instructions a
+    // round, the same permutation.
+    static __host__ __device__ __forceinline__ uint32_t hash(uint32_t v, uint32_t stored_key) {
+        uint32_t x = v ^ stored_key;
+        x *= 0x7feb352du;
+        x ^= x >> 15;
+        return x * 0x846ca68bu;
     }
 
     __host__ __device__ __forceinline__ uint32_t encrypt(uint32_t x) const {
         uint32_t L = x >> hr, R = x & maskR;
 #pragma unroll
         for (int i = 0; i < kFeistelRounds; i += 2) {
-            L ^= feistel_f(R, hl, k[i]) & maskL;
-            R ^= feistel_f(L, hr, k[i + 1]) & maskR;
+            L ^= (hash(R, k[i]) >> shL) & maskL;
+            R ^= (hash(L, k[i + 1]) >> shR) & maskR;
         }
         return (L << hr) | R;
     }

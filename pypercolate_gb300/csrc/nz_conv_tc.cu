@@ -141,13 +141,13 @@ __device__ __forceinline__ const raw_word<S> *raw_plane(const NzRecords &rec) {
 // clamped to the last row so that every load is in bounds and unconditional
 // (all 32 in flight at once); rows past the end are zeroed on conversion.
 template <int S>
-__device__ __forceinline__ void load_chunk(const NzRecords &rec, size_t base, size_t stride, uint32_t k0,
+__device__ __forceinline__ void load_chunk(const NzRecords &rec, bool tiled, uint32_t first, int32_t r, uint32_t k0,
                                            uint32_t last, raw_word<S> (&raw)[kTcK],
                                            uint64_t (&hi)[S == 6 ? kTcK : 1]) {
     const raw_word<S> *plane = raw_plane<S>(rec);
 #pragma unroll
     for (int k = 0; k < kTcK; ++k) {
-        const size_t off = base + (size_t)min(k0 + (uint32_t)k, last) * stride;
+        const size_t off = record_off(rec, tiled, first + min(k0 + (uint32_t)k, last), r);
         raw[k] = plane[off];
         if constexpr (S == 6) hi[k] = rec.m4_hi[off];
     }
@@ -183,8 +183,8 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
     const uint32_t tmem = sh.tmem;
     const uint32_t rows = nhi - nlo, last = rows - 1;
     const uint32_t nchunks = (rows + kTcK - 1) / kTcK;
-    const size_t stride = p.rec.run_stride;
-    const size_t base = (size_t)(nlo - p.n_begin) * stride + (size_t)(live ? r : 0);
+    const uint32_t first = nlo - p.n_begin;
+    const int32_t run = live ? r : 0;
     // thread t's row of A: 8-row group t / 8, row t % 8 of each core matrix
     const int a_off = (t >> 3) * (int)(kSbo / 4) + (t & 7) * 4;
     // weights staged by thread t: probability j = t / 4, rows (t % 4) kTcK / 4
@@ -212,7 +212,7 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
     };
     raw_word<S> raw[kTcK];
     uint64_t raw_hi[S == 6 ? kTcK : 1];
-    load_chunk<S>(p.rec, base, stride, 0, last, raw, raw_hi);
+    load_chunk<S>(p.rec, p.tiled, first, run, 0, last, raw, raw_hi);
     bool bad = false;
     uint32_t ch = 0;
     for (; ch < nchunks; ++ch) {
@@ -228,7 +228,7 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
             }
             // the next chunk's loads fly while this one is staged, multiplied
             // and drained
-            if (ch + 1 < nchunks) load_chunk<S>(p.rec, base, stride, (ch + 1) * kTcK, last, raw, raw_hi);
+            if (ch + 1 < nchunks) load_chunk<S>(p.rec, p.tiled, first, run, (ch + 1) * kTcK, last, raw, raw_hi);
             float *ah = sh.a[st][0] + a_off, *al = sh.a[st][1] + a_off;
 #pragma unroll
             for (int kb = 0; kb < kTcK / 4; ++kb) {

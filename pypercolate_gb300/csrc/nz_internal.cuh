@@ -21,11 +21,15 @@ struct UfParams {
     const uint32_t *perms;  // [n_runs][M] otherwise
     NzRecords rec;          // row n of run r at plane[(n - n_begin) * run_stride + r]
     uint32_t *errors;       // if set: +1 per run whose state is corrupt after its last row
+    const uint32_t *init_flag;  // explicit edge lists: nonzero if a node touches both sides (or null)
+    bool tiled;             // rec is tiled: row i of run r at plane[((i / 32) * run_stride + r) * 32 + i % 32]
 };
 
 // nz_uf.cu
-void launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
-                      uint32_t *flag_scratch, cudaStream_t s);
+// sets up the runs as far as launch_uf_window does not do so itself; returns
+// UfParams::init_flag
+const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
+                                 uint32_t *flag_scratch, cudaStream_t s);
 void launch_uf_window(const UfParams &p, int perm_mode, bool span, int block, cudaStream_t s);
 void launch_philox_perms(uint32_t M, int32_t n_runs, uint64_t key, uint64_t run0, uint32_t *out,
                          cudaStream_t s);
@@ -35,6 +39,10 @@ void launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t n_runs
                             uint32_t *state_out, cudaStream_t s);
 void launch_pack_rows(const NzRecords &rec, int32_t run, uint32_t N, uint32_t M, int32_t spanning,
                       uint8_t *rows, cudaStream_t s);
+
+// nz_ufg.cu: bond percolation with a thread block per run (which initialises
+// the run in the window that begins at row 0)
+void launch_uf_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
 
 // nz_lattice.cu: site percolation and the torus (dispatched from nz_uf.cu)
 bool lattice_extension(const GraphDev &g);
@@ -55,6 +63,7 @@ void launch_canonical_rows(const uint8_t *rows, uint32_t M, int32_t spanning, co
 
 struct ConvParams {
     NzRecords rec;           // window records, row n at (n - n_begin)
+    bool tiled;              // as UfParams::tiled
     uint32_t n_begin, n_end; // window rows
     uint32_t N;
     int32_t n_runs;
@@ -90,6 +99,7 @@ void launch_reduce_runs(const double *stats, int32_t n_runs, int32_t P, uint64_t
 
 struct MicroParams {
     NzRecords rec;
+    bool tiled;  // as UfParams::tiled
     uint32_t n_begin, n_end;
     uint32_t N;
     int32_t n_runs;

@@ -35,10 +35,10 @@
 
 #include "nz_common.cuh"
 #include "nz_internal.cuh"
+#include "nz_wide.cuh"
 
 namespace nz {
 
-typedef unsigned __int128 u128;
 constexpr uint32_t kSizeTag = 0x53495A45u;  // "SIZE"
 
 
@@ -395,70 +395,6 @@ __global__ void __launch_bounds__(256, 3) mix_uf_kernel(MixDev m, const uint32_t
 }
 
 // ---------------------------------------------------------------- reduction
-// Unsigned 256-bit helpers (4 little-endian 64-bit limbs).
-struct U256 { uint64_t w[4]; };
-
-__device__ __forceinline__ void u256_add(U256 &a, const U256 &b) {
-    uint64_t c = 0;
-    for (int i = 0; i < 4; ++i) {
-        const uint64_t s = a.w[i] + b.w[i];
-        const uint64_t c1 = s < a.w[i];
-        const uint64_t s2 = s + c;
-        const uint64_t c2 = s2 < s;
-        a.w[i] = s2;
-        c = c1 | c2;
-    }
-}
-__device__ __forceinline__ U256 u256_from_u128(u128 x) {
-    U256 r = {{(uint64_t)x, (uint64_t)(x >> 64), 0, 0}};
-    return r;
-}
-// a (< 2^128) squared
-__device__ __forceinline__ U256 u128_sq(u128 a) {
-    const uint64_t lo = (uint64_t)a, hi = (uint64_t)(a >> 64);
-    const u128 ll = (u128)lo * lo, lh = (u128)lo * hi, hh = (u128)hi * hi;
-    U256 r = u256_from_u128(ll);
-    U256 mid = {{0, (uint64_t)lh, (uint64_t)(lh >> 64), 0}};
-    u256_add(r, mid);
-    u256_add(r, mid);
-    U256 top = {{0, 0, (uint64_t)hh, (uint64_t)(hh >> 64)}};
-    u256_add(r, top);
-    return r;
-}
-// a * k for k < 2^64
-__device__ __forceinline__ U256 u256_mul64(const U256 &a, uint64_t k) {
-    U256 r = {{0, 0, 0, 0}};
-    u128 carry = 0;
-    for (int i = 0; i < 4; ++i) {
-        const u128 p = (u128)a.w[i] * k + carry;
-        r.w[i] = (uint64_t)p;
-        carry = p >> 64;
-    }
-    return r;
-}
-// a - b (a >= b)
-__device__ __forceinline__ U256 u256_sub(const U256 &a, const U256 &b) {
-    U256 r;
-    uint64_t borrow = 0;
-    for (int i = 0; i < 4; ++i) {
-        const uint64_t d = a.w[i] - b.w[i];
-        const uint64_t b1 = a.w[i] < b.w[i];
-        const uint64_t d2 = d - borrow;
-        const uint64_t b2 = d < borrow;
-        r.w[i] = d2;
-        borrow = b1 | b2;
-    }
-    return r;
-}
-__device__ __forceinline__ double u256_to_f64(const U256 &a) {
-    const double t64 = 18446744073709551616.0;
-    return ((a.w[3] * t64 + (double)a.w[2]) * t64 + (double)a.w[1]) * t64 + (double)a.w[0];
-}
-__device__ __forceinline__ double u128_f64(u128 x) {
-    return fma((double)(uint64_t)(x >> 64), 18446744073709551616.0, (double)(uint64_t)x);
-}
-
-
 // grid (classes, ceil(F / 32)); thread = checkpoint j; loop over the class's runs.
 __global__ void mix_reduce_kernel(MixDev m, const uint32_t *counts, const uint32_t *offsets, MixRec rec,
                                   MixAccum acc, uint32_t n_classes) {

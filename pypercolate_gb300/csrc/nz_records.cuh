@@ -52,6 +52,41 @@ __device__ __forceinline__ uint64_t record_m2(const NzRecords &rec, size_t off) 
     return rec.narrow ? (uint64_t)reinterpret_cast<const uint32_t *>(rec.m2)[off] : rec.m2[off];
 }
 
+// Where row i of run r lies in a window's planes.  n-major: runs next to each
+// other.  Tiled (bond ensembles): 32 rows of a run next to each other, which is
+// what a block working on one run writes and a thread summing over a run's
+// rows reads.
+__device__ __forceinline__ size_t record_off(const NzRecords &rec, bool tiled, uint32_t i, int32_t r) {
+    return tiled ? ((size_t)(i >> 5) * rec.run_stride + r) * 32 + (i & 31u) : (size_t)i * rec.run_stride + r;
+}
+
+// The raw words of 8 consecutive rows of one run in a tiled plane (off: the
+// first row's place, a multiple of 8 rows), in 16-byte loads.
+__device__ __forceinline__ void load_rows8(const uint32_t *plane, size_t off, uint32_t (&q)[8]) {
+    const uint4 *v = reinterpret_cast<const uint4 *>(plane + off);
+    const uint4 a = v[0], b = v[1];
+    q[0] = a.x; q[1] = a.y; q[2] = a.z; q[3] = a.w;
+    q[4] = b.x; q[5] = b.y; q[6] = b.z; q[7] = b.w;
+}
+__device__ __forceinline__ void load_rows8(const uint64_t *plane, size_t off, uint64_t (&q)[8]) {
+    const ulonglong2 *v = reinterpret_cast<const ulonglong2 *>(plane + off);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const ulonglong2 a = v[k];
+        q[2 * k] = a.x;
+        q[2 * k + 1] = a.y;
+    }
+}
+__device__ __forceinline__ void load_rows8(const uint16_t *plane, size_t off, uint16_t (&q)[8]) {
+    const uint4 a = *reinterpret_cast<const uint4 *>(plane + off);
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        q[2 * k] = (uint16_t)w[k];
+        q[2 * k + 1] = (uint16_t)(w[k] >> 16);
+    }
+}
+
 // writes m0 and m2 of a record in either layout
 __device__ __forceinline__ void put_m0_m2(const NzRecords &rec, size_t off, uint32_t m0, uint64_t m2) {
     if (rec.narrow) {
