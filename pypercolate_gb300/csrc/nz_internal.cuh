@@ -33,12 +33,14 @@ const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *no
 void launch_uf_window(const UfParams &p, int perm_mode, bool span, int block, cudaStream_t s);
 void launch_philox_perms(uint32_t M, int32_t n_runs, uint64_t key, uint64_t run0, uint32_t *out,
                          cudaStream_t s);
+void launch_pack_rows(const NzRecords &rec, int32_t run, uint32_t N, uint32_t M, int32_t spanning,
+                      uint8_t *rows, cudaStream_t s);
+
+// nz_mt.cu: numpy's permutations
 void launch_mt_perms(uint32_t M, int32_t n_runs, const uint32_t *seed_words, const int32_t *seed_len,
                      int32_t stride, uint32_t *out, cudaStream_t s);
 void launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t n_runs, uint32_t *out,
                             uint32_t *state_out, cudaStream_t s);
-void launch_pack_rows(const NzRecords &rec, int32_t run, uint32_t N, uint32_t M, int32_t spanning,
-                      uint8_t *rows, cudaStream_t s);
 
 // nz_ufg.cu: bond percolation with a thread block per run (which initialises
 // the run in the window that begins at row 0)
