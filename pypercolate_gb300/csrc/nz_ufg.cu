@@ -1,260 +1,16 @@
-// nz_ufg.cu -- Newman-Ziff bond percolation, one run per thread block.
-//
-// Replaces the hot loop of percolate/hpc.py:249-307 (bond_sample_states).
-// The bonds of a run are added in batches of B = 64 W (W warps, two
-// consecutive bonds per thread) instead of one at a time, with the statistics
-// after every single bond unchanged:
-//
-//   1. every thread finds the roots of its bonds' ends as they stand at the
-//      start of the round (read-only, so the order of the threads does not
-//      matter) and points the start nodes at their root;
-//   2. a bond inside one cluster is done: it stays inside one cluster.  Every
-//      other bond claims its two roots for its position in the batch (an
-//      atomicMin into a hash table).  A bond that holds both claims shares no
-//      root with an earlier unfinished bond, so its two clusters are exactly
-//      what they are when its turn comes: it joins them and notes their sizes.
-//      The others go into the next round.  The earliest unfinished bond always
-//      succeeds, so a batch ends;
-//   3. the largest cluster G is not claimed: below it the bonds of a batch
-//      would queue up for it.  A bond (G, c) joins c to G and notes |c| alone;
-//      G's size at each bond is G's size at the batch start plus a prefix sum.
-//   4. the totals after each bond are prefix sums over the batch of what each
-//      bond noted.  They run over U_k = sum of s^k over all clusters but G, in
-//      which a join with G is a mere -|c|^k; T_k = U_k + |G|^k, and the
-//      reference's moments are T_k - (largest)^k.
-//
-// Integers are exact throughout, so the records equal those of adding one
-// bond at a time, whatever the shape of the trees.
-//
-// A run needs few rounds (CPU count of this scheme at L = 256: 1.8 rounds per
-// batch of 64, 2.6 per 256, 4.7 per 1024), so one run keeps a whole block
-// busy, and a block's node words fit where one thread's 10^5 runs never could:
-// up to N = 65,536 nodes in shared memory, as 16 bits (parent, or size - 1 of
-// a root) and 8 bits (root, sides) per node; beyond, as the 32-bit words of
-// nz_common.cuh in global memory, of which the resident blocks' ones stay
-// near L2's size.
+// nz_ufg.cu -- per-step records of bond percolation, one run per thread block
+// (nz_group.cuh).
 #include <cstdint>
 
 #include "nz_common.cuh"
+#include "nz_group.cuh"
 #include "nz_internal.cuh"
 #include "nz_records.cuh"
 
 namespace nz {
 namespace {
 
-constexpr int kE = 2;                         // bonds per thread and batch
-constexpr uint32_t kSharedNodes = 65536;      // largest N whose nodes live in shared memory
-constexpr int kMaxHops = 4096;                // guards against corrupted node words only
-constexpr uint32_t kTagBits = 11;             // position in the batch (B <= 2048)
-constexpr uint32_t kStampTop = (1u << (32 - kTagBits)) - 2u;
-
-// Node words of one run.  load() gives the word format of nz_common.cuh
-// (root: bit 31, sides 29..30, size; else the parent), sizes less one in
-// shared memory.
-template <bool SHARED>
-struct Nodes;
-
-template <>
-struct Nodes<true> {
-    uint16_t *val;
-    uint8_t *flag;
-    __device__ __forceinline__ uint32_t load(uint32_t x) const { return ((uint32_t)flag[x] << 24) | val[x]; }
-    __device__ __forceinline__ void shorten(uint32_t x, uint32_t parent) const { val[x] = (uint16_t)parent; }
-    __device__ __forceinline__ void link(uint32_t x, uint32_t parent) const {
-        val[x] = (uint16_t)parent;
-        flag[x] = 0;
-    }
-    __device__ __forceinline__ void set_root(uint32_t x, uint32_t size, uint32_t sides) const {
-        val[x] = (uint16_t)(size - 1u);
-        flag[x] = (uint8_t)(0x80u | (sides << 5));
-    }
-    static __device__ __forceinline__ uint32_t size(uint32_t w) { return (w & kSizeMask) + 1u; }
-};
-
-template <>
-struct Nodes<false> {
-    uint32_t *w;
-    // weak accesses that the compiler neither repeats nor caches: other
-    // threads of the block shorten paths meanwhile (any word read is an ancestor)
-    __device__ __forceinline__ uint32_t load(uint32_t x) const {
-        uint32_t v;
-        asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(w + x));
-        return v;
-    }
-    __device__ __forceinline__ void put(uint32_t x, uint32_t v) const {
-        asm volatile("st.global.u32 [%0], %1;" ::"l"(w + x), "r"(v));
-    }
-    __device__ __forceinline__ void shorten(uint32_t x, uint32_t parent) const { put(x, parent); }
-    __device__ __forceinline__ void link(uint32_t x, uint32_t parent) const { put(x, parent); }
-    __device__ __forceinline__ void set_root(uint32_t x, uint32_t size, uint32_t sides) const {
-        put(x, make_root(size, sides));
-    }
-    static __device__ __forceinline__ uint32_t size(uint32_t w) { return root_size(w); }
-};
-
-// What a stretch of bonds adds to the totals.  Up to N = 65,536, sum s^2 is
-// needed modulo 2^32 (sum' s^2 <= N^2 / 4) and sum s^4 modulo 2^64 (sum' s^4
-// < 2^64); beyond, modulo 2^64 and 2^96.
-template <bool NARROW>
-struct Sums;
-
-template <>
-struct Sums<true> {
-    uint32_t g, u2;  // |G|, sum s^2 without G
-    uint64_t u3, u4;
-    __device__ __forceinline__ void zero() { g = u2 = 0; u3 = u4 = 0; }
-    __device__ __forceinline__ void add(const Sums &o) { g += o.g; u2 += o.u2; u3 += o.u3; u4 += o.u4; }
-    __device__ __forceinline__ Sums up(int d) const {
-        Sums r;
-        r.g = __shfl_up_sync(0xffffffffu, g, d);
-        r.u2 = __shfl_up_sync(0xffffffffu, u2, d);
-        r.u3 = __shfl_up_sync(0xffffffffu, u3, d);
-        r.u4 = __shfl_up_sync(0xffffffffu, u4, d);
-        return r;
-    }
-    // clusters a and b, neither of them G, become one
-    __device__ __forceinline__ void join(uint32_t a, uint32_t b) {
-        const uint32_t s = a + b, ab = a * b;  // a + b <= 2^16: ab < 2^31
-        g = 0;
-        u2 = 2u * ab;
-        u3 = 3ull * ((uint64_t)ab * s);
-        u4 = (uint64_t)ab * (4ull * ((uint64_t)s * s) - 2u * ab);
-    }
-    // cluster b becomes part of G
-    __device__ __forceinline__ void absorb(uint32_t b) {
-        const uint64_t b2 = (uint64_t)b * b;
-        g = b;
-        u2 = 0u - (uint32_t)b2;
-        u3 = 0ull - b2 * b;
-        u4 = 0ull - b2 * b2;
-    }
-    // += s^k
-    __device__ __forceinline__ void plus_powers(uint32_t s) {
-        const uint64_t s2 = (uint64_t)s * s;
-        u2 += (uint32_t)s2;
-        u3 += s2 * s;
-        u4 += s2 * s2;
-    }
-    __device__ __forceinline__ void minus_powers(uint32_t s) {
-        const uint64_t s2 = (uint64_t)s * s;
-        u2 -= (uint32_t)s2;
-        u3 -= s2 * s;
-        u4 -= s2 * s2;
-    }
-    __device__ __forceinline__ void load(const RunState &st) {
-        u2 = (uint32_t)st.t2;
-        u3 = st.t3;
-        u4 = st.t4_lo;
-    }
-    __device__ __forceinline__ void store(RunState &st) const {
-        st.t2 = u2;
-        st.t3 = u3;
-        st.t4_lo = u4;
-        st.t4_hi = 0;
-    }
-    __device__ __forceinline__ uint64_t m2() const { return u2; }
-    __device__ __forceinline__ uint32_t m4_hi() const { return 0u; }
-};
-
-template <>
-struct Sums<false> {
-    uint32_t g, u4x;  // |G|; bits 64..95 of sum s^4
-    uint64_t u2, u3, u4;
-    __device__ __forceinline__ void zero() { g = u4x = 0; u2 = u3 = u4 = 0; }
-    __device__ __forceinline__ void add4(uint64_t lo, uint32_t hi) {
-        const uint64_t n = u4 + lo;
-        u4x += hi + (n < lo ? 1u : 0u);
-        u4 = n;
-    }
-    __device__ __forceinline__ void sub4(uint64_t lo, uint32_t hi) {
-        const uint64_t n = u4 - lo;
-        u4x -= hi + (u4 < lo ? 1u : 0u);
-        u4 = n;
-    }
-    __device__ __forceinline__ void add(const Sums &o) {
-        g += o.g;
-        u2 += o.u2;
-        u3 += o.u3;
-        add4(o.u4, o.u4x);
-    }
-    __device__ __forceinline__ Sums up(int d) const {
-        Sums r;
-        r.g = __shfl_up_sync(0xffffffffu, g, d);
-        r.u4x = __shfl_up_sync(0xffffffffu, u4x, d);
-        r.u2 = __shfl_up_sync(0xffffffffu, u2, d);
-        r.u3 = __shfl_up_sync(0xffffffffu, u3, d);
-        r.u4 = __shfl_up_sync(0xffffffffu, u4, d);
-        return r;
-    }
-    __device__ __forceinline__ void join(uint32_t a, uint32_t b) {
-        const uint64_t s = (uint64_t)a + b, ab = (uint64_t)a * b, q = 4ull * s * s - 2ull * ab;
-        g = 0;
-        u2 = 2ull * ab;
-        u3 = 3ull * ab * s;
-        u4 = ab * q;
-        u4x = (uint32_t)__umul64hi(ab, q);
-    }
-    __device__ __forceinline__ void absorb(uint32_t b) {
-        zero();
-        g = b;
-        minus_powers(b);
-    }
-    __device__ __forceinline__ void plus_powers(uint32_t s) {
-        const uint64_t s2 = (uint64_t)s * s;
-        u2 += s2;
-        u3 += s2 * s;
-        add4(s2 * s2, (uint32_t)__umul64hi(s2, s2));
-    }
-    __device__ __forceinline__ void minus_powers(uint32_t s) {
-        const uint64_t s2 = (uint64_t)s * s;
-        u2 -= s2;
-        u3 -= s2 * s;
-        sub4(s2 * s2, (uint32_t)__umul64hi(s2, s2));
-    }
-    __device__ __forceinline__ void load(const RunState &st) {
-        u2 = st.t2;
-        u3 = st.t3;
-        u4 = st.t4_lo;
-        u4x = (uint32_t)st.t4_hi;
-    }
-    __device__ __forceinline__ void store(RunState &st) const {
-        st.t2 = u2;
-        st.t3 = u3;
-        st.t4_lo = u4;
-        st.t4_hi = u4x;
-    }
-    __device__ __forceinline__ uint64_t m2() const { return u2; }
-    __device__ __forceinline__ uint32_t m4_hi() const { return u4x; }
-};
-
-__device__ __forceinline__ void decode_any(const GraphDev &g, bool shared, uint32_t e, uint32_t &u, uint32_t &v) {
-    if (g.kind == NZ_GRAPH_GRID2D) {
-        // shared memory: row-major node ids; global memory: the tiled slots
-        if (shared) decode_edge<NZ_GRAPH_GRID2D>(g, e, u, v);
-        else decode_edge_slots<NZ_GRAPH_GRID2D>(g, e, u, v);
-    } else if (g.kind == NZ_GRAPH_CHAIN1D) {
-        decode_edge<NZ_GRAPH_CHAIN1D>(g, e, u, v);
-    } else {
-        decode_edge<NZ_GRAPH_EDGES>(g, e, u, v);
-        if (u >= g.N || v >= g.N) u = v = 0;  // invalid edge list: no bond
-    }
-}
-
-__device__ __forceinline__ uint32_t sides_any(const GraphDev &g, uint32_t i) {
-    if (g.kind == NZ_GRAPH_GRID2D) return node_sides<NZ_GRAPH_GRID2D>(g, i);
-    if (g.kind == NZ_GRAPH_CHAIN1D) return node_sides<NZ_GRAPH_CHAIN1D>(g, i);
-    return node_sides<NZ_GRAPH_EDGES>(g, i);
-}
-
-template <int W, bool NARROW>
-struct GroupShared {
-    Sums<NARROW> carry[2];  // totals after the last finished batch, double-buffered
-    Sums<NARROW> warp[W];   // what each warp's bonds add
-    uint32_t clusters[2];
-    uint32_t joins[W], top[W], sides[W];
-    uint32_t first[4];  // span search: first bond that joins both sides / adds side 0 / side 1 to G / joins at all
-    uint32_t winner, g_root, g_sides;
-};
+using namespace group;
 
 // Rows i0, i0 + 1 of run r (window rows; i0 is even).  Tiled: element (i, r)
 // of a plane is at ((i / 32) * run_stride + r) * 32 + i % 32, so a warp's 64
@@ -293,420 +49,40 @@ __device__ __forceinline__ void put_rows(const NzRecords &rec, bool tiled, uint3
     }
 }
 
-// bytes of a run's nodes in shared memory (and of the copy kept in its node
-// words between windows): the 16-bit values, then the flags, each padded to
-// a word
-__host__ __device__ __forceinline__ uint32_t val_bytes(uint32_t N) { return (2u * N + 3u) & ~3u; }
-__host__ __device__ __forceinline__ uint32_t flag_bytes(uint32_t N) { return (N + 3u) & ~3u; }
+struct RowSink {
+    NzRecords rec;
+    bool tiled;
+    int32_t r;
+    uint32_t rows;
+    __device__ __forceinline__ bool wants(uint32_t, uint32_t) const { return true; }
+    template <bool NARROW>
+    __device__ __forceinline__ void put(uint32_t i0, const uint32_t (&ms)[kE], const uint32_t (&m0)[kE],
+                                        const Sums<NARROW> (&m)[kE], const uint32_t (&e)[kE]) const {
+        put_rows<NARROW>(rec, tiled, i0, rows, r, ms, m0, m, e);
+    }
+};
 
 // Block r runs the bonds of rows [n_begin, n_end) of run r.
 template <int W, bool SHARED>
-__global__ void __launch_bounds__(32 * W) uf_group_kernel(UfParams p, uint32_t claim_mask, bool given, bool spanning) {
-    constexpr bool NARROW = SHARED;
-    constexpr uint32_t B = 32u * W * kE;
+__global__ void __launch_bounds__(32 * W, 24 / W) uf_group_kernel(UfParams p, uint32_t claim_count, bool given, bool spanning) {
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ GroupShared<W, NARROW> sh;
-    uint32_t *claims = reinterpret_cast<uint32_t *>(smem);
-    const GraphDev &g = p.g;
-    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    __shared__ GroupShared<W, SHARED> sh;
     const int32_t r = blockIdx.x;
-    RunState *state = p.state + r;
-    uint32_t *home = p.nodes + (size_t)r * g.slots;  // the run's node words between windows
-    Nodes<SHARED> nd;
-    if constexpr (SHARED) {
-        uint8_t *base = smem + (size_t)(claim_mask + 1u) * 4u;
-        nd.val = reinterpret_cast<uint16_t *>(base);
-        nd.flag = base + val_bytes(g.N);
-    } else {
-        nd.w = home;
-    }
-    for (uint32_t i = t; i <= claim_mask; i += 32u * W) claims[i] = 0xffffffffu;
-
-    // ---- state at the start of the window
-    bool span = false, init_both = false, corrupt = false;
-    if (p.n_begin == 0) {
-        if constexpr (SHARED) {
-            for (uint32_t i = t; i < g.N; i += 32u * W) nd.set_root(i, 1u, sides_any(g, i));
-        } else {
-            for (uint32_t j = t; j < g.slots; j += 32u * W) {
-                uint32_t i = j;
-                if (g.kind == NZ_GRAPH_GRID2D && kGridTiled) {
-                    const uint32_t tile = j >> 3, w = j & 7u;
-                    const uint32_t tr = tile / g.tile_cols, tc = tile - tr * g.tile_cols;
-                    const uint32_t row = 2u * tr + (w >> 2), col = 4u * tc + (w & 3u);
-                    if (row >= g.L || col >= g.L) continue;  // a padding slot, never read
-                    i = row * g.L + col;
-                }
-                nd.set_root(j, 1u, sides_any(g, i));
-            }
-        }
-        init_both = p.init_flag && *p.init_flag;
-        if (t == 0) {
-            sh.g_root = 0;
-            sh.g_sides = sides_any(g, 0);
-            Sums<NARROW> c;  // N clusters of one node, one of them G
-            c.zero();
-            RunState all;
-            all.t2 = all.t3 = all.t4_lo = g.N;
-            all.t4_hi = 0;
-            c.load(all);
-            c.minus_powers(1u);
-            c.g = 1;
-            sh.carry[0] = c;
-            sh.clusters[0] = g.N;
-        }
-    } else {
-        const RunState st = *state;
-        span = (st.flags & kFlagSpan) != 0;
-        init_both = (st.flags & kFlagInitBoth) != 0;
-        corrupt = (st.flags & kFlagCorrupt) != 0;
-        if constexpr (SHARED) {
-            const uint32_t words = (val_bytes(g.N) + flag_bytes(g.N)) / 4u;
-            uint32_t *dst = reinterpret_cast<uint32_t *>(nd.val);
-            for (uint32_t i = t; i < words; i += 32u * W) dst[i] = home[i];
-        }
-        if (t == 0) {
-            Sums<NARROW> c;
-            c.load(st);
-            c.minus_powers(st.max);
-            c.g = st.max;
-            sh.carry[0] = c;
-            sh.clusters[0] = st.t0;
-            sh.g_root = st.pad;
-            sh.g_sides = (st.flags >> 8) & 3u;
-        }
-    }
-    if (t < 4) sh.first[t] = 0xffffffffu;
-    if (t == 0) sh.winner = 0xffffffffu;
-    __syncthreads();
-    uint32_t G = sh.g_root, g_size = sh.carry[0].g, g_sides = sh.g_sides;
-    uint32_t cur = 0;  // sh.carry buffer in use
-    uint32_t stamp = kStampTop;
-
-    FeistelPerm fp;
-    const uint32_t *perm = nullptr;
-    if (given) perm = p.perms + (size_t)r * g.M;
-    else fp.init(p.key, p.run0 + (uint64_t)r, g.M);
-    const NzRecords rec = p.rec;
-    const uint32_t rows = p.n_end - p.n_begin;
-    const uint32_t hash_shift = __clz(claim_mask);  // top bits of a multiplicative hash, as many as the mask has
-
-    for (uint32_t base = 0; base < rows; base += B) {
-        const uint32_t i0 = base + t * kE;
-        // ---- 1. the bonds of rows i0, i0 + 1 and the roots of their ends
-        uint32_t edge[kE], start[2 * kE], x[2 * kE], w[2 * kE], first_w[2 * kE];
-        bool open[kE];
-#pragma unroll
-        for (int k = 0; k < kE; ++k) {
-            const uint32_t n = p.n_begin + i0 + k;
-            open[k] = i0 + k < rows && n > 0;
-            edge[k] = 0;
-            start[2 * k] = start[2 * k + 1] = 0;
-            if (open[k]) {
-                const uint32_t e = given ? __ldg(perm + (n - 1u)) : fp.at(n - 1u);
-                edge[k] = e;
-                if (given && e >= g.M) open[k] = false;  // caller-supplied index out of range: no bond
-                else decode_any(g, SHARED, e, start[2 * k], start[2 * k + 1]);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 2 * kE; ++c) {
-            x[c] = start[c];
-            w[c] = nd.load(x[c]);
-            first_w[c] = w[c];
-        }
-        auto climb = [&]() {
-            for (int hops = 0; hops < kMaxHops; ++hops) {
-                bool more = false;
-#pragma unroll
-                for (int c = 0; c < 2 * kE; ++c) {
-                    if (!is_root(w[c])) {
-                        x[c] = w[c];
-                        w[c] = nd.load(x[c]);
-                        more |= !is_root(w[c]);
-                    }
-                }
-                if (!more) return;
-            }
-            corrupt = true;
-#pragma unroll
-            for (int c = 0; c < 2 * kE; ++c)
-                if (!is_root(w[c])) x[c & ~1] = x[c | 1];  // a bond that cannot be placed joins nothing
-        };
-        climb();
-#pragma unroll
-        for (int c = 0; c < 2 * kE; ++c)
-            if (!is_root(first_w[c]) && first_w[c] != x[c]) nd.shorten(start[c], x[c]);
-
-        // ---- 2., 3. rounds of joins
-        Sums<NARROW> d[kE];
-        uint32_t formed[kE], sd[kE], kind[kE];  // kind: 0 no join, 1 two clusters, 2 with G
-#pragma unroll
-        for (int k = 0; k < kE; ++k) {
-            d[k].zero();
-            formed[k] = sd[k] = kind[k] = 0;
-        }
-        bool any_join = false;
-        for (uint32_t round = 0; round <= B; ++round) {
-            const uint32_t tag = (stamp << kTagBits) | (t * kE);
-            bool wants = false;
-            uint32_t h[2 * kE];
-#pragma unroll
-            for (int c = 0; c < 2 * kE; ++c) h[c] = g.slots <= claim_mask + 1u ? x[c] : (x[c] * 0x9E3779B1u) >> hash_shift;
-#pragma unroll
-            for (int k = 0; k < kE; ++k) {
-                open[k] = open[k] && x[2 * k] != x[2 * k + 1];
-                if (!open[k]) continue;
-                wants = true;
-                if (x[2 * k] != G) atomicMin(claims + h[2 * k], tag + k);
-                if (x[2 * k + 1] != G) atomicMin(claims + h[2 * k + 1], tag + k);
-            }
-            if (!__syncthreads_or(wants)) break;
-            any_join = true;
-            wants = false;
-#pragma unroll
-            for (int k = 0; k < kE; ++k) {
-                if (!open[k]) continue;
-                const uint32_t xu = x[2 * k], xv = x[2 * k + 1];
-                const bool gu = xu == G, gv = xv == G;
-                if ((!gu && claims[h[2 * k]] != tag + k) || (!gv && claims[h[2 * k + 1]] != tag + k)) {
-                    wants = true;
-                    continue;
-                }
-                open[k] = false;
-                const uint32_t a = nd.size(w[2 * k]), b = nd.size(w[2 * k + 1]);
-                if (gu || gv) {
-                    const uint32_t c = gu ? xv : xu, wc = gu ? w[2 * k + 1] : w[2 * k];
-                    nd.link(c, G);
-                    kind[k] = 2;
-                    d[k].absorb(gu ? b : a);
-                    sd[k] = root_sides(wc);
-                } else {
-                    const bool keep_u = a >= b;
-                    kind[k] = 1;
-                    sd[k] = root_sides(w[2 * k]) | root_sides(w[2 * k + 1]);
-                    nd.link(keep_u ? xv : xu, keep_u ? xu : xv);
-                    nd.set_root(keep_u ? xu : xv, a + b, sd[k]);
-                    d[k].join(a, b);
-                    formed[k] = a + b;
-                }
-            }
-            if (--stamp == 0) {  // stamps used up: start over with a clean table
-                __syncthreads();
-                for (uint32_t i = t; i <= claim_mask; i += 32u * W) claims[i] = 0xffffffffu;
-                stamp = kStampTop;
-            }
-            if (!__syncthreads_or(wants)) break;
-            // the roots of unfinished bonds may have been joined to others
-#pragma unroll
-            for (int c = 0; c < 2 * kE; ++c)
-                if (open[c >> 1]) w[c] = nd.load(x[c]);
-            climb();
-        }
-
-        // ---- 4. totals after every bond
-        uint32_t ms[kE], m0[kE];
-        Sums<NARROW> m[kE];
-        if (!any_join) {
-            const Sums<NARROW> c = sh.carry[cur];
-            const uint32_t cl = sh.clusters[cur] - 1u;
-#pragma unroll
-            for (int k = 0; k < kE; ++k) {
-                m[k] = c;
-                m0[k] = cl;
-                ms[k] = g_size | (span ? kSpanBit : 0u);
-            }
-        } else {
-            // prefix sums over the thread's bonds, then over the warp
-            uint32_t top[kE];
-            top[0] = formed[0];
-#pragma unroll
-            for (int k = 1; k < kE; ++k) {
-                top[k] = formed[k];
-                d[k].add(d[k - 1]);
-                top[k] = max(top[k], top[k - 1]);
-            }
-            Sums<NARROW> inc = d[kE - 1];
-            uint32_t tmax = top[kE - 1], joins = 0;
-#pragma unroll
-            for (int k = 0; k < kE; ++k) joins += kind[k] != 0 ? 1u : 0u;
-            uint32_t njoin = joins;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const Sums<NARROW> y = inc.up(o);
-                const uint32_t ym = __shfl_up_sync(0xffffffffu, tmax, o), yj = __shfl_up_sync(0xffffffffu, njoin, o);
-                if (lane >= (uint32_t)o) {
-                    inc.add(y);
-                    tmax = max(tmax, ym);
-                    njoin += yj;
-                }
-            }
-            uint32_t sall = 0;
-#pragma unroll
-            for (int k = 0; k < kE; ++k) sall |= sd[k];
-            sall = __reduce_or_sync(0xffffffffu, sall);
-            if (lane == 31) {
-                sh.warp[warp] = inc;
-                sh.top[warp] = tmax;
-                sh.joins[warp] = njoin;
-                sh.sides[warp] = sall;
-            }
-            __syncthreads();
-            // before this thread's bonds: the carry, the earlier warps, the
-            // earlier lanes
-            Sums<NARROW> pre = sh.carry[cur];
-            uint32_t ptop = 0, pj = 0;
-            for (uint32_t q = 0; q < warp; ++q) {
-                pre.add(sh.warp[q]);
-                ptop = max(ptop, sh.top[q]);
-                pj += sh.joins[q];
-            }
-            {
-                const Sums<NARROW> y = inc.up(1);
-                const uint32_t ym = __shfl_up_sync(0xffffffffu, tmax, 1);
-                if (lane > 0) {
-                    pre.add(y);
-                    ptop = max(ptop, ym);
-                }
-                pj += njoin - joins;
-            }
-            const uint32_t cl = sh.clusters[cur];
-            // the whole batch: G's new size, the largest other cluster formed
-            uint32_t top_all = 0, sides_all = g_sides;
-#pragma unroll
-            for (int q = 0; q < W; ++q) {
-                top_all = max(top_all, sh.top[q]);
-                sides_all |= sh.sides[q];
-            }
-            // first row (of the batch) at which a cluster spans
-            uint32_t span_row = span ? 0u : 0xffffffffu;
-            if (spanning && !span && (sides_all == 3u || init_both)) {
-#pragma unroll
-                for (int k = 0; k < kE; ++k) {
-                    if (kind[k] == 0) continue;
-                    const uint32_t row = t * kE + k;
-                    if (init_both) atomicMin(&sh.first[3], row);
-                    if (kind[k] == 1) {
-                        if (sd[k] == 3u) atomicMin(&sh.first[0], row);
-                    } else {
-                        if (sd[k] & 1u) atomicMin(&sh.first[1], row);
-                        if (sd[k] & 2u) atomicMin(&sh.first[2], row);
-                    }
-                }
-                __syncthreads();
-                // a node that touches both sides: the first join of all; else G
-                // spans from the join that brings it its missing side
-                const uint32_t f1 = (g_sides & 1u) ? 0u : sh.first[1], f2 = (g_sides & 2u) ? 0u : sh.first[2];
-                span_row = init_both ? sh.first[3] : min(sh.first[0], max(f1, f2));
-                __syncthreads();
-                if (t < 4) sh.first[t] = 0xffffffffu;
-            }
-#pragma unroll
-            for (int k = 0; k < kE; ++k) {
-                m[k] = pre;
-                m[k].add(d[k]);
-                pj += kind[k] != 0 ? 1u : 0u;
-                m0[k] = cl - pj - 1u;
-                const uint32_t gs = m[k].g, largest = max(gs, max(ptop, top[k]));
-                if (largest != gs) {  // moments leave out the largest cluster, which is not G here
-                    m[k].plus_powers(gs);
-                    m[k].minus_powers(largest);
-                }
-                ms[k] = largest | (t * kE + k >= span_row ? kSpanBit : 0u);
-            }
-            if (t == 32u * W - 1u) {
-                Sums<NARROW> c = pre;
-                c.add(d[kE - 1]);
-                sh.carry[cur ^ 1u] = c;
-                sh.clusters[cur ^ 1u] = cl - pj;
-            }
-            span = span || span_row != 0xffffffffu;
-            uint32_t grown = g_size;
-#pragma unroll
-            for (int q = 0; q < W; ++q) grown += sh.warp[q].g;
-            // sides that G has now: those of the clusters it took in
-            uint32_t gsd = 0;
-#pragma unroll
-            for (int k = 0; k < kE; ++k) gsd |= kind[k] == 2 ? sd[k] : 0u;
-            g_size = grown;
-            cur ^= 1u;
-            if (sides_all != g_sides) {
-                const bool s1 = __syncthreads_or(gsd & 1u), s2 = __syncthreads_or(gsd & 2u);
-                g_sides |= (s1 ? 1u : 0u) | (s2 ? 2u : 0u);
-            }
-            if (top_all > g_size) {
-                // another cluster is the largest now: it becomes G
-#pragma unroll
-                for (int k = 0; k < kE; ++k)
-                    if (formed[k] == top_all) atomicMin(&sh.winner, t * kE + k);
-                __syncthreads();
-                const uint32_t win = sh.winner;
-                if (win / kE == t) {
-                    uint32_t root = x[0];
-#pragma unroll
-                    for (int k = 1; k < kE; ++k)
-                        if (win % kE == (uint32_t)k) root = x[2 * k];
-                    uint32_t wr = nd.load(root);
-                    for (int hops = 0; hops < kMaxHops && !is_root(wr); ++hops) {
-                        root = wr;
-                        wr = nd.load(root);
-                    }
-                    nd.set_root(G, g_size, g_sides);
-                    sh.g_root = root;
-                    sh.g_sides = root_sides(wr);
-                    Sums<NARROW> c = sh.carry[cur];
-                    c.plus_powers(g_size);
-                    c.minus_powers(top_all);
-                    c.g = top_all;
-                    sh.carry[cur] = c;
-                }
-                __syncthreads();
-                if (t == 0) sh.winner = 0xffffffffu;
-                G = sh.g_root;
-                g_sides = sh.g_sides;
-                g_size = top_all;
-            }
-        }
-        put_rows<NARROW>(rec, p.tiled, i0, rows, r, ms, m0, m, edge);
-    }
-
-    // ---- state at the end of the window
-    const bool last = p.n_end == g.M + 1u;
-    __syncthreads();
-    if (!last) {
-        if (t == 0) nd.set_root(G, g_size, g_sides);
-        __syncthreads();
-        if constexpr (SHARED) {
-            const uint32_t words = (val_bytes(g.N) + flag_bytes(g.N)) / 4u;
-            const uint32_t *src = reinterpret_cast<const uint32_t *>(nd.val);
-            for (uint32_t i = t; i < words; i += 32u * W) home[i] = src[i];
-        }
-    }
-    const bool bad = __syncthreads_or(corrupt);
-    if (t == 0) {
-        RunState st;
-        Sums<NARROW> c = sh.carry[cur];
-        c.plus_powers(g_size);
-        c.store(st);
-        st.t0 = sh.clusters[cur];
-        st.max = g_size;
-        st.flags = (span ? kFlagSpan : 0u) | (init_both ? kFlagInitBoth : 0u) | (bad ? kFlagCorrupt : 0u) |
-                   (g_sides << 8);
-        st.pad = G;
-        *state = st;
-        if (p.errors && bad && last) atomicAdd(p.errors, 1u);
-    }
-}
-
-// claims: one word per node where that is few, else enough that bonds of one
-// batch seldom share a word
-template <int W, bool SHARED>
-uint32_t claim_words(uint32_t slots) {
-    constexpr uint32_t kMost = SHARED ? 4096u : 8192u;
-    constexpr uint32_t kEnough = 32u * W * kE * 16u < kMost ? 32u * W * kE * 16u : kMost;
-    uint32_t claims = 32;
-    while (claims < slots && claims < kEnough) claims <<= 1;
-    return claims;
+    Claims<W> claims;
+    claims.init(reinterpret_cast<uint32_t *>(smem), claim_count);
+    Run run;
+    run.perm = given ? p.perms + (size_t)r * p.g.M : nullptr;
+    run.key = p.key;
+    run.id = p.run0 + (uint64_t)r;
+    run.home = p.nodes + (size_t)r * p.g.slots;
+    run.state = p.state + r;
+    run.n_begin = p.n_begin;
+    run.n_end = p.n_end;
+    run.spanning = spanning;
+    run.init_both = p.init_flag && *p.init_flag;
+    RowSink sink{p.rec, p.tiled, r, p.n_end - p.n_begin};
+    const bool bad = group_run<W, SHARED>(p.g, run, sh, claims, smem + (size_t)claim_count * 4u, sink);
+    if (bad && p.errors && threadIdx.x == 0) atomicAdd(p.errors, 1u);
 }
 
 template <int W, bool SHARED>
@@ -716,21 +92,28 @@ void launch_group(const UfParams &p, bool given, bool span, cudaStream_t s) {
     if (SHARED) smem += val_bytes(p.g.N) + flag_bytes(p.g.N);
     if (smem > 40 * 1024)
         cudaFuncSetAttribute(uf_group_kernel<W, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    uf_group_kernel<W, SHARED><<<p.n_runs, 32 * W, smem, s>>>(p, claims - 1u, given, span);
+    uf_group_kernel<W, SHARED><<<p.n_runs, 32 * W, smem, s>>>(p, claims, given, span);
 }
 
-// Warps per run: enough for about kWarpsPerSm of them on every SM with the
-// runs that are there and that fit, and batches of at most an eighth of a run.
-constexpr int kWarpsPerSm = 16;
+// Warps per run.  In shared memory: kWarpsPerSm warps on every SM (80 registers
+// a thread) with the runs that are there and that fit, and batches of at most
+// an eighth of a run.  More warps per SM beat smaller batches until there are
+// about 24 (ms by warps per run 1, 2, 4, 8: 4,000 runs of 97 x 97, 6 to an SM,
+// 6.5, 4.1, 3.3, 3.6; 20,000 runs of 32 x 32, 24 to an SM, 1.1, 1.4, 1.9, 3.0).
+// In global memory: 12 warps, two runs to an SM, so that the nodes of the
+// resident runs stay near L2's size (200 runs of 512 x 512: 18.6, 11.1, 9.3,
+// 10.7 ms with 4, 8, 12, 24), 24 where there are no more runs than SMs.
+constexpr int kWarpsPerSm = 24;
+constexpr int kWarpChoices[8] = {1, 2, 3, 4, 6, 8, 12, 24};
 int group_warps(const UfParams &p) {
     const uint32_t N = p.g.N;
-    const bool shared = N <= kSharedNodes;
+    if (N > kSharedNodes) return p.n_runs <= 152 ? 24 : 12;
     int runs = (p.n_runs + 151) / 152;
-    const int fit = shared ? (int)(220u * 1024u / (val_bytes(N) + flag_bytes(N) + 5120u)) : 32;
+    const int fit = (int)(226u * 1024u / (val_bytes(N) + flag_bytes(N) + 6144u));
     runs = runs < fit ? runs : fit;
-    if (runs < 1) runs = 1;
     int w = 1;
-    while (w < 16 && 2 * w * runs <= kWarpsPerSm && 64u * 2u * w * 8u <= p.g.M) w *= 2;
+    for (int c : kWarpChoices)
+        if (c * runs <= kWarpsPerSm && 64u * c * 8u <= p.g.M) w = c;
     return w;
 }
 
@@ -743,14 +126,17 @@ void launch_uf_groups(const UfParams &p, bool given, bool span, cudaStream_t s) 
         switch (warps) {
             case 1: launch_group<1, true>(p, given, span, s); break;
             case 2: launch_group<2, true>(p, given, span, s); break;
+            case 3: launch_group<3, true>(p, given, span, s); break;
             case 4: launch_group<4, true>(p, given, span, s); break;
+            case 6: launch_group<6, true>(p, given, span, s); break;
             case 8: launch_group<8, true>(p, given, span, s); break;
-            default: launch_group<16, true>(p, given, span, s); break;
+            case 12: launch_group<12, true>(p, given, span, s); break;
+            default: launch_group<24, true>(p, given, span, s); break;
         }
+    } else if (warps == 12) {
+        launch_group<12, false>(p, given, span, s);
     } else {
-        if (warps <= 4) launch_group<4, false>(p, given, span, s);
-        else if (warps <= 8) launch_group<8, false>(p, given, span, s);
-        else launch_group<16, false>(p, given, span, s);
+        launch_group<24, false>(p, given, span, s);
     }
 }
 
