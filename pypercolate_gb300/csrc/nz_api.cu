@@ -775,9 +775,10 @@ size_t mix_layout(Carver &c, const NzMixSpec &sp, int32_t n_runs, int32_t T, Mix
     L.offsets = c.take<uint32_t>(n_classes);
     L.cursor = c.take<uint32_t>(n_classes);
     L.queue = c.take<uint32_t>(n_runs);
-    L.head = c.take<uint32_t>(1);
-    L.slot_off = c.take<uint64_t>((size_t)T + 1);
+    L.begin = c.take<uint32_t>(kMixSegments + 1);
+    L.head = c.take<uint32_t>(kMixSegments);
     L.nodes = c.take<uint32_t>((size_t)T * nmax);
+    L.home_words = nmax;
     L.fused = sp.reduction == NZ_MIX_REDUCE_FUSED;
     L.rec = MixRec{};
     L.cells = nullptr;
@@ -830,8 +831,6 @@ int nz_mix(const NzMixSpec *spec, const uint32_t *thr_grid, const uint32_t *thr_
     L.m.thr_chain = thr_chain;
     L.m.F = spec->checkpoints;
     L.T = threads;
-    L.block = block;
-    L.smem_words = smem_words;
     L.acc.count = out->count;
     L.acc.span = out->span;
     L.acc.sum_lo = out->sum_lo;

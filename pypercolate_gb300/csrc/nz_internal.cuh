@@ -154,13 +154,14 @@ struct MixAccum {
     double *m2;
     uint32_t *errors;
 };
+constexpr int kMixSegments = 5;  // parts of the queue by lattice size
 struct MixLaunch {
     MixDev m;
-    uint32_t *cls, *counts, *order, *offsets, *cursor, *queue, *head;
-    uint64_t *slot_off;
-    uint32_t *nodes;
-    int32_t T, block;
-    uint32_t smem_words;
+    uint32_t *cls, *counts, *order, *offsets, *cursor, *queue;
+    uint32_t *begin, *head;  // [kMixSegments + 1], [kMixSegments]
+    uint32_t *nodes;         // [T][home_words]
+    uint64_t home_words;
+    int32_t T;
     bool fused;       // NZ_MIX_REDUCE_FUSED: cells, else records + mix_reduce_kernel
     MixRec rec;       // [n_runs][F] per plane (records only)
     uint64_t *cells;  // [classes][F][kMixCellWords] (fused only)

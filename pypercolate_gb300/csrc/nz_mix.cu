@@ -14,12 +14,14 @@
 //                           S = l for a chain, grid_slots(L) >= L^2 for a
 //                           grid, whose sites sit in 4 x 2 blocks per sector;
 //   3. mix_scatter_kernel : run ids bucketed into a queue sorted by S desc;
-//   4. mix_slots_kernel   : node-slot offsets of the T persistent threads;
-//   5. mix_uf_kernel      : persistent union-find.  Thread t runs queue[t]
-//      first (its node slot is sized for it), then claims further items with
-//      an atomic counter; S only decreases along the queue, so every later
-//      item fits the slot.  Small items (S words <= smem slot) run in shared
-//      memory.  At F evenly spaced occupation checkpoints
+//   4. mix_segments_kernel: where in the queue the lattices stop needing more
+//      than 65,536, 16,384, 4,096 and 1,024 node words;
+//   5. mix_group_kernel   : the union-find, one launch per segment of the queue,
+//      a run per thread block (nz_group.cuh) with as many warps as fill the SMs
+//      with the blocks that fit there: node words in global memory above
+//      65,536, in shared memory below.  The blocks stay and claim runs with an
+//      atomic counter, the largest lattices first.
+//      At F evenly spaced occupation checkpoints
 //      n_j = floor(j M / (F - 1)) each run either writes its exact
 //      statistics (records) or, with the fused reduction, adds them and
 //      their squares into its class's cell j itself (integer atomics of
@@ -30,10 +32,12 @@
 //      mix_finalize_kernel: the same sums and M2 from the fused cells.
 //   Both reductions give identical results; which is faster depends on the
 //   mix of lattices (many runs per lattice favour the fused one).
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
 #include "nz_common.cuh"
+#include "nz_group.cuh"
 #include "nz_internal.cuh"
 #include "nz_wide.cuh"
 
@@ -83,8 +87,8 @@ __global__ void mix_class_kernel(MixDev m, uint32_t *cls, uint32_t *counts) {
 // Position of every class in the order "node words S descending, grids
 // before chains on equal S" (grid S = grid_slots(L) and chain S = l are
 // non-decreasing in the length).  Ordering by the words a run needs -- not
-// by M -- is what makes the persistent threads' node slots safe: every item
-// after position t needs at most the words of item t.
+// by M -- makes the queue's segments (lattices that need at most so many
+// words) contiguous.
 __global__ void mix_order_kernel(MixDev m, uint32_t *order) {
     const uint32_t n_classes = m.n_grid + m.n_chain;
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n_classes; c += gridDim.x * blockDim.x) {
@@ -111,8 +115,6 @@ __global__ void mix_order_kernel(MixDev m, uint32_t *order) {
         order[rank] = c;
     }
 }
-
-__global__ void mix_head_kernel(uint32_t *head, uint32_t v) { *head = v; }
 
 // Single block: exclusive scan of counts taken in the order `order` (classes
 // by N descending) -> offsets[c]; also the cursor copy used by the scatter.
@@ -149,39 +151,31 @@ __global__ void mix_scatter_kernel(int32_t n_runs, const uint32_t *cls, uint32_t
         queue[atomicAdd(&cursor[cls[r]], 1u)] = (uint32_t)r;
 }
 
-// Node-slot offsets (in words) of the T persistent threads: exclusive scan of
-// the words of queue[t]'s class for t < T (single block).
-__global__ void mix_slots_kernel(MixDev m, const uint32_t *queue, const uint32_t *cls, int32_t T,
-                                 uint64_t *slot_off) {
-    __shared__ uint64_t s[1024];
-    __shared__ uint64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int32_t base = 0; base < T; base += 1024) {
-        const int32_t t = base + threadIdx.x;
-        uint64_t v = 0;
-        if (t < T && t < m.n_runs) v = class_slots(m, cls[queue[t]]);
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {
-            const uint64_t y = threadIdx.x >= (unsigned)off ? s[threadIdx.x - off] : 0ull;
-            __syncthreads();
-            s[threadIdx.x] += y;
-            __syncthreads();
-        }
-        if (t < T) slot_off[t] = carry + s[threadIdx.x] - v;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry += s[1023];
-        __syncthreads();
-        if (threadIdx.x == 0 && base + 1024 >= T) slot_off[T] = carry;
-    }
+// Segment k of the queue: runs whose lattices need at most segment_words(k - 1)
+// node words (any, for k = 0) but more than segment_words(k).
+constexpr int kSegments = kMixSegments;
+__host__ __device__ constexpr uint32_t segment_words(int k) {
+    return k == 0 ? group::kSharedNodes : k == 1 ? 16384u : k == 2 ? 4096u : k == 3 ? 1024u : 0u;
 }
 
-
-__device__ __forceinline__ void add128m(uint64_t &lo, uint64_t &hi, uint64_t blo, uint64_t bhi) {
-    const uint64_t nlo = lo + blo;
-    hi += bhi + (nlo < lo ? 1ull : 0ull);
-    lo = nlo;
+// begin[k] and head[k] = the first queue position of segment k, begin[kSegments]
+// = n_runs: class order[k] starts segment j if it is the first class in the
+// order with at most segment_words(j - 1) words.
+__global__ void mix_segments_kernel(MixDev m, const uint32_t *order, const uint32_t *offsets, uint32_t *begin,
+                                    uint32_t *head) {
+    const uint32_t n_classes = m.n_grid + m.n_chain;
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) {
+        begin[0] = head[0] = 0;
+        begin[kSegments] = (uint32_t)m.n_runs;
+    }
+    if (k > n_classes) return;
+    // position n_classes stands for "no class left"
+    const uint32_t at = k < n_classes ? offsets[order[k]] : (uint32_t)m.n_runs;
+    const uint32_t words = k < n_classes ? class_slots(m, order[k]) : 0u;
+    const uint32_t above = k > 0 ? class_slots(m, order[k - 1]) : 0xffffffffu;
+    for (int j = 1; j < kSegments; ++j)
+        if (words <= segment_words(j - 1) && above > segment_words(j - 1)) begin[j] = head[j] = at;
 }
 
 // ------------------------------------------------------- fused reduction
@@ -262,13 +256,31 @@ struct MixSink {
     MixRec rec;
     size_t rec_base;
     uint64_t *cells;
-    __device__ __forceinline__ void put(uint32_t j, uint32_t mx, bool span, uint32_t m0, uint64_t m2, uint64_t m3,
-                                        uint64_t m4lo, uint32_t m4hi) const {
+    uint32_t F, M;
+    uint32_t base, batch;  // rows of the current batch
+    uint32_t j, target;    // next checkpoint and its row
+    bool dense;            // a checkpoint every 8 rows or more often
+
+    __device__ __forceinline__ uint32_t row_of(uint32_t jj) const {
+        return (uint32_t)(((uint64_t)jj * M) / (F - 1u));
+    }
+    __device__ __forceinline__ void start() {
+        j = target = 0;
+        dense = (uint64_t)(F - 1u) * 8u >= M;
+    }
+    __device__ __forceinline__ bool wants(uint32_t first, uint32_t rows) {
+        base = first;
+        batch = rows;
+        return dense || (j < F && target < first + rows);
+    }
+    __device__ __forceinline__ void write(uint32_t jj, uint32_t ms, uint32_t m0, uint64_t m2, uint64_t m3,
+                                          uint64_t m4lo, uint32_t m4hi) const {
         if (FUSED) {
-            mix_checkpoint(cells + (size_t)j * kMixCellWords, mx, span, m0, m2, m3, m4lo, m4hi);
+            mix_checkpoint(cells + (size_t)jj * kMixCellWords, ms & ~kSpanBit, (ms & kSpanBit) != 0, m0, m2, m3, m4lo,
+                           m4hi);
         } else {
-            const size_t off = rec_base + j;
-            rec.max_span[off] = mx | (span ? kSpanBit : 0u);
+            const size_t off = rec_base + jj;
+            rec.max_span[off] = ms;
             rec.m0[off] = m0;
             rec.m2[off] = m2;
             rec.m3[off] = m3;
@@ -276,121 +288,81 @@ struct MixSink {
             rec.m4_hi[off] = m4hi;
         }
     }
-};
-
-// One complete run in `node` (global or shared), delivering its checkpoints.
-template <int KIND, bool FUSED>
-__device__ void mix_run(const MixDev &m, uint64_t key, uint32_t run, uint32_t L, uint32_t N, uint32_t M, uint32_t *node,
-                        const MixSink<FUSED> &out) {
-    GraphDev g;
-    g.kind = KIND; g.site = 0; g.wrap = 0; g.L = L; g.N = N; g.M = M;
-    g.tile_cols = KIND == NZ_GRAPH_GRID2D ? (L + 3u) >> 2 : 0u;  // grids in the tiled layout
-    g.slots = KIND == NZ_GRAPH_GRID2D ? grid_slots(L) : N;
-    g.two_l_m1 = KIND == NZ_GRAPH_GRID2D ? 2u * L - 1u : 1u;
-    g.row_edges = KIND == NZ_GRAPH_GRID2D ? (L - 1u) * g.two_l_m1 : 0u;
-    g.inv_two_l_m1 = 1.0f / (float)g.two_l_m1;
-    g.eu = g.ev = nullptr; g.side = nullptr;
-    for (uint32_t i = 0; i < N; ++i) node[node_slot<KIND>(g, i)] = make_root(1u, node_sides<KIND>(g, i));
-    FeistelPerm fp;
-    fp.init(key, run, M);
-    uint64_t t2 = N, t3 = N, t4lo = N, t4hi = 0;
-    uint32_t t0 = N, mx = 1;
-    uint64_t mx2 = 1, mx3 = 1, mx4lo = 1, mx4hi = 0;
-    bool span = false;
-    const uint32_t Fm1 = (uint32_t)m.F - 1u;
-    uint32_t j = 0;
-    // checkpoint j is the row n_j = floor(j * M / (F - 1))
-    auto next_row = [&](uint32_t jj) -> uint32_t {
-        return (uint32_t)(((uint64_t)jj * M) / Fm1);
-    };
-    uint32_t target = next_row(0);
-    for (uint32_t n = 0; n <= M; ++n) {
-        if (n > 0) {
-            const uint32_t e = fp.at(n - 1u);
-            uint32_t u, v;
-            decode_edge_slots<KIND>(g, e, u, v);
-            uint32_t xu = u, xv = v;
-            uint32_t wu = node[xu], wv = node[xv];
-            for (int hops = 0; !(is_root(wu) && is_root(wv)); ++hops) {
-                if (hops >= 64) { wu = wv = make_root(0, 0); xu = xv; break; }
-                if (!is_root(wu)) {
-                    const uint32_t nu = node[wu];
-                    if (!is_root(nu)) node[xu] = nu;
-                    xu = wu; wu = nu;
-                }
-                if (!is_root(wv)) {
-                    const uint32_t nv = node[wv];
-                    if (!is_root(nv)) node[xv] = nv;
-                    xv = wv; wv = nv;
-                }
+    template <bool NARROW>
+    __device__ __forceinline__ void put(uint32_t i0, const uint32_t (&ms)[group::kE], const uint32_t (&m0)[group::kE],
+                                        const group::Sums<NARROW> (&m)[group::kE], const uint32_t (&)[group::kE]) {
+        if (dense) {
+            // every thread looks up the checkpoints of its rows (several
+            // share a row when F - 1 > M)
+#pragma unroll
+            for (int k = 0; k < group::kE; ++k) {
+                const uint32_t n = i0 + k;
+                if (n > M) break;
+                uint32_t jj = M > 0 ? (uint32_t)(((uint64_t)n * (F - 1u) + M - 1u) / M) : 0u;
+                for (; jj < F && row_of(jj) == n; ++jj)
+                    write(jj, ms[k], m0[k], m[k].m2(), m[k].u3, m[k].u4, m[k].m4_hi());
             }
-            if (xu != xv) {
-                const uint32_t a = root_size(wu), b = root_size(wv);
-                const uint32_t sides = root_sides(wu) | root_sides(wv);
-                const uint32_t s = a + b;
-                uint32_t big = xu, small = xv;
-                if (a < b) { big = xv; small = xu; }
-                node[small] = big;
-                node[big] = make_root(s, sides);
-                t0 -= 1u;
-                const uint64_t ab = (uint64_t)a * b;
-                t2 += 2ull * ab;
-                t3 += 3ull * ab * s;
-                const uint64_t q = 4ull * a * a + 6ull * ab + 4ull * b * b;
-                add128m(t4lo, t4hi, ab * q, __umul64hi(ab, q));
-                if (s > mx) {
-                    mx = s; mx2 = (uint64_t)mx * mx; mx3 = mx2 * mx;
-                    mx4lo = mx3 * mx; mx4hi = __umul64hi(mx3, (uint64_t)mx);
-                }
-                if (sides == 3u) span = true;
-            }
+            return;
         }
-        if (n == target) {
-            const uint64_t m4lo = t4lo - mx4lo;
-            const uint32_t m4hi = (uint32_t)(t4hi - mx4hi - (t4lo < mx4lo ? 1ull : 0ull));
-            // several checkpoints share row n when F - 1 > M
-            while (j < (uint32_t)m.F && n == target) {
-                out.put(j, mx, span, t0 - 1u, t2 - mx2, t3 - mx3, m4lo, m4hi);
-                ++j;
-                if (j < (uint32_t)m.F) target = next_row(j);
-            }
+        // the block walks the batch's checkpoints; the row's thread writes
+        while (j < F && target < base + batch) {
+#pragma unroll
+            for (int k = 0; k < group::kE; ++k)
+                if (i0 + k == target) write(j, ms[k], m0[k], m[k].m2(), m[k].u3, m[k].u4, m[k].m4_hi());
+            ++j;
+            if (j < F) target = row_of(j);
         }
     }
-}
+};
 
-// (256, 3): at most 85 registers (80 used by either reduction), so that 6
-// CTAs of 128 threads stay resident per SM
-template <bool FUSED>
-__global__ void __launch_bounds__(256, 3) mix_uf_kernel(MixDev m, const uint32_t *queue, const uint32_t *cls,
-                                                        int32_t T, const uint64_t *slot_off, uint32_t *nodes,
-                                                        uint32_t smem_words, uint32_t *head, MixRec rec,
-                                                        uint64_t *cells, uint32_t *errors) {
-    extern __shared__ uint32_t s_nodes[];
-    const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T || t >= m.n_runs) return;
-    const uint64_t key = *m.key_ptr;
-    uint32_t *gslot = nodes + slot_off[t];
-    const uint64_t slot_words = slot_off[t + 1] - slot_off[t];
-    uint32_t *sslot = smem_words ? s_nodes + (size_t)threadIdx.x * smem_words : nullptr;
-    uint32_t pos = (uint32_t)t;
-    while (pos < (uint32_t)m.n_runs) {
-        const uint32_t run = queue[pos];
+template <int W, bool SHARED, bool FUSED>
+__global__ void __launch_bounds__(32 * W, 24 / W) mix_group_kernel(MixLaunch p, int segment, uint32_t claim_count,
+                                                                   uint64_t home_words) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ group::GroupShared<W, SHARED> sh;
+    __shared__ GraphDev g;
+    __shared__ uint32_t s_pos;
+    group::Claims<W> claims;
+    claims.init(reinterpret_cast<uint32_t *>(smem), claim_count);
+    const uint32_t end = p.begin[segment + 1];
+    group::Run run;
+    run.perm = nullptr;
+    run.key = *p.m.key_ptr;
+    run.home = SHARED ? nullptr : p.nodes + (size_t)blockIdx.x * home_words;
+    run.state = nullptr;
+    run.n_begin = 0;
+    run.spanning = true;
+    run.init_both = false;
+    for (;;) {
+        if (threadIdx.x == 0) s_pos = atomicAdd(p.head + segment, 1u);
+        __syncthreads();
+        const uint32_t pos = s_pos;
+        if (pos >= end) break;
+        const uint32_t id = p.queue[pos], cls = p.cls[id];
         uint32_t kind, L, N, M;
-        class_graph(m, cls[run], kind, L, N, M);
-        const uint32_t words = class_slots(m, cls[run]);
-        uint32_t *node = (sslot && words <= smem_words) ? sslot : gslot;
-        if (node == gslot && words > slot_words) {  // cannot happen with the words-descending queue
-            atomicAdd(errors, 1u);
-            pos = atomicAdd(head, 1u);
-            continue;
+        class_graph(p.m, cls, kind, L, N, M);
+        if (threadIdx.x == 0) {
+            g.kind = (int32_t)kind; g.site = 0; g.wrap = 0; g.L = L; g.N = N; g.M = M;
+            g.slots = class_slots(p.m, cls);
+            g.tile_cols = kind == NZ_GRAPH_GRID2D ? (L + 3u) >> 2 : 0u;
+            g.two_l_m1 = kind == NZ_GRAPH_GRID2D ? 2u * L - 1u : 1u;
+            g.row_edges = kind == NZ_GRAPH_GRID2D ? (L - 1u) * g.two_l_m1 : 0u;
+            g.inv_two_l_m1 = 1.0f / (float)g.two_l_m1;
+            g.eu = g.ev = nullptr; g.side = nullptr;
         }
-        MixSink<FUSED> out;
-        out.rec = rec;
-        out.rec_base = (size_t)pos * (uint32_t)m.F;
-        out.cells = cells + (size_t)cls[run] * (uint32_t)m.F * kMixCellWords;
-        if (kind == NZ_GRAPH_GRID2D) mix_run<NZ_GRAPH_GRID2D, FUSED>(m, key, run, L, N, M, node, out);
-        else mix_run<NZ_GRAPH_CHAIN1D, FUSED>(m, key, run, L, N, M, node, out);
-        pos = atomicAdd(head, 1u);
+        __syncthreads();
+        run.id = id;
+        run.n_end = M + 1u;
+        MixSink<FUSED> sink;
+        sink.rec = p.rec;
+        sink.rec_base = (size_t)pos * (uint32_t)p.m.F;
+        sink.cells = FUSED ? p.cells + (size_t)cls * (uint32_t)p.m.F * kMixCellWords : nullptr;
+        sink.F = (uint32_t)p.m.F;
+        sink.M = M;
+        sink.start();
+        const bool bad = group::group_run<W, SHARED>(g, run, sh, claims, smem + (size_t)claim_count * 4u, sink);
+        if (bad && threadIdx.x == 0) atomicAdd(p.acc.errors, 1u);
+        __syncthreads();
     }
 }
 
@@ -500,6 +472,40 @@ __global__ void mix_finalize_kernel(MixDev m, const uint32_t *counts, const uint
 
 // ---------------------------------------------------------------- launchers
 
+// Segment `segment` with W warps per run; `words`: the most node words one of
+// its runs needs; per_sm: blocks that fit on an SM.
+template <int W, bool SHARED, bool FUSED>
+static int launch_segment(const MixLaunch &p, int segment, uint32_t words, int per_sm, cudaStream_t s) {
+    const uint32_t claims = group::claim_words<W, SHARED>(words);
+    const size_t smem = (size_t)claims * 4u + (SHARED ? group::val_bytes(words) + group::flag_bytes(words) : 0u);
+    if (smem > 40 * 1024 &&
+        cudaFuncSetAttribute(mix_group_kernel<W, SHARED, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem) != cudaSuccess)
+        return NZ_ERR_INVALID;
+    int blocks = 152 * per_sm;
+    if (blocks > p.m.n_runs) blocks = p.m.n_runs;
+    if (!SHARED && blocks > p.T) blocks = p.T;  // one node array each
+    mix_group_kernel<W, SHARED, FUSED><<<blocks, 32 * W, smem, s>>>(p, segment, claims, p.home_words);
+    return NZ_OK;
+}
+
+template <bool FUSED>
+static int launch_segments(const MixLaunch &p, cudaStream_t s) {
+    const uint64_t most = std::max<uint64_t>(grid_slots(p.m.grid_max), p.m.chain_max);
+    const uint64_t least = std::min<uint64_t>(grid_slots(p.m.grid_min), p.m.chain_min);
+    int st = NZ_OK;
+    // a segment that no lattice of the ranges can fall into is not launched
+    auto used = [&](int k) {
+        return (k == 0 || least <= segment_words(k - 1)) && most > segment_words(k);
+    };
+    if (used(0)) st = launch_segment<12, false, FUSED>(p, 0, (uint32_t)most, 2, s);
+    if (st == NZ_OK && used(1)) st = launch_segment<24, true, FUSED>(p, 1, segment_words(0), 1, s);
+    if (st == NZ_OK && used(2)) st = launch_segment<8, true, FUSED>(p, 2, segment_words(1), 3, s);
+    if (st == NZ_OK && used(3)) st = launch_segment<2, true, FUSED>(p, 3, segment_words(2), 11, s);
+    if (st == NZ_OK && used(4)) st = launch_segment<1, true, FUSED>(p, 4, segment_words(3), 24, s);
+    return st;
+}
+
 int launch_mix(const MixLaunch &p, cudaStream_t s) {
     const uint32_t n_classes = p.m.n_grid + p.m.n_chain;
     if (cudaMemsetAsync(p.counts, 0, sizeof(uint32_t) * n_classes, s) != cudaSuccess) return NZ_ERR_CUDA;
@@ -510,30 +516,18 @@ int launch_mix(const MixLaunch &p, cudaStream_t s) {
     mix_order_kernel<<<(n_classes + 255) / 256, 256, 0, s>>>(p.m, p.order);
     mix_offsets_kernel<<<1, 1024, 0, s>>>(p.counts, p.order, n_classes, p.offsets, p.cursor);
     mix_scatter_kernel<<<blocks, 256, 0, s>>>(p.m.n_runs, p.cls, p.cursor, p.queue);
-    mix_slots_kernel<<<1, 1024, 0, s>>>(p.m, p.queue, p.cls, p.T, p.slot_off);
-    const uint32_t first_free = (uint32_t)(p.T < p.m.n_runs ? p.T : p.m.n_runs);
-    mix_head_kernel<<<1, 1, 0, s>>>(p.head, first_free);
-    const size_t smem = (size_t)p.smem_words * 4u * (size_t)p.block;
-    const unsigned grid = (unsigned)((p.T + p.block - 1) / p.block);
+    mix_segments_kernel<<<(n_classes + 256) / 256, 256, 0, s>>>(p.m, p.order, p.offsets, p.begin, p.head);
     if (p.fused) {
         const size_t cells = (size_t)n_classes * (uint32_t)p.m.F;
         if (cudaMemsetAsync(p.cells, 0, cells * kMixCellWords * sizeof(uint64_t), s) != cudaSuccess)
             return NZ_ERR_CUDA;
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(mix_uf_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                cudaSuccess)
-            return NZ_ERR_INVALID;
-        mix_uf_kernel<true><<<grid, p.block, smem, s>>>(p.m, p.queue, p.cls, p.T, p.slot_off, p.nodes, p.smem_words,
-                                                        p.head, p.rec, p.cells, p.acc.errors);
+        const int st = launch_segments<true>(p, s);
+        if (st != NZ_OK) return st;
         mix_finalize_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(p.m, p.counts, p.cells, p.acc,
                                                                             n_classes);
     } else {
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(mix_uf_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                cudaSuccess)
-            return NZ_ERR_INVALID;
-        mix_uf_kernel<false><<<grid, p.block, smem, s>>>(p.m, p.queue, p.cls, p.T, p.slot_off, p.nodes,
-                                                         p.smem_words, p.head, p.rec, p.cells, p.acc.errors);
+        const int st = launch_segments<false>(p, s);
+        if (st != NZ_OK) return st;
         dim3 rg(n_classes, (p.m.F + 31) / 32);
         mix_reduce_kernel<<<rg, 32, 0, s>>>(p.m, p.counts, p.offsets, p.rec, p.acc, n_classes);
     }
