@@ -10,6 +10,7 @@
 //
 // Parameter layout (one flat FP32 buffer, mirrored as BF16 for products):
 // for layer l = 0..n_layers-1: W_l [in_l][out_l] row-major, then b_l [out_l].
+#include <algorithm>
 #include <cstdint>
 #include <cuda_bf16.h>
 
@@ -28,38 +29,57 @@ __device__ __forceinline__ float gelu_grad(float z) {
 // GEMM on the tensor cores: tcgen05.mma kind::f16 with BF16 operands and an
 // FP32 accumulator in TMEM
 // ---------------------------------------------------------------------
-// C[m][n] = sum_k A(m, k) B(k, n) (+ bias[n]); A(m, k) = A[m * sam + k * sak]
-// (FP32, rounded to BF16 as it is staged), B(k, n) = B[k * sbk + n * sbn]
-// (BF16, or FP32 rounded to BF16).  epilogue 0: C = acc (+ bias); 1: Z = acc
-// + bias, C = GELU(Z).  accumulate: C += instead of C =.
+// C[m][n] = sum_k A(m, k) B(k, n), with the epilogues of GemmOut; A(m, k) =
+// A[m * sam + k * sak] (FP32, rounded to BF16 as it is staged), B(k, n) =
+// B[k * sbk + n * sbn] (BF16, or FP32 rounded to BF16).
 //
-// One CTA of 128 threads per 128 x ntile tile of C (ntile <= 128, a multiple
-// of 16): the threads stage 64-deep K chunks of A (128 rows) and B (ntile
-// rows) into shared memory as BF16 in the canonical no-swizzle K-major
-// layout (8-row x 16-byte core matrices, K-adjacent ones 128 bytes apart,
-// 8-row groups 1 KB apart), double-buffered; one thread issues four
-// 128 x ntile x 16 MMAs per chunk and commits them to the chunk's mbarrier;
-// thread t reads row t of the accumulator out of TMEM (tcgen05.ld, lane t)
-// for the epilogue.  Every mbarrier wait gives up after 1 s: the tile is
-// then written as NaN and counted in g_mlp_errors (nz_mlp_take_errors).
+// One CTA of 256 threads per 128 x ntile tile of C (ntile 16, 32 or 64): the
+// threads stage 64-deep K chunks of A (128 rows) and B (ntile rows) into shared
+// memory as BF16 in the canonical no-swizzle K-major layout (8-row x 16-byte
+// core matrices, K-adjacent ones 128 bytes apart, 8-row groups 1 KB apart),
+// double-buffered; one thread issues four 128 x ntile x 16 MMAs per chunk and
+// commits them to the chunk's mbarrier; thread t reads row t % 128 of the
+// accumulator out of TMEM (tcgen05.ld) for the epilogue, threads 128 .. 255 the
+// upper half of the columns.  Every mbarrier wait gives up after 1 s: the tile
+// is then written as NaN and counted in g_mlp_errors (nz_mlp_take_errors).
+//
+// These GEMMs are tiny (batch 4096 x 128 x 128); the staging bounds them.  A
+// thread stages 8 consecutive K of one row at a time: two 16-byte loads where K
+// is contiguous in memory, else 8 loads that are coalesced over the rows, and
+// one 16-byte shared-memory store whose 8-lane phases cover 128 bytes; all loads
+// of a chunk, and of the epilogue, are issued before the first is used.  A
+// launch takes 8 to 12 us; one element at a time, with two divisions each and
+// 2-byte stores, it took 38.  64-column tiles put 64 CTAs on a batch of 4096.
 constexpr int kGM = 128;   // rows of C per CTA (TMEM lanes)
 constexpr int kGK = 64;    // K per staged chunk: 4 MMAs of K = 16
-constexpr int kGN = 128;   // largest column tile
+constexpr int kGN = 64;    // largest column tile
+constexpr int kGThreads = 256;
 constexpr uint32_t kGSbo = (kGK / 8) * tc::kCoreBytes;
 
 struct GemmSmem {
     __nv_bfloat16 a[2][kGM * kGK];
     __nv_bfloat16 b[2][kGN * kGK];
+    float part[kGThreads];
+    float bias[kGN];
     uint64_t mbar[2];
     uint32_t tmem;
 };
 
 __device__ uint32_t g_mlp_errors;  // tiles whose mbarrier waits gave up
 
-// element (row, k) of a staged K-major operand, in BF16 units
-__device__ __forceinline__ int kmajor_idx(int row, int k) {
-    return (row >> 3) * (int)(kGSbo / 2) + (k >> 3) * 64 + (row & 7) * 8 + (k & 7);
-}
+// Where the product goes.  kPlain: C = acc (+ bias), and Z too if given.  kGelu:
+// Z = acc + bias, C = GELU(Z).  kBack: C = acc * GELU'(Z) (the gradient of the
+// layer's pre-activations from that of its activations).
+enum class Epi { kPlain, kGelu, kBack };
+struct GemmOut {
+    Epi epi;
+    const float *bias;
+    float *Z;
+    float *C;
+    int ldc;
+    int64_t slice;   // floats from one K slice's C to the next
+    float *colsum;   // sums over K of B's FP32 values (the bias gradient), at slice * `slice`; or null
+};
 
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B BF16
 // (bits 7-9, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits
@@ -75,22 +95,101 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uin
         ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
 
-__global__ void __launch_bounds__(kGM) mlp_gemm_kernel(int M, int N, int K, const float *A, int sam, int sak,
-                                                       const float *Bf, const __nv_bfloat16 *Bh, int sbk, int sbn,
-                                                       const float *bias, int epilogue, float *Z, float *C,
-                                                       int ldc, int accumulate, int ntile, int k_split) {
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+
+// The 8 values (row, k0 .. k0 + 7) of an operand, zero outside rows x K, as
+// BF16 bits or FP32.  WIDE: K contiguous, every row and k0 at a 16-byte
+// boundary, K a multiple of 8.  Branch-free, so that a thread's loads overlap.
+template <bool WIDE, class T>
+__device__ __forceinline__ void load8(const T *src, int64_t s_row, int64_t s_k, int row, int rows, int k0, int K,
+                                      float (&v)[8]) {
+    const bool in = row < rows && k0 < K;
+    const T *p = src + (in ? row * s_row + k0 * s_k : 0);
+    if constexpr (WIDE && sizeof(T) == 4) {
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 a = in ? reinterpret_cast<const float4 *>(p)[0] : zero;
+        const float4 b = in ? reinterpret_cast<const float4 *>(p)[1] : zero;
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else if constexpr (WIDE) {
+        const uint4 a = in ? *reinterpret_cast<const uint4 *>(p) : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[2 * i] = __uint_as_float(w[i] << 16);
+            v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = in && k0 + i < K ? (float)p[i * s_k] : 0.0f;
+    }
+}
+
+// One K chunk of an operand (`rows` of its source's rows from row0 on, `tile`
+// <= TILE of them staged) into core matrices, all its loads before the first
+// store.  colsum: += this thread's values of row t % tile.
+template <int TILE, bool WIDE, bool COLSUM, class T>
+__device__ __forceinline__ void stage_operand(__nv_bfloat16 *dst, const T *src, int64_t s_row, int64_t s_k, int row0,
+                                              int rows, int tile, int k0, int K, float &colsum) {
+    const bool k_fast = s_k == 1 && !COLSUM;
+    // items: (row, group of 8 k).  K contiguous: 8 rows x 4 groups per warp
+    // (128 contiguous bytes of each row); else 32 rows per warp
+    constexpr int kItems = TILE * (kGK / 8) / kGThreads;
+    float v[kItems][8];
+    int at[kItems];
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        const int i = threadIdx.x + q * kGThreads;
+        const int row = k_fast ? (i & 7) + ((i >> 6) << 3) : i % tile;
+        const int kc = k_fast ? (i >> 3) & 7 : i / tile;
+        at[q] = i < tile * (kGK / 8) ? (row >> 3) * (int)(kGSbo / 2) + kc * 64 + (row & 7) * 8 : -1;
+        load8<WIDE>(src, s_row, s_k, row0 + row, at[q] >= 0 ? rows : 0, k0 + kc * 8, K, v[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        if (COLSUM) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) colsum += v[q][k];
+        }
+        if (at[q] >= 0)
+            *reinterpret_cast<uint4 *>(dst + at[q]) =
+                make_uint4(pack_bf16(v[q][0], v[q][1]), pack_bf16(v[q][2], v[q][3]), pack_bf16(v[q][4], v[q][5]),
+                           pack_bf16(v[q][6], v[q][7]));
+    }
+}
+
+template <class T>
+struct GemmIn {
+    const float *A;
+    int sam, sak;
+    const T *B;
+    int sbk, sbn;
+};
+
+// A_WIDE, B_WIDE: operands with K contiguous, in 16-byte loads; B of type T
+template <bool A_WIDE, bool B_WIDE, class T>
+__global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K, GemmIn<T> in, GemmOut out, int ntile,
+                                                             int k_split) {
     extern __shared__ __align__(1024) uint8_t gemm_smem[];
     GemmSmem &sh = *reinterpret_cast<GemmSmem *>(gemm_smem);
     const int t = threadIdx.x, warp = t >> 5;
     const int m0 = blockIdx.y * kGM, n0 = blockIdx.x * ntile;
     // split-K: this CTA's K range [kb, kb + k_split); its tile goes to slice
-    // blockIdx.z of C (M x ldc floats per slice)
+    // blockIdx.z of C
     const int kb = blockIdx.z * k_split;
-    if (gridDim.z > 1) {
-        K = min(K - kb, k_split);
-        C += (size_t)blockIdx.z * M * ldc;
-    }
-    const uint32_t cols = ntile <= 32 ? 32u : (ntile <= 64 ? 64u : 128u);  // TMEM: power of two >= 32
+    K = min(K - kb, k_split);
+    float *C = out.C + blockIdx.z * out.slice;
+    const float *A = in.A + (int64_t)kb * in.sak;
+    const uint32_t cols = ntile <= 32 ? 32u : 64u;  // TMEM: power of two >= 32
+    if (t < ntile) sh.bias[t] = out.bias && n0 + t < N ? out.bias[n0 + t] : 0.0f;
+    // rows t % 128 of C; threads 128 .. 255 take columns 32 .. 63
+    const int m = m0 + (t & 127), j0 = (t >> 7) * 32;
+    const int64_t row = (int64_t)m * out.ldc + n0 + j0;
+    const bool whole = ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(out.Z)) & 15u) == 0 &&
+                       n0 + j0 + 32 <= N && ntile >= 32 && (out.ldc & 3) == 0;
     if (warp == 0) tc::tmem_alloc(tc::smem_u32(&sh.tmem), cols);
     if (t == 0) {
         tc::mbar_init(tc::smem_u32(&sh.mbar[0]));
@@ -102,30 +201,13 @@ __global__ void __launch_bounds__(kGM) mlp_gemm_kernel(int M, int N, int K, cons
     tc::fence_after();
     const uint32_t tmem = sh.tmem;
     const int nch = (K + kGK - 1) / kGK;
-    // thread index -> element: K fastest when K is the contiguous dimension
-    // of the source, else rows fastest (coalesced global loads either way)
-    const bool a_kfast = sak == 1, b_kfast = sbk == 1;
+    constexpr bool kSums = sizeof(T) == 4;  // FP32 B: the gradient of the pre-activations
+    float colsum = 0.0f, none = 0.0f;
+    const bool sums = kSums && out.colsum && blockIdx.y == 0;
+    const T *B = in.B + (int64_t)kb * in.sbk;
     auto stage = [&](int c, int buf) {
-        const int k0 = c * kGK;
-        __nv_bfloat16 *sa = sh.a[buf], *sb = sh.b[buf];
-        for (int i = t; i < kGM * kGK; i += kGM) {
-            const int r = a_kfast ? i / kGK : i % kGM;
-            const int k = a_kfast ? i % kGK : i / kGM;
-            const int gm = m0 + r, gk = k0 + k;
-            const float v = (gm < M && gk < K) ? A[(size_t)gm * sam + (size_t)(kb + gk) * sak] : 0.0f;
-            sa[kmajor_idx(r, k)] = __float2bfloat16_rn(v);
-        }
-        for (int i = t; i < ntile * kGK; i += kGM) {
-            const int r = b_kfast ? i / kGK : i % ntile;
-            const int k = b_kfast ? i % kGK : i / ntile;
-            const int gn = n0 + r, gk = k0 + k;
-            __nv_bfloat16 v = __float2bfloat16_rn(0.0f);
-            if (gn < N && gk < K) {
-                const size_t idx = (size_t)(kb + gk) * sbk + (size_t)gn * sbn;
-                v = Bh ? Bh[idx] : __float2bfloat16_rn(Bf[idx]);
-            }
-            sb[kmajor_idx(r, k)] = v;
-        }
+        stage_operand<kGM, A_WIDE, false>(sh.a[buf], A, in.sam, in.sak, m0, M, kGM, c * kGK, K, none);
+        stage_operand<kGN, B_WIDE, kSums>(sh.b[buf], B, in.sbn, in.sbk, n0, N, ntile, c * kGK, K, colsum);
     };
     stage(0, 0);
     bool bad = false;
@@ -155,30 +237,65 @@ __global__ void __launch_bounds__(kGM) mlp_gemm_kernel(int M, int N, int K, cons
     }
     // MMAs complete in order: the last chunk issued covers them all
     if (c > 0 && !tc::mbar_wait(tc::smem_u32(&sh.mbar[(c - 1) & 1]), ((c - 1) >> 1) & 1)) bad = true;
+    sh.part[t] = colsum;
     tc::fence_before();
     const bool any_bad = __syncthreads_or(bad) || c < nch;
     tc::fence_after();
-    const int m = m0 + t;
-    if (!any_bad) {
-        for (int j0 = 0; j0 < ntile; j0 += 32) {
-            float v[32];
-            tc::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)j0, v);
-            if (m < M) {
+    if (j0 < ntile) {
+        float v[32], z[32];
+        // all loads of the epilogue before its first store
+        if (out.epi == Epi::kBack && m < M) {
+            if (whole) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    const float4 q = *reinterpret_cast<const float4 *>(out.Z + row + j);
+                    z[j] = q.x; z[j + 1] = q.y; z[j + 2] = q.z; z[j + 3] = q.w;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) z[j] = j0 + j < ntile && n0 + j0 + j < N ? out.Z[row + j] : 0.0f;
+            }
+        }
+        if (any_bad) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __int_as_float(0x7fc00000);
+            if (t == 0) atomicAdd(&g_mlp_errors, 1u);
+        } else {
+            tc::tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)j0, v);
+        }
+        if (m < M) {
+            const bool store_z = out.Z && out.epi != Epi::kBack;
+            if (out.epi == Epi::kBack) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] *= gelu_grad(z[j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) z[j] = v[j] + (j0 + j < ntile ? sh.bias[j0 + j] : 0.0f);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = out.epi == Epi::kGelu ? gelu(z[j]) : z[j];
+            }
+            if (whole) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    *reinterpret_cast<float4 *>(C + row + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    if (store_z)
+                        *reinterpret_cast<float4 *>(out.Z + row + j) = make_float4(z[j], z[j + 1], z[j + 2], z[j + 3]);
+                }
+            } else {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
-                    const int n = n0 + j0 + j;
-                    if (j0 + j >= ntile || n >= N) continue;
-                    float x = v[j] + (bias ? bias[n] : 0.0f);
-                    const size_t o = (size_t)m * ldc + n;
-                    if (epilogue == 1) { Z[o] = x; x = gelu(x); }
-                    C[o] = accumulate ? C[o] + x : x;
+                    if (j0 + j >= ntile || n0 + j0 + j >= N) continue;
+                    C[row + j] = v[j];
+                    if (store_z) out.Z[row + j] = z[j];
                 }
             }
         }
-    } else {
-        if (m < M)
-            for (int j = 0; j < ntile && n0 + j < N; ++j) C[(size_t)m * ldc + n0 + j] = __int_as_float(0x7fc00000);
-        if (t == 0) atomicAdd(&g_mlp_errors, 1u);
+    }
+    // column sums: the threads that staged one column, in order
+    if (sums && t < ntile && n0 + t < N) {
+        float x = 0.0f;
+        for (int q = t; q < kGThreads; q += ntile) x += sh.part[q];
+        out.colsum[blockIdx.z * out.slice + n0 + t] = any_bad ? __int_as_float(0x7fc00000) : x;
     }
     tc::fence_before();
     __syncthreads();
@@ -188,71 +305,46 @@ __global__ void __launch_bounds__(kGM) mlp_gemm_kernel(int M, int N, int K, cons
     }
 }
 
-// slices[z][m][n] summed over z in order into C (deterministic split-K)
-__global__ void splitk_sum_kernel(const float *slices, int splits, int M, int N, int ldc, float *C) {
-    const int64_t total = (int64_t)M * N;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int m = (int)(i / N), n = (int)(i % N);
+// slices of `count` values, `stride` floats apart, summed in order into out
+// (deterministic split-K): the weight gradient and, after it, the bias gradient
+__global__ void splitk_sum_kernel(const float *slices, int splits, int64_t stride, int64_t count, float *out) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
         float acc = 0.0f;
-        for (int z = 0; z < splits; ++z) acc += slices[(size_t)z * M * ldc + (size_t)m * ldc + n];
-        C[(size_t)m * ldc + n] = acc;
+#pragma unroll 8
+        for (int z = 0; z < splits; ++z) acc += slices[z * stride + i];
+        out[i] = acc;
     }
 }
 
-// C = A B (+ bias, epilogue).  With `partial` (room for `splits` x M x ldc
-// floats) and splits > 1, K is split over that many CTAs per tile, for GEMMs
-// with few output tiles and a long K (the weight gradients: K = batch); the
-// slices are then summed in order (no bias, no epilogue, C overwritten).
-static void gemm(int M, int N, int K, const float *A, int sam, int sak, const float *Bf, const __nv_bfloat16 *Bh,
-                 int sbk, int sbn, const float *bias, int epilogue, float *Z, float *C, int ldc, int accumulate,
-                 cudaStream_t s, float *partial = nullptr, int splits = 1) {
+// Launches the product; `splits` K slices of k_split (1 slice: k_split = K).
+template <class T>
+static void gemm(int M, int N, int K, const GemmIn<T> &in, const GemmOut &out, int splits, int k_split,
+                 cudaStream_t s) {
     if (M <= 0 || N <= 0) return;
-    const int ntile = N >= kGN ? kGN : ((N + 15) / 16) * 16;
-    int k_split = K;
-    if (partial && splits > 1) {
-        k_split = ((K + splits - 1) / splits + kGK - 1) / kGK * kGK;
-        splits = (K + k_split - 1) / k_split;
-    }
-    if (splits < 2) { partial = nullptr; splits = 1; k_split = K; }
-    // above 48 KB of dynamic shared memory the launch needs the attribute,
-    // which belongs to the function in the current device's context
-    cudaFuncSetAttribute(mlp_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GemmSmem));
-    dim3 grid((N + ntile - 1) / ntile, (M + kGM - 1) / kGM, splits);
-    mlp_gemm_kernel<<<grid, kGM, sizeof(GemmSmem), s>>>(M, N, K, A, sam, sak, Bf, Bh, sbk, sbn,
-                                                         partial ? nullptr : bias, partial ? 0 : epilogue, Z,
-                                                         partial ? partial : C, ldc, partial ? 0 : accumulate,
-                                                         ntile, k_split);
-    if (partial) {
-        const int64_t total = (int64_t)M * N;
-        const int blocks = (int)((total + 255) / 256 > 1024 ? 1024 : (total + 255) / 256);
-        splitk_sum_kernel<<<blocks, 256, 0, s>>>(partial, splits, M, N, ldc, C);
+    const int ntile = N > 32 ? kGN : (N > 16 ? 32 : 16);
+    auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    // slices begin at multiples of kGK, so every 8-k group does at one of 8
+    const bool a_wide = in.sak == 1 && (in.sam & 3) == 0 && (K & 7) == 0 && aligned(in.A);
+    const bool b_wide = sizeof(T) == 2 && in.sbk == 1 && (K & 7) == 0 && (in.sbn & 7) == 0 && aligned(in.B);
+    auto launch = [&](auto *kernel) {
+        // above 48 KB of dynamic shared memory the launch needs the attribute,
+        // which belongs to the function in the current device's context
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GemmSmem));
+        dim3 grid((N + ntile - 1) / ntile, (M + kGM - 1) / kGM, splits);
+        kernel<<<grid, kGThreads, sizeof(GemmSmem), s>>>(M, N, K, in, out, ntile, k_split);
+    };
+    if constexpr (sizeof(T) == 2) {
+        if (a_wide && b_wide) launch(mlp_gemm_kernel<true, true, T>);
+        else if (a_wide) launch(mlp_gemm_kernel<true, false, T>);
+        else launch(mlp_gemm_kernel<false, false, T>);
+    } else {
+        launch(mlp_gemm_kernel<false, false, T>);
     }
 }
 
 __global__ void to_bf16_kernel(const float *a, __nv_bfloat16 *b, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         b[i] = __float2bfloat16_rn(a[i]);
-}
-
-// dZ = dH * GELU'(Z)
-__global__ void gelu_back_kernel(const float *Z, const float *dH, float *dZ, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dZ[i] = dH[i] * gelu_grad(Z[i]);
-}
-
-// db[o] = sum_b dZ[b][o]
-__global__ void bias_grad_kernel(const float *dZ, int B, int N, float *db) {
-    const int o = blockIdx.x;
-    float s = 0.0f;
-    for (int b = threadIdx.x; b < B; b += blockDim.x) s += dZ[(size_t)b * N + o];
-    __shared__ float red[256];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 128; off > 0; off >>= 1) {
-        if (threadIdx.x < (unsigned)off) red[threadIdx.x] += red[threadIdx.x + off];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) db[o] = red[0];
 }
 
 // Weighted squared error: loss = sum_{b,o} w[b][o] (y - t)^2 / B ; dY = 2 w (y - t) / B
@@ -348,8 +440,8 @@ int nz_mlp_forward(const int32_t *widths, int32_t n_layers, int32_t batch, const
         const int K = widths[l], N = widths[l + 1];
         const bool last = l == n_layers - 1;
         float *zl = z + act, *hl = last ? y : h + act;
-        gemm(batch, N, K, in, K, 1, nullptr, pb + wo[l], N, 1, params + bo[l], last ? 0 : 1, zl, hl, N, 0, s);
-        if (last) cudaMemcpyAsync(zl, y, sizeof(float) * (size_t)batch * N, cudaMemcpyDeviceToDevice, s);
+        const GemmIn<__nv_bfloat16> g{in, K, 1, pb + wo[l], N, 1};
+        gemm(batch, N, K, g, GemmOut{last ? Epi::kPlain : Epi::kGelu, params + bo[l], zl, hl, N, 0, nullptr}, 1, K, s);
         in = hl;
         act += (int64_t)batch * N;
     }
@@ -378,27 +470,42 @@ int nz_mlp_backward(const int32_t *widths, int32_t n_layers, int32_t batch, cons
     const __nv_bfloat16 *pb = reinterpret_cast<const __nv_bfloat16 *>(params_bf16);
     int wmax = 0;
     for (int l = 0; l <= n_layers; ++l) wmax = widths[l] > wmax ? widths[l] : wmax;
-    float *dZ = scratch, *dA = scratch + (size_t)batch * wmax;
     int64_t act_off[kMaxLayers];
     int64_t a = 0;
     for (int l = 0; l < n_layers; ++l) { act_off[l] = a; a += (int64_t)batch * widths[l + 1]; }
-    // dZ of the last (linear) layer = dy
-    cudaMemcpyAsync(dZ, dy, sizeof(float) * (size_t)batch * widths[n_layers], cudaMemcpyDeviceToDevice, s);
+    // dZ of the last (linear) layer = dy; the other layers' in turn in the two
+    // halves of the scratch, whose other half holds the weight gradient's slices
+    const int64_t half = (int64_t)batch * wmax;
+    const float *dZ = dy;
+    int other = 0;  // the half that dZ is not in
     for (int l = n_layers - 1; l >= 0; --l) {
         const int K = widths[l], N = widths[l + 1];
-        const float *A = l == 0 ? x : h + act_off[l - 1];
-        // dW[K][N] = A^T dZ  (reduction over the batch), split over the batch
-        // into slices held in the dA half of the scratch (free until the dA
-        // GEMM below): splits * K * N <= batch * wmax floats
-        const int64_t room = (int64_t)batch * wmax / ((int64_t)K * N);
-        const int splits = (int)(room < 32 ? room : 32);
-        gemm(K, N, batch, A, 1, K, dZ, nullptr, N, 1, nullptr, 0, nullptr, grads + wo[l], N, 0, s, dA, splits);
-        bias_grad_kernel<<<N, 256, 0, s>>>(dZ, batch, N, grads + bo[l]);
+        float *spare = scratch + other * half;
+        // dW[K][N] = A^T dZ and db[N] = column sums of dZ: the reduction over
+        // the batch is split into up to 16 slices (dW, then db), summed in
+        // order; 32 slices would not leave room for db at K = N = wmax
+        const int64_t per_slice = (int64_t)K * N + N;
+        int splits = (int)std::min<int64_t>(16, half / per_slice);
+        int k_split = batch;
+        if (splits > 1) {
+            k_split = ((batch + splits - 1) / splits + kGK - 1) / kGK * kGK;
+            splits = (batch + k_split - 1) / k_split;
+        }
+        if (splits < 2) { splits = 1; k_split = batch; }
+        float *dst = splits > 1 ? spare : grads + wo[l];
+        const GemmIn<float> g{l == 0 ? x : h + act_off[l - 1], 1, K, dZ, N, 1};
+        gemm(K, N, batch, g, GemmOut{Epi::kPlain, nullptr, nullptr, dst, N, per_slice, dst + (int64_t)K * N}, splits,
+             k_split, s);
+        if (splits > 1)
+            splitk_sum_kernel<<<blocks_for(per_slice), 256, 0, s>>>(spare, splits, per_slice, per_slice,
+                                                                   grads + wo[l]);
         if (l == 0) break;
-        // dA[batch][K] = dZ W^T  (W[K][N]: B(k=n, n=k) = W[k][n] -> sbk = 1, sbn = N)
-        gemm(batch, K, N, dZ, N, 1, nullptr, pb + wo[l], 1, N, nullptr, 0, nullptr, dA, K, 0, s);
-        const int64_t cnt = (int64_t)batch * K;
-        gelu_back_kernel<<<blocks_for(cnt), 256, 0, s>>>(z + act_off[l - 1], dA, dZ, cnt);
+        // dZ of layer l - 1 = (dZ W^T) * GELU'(z)  (W[K][N]: B(k=n, n=k) = W[k][n])
+        const GemmIn<__nv_bfloat16> b{dZ, N, 1, pb + wo[l], 1, N};
+        gemm(batch, K, N, b, GemmOut{Epi::kBack, nullptr, const_cast<float *>(z) + act_off[l - 1], spare, K, 0, nullptr},
+             1, N, s);
+        dZ = spare;
+        other ^= 1;
     }
     return cudaGetLastError() == cudaSuccess ? NZ_OK : NZ_ERR_CUDA;
 }
