@@ -513,7 +513,7 @@ size_t ensemble_layout(Carver &c, const GraphDev &g, int32_t n_runs, int32_t P, 
     L.state = c.take<RunState>((size_t)n_runs);
     L.flag = c.take<uint32_t>(4);
     // bond ensembles write tiled records: whole tiles of 32 rows
-    const size_t rows = lattice_extension(g) ? (size_t)L.window : ((size_t)L.window + 31) / 32 * 32;
+    const size_t rows = g.site ? (size_t)L.window : ((size_t)L.window + 31) / 32 * 32;
     const size_t plane = rows * n_runs;
     for (int b = 0; b < 2; ++b) {
         NzRecords &r = L.rec[b];
@@ -641,7 +641,7 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
     up.run0 = run0;
     up.perms = nullptr;
     up.init_flag = nullptr;
-    up.tiled = !lattice_extension(g);
+    up.tiled = !g.site;
     up.errors = L.flag + 1;  // zeroed in the set-up; read by nz_ensemble_errors
     ConvParams cp;
     cp.tiled = up.tiled;

@@ -40,6 +40,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include "nz_common.cuh"
 
@@ -48,6 +49,7 @@ namespace group {
 
 constexpr int kE = 2;                         // bonds per thread and batch
 constexpr uint32_t kSharedNodes = 65536;      // largest N whose nodes live in shared memory
+constexpr uint32_t kSharedTorus = 16384;      // the same on the torus
 constexpr int kMaxHops = 4096;                // guards against corrupted node words only
 constexpr uint32_t kTagBits = 11;             // position in the batch (B <= 2048)
 constexpr uint32_t kStampTop = (1u << (32 - kTagBits)) - 2u;
@@ -55,11 +57,11 @@ constexpr uint32_t kStampTop = (1u << (32 - kTagBits)) - 2u;
 // Node words of one run.  load() gives the word format of nz_common.cuh
 // (root: bit 31, sides 29..30, size; else the parent), sizes less one in
 // shared memory.
-template <bool SHARED>
+template <bool SHARED, bool TORUS>
 struct Nodes;
 
 template <>
-struct Nodes<true> {
+struct Nodes<true, false> {
     uint16_t *val;
     uint8_t *flag;
     __device__ __forceinline__ uint32_t load(uint32_t x) const { return ((uint32_t)flag[x] << 24) | val[x]; }
@@ -76,7 +78,7 @@ struct Nodes<true> {
 };
 
 template <>
-struct Nodes<false> {
+struct Nodes<false, false> {
     uint32_t *w;
     // weak accesses that the compiler neither repeats nor caches: other
     // threads of the block shorten paths meanwhile (any word read is an ancestor)
@@ -106,6 +108,54 @@ __device__ __forceinline__ uint64_t warp_sum(uint64_t v, uint32_t &over) {
     over = (uint32_t)(hi >> 32);
     return (hi << 32) | (uint32_t)lo;
 }
+
+// On the torus every node but a root also has its displacement (dx, dy) from its
+// parent, as one integer dx S + dy, which adds and compares like the pair: S =
+// 2^16 in 32 bits in shared memory (up to N = 16,384 nodes, where every
+// difference that is formed, of at most 2 N - 1 steps, fits 16 bits), S = 2^32
+// in 64 bits beyond.  Parent and displacement are two words, so a start node is
+// only pointed at its root while no thread climbs.
+template <>
+struct Nodes<true, true> : Nodes<true, false> {
+    typedef int32_t Disp;
+    static constexpr int kShift = 16;
+    Disp *off;
+    __device__ __forceinline__ Disp disp(uint32_t x) const { return off[x]; }
+    __device__ __forceinline__ void set_disp(uint32_t x, Disp d) const { off[x] = d; }
+    static __device__ __forceinline__ int32_t dy(Disp d) { return (int16_t)(d & 0xffff); }
+    static __device__ __forceinline__ int32_t dx(Disp d) { return (d - dy(d)) >> kShift; }
+};
+
+template <>
+struct Nodes<false, true> {
+    typedef int64_t Disp;
+    static constexpr int kShift = 32;
+    uint4 *cell;  // x: node word; z, w: displacement
+    __device__ __forceinline__ uint32_t load(uint32_t x) const {
+        uint32_t v;
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(&cell[x].x));
+        return v;
+    }
+    __device__ __forceinline__ void put(uint32_t x, uint32_t v) const {
+        asm volatile("st.global.u32 [%0], %1;" ::"l"(&cell[x].x), "r"(v));
+    }
+    __device__ __forceinline__ void shorten(uint32_t x, uint32_t parent) const { put(x, parent); }
+    __device__ __forceinline__ void link(uint32_t x, uint32_t parent) const { put(x, parent); }
+    __device__ __forceinline__ void set_root(uint32_t x, uint32_t size, uint32_t sides) const {
+        put(x, make_root(size, sides));
+    }
+    static __device__ __forceinline__ uint32_t size(uint32_t w) { return root_size(w); }
+    __device__ __forceinline__ Disp disp(uint32_t x) const {
+        Disp v;
+        asm volatile("ld.global.s64 %0, [%1];" : "=l"(v) : "l"(&cell[x].z));
+        return v;
+    }
+    __device__ __forceinline__ void set_disp(uint32_t x, Disp d) const {
+        asm volatile("st.global.s64 [%0], %1;" ::"l"(&cell[x].z), "l"(d));
+    }
+    static __device__ __forceinline__ int32_t dy(Disp d) { return (int32_t)(d & 0xffffffffll); }
+    static __device__ __forceinline__ int32_t dx(Disp d) { return (int32_t)((d - dy(d)) >> kShift); }
+};
 
 // What a stretch of bonds adds to the totals.  Up to N = 65,536, sum s^2 is
 // needed modulo 2^32 (sum' s^2 <= N^2 / 4) and sum s^4 modulo 2^64 (sum' s^4
@@ -274,11 +324,26 @@ __device__ __forceinline__ void decode_any(const GraphDev &g, bool shared, uint3
     }
 }
 
+// Bonds of the torus: e < N to the right neighbour, else to the one below;
+// `down` says which.
+__device__ __forceinline__ void decode_torus(const GraphDev &g, uint32_t e, uint32_t &u, uint32_t &v, bool &down) {
+    down = e >= g.N;
+    u = down ? e - g.N : e;
+    const uint32_t row = u / g.L, col = u - row * g.L;
+    v = down ? (row + 1u == g.L ? 0u : row + 1u) * g.L + col : row * g.L + (col + 1u == g.L ? 0u : col + 1u);
+}
+
 __device__ __forceinline__ uint32_t sides_any(const GraphDev &g, uint32_t i) {
     if (g.kind == NZ_GRAPH_GRID2D) return node_sides<NZ_GRAPH_GRID2D>(g, i);
     if (g.kind == NZ_GRAPH_CHAIN1D) return node_sides<NZ_GRAPH_CHAIN1D>(g, i);
+    if (g.kind == NZ_GRAPH_TORUS2D) return 0u;
     return node_sides<NZ_GRAPH_EDGES>(g, i);
 }
+
+template <bool SHARED, bool TORUS>
+struct DispOf {
+    typedef typename std::conditional<SHARED, int32_t, int64_t>::type type;
+};
 
 template <int W, bool NARROW>
 struct GroupShared {
@@ -287,6 +352,7 @@ struct GroupShared {
     uint32_t clusters[2];
     uint32_t joins[W], top[W], sides[W];
     uint32_t first[4];  // span search: first bond that joins both sides / adds side 0 / side 1 to G / joins at all
+    uint32_t wrap[2];       // torus: first window row at which a cluster wraps along x / y
     uint32_t winner, g_root, g_sides;
     FeistelPerm fp;         // the run's keyed permutation: its registers are needed elsewhere
 };
@@ -296,6 +362,15 @@ struct GroupShared {
 // a word
 __host__ __device__ __forceinline__ uint32_t val_bytes(uint32_t N) { return (2u * N + 3u) & ~3u; }
 __host__ __device__ __forceinline__ uint32_t flag_bytes(uint32_t N) { return (N + 3u) & ~3u; }
+template <bool TORUS>
+__host__ __device__ __forceinline__ uint32_t node_bytes(uint32_t N) {
+    return val_bytes(N) + flag_bytes(N) + (TORUS ? 4u * N : 0u);
+}
+// numbers that node ids run up to
+template <bool SHARED, bool TORUS>
+__host__ __device__ __forceinline__ uint32_t node_count(const GraphDev &g) {
+    return SHARED || TORUS ? g.N : g.slots;
+}
 
 // claims: one word per node where that is few, else enough that bonds of one
 // batch seldom share a word
@@ -341,19 +416,25 @@ struct Run {
 // rows to `sink`: wants(base, B) says (for the whole block alike) whether rows
 // base .. base + B - 1 of the window are wanted, put(i0, ...) takes this
 // thread's rows i0 .. i0 + kE - 1 (rows past the window's end among them).
-// `nodes`: shared memory for val_bytes + flag_bytes of the run (SHARED only).
+// `nodes`: shared memory for node_bytes of the run (SHARED only).  TORUS: the
+// flag of a row says that a cluster wraps (g.wrap); other lattices: that one
+// spans.
 // Every thread of the block calls it and may call it again at once.  Returns
 // whether the run is finished and was found corrupt.
-template <int W, bool SHARED, class Sink>
+template <int W, bool SHARED, bool TORUS, class Sink>
 __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, GroupShared<W, SHARED> &sh,
                                           Claims<W> &claims, uint8_t *nodes, Sink &sink) {
     constexpr bool NARROW = SHARED;
     constexpr uint32_t B = 32u * W * kE;
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-    Nodes<SHARED> nd;
+    typedef Nodes<SHARED, TORUS> NodesT;
+    NodesT nd;
     if constexpr (SHARED) {
         nd.val = reinterpret_cast<uint16_t *>(nodes);
         nd.flag = nodes + val_bytes(g.N);
+        if constexpr (TORUS) nd.off = reinterpret_cast<int32_t *>(nodes + val_bytes(g.N) + flag_bytes(g.N));
+    } else if constexpr (TORUS) {
+        nd.cell = reinterpret_cast<uint4 *>(run.home);
     } else {
         nd.w = run.home;
     }
@@ -364,7 +445,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
         if constexpr (SHARED) {
             for (uint32_t i = t; i < g.N; i += 32u * W) nd.set_root(i, 1u, sides_any(g, i));
         } else {
-            for (uint32_t j = t; j < g.slots; j += 32u * W) {
+            for (uint32_t j = t; j < node_count<SHARED, TORUS>(g); j += 32u * W) {
                 uint32_t i = j;
                 if (g.kind == NZ_GRAPH_GRID2D && kGridTiled) {
                     const uint32_t tile = j >> 3, w = j & 7u;
@@ -377,6 +458,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             }
         }
         init_both = run.init_both;
+        if (t < 2) sh.wrap[t] = 0xffffffffu;
         if (t == 0) {
             sh.g_root = 0;
             sh.g_sides = sides_any(g, 0);
@@ -396,8 +478,9 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
         span = (st.flags & kFlagSpan) != 0;
         init_both = (st.flags & kFlagInitBoth) != 0;
         corrupt = (st.flags & kFlagCorrupt) != 0;
+        if (t < 2) sh.wrap[t] = (st.flags & (t == 0 ? kFlagWrapX : kFlagWrapY)) ? 0u : 0xffffffffu;
         if constexpr (SHARED) {
-            const uint32_t words = (val_bytes(g.N) + flag_bytes(g.N)) / 4u;
+            const uint32_t words = node_bytes<TORUS>(g.N) / 4u;
             uint32_t *dst = reinterpret_cast<uint32_t *>(nd.val);
             for (uint32_t i = t; i < words; i += 32u * W) dst[i] = run.home[i];
         }
@@ -428,6 +511,13 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
     // M well below its power of two: cycle walks are common (the domain is
     // 1.8 M at L = 97, within 1.01 M at L = 2^k)
     const bool walks = !given && (sh.fp.maskR + 1ull) * (sh.fp.maskL + 1ull) > g.M + g.M / 8ull;
+
+    // (dx, dy) of a bond of the torus
+    auto step = [](bool is_down) {
+        typedef typename DispOf<SHARED, TORUS>::type D;
+        return is_down ? (D)1 : (D)((D)1 << (SHARED ? 16 : 32));
+    };
+    (void)step;
 
     for (uint32_t base = 0; base < rows; base += B) {
         const uint32_t i0 = base + t * kE;
@@ -471,7 +561,8 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             }
         }
         uint32_t start[2 * kE], x[2 * kE], w[2 * kE], first_w[2 * kE];
-        bool open[kE];
+        bool open[kE], down[kE] = {};
+        typename DispOf<SHARED, TORUS>::type pos[2 * kE] = {};  // displacement of each end from x
 #pragma unroll
         for (int k = 0; k < kE; ++k) {
             const uint32_t n = run.n_begin + i0 + k;
@@ -481,6 +572,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                 if (given) edge[k] = __ldg(run.perm + (n - 1u));
                 const uint32_t e = edge[k];
                 if (given && e >= g.M) open[k] = false;  // caller-supplied index out of range: no bond
+                else if constexpr (TORUS) decode_torus(g, e, start[2 * k], start[2 * k + 1], down[k]);
                 else decode_any(g, SHARED, e, start[2 * k], start[2 * k + 1]);
             } else {
                 edge[k] = 0;
@@ -498,6 +590,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
 #pragma unroll
                 for (int c = 0; c < 2 * kE; ++c) {
                     if (!is_root(w[c])) {
+                        if constexpr (TORUS) pos[c] += nd.disp(x[c]);
                         x[c] = w[c];
                         w[c] = nd.load(x[c]);
                         more |= !is_root(w[c]);
@@ -511,9 +604,11 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                 if (!is_root(w[c])) x[c & ~1] = x[c | 1];  // a bond that cannot be placed joins nothing
         };
         climb();
+        if constexpr (!TORUS) {
 #pragma unroll
-        for (int c = 0; c < 2 * kE; ++c)
-            if (!is_root(first_w[c]) && first_w[c] != x[c]) nd.shorten(start[c], x[c]);
+            for (int c = 0; c < 2 * kE; ++c)
+                if (!is_root(first_w[c]) && first_w[c] != x[c]) nd.shorten(start[c], x[c]);
+        }
 
         // ---- 2., 3. rounds of joins
         Sums<NARROW> d[kE];
@@ -529,9 +624,21 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             bool wants = false;
             uint32_t h[2 * kE];
 #pragma unroll
-            for (int c = 0; c < 2 * kE; ++c) h[c] = g.slots <= claims.mask + 1u ? x[c] : (x[c] * 0x9E3779B1u) >> claims.shift;
+            for (int c = 0; c < 2 * kE; ++c) h[c] = node_count<SHARED, TORUS>(g) <= claims.mask + 1u ? x[c] : (x[c] * 0x9E3779B1u) >> claims.shift;
 #pragma unroll
             for (int k = 0; k < kE; ++k) {
+                if constexpr (TORUS) {
+                    // a bond inside one cluster closes a loop, which winds
+                    // around the torus where the two ways around it differ
+                    if (open[k] && x[2 * k] == x[2 * k + 1]) {
+                        const auto d = pos[2 * k] + step(down[k]) - pos[2 * k + 1];
+                        if (d != 0) {
+                            const uint32_t row = i0 + k;
+                            if (NodesT::dx(d) != 0 && row < sh.wrap[0]) atomicMin(&sh.wrap[0], row);
+                            if (NodesT::dy(d) != 0 && row < sh.wrap[1]) atomicMin(&sh.wrap[1], row);
+                        }
+                    }
+                }
                 open[k] = open[k] && x[2 * k] != x[2 * k + 1];
                 if (!open[k]) continue;
                 wants = true;
@@ -541,6 +648,16 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             if (!__syncthreads_or(wants)) break;
             any_join = true;
             wants = false;
+            if constexpr (TORUS) {
+                if (round == 0) {
+#pragma unroll
+                    for (int c = 0; c < 2 * kE; ++c)
+                        if (!is_root(first_w[c]) && first_w[c] != x[c]) {
+                            nd.shorten(start[c], x[c]);
+                            nd.set_disp(start[c], pos[c]);
+                        }
+                }
+            }
 #pragma unroll
             for (int k = 0; k < kE; ++k) {
                 if (!open[k]) continue;
@@ -552,6 +669,12 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                 }
                 open[k] = false;
                 const uint32_t a = nd.size(w[2 * k]), b = nd.size(w[2 * k + 1]);
+                if constexpr (TORUS) {
+                    // position of v's root as seen from u's
+                    const auto d = pos[2 * k] + step(down[k]) - pos[2 * k + 1];
+                    const bool under_u = gu || (!gv && a >= b);
+                    nd.set_disp(under_u ? xv : xu, under_u ? d : -d);
+                }
                 if (gu || gv) {
                     const uint32_t c = gu ? xv : xu, wc = gu ? w[2 * k + 1] : w[2 * k];
                     nd.link(c, G);
@@ -582,6 +705,15 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
 
         // ---- 4. totals after every bond
         const bool want = sink.wants(base, B);
+        // torus: first window row whose flag is set (a later row of another
+        // thread's next batch may be in already; it does not reach these rows)
+        uint32_t wrap_row = 0xffffffffu;
+        if constexpr (TORUS) {
+            if (run.spanning) {
+                const uint32_t rx = sh.wrap[0], ry = sh.wrap[1];
+                wrap_row = g.wrap == 0 ? min(rx, ry) : g.wrap == 1 ? rx : g.wrap == 2 ? ry : max(rx, ry);
+            }
+        }
         uint32_t ms[kE], m0[kE];
         Sums<NARROW> m[kE];
         if (!any_join) {
@@ -591,7 +723,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             for (int k = 0; k < kE; ++k) {
                 m[k] = c;
                 m0[k] = cl;
-                ms[k] = g_size | (span ? kSpanBit : 0u);
+                ms[k] = g_size | (span || i0 + k >= wrap_row ? kSpanBit : 0u);
             }
         } else {
             // prefix sums over the thread's bonds, then over the warp
@@ -681,7 +813,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             const uint32_t cl = sh.clusters[cur];
             // first row (of the batch) at which a cluster spans
             uint32_t span_row = span ? 0u : 0xffffffffu;
-            if (run.spanning && !span && (sides_all == 3u || init_both)) {
+            if (!TORUS && run.spanning && !span && (sides_all == 3u || init_both)) {
 #pragma unroll
                 for (int k = 0; k < kE; ++k) {
                     if (kind[k] == 0) continue;
@@ -714,7 +846,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                     m[k].plus_powers(gs);
                     m[k].minus_powers(largest);
                 }
-                ms[k] = largest | (t * kE + k >= span_row ? kSpanBit : 0u);
+                ms[k] = largest | (t * kE + k >= span_row || i0 + k >= wrap_row ? kSpanBit : 0u);
             }
             if (t == 32u * W - 1u) {
                 Sums<NARROW> c = pre;
@@ -776,7 +908,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
         if (t == 0) nd.set_root(G, g_size, g_sides);
         __syncthreads();
         if constexpr (SHARED) {
-            const uint32_t words = (val_bytes(g.N) + flag_bytes(g.N)) / 4u;
+            const uint32_t words = node_bytes<TORUS>(g.N) / 4u;
             const uint32_t *src = reinterpret_cast<const uint32_t *>(nd.val);
             for (uint32_t i = t; i < words; i += 32u * W) run.home[i] = src[i];
         }
@@ -791,6 +923,8 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
         st.max = g_size;
         st.flags = (span ? kFlagSpan : 0u) | (init_both ? kFlagInitBoth : 0u) | (bad ? kFlagCorrupt : 0u) |
                    (g_sides << 8);
+        if (TORUS)
+            st.flags |= (sh.wrap[0] != 0xffffffffu ? kFlagWrapX : 0u) | (sh.wrap[1] != 0xffffffffu ? kFlagWrapY : 0u);
         st.pad = G;
         *run.state = st;
     }

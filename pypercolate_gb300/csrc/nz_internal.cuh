@@ -46,8 +46,7 @@ void launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t n_runs
 // the run in the window that begins at row 0)
 void launch_uf_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
 
-// nz_lattice.cu: site percolation and the torus (dispatched from nz_uf.cu)
-bool lattice_extension(const GraphDev &g);
+// nz_lattice.cu: site percolation (dispatched from nz_uf.cu)
 void launch_init_lattice_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
                               cudaStream_t s);
 void launch_lattice_window(const UfParams &p, int perm_mode, bool span, int block, cudaStream_t s);

@@ -1,10 +1,11 @@
-// nz_lattice.cu -- site percolation, and wrapping on the periodic square lattice.
+// nz_lattice.cu -- site percolation on the grid, the chain and the torus.
 //
-// Extensions that the reference lists as to-do (percolate/__init__.py:68-78;
+// An extension that the reference lists as to-do (percolate/__init__.py:68-78;
 // percolate/percolate.py:210-211 rejects every model but 'bond'), built on
-// the union-find of nz_uf.cu and writing the same per-step records, so the
+// the union-find's node words and writing the same per-step records, so the
 // fused microcanonical reductions, the canonical convolution and every other
-// consumer of records apply unchanged.
+// consumer of records apply unchanged.  (Bond percolation, on the torus too, is
+// in nz_group.cuh.)
 //
 // Site percolation (Newman & Ziff, Phys. Rev. Lett. 85, 4104 (2000); Phys.
 // Rev. E 64, 016706 (2001), Sec. II): step n occupies the n-th site of a
@@ -127,11 +128,9 @@ __device__ __forceinline__ void link(uint32_t *node, uint32_t u, uint32_t v, Tal
     if (SPAN && sides == 3u) t.st.flags |= kFlagSpan;
 }
 
-// Site kernel at most 56 registers (9 CTAs of 128 per SM), like the bond
-// union-find: beside the convolution of the previous window this measured
-// 5.84e9 against 5.47e9 site additions/s (L = 256, 100,000 runs).  The torus
-// kernel is not capped (72 registers for bonds, 78 for sites; capped, the
-// 78-register bond kernel of the time spilled and measured 18 % slower).
+// Site kernel at most 56 registers (9 CTAs of 128 per SM): beside the
+// convolution of the previous window this measured 5.84e9 against 5.47e9 site
+// additions/s (L = 256, 100,000 runs).  The torus kernel is not capped.
 #ifndef NZ_SITE_MIN_BLOCKS
 #define NZ_SITE_MIN_BLOCKS 9
 #endif
@@ -254,8 +253,8 @@ __device__ __forceinline__ void link_torus(uint4 *cell, uint32_t u, uint32_t v, 
     t.merge(a, b);
 }
 
-template <bool SITE, int PERM, bool SPAN>
-__global__ void __launch_bounds__(256) torus_window_kernel(UfParams p) {
+template <int PERM, bool SPAN>
+__global__ void __launch_bounds__(256) torus_site_window_kernel(UfParams p) {
     const int32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= p.n_runs) return;
     const GraphDev &g = p.g;
@@ -268,51 +267,29 @@ __global__ void __launch_bounds__(256) torus_window_kernel(UfParams p) {
     else perm = p.perms + (size_t)r * g.M;
     const NzRecords rec = p.rec;
     const uint32_t L = g.L;
-    // bond model: the next step's index is computed while this step's first
-    // loads are in flight (7.3e9 against 7.0e9 bond additions/s at L = 256);
-    // the site model measured 2 % slower that way and computes it in place
-    uint32_t e_next = 0;
-    if (!SITE) {
-        const uint32_t first = p.n_begin > 0 ? p.n_begin - 1u : 0u;
-        if (first < g.M) e_next = step_index<PERM>(fp, perm, first);
-    }
     for (uint32_t n = p.n_begin; n < p.n_end; ++n) {
         uint32_t e = 0;
         if (n > 0) {
-            bool advanced = false;
-            if (SITE) {
-                e = step_index<PERM>(fp, perm, n - 1u);
-                if (e < g.N) {
-                    const uint4 ce = cell[e];
-                    if (ce.x == kEmpty) {
-                        const uint4 occupied = make_uint4(make_root(1u, 0u), 0u, 0u, 0u);
-                        cell[e] = occupied;
-                        t.add_single();
-                        const uint32_t row = e / L, col = e - row * L;
-                        const uint32_t right = row * L + (col + 1u == L ? 0u : col + 1u);
-                        const uint32_t left = row * L + (col == 0u ? L - 1u : col - 1u);
-                        const uint32_t down = (row + 1u == L ? 0u : row + 1u) * L + col;
-                        const uint32_t up = (row == 0u ? L - 1u : row - 1u) * L + col;
-                        // this site's cell is re-read for every link: an earlier link
-                        // may have hung it below another root
-                        if (cell[right].x != kEmpty) link_torus(cell, e, right, cell[e], cell[right], 1, 0, t);
-                        if (cell[left].x != kEmpty) link_torus(cell, e, left, cell[e], cell[left], -1, 0, t);
-                        if (cell[down].x != kEmpty) link_torus(cell, e, down, cell[e], cell[down], 0, 1, t);
-                        if (cell[up].x != kEmpty) link_torus(cell, e, up, cell[e], cell[up], 0, -1, t);
-                    }
+            e = step_index<PERM>(fp, perm, n - 1u);
+            if (e < g.N) {
+                const uint4 ce = cell[e];
+                if (ce.x == kEmpty) {
+                    const uint4 occupied = make_uint4(make_root(1u, 0u), 0u, 0u, 0u);
+                    cell[e] = occupied;
+                    t.add_single();
+                    const uint32_t row = e / L, col = e - row * L;
+                    const uint32_t right = row * L + (col + 1u == L ? 0u : col + 1u);
+                    const uint32_t left = row * L + (col == 0u ? L - 1u : col - 1u);
+                    const uint32_t down = (row + 1u == L ? 0u : row + 1u) * L + col;
+                    const uint32_t up = (row == 0u ? L - 1u : row - 1u) * L + col;
+                    // this site's cell is re-read for every link: an earlier link
+                    // may have hung it below another root
+                    if (cell[right].x != kEmpty) link_torus(cell, e, right, cell[e], cell[right], 1, 0, t);
+                    if (cell[left].x != kEmpty) link_torus(cell, e, left, cell[e], cell[left], -1, 0, t);
+                    if (cell[down].x != kEmpty) link_torus(cell, e, down, cell[e], cell[down], 0, 1, t);
+                    if (cell[up].x != kEmpty) link_torus(cell, e, up, cell[e], cell[up], 0, -1, t);
                 }
-            } else if ((e = e_next) < g.M) {
-                const bool vertical = e >= g.N;
-                const uint32_t u = vertical ? e - g.N : e;
-                const uint32_t row = u / L, col = u - row * L;
-                const uint32_t v = vertical ? (row + 1u == L ? 0u : row + 1u) * L + col
-                                            : row * L + (col + 1u == L ? 0u : col + 1u);
-                const uint4 cu = cell[u], cv = cell[v];
-                if (n < g.M) e_next = step_index<PERM>(fp, perm, n);
-                advanced = true;
-                link_torus(cell, u, v, cu, cv, vertical ? 0 : 1, vertical ? 1 : 0, t);
             }
-            if (!SITE && !advanced && n < g.M) e_next = step_index<PERM>(fp, perm, n);
         }
         const size_t off = (size_t)(n - p.n_begin) * rec.run_stride + r;
         t.write(rec, off, SPAN && wraps(t.st.flags, g.wrap), e);
@@ -335,14 +312,13 @@ __global__ void init_torus_cells_kernel(uint64_t total, uint32_t word, uint4 *ce
         cells[i] = make_uint4(word, 0u, 0u, 0u);
 }
 
-// bond model: N clusters of one node; site model: nothing occupied
-__global__ void init_lattice_state_kernel(int32_t n_runs, uint32_t N, uint32_t site, RunState *state) {
+// nothing occupied
+__global__ void init_lattice_state_kernel(int32_t n_runs, RunState *state) {
     const int32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n_runs) return;
     RunState s;
-    const uint32_t c = site ? 0u : N;
-    s.t2 = c; s.t3 = c; s.t4_lo = c; s.t4_hi = 0;
-    s.t0 = c; s.max = site ? 0u : 1u; s.flags = 0u; s.pad = 0;
+    s.t2 = s.t3 = s.t4_lo = s.t4_hi = 0;
+    s.t0 = s.max = s.flags = s.pad = 0u;
     state[r] = s;
 }
 
@@ -359,18 +335,17 @@ void launch_site_k(const UfParams &p, bool span, int block, cudaStream_t s) {
     else site_window_kernel<KIND, PERM, false><<<grid, block, 0, s>>>(p);
 }
 
-template <bool SITE, int PERM>
+template <int PERM>
 void launch_torus_k(const UfParams &p, bool span, int block, cudaStream_t s) {
     dim3 grid((p.n_runs + block - 1) / block);
-    if (span) torus_window_kernel<SITE, PERM, true><<<grid, block, 0, s>>>(p);
-    else torus_window_kernel<SITE, PERM, false><<<grid, block, 0, s>>>(p);
+    if (span) torus_site_window_kernel<PERM, true><<<grid, block, 0, s>>>(p);
+    else torus_site_window_kernel<PERM, false><<<grid, block, 0, s>>>(p);
 }
 
 template <int PERM>
 void launch_lattice_perm(const UfParams &p, bool span, int block, cudaStream_t s) {
     if (p.g.kind == NZ_GRAPH_TORUS2D) {
-        if (p.g.site) launch_torus_k<true, PERM>(p, span, block, s);
-        else launch_torus_k<false, PERM>(p, span, block, s);
+        launch_torus_k<PERM>(p, span, block, s);
     } else if (p.g.kind == NZ_GRAPH_GRID2D) {
         launch_site_k<NZ_GRAPH_GRID2D, PERM>(p, span, block, s);
     } else {
@@ -380,18 +355,15 @@ void launch_lattice_perm(const UfParams &p, bool span, int block, cudaStream_t s
 
 }  // namespace
 
-bool lattice_extension(const GraphDev &g) { return g.site || g.kind == NZ_GRAPH_TORUS2D; }
-
 void launch_init_lattice_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
                               cudaStream_t s) {
     // every word of the runs' node arrays (the grid's layout has padding slots)
     const uint64_t total = (uint64_t)n_runs * (g.kind == NZ_GRAPH_TORUS2D ? g.N : g.slots);
     if (g.kind == NZ_GRAPH_TORUS2D)
-        init_torus_cells_kernel<<<grid_for(total), 256, 0, s>>>(total, g.site ? kEmpty : make_root(1u, 0u),
-                                                                 reinterpret_cast<uint4 *>(nodes));
+        init_torus_cells_kernel<<<grid_for(total), 256, 0, s>>>(total, kEmpty, reinterpret_cast<uint4 *>(nodes));
     else
         init_site_nodes_kernel<<<grid_for(total), 256, 0, s>>>(total, nodes);
-    init_lattice_state_kernel<<<(n_runs + 255) / 256, 256, 0, s>>>(n_runs, g.N, g.site, state);
+    init_lattice_state_kernel<<<(n_runs + 255) / 256, 256, 0, s>>>(n_runs, state);
 }
 
 void launch_lattice_window(const UfParams &p, int perm_mode, bool span, int block, cudaStream_t s) {

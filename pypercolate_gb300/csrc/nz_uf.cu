@@ -1,8 +1,8 @@
 // nz_uf.cu -- permutations, reference rows and the union-find's dispatch.
 //
 // Bond percolation (percolate/hpc.py:249-307, bond_sample_states) runs in
-// nz_ufg.cu, site percolation and the torus in nz_lattice.cu; all of them
-// write the per-step records that the consumers share.
+// nz_ufg.cu, site percolation in nz_lattice.cu; both write the per-step records
+// that the consumers share.
 #include <cstdint>
 
 #include "nz_common.cuh"
@@ -60,7 +60,7 @@ __global__ void pack_rows_kernel(NzRecords rec, int32_t run, uint32_t N, uint32_
 // ------------------------------------------------------------ launchers
 const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
                                  uint32_t *flag_scratch, cudaStream_t s) {
-    if (lattice_extension(g)) {
+    if (g.site) {
         launch_init_lattice_runs(g, n_runs, nodes, state, s);
         return nullptr;
     }
@@ -72,7 +72,7 @@ const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *no
 }
 
 void launch_uf_window(const UfParams &p, int perm_mode, bool span, int block, cudaStream_t s) {
-    if (lattice_extension(p.g)) launch_lattice_window(p, perm_mode, span, block, s);
+    if (p.g.site) launch_lattice_window(p, perm_mode, span, block, s);
     else launch_uf_groups(p, perm_mode != NZ_PERM_PHILOX, span, s);
 }
 

@@ -63,7 +63,7 @@ struct RowSink {
 };
 
 // Block r runs the bonds of rows [n_begin, n_end) of run r.
-template <int W, bool SHARED>
+template <int W, bool SHARED, bool TORUS>
 __global__ void __launch_bounds__(32 * W, 24 / W) uf_group_kernel(UfParams p, uint32_t claim_count, bool given, bool spanning) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ GroupShared<W, SHARED> sh;
@@ -81,18 +81,19 @@ __global__ void __launch_bounds__(32 * W, 24 / W) uf_group_kernel(UfParams p, ui
     run.spanning = spanning;
     run.init_both = p.init_flag && *p.init_flag;
     RowSink sink{p.rec, p.tiled, r, p.n_end - p.n_begin};
-    const bool bad = group_run<W, SHARED>(p.g, run, sh, claims, smem + (size_t)claim_count * 4u, sink);
+    const bool bad = group_run<W, SHARED, TORUS>(p.g, run, sh, claims, smem + (size_t)claim_count * 4u, sink);
     if (bad && p.errors && threadIdx.x == 0) atomicAdd(p.errors, 1u);
 }
 
-template <int W, bool SHARED>
+template <int W, bool SHARED, bool TORUS>
 void launch_group(const UfParams &p, bool given, bool span, cudaStream_t s) {
-    const uint32_t claims = claim_words<W, SHARED>(p.g.slots);
+    const uint32_t claims = claim_words<W, SHARED>(node_count<SHARED, TORUS>(p.g));
     size_t smem = (size_t)claims * 4u;
-    if (SHARED) smem += val_bytes(p.g.N) + flag_bytes(p.g.N);
+    if (SHARED) smem += node_bytes<TORUS>(p.g.N);
     if (smem > 40 * 1024)
-        cudaFuncSetAttribute(uf_group_kernel<W, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    uf_group_kernel<W, SHARED><<<p.n_runs, 32 * W, smem, s>>>(p, claims, given, span);
+        cudaFuncSetAttribute(uf_group_kernel<W, SHARED, TORUS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
+    uf_group_kernel<W, SHARED, TORUS><<<p.n_runs, 32 * W, smem, s>>>(p, claims, given, span);
 }
 
 // Warps per run.  In shared memory: kWarpsPerSm warps on every SM (80 registers
@@ -107,9 +108,10 @@ constexpr int kWarpsPerSm = 24;
 constexpr int kWarpChoices[8] = {1, 2, 3, 4, 6, 8, 12, 24};
 int group_warps(const UfParams &p) {
     const uint32_t N = p.g.N;
-    if (N > kSharedNodes) return p.n_runs <= 152 ? 24 : 12;
+    const bool torus = p.g.kind == NZ_GRAPH_TORUS2D;
+    if (N > (torus ? kSharedTorus : kSharedNodes)) return p.n_runs <= 152 ? 24 : 12;
     int runs = (p.n_runs + 151) / 152;
-    const int fit = (int)(226u * 1024u / (val_bytes(N) + flag_bytes(N) + 6144u));
+    const int fit = (int)(226u * 1024u / ((torus ? node_bytes<true>(N) : node_bytes<false>(N)) + 6144u));
     runs = runs < fit ? runs : fit;
     int w = 1;
     for (int c : kWarpChoices)
@@ -117,27 +119,33 @@ int group_warps(const UfParams &p) {
     return w;
 }
 
+template <bool TORUS>
+void launch_groups(const UfParams &p, bool given, bool span, cudaStream_t s) {
+    const int warps = group_warps(p);
+    if (p.g.N <= (TORUS ? kSharedTorus : kSharedNodes)) {
+        switch (warps) {
+            case 1: launch_group<1, true, TORUS>(p, given, span, s); break;
+            case 2: launch_group<2, true, TORUS>(p, given, span, s); break;
+            case 3: launch_group<3, true, TORUS>(p, given, span, s); break;
+            case 4: launch_group<4, true, TORUS>(p, given, span, s); break;
+            case 6: launch_group<6, true, TORUS>(p, given, span, s); break;
+            case 8: launch_group<8, true, TORUS>(p, given, span, s); break;
+            case 12: launch_group<12, true, TORUS>(p, given, span, s); break;
+            default: launch_group<24, true, TORUS>(p, given, span, s); break;
+        }
+    } else if (warps == 12) {
+        launch_group<12, false, TORUS>(p, given, span, s);
+    } else {
+        launch_group<24, false, TORUS>(p, given, span, s);
+    }
+}
+
 }  // namespace
 
 void launch_uf_groups(const UfParams &p, bool given, bool span, cudaStream_t s) {
     if (p.n_runs <= 0) return;
-    const int warps = group_warps(p);
-    if (p.g.N <= kSharedNodes) {
-        switch (warps) {
-            case 1: launch_group<1, true>(p, given, span, s); break;
-            case 2: launch_group<2, true>(p, given, span, s); break;
-            case 3: launch_group<3, true>(p, given, span, s); break;
-            case 4: launch_group<4, true>(p, given, span, s); break;
-            case 6: launch_group<6, true>(p, given, span, s); break;
-            case 8: launch_group<8, true>(p, given, span, s); break;
-            case 12: launch_group<12, true>(p, given, span, s); break;
-            default: launch_group<24, true>(p, given, span, s); break;
-        }
-    } else if (warps == 12) {
-        launch_group<12, false>(p, given, span, s);
-    } else {
-        launch_group<24, false>(p, given, span, s);
-    }
+    if (p.g.kind == NZ_GRAPH_TORUS2D) launch_groups<true>(p, given, span, s);
+    else launch_groups<false>(p, given, span, s);
 }
 
 }  // namespace nz

@@ -89,3 +89,72 @@ def test_windows_leave_the_sums_alone(gpu, kind, L, window):
     assert (a['sums'] == b['sums']).all()
     np.testing.assert_array_equal(a['m2'], b['m2'])
     np.testing.assert_allclose(ma, mb, rtol=1e-12)  # FP64 sums of < 2^17 terms in another order
+
+
+# 128: the last torus in shared memory; wrapping criteria, and one and two
+# nodes to a side, where bonds are loops and doubled
+@pytest.mark.parametrize('wrap', ['either', 'x', 'y', 'both'])
+@pytest.mark.parametrize('L,runs', [(1, 2), (2, 40), (3, 2000), (20, 60), (33, 700), (128, 2), (129, 2)])
+def test_torus_matches_census(gpu, oracle, L, runs, wrap):
+    from pypercolate_gb300 import lattice
+    host = lattice.sample_records('torus', L, wrap=wrap, n_runs=runs, key=23, run0=3)
+    M = 2 * L * L
+    for r in sorted({0, runs - 1} if L < 100 else {runs - 1}):
+        perm = oracle.philox_permutation(23, 3 + r, M)
+        assert np.array_equal(host['edge'][1:, r], perm)
+        if L <= 33:  # the census is a search of the lattice per step
+            ref = oracle.lattice_census('torus', L, perm, wrap=wrap)
+            for plane in ('max_span', 'm0', 'm2', 'm3', 'm4_lo'):
+                assert np.array_equal(host[plane][:, r], ref[plane]), plane
+        else:
+            eu, ev = _torus_edges(L)
+            ref = oracle.sample_states(L * L, M, eu, ev, np.zeros(L * L, np.uint8), False, perm)
+            assert np.array_equal(host['max_span'][:, r] & 0x7fffffff, ref['max'])
+            assert np.array_equal(host['m4_lo'][:, r], ref['moments_u64'][:, 4])
+            assert np.array_equal((host['max_span'][:, r] >> 31).astype(bool), _wraps(L, perm, wrap))
+
+
+def _torus_edges(L):
+    n = np.arange(L * L)
+    row, col = n // L, n % L
+    return (np.concatenate([n, n]).astype(np.uint32),
+            np.concatenate([row * L + (col + 1) % L, (row + 1) % L * L + col]).astype(np.uint32))
+
+
+def _wraps(L, perm, wrap):
+    """Wrapping flags by a union-find with positions, one bond at a time."""
+    N = L * L
+    eu, ev = (a.astype(int).tolist() for a in _torus_edges(L))
+    parent, off, size = list(range(N)), [(0, 0)] * N, [1] * N
+    wx = wy = False
+    out = [False]
+    for e in perm.tolist():
+        u, v, pos = eu[e], ev[e], []
+        for x in (u, v):
+            px = py = 0
+            while parent[x] != x:
+                px, py, x = px + off[x][0], py + off[x][1], parent[x]
+            pos.append((x, px, py))
+        (a, ax, ay), (b, bx, by) = pos
+        dx, dy = ax + (e < N) - bx, ay + (e >= N) - by
+        if a == b:
+            wx, wy = wx or dx != 0, wy or dy != 0
+        elif size[a] >= size[b]:
+            parent[b], off[b], size[a] = a, (dx, dy), size[a] + size[b]
+        else:
+            parent[a], off[a], size[b] = b, (-dx, -dy), size[a] + size[b]
+        out.append({'either': wx or wy, 'x': wx, 'y': wy, 'both': wx and wy}[wrap])
+    return np.array(out)
+
+
+def test_torus_windows(gpu):
+    from pypercolate_gb300.ensemble import Ensemble
+    for L, window in ((24, 100), (130, 20000)):
+        got = []
+        for w in (0, window):
+            e = Ensemble('torus', L, [0.4, 0.5], precision='fp64', wrap='both', window=w)
+            e.run(40, key=3)
+            assert e.errors() == 0
+            got.append(e.micro_sums())
+        assert np.array_equal(got[0]['span_count'], got[1]['span_count'])
+        assert (got[0]['sums'] == got[1]['sums']).all()
