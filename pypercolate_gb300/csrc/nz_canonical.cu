@@ -11,6 +11,7 @@
 #include <type_traits>
 
 #include "nz_common.cuh"
+#include "nz_conv.cuh"
 #include "nz_internal.cuh"
 #include "nz_math.cuh"
 #include "nz_records.cuh"
@@ -271,7 +272,6 @@ constexpr int kConvRuns = 128;         // runs per CTA (one per thread)
 // earlier FP64-accumulated kernels); 16 is an autotuner candidate for the
 // m0 / m3 / m4 kernel
 constexpr int kConvPT = 8;
-constexpr int kConvChunk = 128;  // rows staged per step, summed in FP32 before the TwoSum add
 // 16 record loads in flight per thread: over the FP32 band (weights >= e^-30
 // of the mode) 1047 against 1052 ms per 100,000-run L = 256 step with 8
 // (over the full e^-80 band 8 had been better: 479 against 512 ms); 32
@@ -280,31 +280,6 @@ constexpr int kConvChunk = 128;  // rows staged per step, summed in FP32 before 
 #define NZ_CONV_BATCH 16
 #endif
 constexpr int kConvBatch = NZ_CONV_BATCH;  // record loads in flight per thread
-
-// Window accumulator of one canonical value.  FP64 path: an FP64 sum.  FP32
-// path: the FP32 partial sums of the row chunks are added into an FP32
-// (sum, compensation) pair by an error-free addition -- as accurate as an
-// FP64 sum of them, without the FP64 pipe, which runs at 1/64 of the FP32
-// rate on this chip.
-template <int PRECISION>
-struct ConvAcc {
-    double v = 0.0;
-    __device__ __forceinline__ void add(double x) { v += x; }
-    __device__ __forceinline__ double value() const { return v; }
-};
-template <>
-struct ConvAcc<1> {
-    float s = 0.0f, c = 0.0f;
-    // chunk sums and the running sum are >= 0: Fast2Sum on the operands
-    // ordered by size is exact (3 additions and a max / min, not TwoSum's 6)
-    __device__ __forceinline__ void add(float x) {
-        const float a = fmaxf(s, x), b = fminf(s, x);
-        const float t = __fadd_rn(a, b);
-        c = __fadd_rn(c, __fsub_rn(b, __fsub_rn(t, a)));
-        s = t;
-    }
-    __device__ __forceinline__ double value() const { return (double)s + (double)c; }
-};
 
 // grid: (run tiles, p tiles, 7 statistics).  Each thread accumulates the
 // kConvPT canonical values of its run for one statistic over the window's
@@ -394,7 +369,7 @@ __device__ __forceinline__ void conv_rows_max(const ConvParams &p, uint32_t c0, 
     }
 }
 
-// ---- the same sums over tiled records.  A chunk's rows are read in groups of
+// ---- the same sums over tiled records (FP64; FP32: nz_conv_tiles.cu).  A chunk's rows are read in groups of
 // 8 (16-byte loads of one run's consecutive rows, kTileAhead groups in flight)
 // from the group that holds its first row; s_w row 0 is that group's first row
 // and rows outside the chunk have zero weights, which leave every FP32 partial
@@ -461,9 +436,8 @@ __device__ __forceinline__ void conv_rows_tiled(const ConvParams &p, uint32_t fi
     for_groups<(sizeof(tile_raw<S>) == 8 ? 2 : kTileAhead), Raw>(
         groups,
         [&](uint32_t k, Raw &q) {
-            const size_t off = record_off(p.rec, true, first + 8 * k, r);
-            load_rows8(tile_plane<S>(p.rec), off, q.q);
-            if constexpr (S == 6) load_rows8(p.rec.m4_hi, off, q.hi);
+            load_rows8(tile_plane<S>(p.rec), p.rec.run_stride, first + 8 * k, r, q.q);
+            if constexpr (S == 6) load_rows8(p.rec.m4_hi, p.rec.run_stride, first + 8 * k, r, q.hi);
         },
         [&](uint32_t k, const Raw &q) {
 #pragma unroll
@@ -490,7 +464,7 @@ __device__ __forceinline__ void conv_rows_max_tiled(const ConvParams &p, uint32_
 #pragma unroll
     for (int j = 0; j < kConvPT; ++j) p0[j] = p1[j] = p3[j] = 0;
     for_groups<kTileAhead, Raw>(
-        groups, [&](uint32_t k, Raw &q) { load_rows8(p.rec.max_span, record_off(p.rec, true, first + 8 * k, r), q.q); },
+        groups, [&](uint32_t k, Raw &q) { load_rows8(p.rec.max_span, p.rec.run_stride, first + 8 * k, r, q.q); },
         [&](uint32_t k, const Raw &q) {
 #pragma unroll
             for (int b = 0; b < 8; ++b) {
@@ -635,66 +609,6 @@ __global__ void NZ_CONV_BOUNDS conv_window_kernel(ConvParams p) {
 // ---------------------------------------------------------------------
 // m2 with compensated FP32 arithmetic
 // ---------------------------------------------------------------------
-// sum' s^2 / N is the susceptibility curve: up to ~2e4 at L = 1024, and its
-// canonical value must come within 1e-6 absolute of the FP64 convolution,
-// i.e. ~5e-11 relative per run.  Plain FP32 sums of 128 products carry
-// ~1e-7, and FP32 weights alone ~2e-9.  So every term is computed from exact
-// two-part operands and summed with its rounding errors kept, after Dot2 of
-// Ogita, Rump & Oishi (2005, "Accurate sum and dot product"):
-//   w = wh + wl        (wh = FP32(w64), wl = FP32(w64 - wh): ~2^-48 relative)
-//   q = qh + ql        (qh = q rounded toward zero to 24 bits, ql = q - qh,
-//                       both exact in FP32 for q < 2^48)
-//   ph = wh qh, eh = fma(wh, qh, -ph)     (TwoProduct: ph + eh = wh qh exactly)
-//   (s, e) = Fast2Sum(max(s, ph), min(s, ph))  (s + e = old s + ph exactly)
-//   c += e + eh + wh ql + wl qh           (wl ql, ~2^-48 of the term, dropped)
-// The run's value is s + c (FP64), about 2^-44 relative; the statistic's
-// curve then inherits FP64-level accuracy from the FP64 run reduction.
-// Only the band's core -- the rows whose weight is >= e^-8 of the mode, +-4
-// standard deviations -- needs this: the tails hold < 1e-4 of the weight,
-// and plain FP32 products summed per chunk keep their error near 1e-11 of
-// the value.  Chunks of rows outside every core of a tile (about a third of
-// a tile's rows) take the plain path.
-struct Dot2Acc {
-    float s = 0.0f, c = 0.0f, tail = 0.0f;
-    // a compensated term.  Every term and the running sum are >= 0, so
-    // ordering the two operands by size (max / min, on the integer pipe)
-    // makes Dekker's Fast2Sum exact: 3 additions instead of TwoSum's 6.
-    __device__ __forceinline__ void add(float wh, float wl, float qh, float ql) {
-        const float ph = __fmul_rn(wh, qh);
-        const float eh = __fmaf_rn(wh, qh, -ph);
-        const float a = fmaxf(s, ph), b = fminf(s, ph);
-        const float t = __fadd_rn(a, b);
-        const float e = __fsub_rn(b, __fsub_rn(t, a));
-        s = t;
-        c = __fadd_rn(c, __fadd_rn(e, eh));
-        c = __fmaf_rn(wh, ql, c);
-        c = __fmaf_rn(wl, qh, c);
-    }
-    // a term of a chunk outside every core: plain FP32 product and sum,
-    // added into the running sum once per chunk by Fast2Sum (so the
-    // compensation stays of the size of the rounding errors it collects)
-    __device__ __forceinline__ void add_tail(float wh, float q) { tail = __fmaf_rn(wh, q, tail); }
-    __device__ __forceinline__ void flush_tail() {
-        const float a = fmaxf(s, tail), b = fminf(s, tail);
-        const float t = __fadd_rn(a, b);
-        c = __fadd_rn(c, __fsub_rn(b, __fsub_rn(t, a)));
-        s = t;
-        tail = 0.0f;
-    }
-    __device__ __forceinline__ double value() const { return (double)s + (double)c; }
-};
-
-// q (< 2^48) as qh + ql, both exact in FP32
-__device__ __forceinline__ void split_u64(uint64_t q, float &qh, float &ql) {
-    qh = __ull2float_rz(q);
-    ql = (float)(int64_t)(q - (uint64_t)qh);
-}
-__device__ __forceinline__ void split_u32(uint32_t q, float &qh, float &ql) {
-    qh = __uint2float_rz(q);
-    ql = (float)(int32_t)(q - (uint32_t)qh);
-}
-
-
 // grid (run tiles, tiles of kM2PT probabilities): each thread the kM2PT m2
 // values of its run.  A chunk of rows that meets the core of any of the
 // tile's probabilities runs the compensated arithmetic on all its rows
@@ -712,10 +626,9 @@ constexpr int kM2Batch = NZ_M2_BATCH;
 // on the same box 8 gave 1085.8 and 1204.7 ms per 100,000-run L = 256 step
 // against 1108.8 and 1224.7 ms for 16 (two boxes); 32 measured 1285 against
 // 1128 ms for 16)
-template <bool NARROW, int kM2PT, bool TILED>
+template <bool NARROW, int kM2PT>
 __global__ void NZ_CONV_BOUNDS conv_m2_comp_kernel(ConvParams p) {
-    constexpr int kRows = kConvChunk + (TILED ? 8 : 0);
-    __shared__ float s_wh[kRows][kM2PT], s_wl[kRows][kM2PT];
+    __shared__ float s_wh[kConvChunk][kM2PT], s_wl[kConvChunk][kM2PT];
     __shared__ uint32_t s_lo[kM2PT], s_len[kM2PT], s_clo[kM2PT], s_clen[kM2PT];
     __shared__ uint32_t s_range[2];
     const int r = blockIdx.x * kConvRuns + threadIdx.x;
@@ -747,13 +660,12 @@ __global__ void NZ_CONV_BOUNDS conv_m2_comp_kernel(ConvParams p) {
 #pragma unroll
         for (int j = 0; j < kM2PT; ++j)
             core |= s_clen[j] && s_clo[j] < c0 + cn && c0 < s_clo[j] + s_clen[j];
-        const uint32_t lead = TILED ? (c0 - p.n_begin) & 7u : 0u;
         __syncthreads();
-        for (int i = threadIdx.x; i < kRows * kM2PT; i += kConvRuns) {
+        for (int i = threadIdx.x; i < kConvChunk * kM2PT; i += kConvRuns) {
             const int rw = i / kM2PT, j = i % kM2PT;
-            const uint32_t n = c0 + rw - lead;
+            const uint32_t n = c0 + rw;
             float vh = 0.0f, vl = 0.0f;
-            if ((uint32_t)rw - lead < cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
+            if (rw < (int)cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
                 const size_t widx = (size_t)(p0 + j) * p.cap + (n - s_lo[j]);
                 vh = p.w32[widx];
                 vl = p.w32lo[widx];
@@ -773,40 +685,6 @@ __global__ void NZ_CONV_BOUNDS conv_m2_comp_kernel(ConvParams p) {
             if constexpr (NARROW) split_u32(w, qh, ql);
             else split_u64(w, qh, ql);
         };
-        if constexpr (TILED) {
-            // a row outside the chunk has zero weights: a compensated term of
-            // zeros leaves (s, c) as they are
-            struct Raw {
-                raw_t q[8];
-            };
-            const uint32_t first = c0 - p.n_begin - lead, groups = (lead + cn + 7u) / 8u;
-            auto load = [&](uint32_t k, Raw &q) { load_rows8(plane, record_off(p.rec, true, first + 8 * k, r), q.q); };
-            if (core) {
-                for_groups<kTileAhead, Raw>(groups, load, [&](uint32_t k, const Raw &q) {
-#pragma unroll
-                    for (int b = 0; b < 8; ++b) {
-                        float qh, ql;
-                        split(q.q[b], qh, ql);
-#pragma unroll
-                        for (int j = 0; j < kM2PT; ++j) acc[j].add(s_wh[8 * k + b][j], s_wl[8 * k + b][j], qh, ql);
-                    }
-                });
-            } else {
-                for_groups<kTileAhead, Raw>(groups, load, [&](uint32_t k, const Raw &q) {
-#pragma unroll
-                    for (int b = 0; b < 8; ++b) {
-                        float qh, ql;
-                        split(q.q[b], qh, ql);
-                        const float v = __fadd_rn(qh, ql);
-#pragma unroll
-                        for (int j = 0; j < kM2PT; ++j) acc[j].add_tail(s_wh[8 * k + b][j], v);
-                    }
-                });
-#pragma unroll
-                for (int j = 0; j < kM2PT; ++j) acc[j].flush_tail();
-            }
-            continue;
-        }
         uint32_t i = 0;
         if (core) {
             for (; i + kM2Batch <= cn; i += kM2Batch) {
@@ -866,19 +744,12 @@ void launch_conv_m2_comp(const ConvParams &p, cudaStream_t s) {
     if (p.n_runs <= 0 || p.P <= 0) return;
     const int pt = p.m2_tile == 16 ? 16 : 8;
     dim3 g((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + pt - 1) / pt, 1);
-    auto launch = [&](auto narrow, auto tile) {
-        constexpr bool N = decltype(narrow)::value;
-        constexpr int PT = decltype(tile)::value;
-        if (p.tiled) conv_m2_comp_kernel<N, PT, true><<<g, kConvRuns, 0, s>>>(p);
-        else conv_m2_comp_kernel<N, PT, false><<<g, kConvRuns, 0, s>>>(p);
-    };
-    using std::integral_constant;
     if (pt == 8) {
-        if (p.rec.narrow) launch(integral_constant<bool, true>(), integral_constant<int, 8>());
-        else launch(integral_constant<bool, false>(), integral_constant<int, 8>());
+        if (p.rec.narrow) conv_m2_comp_kernel<true, 8><<<g, kConvRuns, 0, s>>>(p);
+        else conv_m2_comp_kernel<false, 8><<<g, kConvRuns, 0, s>>>(p);
     } else {
-        if (p.rec.narrow) launch(integral_constant<bool, true>(), integral_constant<int, 16>());
-        else launch(integral_constant<bool, false>(), integral_constant<int, 16>());
+        if (p.rec.narrow) conv_m2_comp_kernel<true, 16><<<g, kConvRuns, 0, s>>>(p);
+        else conv_m2_comp_kernel<false, 16><<<g, kConvRuns, 0, s>>>(p);
     }
 }
 
@@ -909,13 +780,23 @@ static void launch_conv_window_pt(const ConvParams &p, int precision, cudaStream
             launch_conv_m2_comp(p, s);
         }
     };
-    if (p.tiled) launch(std::integral_constant<Layout, Layout::kTiled>());
-    else if (p.rec.site) launch(std::integral_constant<Layout, Layout::kSite>());
+    if (p.rec.site) launch(std::integral_constant<Layout, Layout::kSite>());
     else launch(std::integral_constant<Layout, Layout::kBond>());
 }
 
 void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
     if (p.n_runs <= 0 || p.P <= 0) return;
+    if (p.tiled) {
+        if (precision != 0) {
+            launch_conv_tiles(p, s);
+        } else {
+            dim3 gmax((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + kConvPT - 1) / kConvPT, 1);
+            dim3 gother(gmax.x, gmax.y, 4);
+            conv_window_kernel<0, Layout::kTiled, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
+            conv_window_kernel<0, Layout::kTiled, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
+        }
+        return;
+    }
     // the FP64 path keeps 8 probabilities per CTA (its accumulators are
     // twice as wide)
     if (precision != 0 && p.conv_tile == 16) launch_conv_window_pt<16>(p, precision, s);
@@ -1362,7 +1243,7 @@ struct MicroSums {
 };
 
 template <bool NARROW>
-__global__ void __launch_bounds__(32 * kMicroWarps) micro_tiled_kernel(MicroParams p) {
+__global__ void __launch_bounds__(32 * kMicroWarps, 2) micro_tiled_kernel(MicroParams p) {
     __shared__ MicroSums<NARROW> s_sum[32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t i = blockIdx.x * 32u + lane, n = p.n_begin + i;
@@ -1374,14 +1255,15 @@ __global__ void __launch_bounds__(32 * kMicroWarps) micro_tiled_kernel(MicroPara
         uint64_t m2, m3, m4;
     };
     auto load = [&](int r) -> Rec {
-        const size_t off = record_off(rec, true, i, r);
+        const size_t o4 = tile_off<4>(rec.run_stride, i, r), o8 = tile_off<8>(rec.run_stride, i, r);
         Rec q;
-        q.ms = rec.max_span[off];
-        q.m0 = NARROW ? (uint32_t)reinterpret_cast<const uint16_t *>(rec.m0)[off] : rec.m0[off];
-        q.m2 = NARROW ? (uint64_t)reinterpret_cast<const uint32_t *>(rec.m2)[off] : rec.m2[off];
-        q.m3 = rec.m3[off];
-        q.m4 = rec.m4_lo[off];
-        q.m4_hi = (!NARROW && rec.m4_hi) ? rec.m4_hi[off] : 0u;
+        q.ms = rec.max_span[o4];
+        q.m0 = NARROW ? (uint32_t)reinterpret_cast<const uint16_t *>(rec.m0)[tile_off<2>(rec.run_stride, i, r)]
+                      : rec.m0[o4];
+        q.m2 = NARROW ? (uint64_t)reinterpret_cast<const uint32_t *>(rec.m2)[o4] : rec.m2[o8];
+        q.m3 = rec.m3[o8];
+        q.m4 = rec.m4_lo[o8];
+        q.m4_hi = (!NARROW && rec.m4_hi) ? rec.m4_hi[o4] : 0u;
         return q;
     };
     auto add = [&](const Rec &q) {

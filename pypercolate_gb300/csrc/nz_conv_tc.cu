@@ -147,9 +147,9 @@ __device__ __forceinline__ void load_chunk(const NzRecords &rec, bool tiled, uin
     const raw_word<S> *plane = raw_plane<S>(rec);
 #pragma unroll
     for (int k = 0; k < kTcK; ++k) {
-        const size_t off = record_off(rec, tiled, first + min(k0 + (uint32_t)k, last), r);
-        raw[k] = plane[off];
-        if constexpr (S == 6) hi[k] = rec.m4_hi[off];
+        const uint32_t i = first + min(k0 + (uint32_t)k, last);
+        raw[k] = plane[record_off<sizeof(raw_word<S>)>(rec, tiled, i, r)];
+        if constexpr (S == 6) hi[k] = rec.m4_hi[record_off<4>(rec, tiled, i, r)];
     }
 }
 
@@ -409,7 +409,8 @@ int launch_conv_window_tc(const ConvParams &p, cudaStream_t s) {
     // m2 needs ~5e-11 relative per run (the susceptibility curve within 1e-6
     // absolute of FP64 at L = 1024), beyond FP32 tensor-core accumulation:
     // it runs on the compensated SIMT kernel
-    launch_conv_m2_comp(p, s);
+    if (p.tiled) launch_conv_tiles_m2(p, s);
+    else launch_conv_m2_comp(p, s);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

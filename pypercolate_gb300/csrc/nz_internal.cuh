@@ -22,7 +22,7 @@ struct UfParams {
     NzRecords rec;          // row n of run r at plane[(n - n_begin) * run_stride + r]
     uint32_t *errors;       // if set: +1 per run whose state is corrupt after its last row
     const uint32_t *init_flag;  // explicit edge lists: nonzero if a node touches both sides (or null)
-    bool tiled;             // rec is tiled: row i of run r at plane[((i / 32) * run_stride + r) * 32 + i % 32]
+    bool tiled;             // rec is tiled (tile_off in nz_records.cuh)
 };
 
 // nz_uf.cu
@@ -92,6 +92,9 @@ int launch_conv_window_tc(const ConvParams &p, cudaStream_t s);
 void launch_narrow_weights_f32(const double *w64, const uint32_t *band_lo, const uint32_t *band_len, int32_t P,
                                int32_t cap, double rel, double rel_core, float *w32, float *w32lo, uint32_t *lo32,
                                uint32_t *len32, uint32_t *core_lo, uint32_t *core_len, cudaStream_t s);
+// nz_conv_tiles.cu: the FP32 convolution of tiled records (all statistics, or m2 alone)
+void launch_conv_tiles(const ConvParams &p, cudaStream_t s);
+void launch_conv_tiles_m2(const ConvParams &p, cudaStream_t s);
 // m2 (statistic 4) of the FP32 paths with compensated products and sums
 void launch_conv_m2_comp(const ConvParams &p, cudaStream_t s);
 // part: scratch [slices][P*7][3] doubles

@@ -52,38 +52,42 @@ __device__ __forceinline__ uint64_t record_m2(const NzRecords &rec, size_t off) 
     return rec.narrow ? (uint64_t)reinterpret_cast<const uint32_t *>(rec.m2)[off] : rec.m2[off];
 }
 
-// Where row i of run r lies in a window's planes.  n-major: runs next to each
-// other.  Tiled (bond ensembles): 32 rows of a run next to each other, which is
-// what a block working on one run writes and a thread summing over a run's
-// rows reads.
-__device__ __forceinline__ size_t record_off(const NzRecords &rec, bool tiled, uint32_t i, int32_t r) {
-    return tiled ? ((size_t)(i >> 5) * rec.run_stride + r) * 32 + (i & 31u) : (size_t)i * rec.run_stride + r;
+// Where row i of run r lies in a tiled plane of BYTES-wide values: 32 rows of a
+// run next to each other (a line of 64, 128 or 256 bytes), which is what a block
+// working on one run writes and a thread summing over a run's rows reads; the
+// lines of a tile's runs follow each other, so that the rows of many runs are
+// one contiguous copy.  Within its line a 16-byte piece is moved by the run's
+// number, so that 8 runs' equal rows, once in shared memory, lie in different
+// banks.
+template <int BYTES>
+__device__ __forceinline__ size_t tile_off(int64_t run_stride, uint32_t i, int32_t r) {
+    constexpr uint32_t kPer = 16 / BYTES;  // rows per 16 bytes
+    const uint32_t turn = BYTES == 2 ? (uint32_t)(r >> 1) & 3u : (uint32_t)r & 7u;
+    const size_t line = ((size_t)(i >> 5) * run_stride + r) * 32;
+    return line + (((((i & 31u) / kPer) ^ turn) * kPer) | (i & (kPer - 1u)));
 }
 
-// The raw words of 8 consecutive rows of one run in a tiled plane (off: the
-// first row's place, a multiple of 8 rows), in 16-byte loads.
-__device__ __forceinline__ void load_rows8(const uint32_t *plane, size_t off, uint32_t (&q)[8]) {
-    const uint4 *v = reinterpret_cast<const uint4 *>(plane + off);
-    const uint4 a = v[0], b = v[1];
-    q[0] = a.x; q[1] = a.y; q[2] = a.z; q[3] = a.w;
-    q[4] = b.x; q[5] = b.y; q[6] = b.z; q[7] = b.w;
+// the same, or n-major (runs next to each other)
+template <int BYTES>
+__device__ __forceinline__ size_t record_off(const NzRecords &rec, bool tiled, uint32_t i, int32_t r) {
+    return tiled ? tile_off<BYTES>(rec.run_stride, i, r) : (size_t)i * rec.run_stride + r;
 }
-__device__ __forceinline__ void load_rows8(const uint64_t *plane, size_t off, uint64_t (&q)[8]) {
-    const ulonglong2 *v = reinterpret_cast<const ulonglong2 *>(plane + off);
+
+// The raw words of rows i .. i + 7 (i a multiple of 8) of one run in a tiled
+// plane, in 16-byte loads.
+template <class T>
+__device__ __forceinline__ void load_rows8(const T *plane, int64_t run_stride, uint32_t i, int32_t r, T (&q)[8]) {
+    constexpr int kPer = 16 / (int)sizeof(T);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const ulonglong2 a = v[k];
-        q[2 * k] = a.x;
-        q[2 * k + 1] = a.y;
-    }
-}
-__device__ __forceinline__ void load_rows8(const uint16_t *plane, size_t off, uint16_t (&q)[8]) {
-    const uint4 a = *reinterpret_cast<const uint4 *>(plane + off);
-    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+    for (int k = 0; k < 8; k += kPer) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(plane + tile_off<sizeof(T)>(run_stride, i + k, r));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        q[2 * k] = (uint16_t)w[k];
-        q[2 * k + 1] = (uint16_t)(w[k] >> 16);
+        for (int b = 0; b < kPer; ++b) {
+            if constexpr (sizeof(T) == 2) q[k + b] = (T)(w[b / 2] >> (16 * (b & 1)));
+            else if constexpr (sizeof(T) == 4) q[k + b] = (T)w[b];
+            else q[k + b] = (T)(((uint64_t)w[2 * b + 1] << 32) | w[2 * b]);
+        }
     }
 }
 

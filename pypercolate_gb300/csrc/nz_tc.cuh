@@ -44,6 +44,17 @@ __device__ __forceinline__ void mbar_init(uint32_t mbar) {
 }
 __device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
+// `bytes` of contiguous global memory into shared memory (all 16-byte aligned),
+// announced to and completed on an mbarrier.
+__device__ __forceinline__ void expect_bytes(uint32_t mbar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t mbar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(mbar)
+                 : "memory");
+}
+
 // Waits for the phase of the given parity; false after kWaitNs.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
     const uint64_t t0 = global_ns();

@@ -12,28 +12,28 @@ namespace {
 
 using namespace group;
 
-// Rows i0, i0 + 1 of run r (window rows; i0 is even).  Tiled: element (i, r)
-// of a plane is at ((i / 32) * run_stride + r) * 32 + i % 32, so a warp's 64
-// rows are contiguous; the planes hold whole tiles.  Otherwise n-major.
+// Rows i0, i0 + 1 of run r (window rows; i0 is even), in tiles or n-major.
+// Both rows lie in one 16-byte piece of a tile, and the planes hold whole tiles.
 template <bool NARROW>
 __device__ __forceinline__ void put_rows(const NzRecords &rec, bool tiled, uint32_t i0, uint32_t rows, int32_t r,
                                          const uint32_t (&ms)[kE], const uint32_t (&m0)[kE],
                                          const Sums<NARROW> (&m)[kE], const uint32_t (&e)[kE]) {
     if (i0 >= rows) return;
     if (tiled) {
-        const size_t off = ((size_t)(i0 >> 5) * rec.run_stride + r) * 32 + (i0 & 31u);
-        *reinterpret_cast<uint2 *>(rec.max_span + off) = make_uint2(ms[0], ms[1]);
+        const size_t o4 = tile_off<4>(rec.run_stride, i0, r), o8 = tile_off<8>(rec.run_stride, i0, r);
+        *reinterpret_cast<uint2 *>(rec.max_span + o4) = make_uint2(ms[0], ms[1]);
         if (rec.narrow) {
-            *reinterpret_cast<uint32_t *>(reinterpret_cast<uint16_t *>(rec.m0) + off) = m0[0] | (m0[1] << 16);
-            *reinterpret_cast<uint2 *>(reinterpret_cast<uint32_t *>(rec.m2) + off) =
+            const size_t o2 = tile_off<2>(rec.run_stride, i0, r);
+            *reinterpret_cast<uint32_t *>(reinterpret_cast<uint16_t *>(rec.m0) + o2) = m0[0] | (m0[1] << 16);
+            *reinterpret_cast<uint2 *>(reinterpret_cast<uint32_t *>(rec.m2) + o4) =
                 make_uint2((uint32_t)m[0].m2(), (uint32_t)m[1].m2());
         } else {
-            *reinterpret_cast<uint2 *>(rec.m0 + off) = make_uint2(m0[0], m0[1]);
-            *reinterpret_cast<ulonglong2 *>(rec.m2 + off) = make_ulonglong2(m[0].m2(), m[1].m2());
+            *reinterpret_cast<uint2 *>(rec.m0 + o4) = make_uint2(m0[0], m0[1]);
+            *reinterpret_cast<ulonglong2 *>(rec.m2 + o8) = make_ulonglong2(m[0].m2(), m[1].m2());
         }
-        *reinterpret_cast<ulonglong2 *>(rec.m3 + off) = make_ulonglong2(m[0].u3, m[1].u3);
-        *reinterpret_cast<ulonglong2 *>(rec.m4_lo + off) = make_ulonglong2(m[0].u4, m[1].u4);
-        if (rec.m4_hi) *reinterpret_cast<uint2 *>(rec.m4_hi + off) = make_uint2(m[0].m4_hi(), m[1].m4_hi());
+        *reinterpret_cast<ulonglong2 *>(rec.m3 + o8) = make_ulonglong2(m[0].u3, m[1].u3);
+        *reinterpret_cast<ulonglong2 *>(rec.m4_lo + o8) = make_ulonglong2(m[0].u4, m[1].u4);
+        if (rec.m4_hi) *reinterpret_cast<uint2 *>(rec.m4_hi + o4) = make_uint2(m[0].m4_hi(), m[1].m4_hi());
         return;
     }
 #pragma unroll
