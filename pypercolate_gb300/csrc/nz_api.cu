@@ -548,7 +548,9 @@ size_t ensemble_layout(Carver &c, const GraphDev &g, int32_t n_runs, int32_t P, 
     L.core_lo32 = c.take<uint32_t>(P);
     L.core_len32 = c.take<uint32_t>(P);
     L.stats = c.take<double>((size_t)n_runs * P * 7);
-    L.slices = n_runs < 1024 ? 1 : (n_runs < 65536 ? 16 : 64);
+    // enough slices to occupy the SMs whatever the run count (1,000 runs, 201 p:
+    // one slice 150 us, 16 slices 20)
+    L.slices = n_runs < 256 ? 1 : (n_runs < 65536 ? 16 : 64);
     // room for the largest tuned slice count
     L.part = c.take<double>((size_t)kMaxSlices * P * 7 * 3);
     return c.used;
@@ -610,15 +612,8 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
 
     {
         ProfScope prof(NZ_PROF_SETUP, s);
-        launch_binomial_weights(M, ps, P, cutoff, L.cap, L.band_lo, L.band_len, L.w64, nullptr, s);
-        if (conv_precision != 0)
-            launch_narrow_weights_f32(L.w64, L.band_lo, L.band_len, P, L.cap, exp(-fmin(cutoff, kConvF32Cutoff)),
-                                      exp(-kConvCoreCutoff), L.w32, L.w32lo, L.band_lo32, L.band_len32,
-                                      L.core_lo32, L.core_len32, s);
         if (cudaMemsetAsync(L.flag, 0, 4 * sizeof(uint32_t), s) != cudaSuccess) return NZ_ERR_CUDA;
         launch_init_runs(g, n_runs, L.nodes, L.state, L.flag, s);
-        if (cudaMemsetAsync(L.stats, 0, sizeof(double) * (size_t)n_runs * P * 7, s) != cudaSuccess)
-            return NZ_ERR_CUDA;
     }
 
     AuxGuard aux{aux_checkout()};
@@ -631,6 +626,18 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
         return NZ_ERR_CUDA;
     JoinGuard joiner1{s, s1, aux.a->join1, true};
     JoinGuard joiner{s, s2, aux.a->join, true};
+    {
+        // the weights are the consumers' alone: beside the first window's
+        // union-find
+        ProfScope prof(NZ_PROF_SETUP, s2);
+        launch_binomial_weights(M, ps, P, cutoff, L.cap, L.band_lo, L.band_len, L.w64, nullptr, s2);
+        if (conv_precision != 0)
+            launch_narrow_weights_f32(L.w64, L.band_lo, L.band_len, P, L.cap, exp(-fmin(cutoff, kConvF32Cutoff)),
+                                      exp(-kConvCoreCutoff), L.w32, L.w32lo, L.band_lo32, L.band_len32,
+                                      L.core_lo32, L.core_len32, s2);
+        if (cudaMemsetAsync(L.stats, 0, sizeof(double) * (size_t)n_runs * P * 7, s2) != cudaSuccess)
+            return NZ_ERR_CUDA;
+    }
 
     UfParams up;
     up.g = g;
