@@ -376,7 +376,7 @@ __host__ __device__ __forceinline__ uint32_t node_count(const GraphDev &g) {
 // batch seldom share a word
 template <int W, bool SHARED>
 __host__ __device__ __forceinline__ uint32_t claim_words(uint32_t slots) {
-    constexpr uint32_t kMost = SHARED ? 4096u : 8192u;
+    constexpr uint32_t kMost = SHARED ? 4096u : 16384u;
     constexpr uint32_t kEnough = 32u * W * kE * 16u < kMost ? 32u * W * kE * 16u : kMost;
     uint32_t claims = 32;
     while (claims < slots && claims < kEnough) claims <<= 1;
@@ -647,6 +647,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             }
             if (!__syncthreads_or(wants)) break;
             any_join = true;
+            const bool wanted = wants;
             wants = false;
             if constexpr (TORUS) {
                 if (round == 0) {
@@ -658,6 +659,9 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                         }
                 }
             }
+            // (a warp with no bond left does without, but in shared memory the
+            // code is faster without the branch)
+            if (SHARED || __any_sync(0xffffffffu, wanted))
 #pragma unroll
             for (int k = 0; k < kE; ++k) {
                 if (!open[k]) continue;
@@ -696,11 +700,14 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                 claims.clear();
             }
             if (!__syncthreads_or(wants)) break;
-            // the roots of unfinished bonds may have been joined to others
+            // the roots of unfinished bonds may have been joined to others (of
+            // many warps, one with none goes straight on to the next barrier)
+            if ((SHARED && W <= 4) || __any_sync(0xffffffffu, wants)) {
 #pragma unroll
-            for (int c = 0; c < 2 * kE; ++c)
-                if (open[c >> 1]) w[c] = nd.load(x[c]);
-            climb();
+                for (int c = 0; c < 2 * kE; ++c)
+                    if (open[c >> 1]) w[c] = nd.load(x[c]);
+                climb();
+            }
         }
 
         // ---- 4. totals after every bond
