@@ -283,6 +283,10 @@ int nz_microcanonical_finalize(const NzMicroAccum *acc, uint32_t num_nodes,
  * With NZ_MICRO_FIELD_MAJOR or-ed in, out is field-major instead:
  * out[j * (M + 1) + n], each value's M + 1 rows contiguous.) */
 #define NZ_MICRO_FIELD_MAJOR 2
+/* With NZ_MICRO_ARRAYS or-ed in, out holds the reference's arrays one after
+ * another: spanning mean[M+1], spanning bounds[M+1][2], max mean[M+1], max
+ * bounds[M+1][2], moments mean[5][M+1], moments bounds[5][M+1][2]. */
+#define NZ_MICRO_ARRAYS 4
 
 /* Adds the runs of a record set (rows n_begin..n_end-1 of all its runs; the
  * records' row 0 is n_begin) to the accumulators: the run-reductions of

@@ -270,7 +270,8 @@ def to_device(arr):
     torch = torch_cuda()
     a = np.ascontiguousarray(arr)
     raw = a.view(np.uint8).reshape(-1) if a.size else np.zeros(1, np.uint8)
-    return torch.from_numpy(raw.copy()).to('cuda')
+    # (the copy to the device is complete when .to returns)
+    return torch.from_numpy(raw if raw.flags.writeable else raw.copy()).to('cuda')
 
 
 def ptr(t):
@@ -280,8 +281,8 @@ def ptr(t):
 def to_host(t, dtype, shape):
     """Device byte buffer -> numpy array of the given dtype/shape."""
     n = int(np.prod(shape)) * np.dtype(dtype).itemsize
-    raw = t[:n].cpu().numpy() if n else np.zeros(0, np.uint8)
-    return raw.view(dtype).reshape(shape).copy()
+    raw = t[:n].cpu().numpy() if n else np.zeros(0, np.uint8)  # memory of its own
+    return raw.view(dtype).reshape(shape)
 
 
 def make_graph(kind, length=0, num_nodes=0, num_edges=0, edge_u=None, edge_v=None,

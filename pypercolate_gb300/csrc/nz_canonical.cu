@@ -1595,9 +1595,19 @@ __global__ void micro_finalize_kernel(NzMicroAccum acc, uint32_t N, uint32_t M, 
     // every row has R runs: one pair of t quantiles per block
     const TPair tq = t_pair_block(1.0 - alpha, R - 1.0, R - 1.0, n <= M);
     if (n > M) return;
-    // value j of row n: out[n * 21 + j], or out[j * (M + 1) + n] field-major
-    const bool fields = (normalize & NZ_MICRO_FIELD_MAJOR) != 0;
-    auto put = [&](int j, double v) { out[fields ? (size_t)j * (M + 1) + n : (size_t)n * 21 + j] = v; };
+    // value j of row n: out[n * 21 + j], out[j * (M + 1) + n] field-major, or in
+    // its array: j / 3 is the statistic, j % 3 its mean, lower or upper bound
+    const bool fields = (normalize & NZ_MICRO_FIELD_MAJOR) != 0, arrays = (normalize & NZ_MICRO_ARRAYS) != 0;
+    const size_t rows = (size_t)M + 1;
+    auto put = [&](int j, double v) {
+        size_t at = fields ? j * rows + n : (size_t)n * 21 + j;
+        if (arrays) {
+            const int f = j / 3, c = j % 3;
+            at = f < 2 ? (c == 0 ? 3 * f * rows + n : (3 * f + 1) * rows + 2 * (size_t)n + c - 1)
+                       : (c == 0 ? (4 + f) * rows + n : (11 + 2 * (f - 2)) * rows + 2 * (size_t)n + c - 1);
+        }
+        out[at] = v;
+    };
     if (spanning) {
         const double k = (double)acc.span_count[n];
         if (half == 0) {

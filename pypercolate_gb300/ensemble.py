@@ -227,7 +227,7 @@ class Ensemble:
         n = int(self.count.cpu().numpy()[0])
         mean = self.mean.cpu().numpy().reshape(self.P, 7)
         m2 = self.m2.cpu().numpy().reshape(self.P, 7)
-        ret = np.empty(self.P, dtype=hpc.canonical_averages_dtype(self.spanning))
+        ret = np.empty(self.P, dtype=hpc._dtype('canonical_averages', self.spanning))
         ret['number_of_runs'] = n
         if self.spanning:
             ret['percolation_probability_mean'] = mean[:, 0]
@@ -249,21 +249,22 @@ class Ensemble:
             raise ValueError('ensemble was created with micro=False')
         torch = nat.torch_cuda()
         out = torch.empty((self.M + 1) * 21, dtype=torch.float64, device='cuda')
-        # normalised, field-major (2 = NZ_MICRO_FIELD_MAJOR): each value's rows contiguous
+        # normalised, the arrays one after another (4 = NZ_MICRO_ARRAYS): one
+        # copy to the host, of which the results are views
         st = nat.lib_handle().nz_microcanonical_finalize(
-            self._micro_struct(), self.N, self.M, int(self.spanning), float(alpha), 1 | 2,
+            self._micro_struct(), self.N, self.M, int(self.spanning), float(alpha), 1 | 4,
             nat.ptr(out), nat.stream_handle())
         nat.check(st, 'nz_microcanonical_finalize')
-        o = out.cpu().numpy().reshape(21, self.M + 1)
-        pair = lambda j: np.stack([o[j], o[j + 1]], axis=1)  # noqa: E731
+        o, rows = out.cpu().numpy(), self.M + 1
+        take = lambda first, *shape: o[first * rows:first * rows + int(np.prod(shape))].reshape(shape)  # noqa: E731
         ret = {'N': self.N, 'M': self.M}
         if self.spanning:
-            ret['spanning_cluster'] = o[0].copy()
-            ret['spanning_cluster_ci'] = pair(1)
-        ret['max_cluster_size'] = o[3].copy()
-        ret['max_cluster_size_ci'] = pair(4)
-        ret['moments'] = o[6:21:3].copy()
-        ret['moments_ci'] = np.stack([pair(7 + 3 * k) for k in range(5)])
+            ret['spanning_cluster'] = take(0, rows)
+            ret['spanning_cluster_ci'] = take(1, rows, 2)
+        ret['max_cluster_size'] = take(3, rows)
+        ret['max_cluster_size_ci'] = take(4, rows, 2)
+        ret['moments'] = take(6, 5, rows)
+        ret['moments_ci'] = take(11, 5, rows, 2)
         return ret
 
     def micro_sums(self):

@@ -29,6 +29,7 @@ are bit-identical to the reference's for the same seed.  The keyword
 ``rng='philox'`` (swallowed by the reference's ``**kwargs``) selects the
 project's Philox-keyed permutation instead, with ``seed`` as the Philox key.
 """
+import functools
 import os
 
 import numpy as np
@@ -82,6 +83,12 @@ def finalized_canonical_averages_dtype(spanning_cluster=True):
                ('moments_mean', '(5,)float64'), ('moments_std', '(5,)float64'),
                ('moments_ci', '(5,2)float64')]
     return _ndarray_dtype(fields)
+
+
+@functools.lru_cache(maxsize=None)
+def _dtype(name, spanning):
+    """np.dtype of a row type (numpy parses the field strings on every use)."""
+    return np.dtype(globals()[name + '_dtype'](spanning))
 
 
 # ---------------------------------------------------------------------------
@@ -227,8 +234,10 @@ def _run_microcanonical(spec, spanning, seeds=None, rng='numpy', key=0, run0=0, 
     lib = nat.lib_handle()
     g = spec.struct()
     if perms is not None:
-        perms = np.ascontiguousarray(perms, dtype=np.uint32).reshape(-1, max(spec.M, 1) if spec.M else 0)
-        n_runs = perms.shape[0]
+        # host rows, or a device tensor of n_runs rows of 32-bit indices
+        if not isinstance(perms, torch.Tensor):
+            perms = np.ascontiguousarray(perms, dtype=np.uint32).reshape(-1, max(spec.M, 1) if spec.M else 0)
+            n_runs = perms.shape[0]
         mode = nat.PERM_GIVEN
     elif rng == 'philox':
         mode = nat.PERM_PHILOX
@@ -242,7 +251,7 @@ def _run_microcanonical(spec, spanning, seeds=None, rng='numpy', key=0, run0=0, 
     d_perm = d_words = d_len = None
     stride = 1
     if mode == nat.PERM_GIVEN:
-        d_perm = nat.to_device(perms)
+        d_perm = perms if isinstance(perms, torch.Tensor) else nat.to_device(perms)
     elif mode == nat.PERM_MT19937:
         ws_list = [_mt_seed_words(s) for s in seeds]
         stride = max(max(len(w) for w, _ in ws_list), 1)
@@ -264,7 +273,7 @@ def _run_microcanonical(spec, spanning, seeds=None, rng='numpy', key=0, run0=0, 
 
 def _pack_rows(rec, run, spec, spanning):
     lib = nat.lib_handle()
-    dt = np.dtype(microcanonical_statistics_dtype(spanning))
+    dt = _dtype('microcanonical_statistics', spanning)
     out = nat.device_empty(dt.itemsize * (spec.M + 1))
     st = lib.nz_pack_microcanonical_rows(rec.struct(), run, spec.N, spec.M, int(bool(spanning)),
                                          nat.ptr(out), nat.stream_handle())
@@ -351,7 +360,7 @@ def bond_canonical_statistics(microcanonical_statistics, convolution_factors, **
     (one row per p) returns one row per p from a single launch."""
     micro = microcanonical_statistics
     spanning = 'has_spanning_cluster' in micro.dtype.names
-    rows = np.ascontiguousarray(micro, dtype=microcanonical_statistics_dtype(spanning)).ravel()
+    rows = np.ascontiguousarray(micro, dtype=_dtype('microcanonical_statistics', spanning)).ravel()
     M = rows.shape[0] - 1
     f = np.asarray(convolution_factors, dtype=np.float64)
     single = f.ndim == 1
@@ -367,7 +376,7 @@ def bond_canonical_statistics(microcanonical_statistics, convolution_factors, **
         nat.stream_handle())
     nat.check(st, 'nz_canonical_statistics_rows')
     vals = out.cpu().numpy().reshape(-1, 7)
-    ret = np.empty(f.shape[0], dtype=canonical_statistics_dtype(spanning))
+    ret = np.empty(f.shape[0], dtype=_dtype('canonical_statistics', spanning))
     if spanning:
         ret['percolation_probability'] = vals[:, 0]
     ret['max_cluster_size'] = vals[:, 1]
@@ -380,8 +389,8 @@ def bond_initialize_canonical_averages(canonical_statistics, **kwargs):
     (percolate/hpc.py:561-635), same shape as the input."""
     cs = canonical_statistics
     spanning = 'percolation_probability' in cs.dtype.names
-    arr = np.ascontiguousarray(cs, dtype=canonical_statistics_dtype(spanning))
-    dt = np.dtype(canonical_averages_dtype(spanning))
+    arr = np.ascontiguousarray(cs, dtype=_dtype('canonical_statistics', spanning))
+    dt = _dtype('canonical_averages', spanning)
     P = arr.size
     d_in = nat.to_device(arr)
     out = nat.device_empty(dt.itemsize * max(P, 1))
@@ -401,7 +410,7 @@ def bond_reduce(row_a, row_b):
         'percolation_probability_m2' in row_a.dtype.names and
         'percolation_probability_m2' in row_b.dtype.names
     )
-    dt = np.dtype(canonical_averages_dtype(spanning))
+    dt = _dtype('canonical_averages', spanning)
     a = np.ascontiguousarray(row_a, dtype=dt)
     b = np.ascontiguousarray(row_b, dtype=dt)
     if a.shape != b.shape:
@@ -421,8 +430,8 @@ def finalize_canonical_averages(number_of_nodes, ps, canonical_averages, alpha):
     ca = canonical_averages
     spanning = ('percolation_probability_mean' in ca.dtype.names and
                 'percolation_probability_m2' in ca.dtype.names)
-    dt_in = np.dtype(canonical_averages_dtype(spanning))
-    dt = np.dtype(finalized_canonical_averages_dtype(spanning))
+    dt_in = _dtype('canonical_averages', spanning)
+    dt = _dtype('finalized_canonical_averages', spanning)
     arr = np.ascontiguousarray(ca, dtype=dt_in)
     P = arr.size
     ps_arr = np.ascontiguousarray(np.broadcast_to(np.asarray(ps, dtype=np.float64), arr.shape)).ravel()

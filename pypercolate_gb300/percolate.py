@@ -173,8 +173,26 @@ def percolation_graph(graph, spanning_cluster=True):
         perc = graph
     ret['perc_graph'] = perc
     ret['num_nodes'] = nx.number_of_nodes(perc)
-    ret['num_edges'] = nx.number_of_edges(perc)
+    ret['num_edges'] = _edges_left(graph, perc)
     return ret
+
+
+def _edges_left(graph, perc):
+    """number_of_edges of perc, the subgraph of `graph` without its auxiliary
+    nodes: of a simple graph, its edges less those that touch a removed node
+    (networkx counts a subgraph's edges through its filters)."""
+    if perc is graph or type(graph) is not nx.Graph:
+        return nx.number_of_edges(perc)
+    gone = {n for n, a in graph.nodes(data=True) if 'span' in a}
+    half = 0  # twice the edges inside `gone`
+    touching = 0
+    for a in gone:
+        for b in graph.adj[a]:
+            if b not in gone:
+                touching += 1
+            else:
+                half += 2 if a == b else 1
+    return graph.number_of_edges() - touching - half // 2
 
 
 def _binomial_pmf(n, p):
@@ -309,8 +327,8 @@ class _MicroAverages:
         chunk = max(1, min(R, _MICRO_RECORD_BUDGET // (36 * (M + 1))))
         for r0 in range(0, R, chunk):
             rc = min(chunk, R - r0)
-            p = perms[r0 * M:(r0 + rc) * M].cpu().numpy().view(np.uint32).reshape(rc, M)
-            rec = hpc._run_microcanonical(spec, self._spanning, perms=p if M else None,
+            rec = hpc._run_microcanonical(spec, self._spanning,
+                                          perms=perms[r0 * M:(r0 + rc) * M] if M else None, n_runs=rc,
                                           seeds=None if M else [0] * rc, with_edge=False)
             nat.check(nat.lib_handle().nz_microcanonical_reduce(
                 rec.struct(), N, M, rc, 0, M + 1, s, nat.stream_handle()),
