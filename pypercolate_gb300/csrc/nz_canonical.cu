@@ -776,20 +776,19 @@ static void launch_conv_window_pt(const ConvParams &p, int precision, cudaStream
     dim3 gmax((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + kConvPT - 1) / kConvPT, 1);
     dim3 gother(gmax.x, (p.P + PT_OTHER - 1) / PT_OTHER, precision == 0 ? 4 : 3);
     // the record model is a template parameter: a run-time test in the row
-    // loop cost 17 % of the kernel's time
-    auto launch = [&](auto layout) {
-        constexpr Layout LAYOUT = decltype(layout)::value;
-        if (precision == 0) {
-            conv_window_kernel<0, LAYOUT, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-            conv_window_kernel<0, LAYOUT, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
-        } else {
-            conv_window_kernel<1, LAYOUT, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-            conv_window_kernel<1, LAYOUT, false, PT_OTHER><<<gother, kConvRuns, 0, s>>>(p);
-            launch_conv_m2_comp(p, s);
-        }
-    };
-    if (p.rec.site) launch(std::integral_constant<Layout, Layout::kSite>());
-    else launch(std::integral_constant<Layout, Layout::kBond>());
+    // loop cost 17 % of the kernel's time.  (In FP32 only site ensembles come
+    // here: bond ensembles write tiles.)
+    if (precision != 0) {
+        conv_window_kernel<1, Layout::kSite, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
+        conv_window_kernel<1, Layout::kSite, false, PT_OTHER><<<gother, kConvRuns, 0, s>>>(p);
+        launch_conv_m2_comp(p, s);
+    } else if (p.rec.site) {
+        conv_window_kernel<0, Layout::kSite, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
+        conv_window_kernel<0, Layout::kSite, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
+    } else {
+        conv_window_kernel<0, Layout::kBond, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
+        conv_window_kernel<0, Layout::kBond, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
+    }
 }
 
 void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
@@ -1640,12 +1639,16 @@ __global__ void micro_finalize_kernel(NzMicroAccum acc, uint32_t N, uint32_t M, 
 
 void launch_micro_finalize(const NzMicroAccum &acc, uint32_t N, uint32_t M, int32_t spanning, double alpha,
                            int32_t normalize, double *out, cudaStream_t s) {
-    // blocks of one warp: the rows with iterated quantiles are neighbours, and
-    // several of their warps on one SM queue for its FP64 unit (the rows of 128
-    // threads on one SM: 1.5 against 0.63 ms for 10^5 runs of 32 x 32, with the
-    // binomial sums of nz_math.cuh in the second figure)
+    // blocks of one warp while that is few blocks: the rows with iterated
+    // quantiles are neighbours, and several of their warps on one SM queue for
+    // its FP64 unit (the rows of 128 threads on one SM: 1.5 against 0.63 ms for
+    // 10^5 runs of 32 x 32, with the binomial sums of nz_math.cuh in the second
+    // figure).  Every block works out its own t quantiles, which the 32,700
+    // one-warp blocks of a 512 x 512 grid pay for (4.5 against 1.7 ms).
     const uint64_t threads = 2ull * ((uint64_t)M + 1);
-    micro_finalize_kernel<<<(unsigned)((threads + 31) / 32), 32, 0, s>>>(acc, N, M, spanning, alpha, normalize, out);
+    const unsigned block = threads <= 80000 ? 32 : 128;
+    micro_finalize_kernel<<<(unsigned)((threads + block - 1) / block), block, 0, s>>>(acc, N, M, spanning, alpha,
+                                                                                     normalize, out);
 }
 
 __global__ void t_quantile_kernel(const double *q, const double *df, int32_t count, double *out) {

@@ -137,24 +137,64 @@ __device__ __forceinline__ const raw_word<S> *raw_plane(const NzRecords &rec) {
     else return rec.m4_lo;
 }
 
-// Loads of chunk rows [k0, k0 + 32) relative to the CTA's first row, each
-// clamped to the last row so that every load is in bounds and unconditional
-// (all 32 in flight at once); rows past the end are zeroed on conversion.
-template <int S>
-__device__ __forceinline__ void load_chunk(const NzRecords &rec, bool tiled, uint32_t first, int32_t r, uint32_t k0,
-                                           uint32_t last, raw_word<S> (&raw)[kTcK],
-                                           uint64_t (&hi)[S == 6 ? kTcK : 1]) {
-    const raw_word<S> *plane = raw_plane<S>(rec);
+// Rows i .. i + kTcK - 1 of a tiled plane out of the 16-byte pieces that hold
+// them (the planes hold whole tiles; pieces past `last`'s are read as that one).
+// How far the first row is into its piece is the same for all chunks of a
+// window.
+template <class T>
+__device__ __forceinline__ void load_pieces(const T *plane, int64_t stride, uint32_t i, uint32_t last, int32_t r,
+                                            T (&q)[kTcK]) {
+    constexpr uint32_t kPer = 16 / sizeof(T);        // rows per piece
+    constexpr int kPieces = kTcK / (int)kPer + 1;
+    const uint32_t skip = i & (kPer - 1u), first = i - skip, end = last & ~(kPer - 1u);
+    T all[kPieces * kPer];
 #pragma unroll
-    for (int k = 0; k < kTcK; ++k) {
-        const uint32_t i = first + min(k0 + (uint32_t)k, last);
-        raw[k] = plane[record_off<sizeof(raw_word<S>)>(rec, tiled, i, r)];
-        if constexpr (S == 6) hi[k] = rec.m4_hi[record_off<4>(rec, tiled, i, r)];
+    for (int k = 0; k < kPieces; ++k) {
+        const uint32_t at = min(first + (uint32_t)k * kPer, end);
+        const uint4 v = *reinterpret_cast<const uint4 *>(plane + tile_off<sizeof(T)>(stride, at, r));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int b = 0; b < (int)kPer; ++b) {
+            if constexpr (sizeof(T) == 2) all[k * kPer + b] = (T)(w[b / 2] >> (16 * (b & 1)));
+            else if constexpr (sizeof(T) == 4) all[k * kPer + b] = (T)w[b];
+            else all[k * kPer + b] = (T)(((uint64_t)w[2 * b + 1] << 32) | w[2 * b]);
+        }
+    }
+    // the pieces moved down by `skip` rows, one power of two at a time
+#pragma unroll
+    for (uint32_t step = kPer / 2; step > 0; step /= 2)
+        if (skip & step) {
+#pragma unroll
+            for (int k = 0; k + (int)step < kPieces * (int)kPer; ++k) all[k] = all[k + step];
+        }
+#pragma unroll
+    for (int k = 0; k < kTcK; ++k) q[k] = all[k];
+}
+
+// Loads of chunk rows [k0, k0 + kTcK) relative to the CTA's first row, each
+// clamped to the last row so that every load is in bounds and unconditional
+// (all in flight at once); rows past the end are zeroed on conversion.  m4 with
+// its high words takes pieces (200 runs at L = 512: 6.7 -> 4.8 ms); the others'
+// kernel is faster without (3.8 against 4.2 ms).
+template <int S, bool TILED>
+__device__ __forceinline__ void load_chunk(const NzRecords &rec, uint32_t first, int32_t r, uint32_t k0, uint32_t last,
+                                           raw_word<S> (&raw)[kTcK], uint32_t (&hi)[S == 6 ? kTcK : 1]) {
+    const raw_word<S> *plane = raw_plane<S>(rec);
+    if constexpr (S == 6 && TILED) {
+        load_pieces(plane, rec.run_stride, first + k0, first + last, r, raw);
+        load_pieces(rec.m4_hi, rec.run_stride, first + k0, first + last, r, hi);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kTcK; ++k) {
+            const uint32_t i = first + min(k0 + (uint32_t)k, last);
+            raw[k] = plane[record_off<sizeof(raw_word<S>)>(rec, TILED, i, r)];
+            if constexpr (S == 6) hi[k] = rec.m4_hi[record_off<4>(rec, TILED, i, r)];
+        }
     }
 }
 
 template <int S>
-__device__ __forceinline__ float raw_value(raw_word<S> w, uint64_t hi, uint32_t held) {
+__device__ __forceinline__ float raw_value(raw_word<S> w, uint32_t hi, uint32_t held) {
     if constexpr (S == 0) return (w & kSpanBit) ? 1.0f : 0.0f;
     else if constexpr (S == 1) return (float)(w & ~kSpanBit);
     else if constexpr (S == 2 || S == 8 || S == 9) return (float)w;
@@ -211,8 +251,8 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
         for (int j = 0; j < kTcP; ++j) acc_c[j] = __fadd_rn(acc_c[j], v[j]);
     };
     raw_word<S> raw[kTcK];
-    uint64_t raw_hi[S == 6 ? kTcK : 1];
-    load_chunk<S>(p.rec, p.tiled, first, run, 0, last, raw, raw_hi);
+    uint32_t raw_hi[S == 6 ? kTcK : 1];
+    load_chunk<S, !SITE>(p.rec, first, run, 0, last, raw, raw_hi);
     bool bad = false;
     uint32_t ch = 0;
     for (; ch < nchunks; ++ch) {
@@ -228,7 +268,7 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
             }
             // the next chunk's loads fly while this one is staged, multiplied
             // and drained
-            if (ch + 1 < nchunks) load_chunk<S>(p.rec, p.tiled, first, run, (ch + 1) * kTcK, last, raw, raw_hi);
+            if (ch + 1 < nchunks) load_chunk<S, !SITE>(p.rec, first, run, (ch + 1) * kTcK, last, raw, raw_hi);
             float *ah = sh.a[st][0] + a_off, *al = sh.a[st][1] + a_off;
 #pragma unroll
             for (int kb = 0; kb < kTcK / 4; ++kb) {
@@ -404,7 +444,8 @@ bool conv_tc_grid_fits(int32_t n_runs, int32_t P) {
 
 int launch_conv_window_tc(const ConvParams &p, cudaStream_t s) {
     if (p.n_runs <= 0 || p.P <= 0) return 0;
-    const cudaError_t e = p.rec.site ? launch_tc<true>(p, s) : launch_tc<false>(p, s);
+    // site ensembles write n-major records, all others tiles
+    const cudaError_t e = p.tiled ? launch_tc<false>(p, s) : launch_tc<true>(p, s);
     if (e != cudaSuccess) return -1;
     // m2 needs ~5e-11 relative per run (the susceptibility curve within 1e-6
     // absolute of FP64 at L = 1024), beyond FP32 tensor-core accumulation:
