@@ -175,7 +175,7 @@ int nz_microcanonical(const NzGraph *graph, int32_t spanning, int32_t n_runs, in
     p.tiled = false;
     {
         ProfScope prof(NZ_PROF_UNION_FIND, s);
-        launch_uf_window(p, mode, spanning != 0, n_runs >= 128 ? 128 : 32, s);
+        launch_uf_window(p, mode, spanning != 0, s);
     }
     return check_launch();
 }
@@ -300,8 +300,6 @@ int nz_canonical_statistics_records(const NzRecords *rec, uint32_t num_nodes, ui
     p.w32 = nullptr;
     p.w32lo = nullptr;
     p.core_lo = p.core_len = nullptr;
-    p.m2_tile = 8;
-    p.conv_tile = 8;
     p.acc = out;
     p.errors = nullptr;
     p.tiled = false;
@@ -512,8 +510,8 @@ size_t ensemble_layout(Carver &c, const GraphDev &g, int32_t n_runs, int32_t P, 
     L.nodes = c.take<uint32_t>((size_t)n_runs * g.slots);
     L.state = c.take<RunState>((size_t)n_runs);
     L.flag = c.take<uint32_t>(4);
-    // bond ensembles write tiled records: whole tiles of 32 rows
-    const size_t rows = g.site ? (size_t)L.window : ((size_t)L.window + 31) / 32 * 32;
+    // tiled records: whole tiles of 32 rows
+    const size_t rows = ((size_t)L.window + 31) / 32 * 32;
     const size_t plane = rows * n_runs;
     for (int b = 0; b < 2; ++b) {
         NzRecords &r = L.rec[b];
@@ -648,7 +646,7 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
     up.run0 = run0;
     up.perms = nullptr;
     up.init_flag = nullptr;
-    up.tiled = !g.site;
+    up.tiled = true;
     up.errors = L.flag + 1;  // zeroed in the set-up; read by nz_ensemble_errors
     ConvParams cp;
     cp.tiled = up.tiled;
@@ -664,8 +662,6 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
     cp.w32lo = L.w32lo;
     cp.core_lo = L.core_lo32;
     cp.core_len = L.core_len32;
-    cp.m2_tile = m2_tile;
-    cp.conv_tile = conv_tile;
     cp.acc = L.stats;
     cp.errors = L.flag + 1;  // with the union-find's corruption count
     MicroParams mp;
@@ -707,7 +703,7 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
         up.n_begin = w0; up.n_end = w1;
         {
             ProfScope prof(NZ_PROF_UNION_FIND, s1);
-            launch_uf_window(up, NZ_PERM_PHILOX, spanning != 0, uf_block, s1);
+            launch_uf_window(up, NZ_PERM_PHILOX, spanning != 0, s1);
         }
         if (cudaEventRecord(aux.a->produced[b], s1) != cudaSuccess ||
             cudaStreamWaitEvent(s2, aux.a->produced[b], 0) != cudaSuccess)

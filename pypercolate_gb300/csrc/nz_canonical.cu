@@ -274,49 +274,35 @@ void launch_band_dot(const uint32_t *band_lo, const uint32_t *band_len, const do
 // =====================================================================
 // Banded convolution of record windows (ensemble path)
 // =====================================================================
-constexpr int kConvRuns = 128;         // runs per CTA (one per thread)
-// probabilities per CTA of the FP32 / FP64 window kernels: 8 by default
-// (8 gave 544 ms, 16 587 ms, 32 1025 ms per 100,000-run step with the
-// earlier FP64-accumulated kernels); 16 is an autotuner candidate for the
-// m0 / m3 / m4 kernel
-constexpr int kConvPT = 8;
-// 16 record loads in flight per thread: over the FP32 band (weights >= e^-30
-// of the mode) 1047 against 1052 ms per 100,000-run L = 256 step with 8
-// (over the full e^-80 band 8 had been better: 479 against 512 ms); 32
-// measured 1229 against 1211 ms (same box)
-#ifndef NZ_CONV_BATCH
-#define NZ_CONV_BATCH 16
-#endif
-constexpr int kConvBatch = NZ_CONV_BATCH;  // record loads in flight per thread
+// FP64 (the FP32 convolution of an ensemble's tiled records: nz_conv_tiles.cu)
+constexpr int kConvRuns = 128;  // runs per CTA (one per thread)
+constexpr int kConvPT = 8;      // probabilities per CTA
+constexpr int kConvBatch = 16;  // record loads in flight per thread
 
 // grid: (run tiles, p tiles, 7 statistics).  Each thread accumulates the
 // kConvPT canonical values of its run for one statistic over the window's
 // rows, with the tile's weights staged in shared memory (zero outside each
-// p's band).  PRECISION 0: FP64 products and sums.  PRECISION 1: FP32
-// products summed in FP32 over kConvChunk rows, then added into a TwoSum
-// pair (ConvAcc<1>).
-template <int PRECISION, int S, bool SITE, int kConvPT>
+// p's band), with FP64 products and sums.
+template <int S, bool SITE>
 __device__ __forceinline__ void conv_rows(const ConvParams &p, uint32_t c0, uint32_t cn, int r,
-                                          const typename std::conditional<PRECISION == 0, double, float>::type (*s_w)[kConvPT],
-                                          ConvAcc<PRECISION> *acc) {
-    using wtype = typename std::conditional<PRECISION == 0, double, float>::type;
-    wtype part[kConvPT];
+                                          const double (*s_w)[kConvPT],
+                                          double *acc) {
+    double part[kConvPT];
 #pragma unroll
     for (int j = 0; j < kConvPT; ++j) part[j] = 0;
     const size_t base = (size_t)(c0 - p.n_begin) * p.rec.run_stride + r;
     // m1 = (sites in clusters) - max: N for bond records, n for site records
-    auto value = [&](uint32_t i) -> wtype {
+    auto value = [&](uint32_t i) -> double {
         const size_t off = base + (size_t)i * p.rec.run_stride;
         const uint32_t held = (S == 3 && SITE) ? c0 + i : p.N;
-        return PRECISION == 0 ? (wtype)record_value<S>(p.rec, off, held)
-                              : (wtype)record_value_f<S>(p.rec, off, held);
+        return (double)record_value<S>(p.rec, off, held);
     };
     // the records of kConvBatch rows are loaded before their products so that
     // that many loads are in flight per thread; each accumulator still adds
     // the rows in increasing order
     uint32_t i = 0;
     for (; i + kConvBatch <= cn; i += kConvBatch) {
-        wtype q[kConvBatch];
+        double q[kConvBatch];
 #pragma unroll
         for (int b = 0; b < kConvBatch; ++b) q[b] = value(i + b);
 #pragma unroll
@@ -325,36 +311,35 @@ __device__ __forceinline__ void conv_rows(const ConvParams &p, uint32_t c0, uint
             for (int j = 0; j < kConvPT; ++j) part[j] = fma(s_w[i + b][j], q[b], part[j]);
     }
     for (; i < cn; ++i) {
-        const wtype q = value(i);
+        const double q = value(i);
 #pragma unroll
         for (int j = 0; j < kConvPT; ++j) part[j] = fma(s_w[i][j], q, part[j]);
     }
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) acc[j].add(part[j]);
+    for (int j = 0; j < kConvPT; ++j) acc[j] += part[j];
 }
 
 // Statistics 0 (spanning), 1 (max) and 3 (m1 = held - max) all come from the
 // max_span plane: one pass loads each word once and feeds the three sets of
 // products (each accumulator adds the same values in the same order as a
 // pass per statistic would).
-template <int PRECISION, bool SITE, int kConvPT>
+template <bool SITE>
 __device__ __forceinline__ void conv_rows_max(const ConvParams &p, uint32_t c0, uint32_t cn, int r,
-                                              const typename std::conditional<PRECISION == 0, double, float>::type (*s_w)[kConvPT],
-                                              ConvAcc<PRECISION> *acc0, ConvAcc<PRECISION> *acc1,
-                                              ConvAcc<PRECISION> *acc3) {
-    using wtype = typename std::conditional<PRECISION == 0, double, float>::type;
-    wtype p0[kConvPT], p1[kConvPT], p3[kConvPT];
+                                              const double (*s_w)[kConvPT],
+                                              double *acc0, double *acc1,
+                                              double *acc3) {
+    double p0[kConvPT], p1[kConvPT], p3[kConvPT];
 #pragma unroll
     for (int j = 0; j < kConvPT; ++j) p0[j] = p1[j] = p3[j] = 0;
     const size_t base = (size_t)(c0 - p.n_begin) * p.rec.run_stride + r;
     auto step = [&](uint32_t i, uint32_t ms) {
         const uint32_t held = SITE ? c0 + i : p.N;
         const uint32_t mx = ms & ~kSpanBit;
-        const wtype q0 = (ms & kSpanBit) ? (wtype)1 : (wtype)0;
-        const wtype q1 = (wtype)mx, q3 = (wtype)(held - mx);
+        const double q0 = (ms & kSpanBit) ? (double)1 : (double)0;
+        const double q1 = (double)mx, q3 = (double)(held - mx);
 #pragma unroll
         for (int j = 0; j < kConvPT; ++j) {
-            const wtype w = s_w[i][j];
+            const double w = s_w[i][j];
             p0[j] = fma(w, q0, p0[j]);  // (dropped at the end without a spanning statistic)
             p1[j] = fma(w, q1, p1[j]);
             p3[j] = fma(w, q3, p3[j]);
@@ -371,16 +356,16 @@ __device__ __forceinline__ void conv_rows_max(const ConvParams &p, uint32_t c0, 
     for (; i < cn; ++i) step(i, p.rec.max_span[base + (size_t)i * p.rec.run_stride]);
 #pragma unroll
     for (int j = 0; j < kConvPT; ++j) {
-        acc0[j].add(p0[j]);
-        acc1[j].add(p1[j]);
-        acc3[j].add(p3[j]);
+        acc0[j] += p0[j];
+        acc1[j] += p1[j];
+        acc3[j] += p3[j];
     }
 }
 
-// ---- the same sums over tiled records (FP64; FP32: nz_conv_tiles.cu).  A chunk's rows are read in groups of
+// ---- the same sums over tiled records.  A chunk's rows are read in groups of
 // 8 (16-byte loads of one run's consecutive rows, kTileAhead groups in flight)
 // from the group that holds its first row; s_w row 0 is that group's first row
-// and rows outside the chunk have zero weights, which leave every FP32 partial
+// and rows outside the chunk have zero weights, which leave every partial
 // sum as it is.  Rows are added in increasing order, chunk by chunk, as above.
 constexpr int kTileAhead = 3;
 
@@ -398,16 +383,10 @@ __device__ __forceinline__ const tile_raw<S> *tile_plane(const NzRecords &rec) {
     else if constexpr (S == 9) return reinterpret_cast<const uint32_t *>(rec.m2);
     else return rec.m4_lo;
 }
-template <int PRECISION, int S>
-__device__ __forceinline__ auto tile_value(tile_raw<S> q, uint32_t hi) {
-    if constexpr (PRECISION == 0) {
-        if constexpr (S == 6) return fma((double)hi, 18446744073709551616.0, (double)q);
-        else return (double)q;
-    } else {
-        if constexpr (S == 6) return fmaf((float)hi, 18446744073709551616.0f, u64_to_f32(q));
-        else if constexpr (sizeof(tile_raw<S>) == 8) return u64_to_f32(q);
-        else return (float)q;
-    }
+template <int S>
+__device__ __forceinline__ double tile_value(tile_raw<S> q, uint32_t hi) {
+    if constexpr (S == 6) return fma((double)hi, 18446744073709551616.0, (double)q);
+    else return (double)q;
 }
 
 // calls step(row group index k, loaded groups) for the 8-row groups of
@@ -429,16 +408,15 @@ __device__ __forceinline__ void for_groups(uint32_t groups, Load load, Step step
     }
 }
 
-template <int PRECISION, int S, int kConvPT>
+template <int S>
 __device__ __forceinline__ void conv_rows_tiled(const ConvParams &p, uint32_t first, uint32_t groups, int r,
-                                                const typename std::conditional<PRECISION == 0, double, float>::type (*s_w)[kConvPT],
-                                                ConvAcc<PRECISION> *acc) {
-    using wtype = typename std::conditional<PRECISION == 0, double, float>::type;
+                                                const double (*s_w)[kConvPT],
+                                                double *acc) {
     struct Raw {
         tile_raw<S> q[8];
         uint32_t hi[S == 6 ? 8 : 1];
     };
-    wtype part[kConvPT];
+    double part[kConvPT];
 #pragma unroll
     for (int j = 0; j < kConvPT; ++j) part[j] = 0;
     for_groups<(sizeof(tile_raw<S>) == 8 ? 2 : kTileAhead), Raw>(
@@ -450,25 +428,24 @@ __device__ __forceinline__ void conv_rows_tiled(const ConvParams &p, uint32_t fi
         [&](uint32_t k, const Raw &q) {
 #pragma unroll
             for (int b = 0; b < 8; ++b) {
-                const wtype v = tile_value<PRECISION, S>(q.q[b], S == 6 ? q.hi[S == 6 ? b : 0] : 0u);
+                const double v = tile_value<S>(q.q[b], S == 6 ? q.hi[S == 6 ? b : 0] : 0u);
 #pragma unroll
                 for (int j = 0; j < kConvPT; ++j) part[j] = fma(s_w[8 * k + b][j], v, part[j]);
             }
         });
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) acc[j].add(part[j]);
+    for (int j = 0; j < kConvPT; ++j) acc[j] += part[j];
 }
 
-template <int PRECISION, int kConvPT>
+template <bool SITE>
 __device__ __forceinline__ void conv_rows_max_tiled(const ConvParams &p, uint32_t first, uint32_t groups, int r,
-                                                    const typename std::conditional<PRECISION == 0, double, float>::type (*s_w)[kConvPT],
-                                                    ConvAcc<PRECISION> *acc0, ConvAcc<PRECISION> *acc1,
-                                                    ConvAcc<PRECISION> *acc3) {
-    using wtype = typename std::conditional<PRECISION == 0, double, float>::type;
+                                                    const double (*s_w)[kConvPT],
+                                                    double *acc0, double *acc1,
+                                                    double *acc3) {
     struct Raw {
         uint32_t q[8];
     };
-    wtype p0[kConvPT], p1[kConvPT], p3[kConvPT];
+    double p0[kConvPT], p1[kConvPT], p3[kConvPT];
 #pragma unroll
     for (int j = 0; j < kConvPT; ++j) p0[j] = p1[j] = p3[j] = 0;
     for_groups<kTileAhead, Raw>(
@@ -477,11 +454,11 @@ __device__ __forceinline__ void conv_rows_max_tiled(const ConvParams &p, uint32_
 #pragma unroll
             for (int b = 0; b < 8; ++b) {
                 const uint32_t mx = q.q[b] & ~kSpanBit;
-                const wtype q0 = (q.q[b] & kSpanBit) ? (wtype)1 : (wtype)0;
-                const wtype q1 = (wtype)mx, q3 = (wtype)(p.N - mx);
+                const double q0 = (q.q[b] & kSpanBit) ? (double)1 : (double)0;
+                const double q1 = (double)mx, q3 = (double)((SITE ? p.n_begin + first + 8 * k + b : p.N) - mx);
 #pragma unroll
                 for (int j = 0; j < kConvPT; ++j) {
-                    const wtype w = s_w[8 * k + b][j];
+                    const double w = s_w[8 * k + b][j];
                     p0[j] = fma(w, q0, p0[j]);
                     p1[j] = fma(w, q1, p1[j]);
                     p3[j] = fma(w, q3, p3[j]);
@@ -490,41 +467,31 @@ __device__ __forceinline__ void conv_rows_max_tiled(const ConvParams &p, uint32_
         });
 #pragma unroll
     for (int j = 0; j < kConvPT; ++j) {
-        acc0[j].add(p0[j]);
-        acc1[j].add(p1[j]);
-        acc3[j].add(p3[j]);
+        acc0[j] += p0[j];
+        acc1[j] += p1[j];
+        acc3[j] += p3[j];
     }
 }
 
 // Each thread accumulates the kConvPT canonical values of its run over the
 // window's rows, with the tile's weights staged in shared memory (zero
-// outside each p's band).  PRECISION 0: FP64 products and sums.  PRECISION 1:
-// FP32 products summed in FP32 over kConvChunk rows, then added into a
-// TwoSum pair (ConvAcc<1>).
+// outside each p's band), in FP64.
 // MAXSET: grid (run tiles, p tiles, 1), statistics 0, 1 and 3 from the
 // max_span plane in one pass; otherwise grid (run tiles, p tiles, 4),
-// statistics 2, 4, 5, 6 (one per z) -- on the FP32 path (run tiles, p
-// tiles, 3), statistics 2, 5, 6, with m2 (4) in conv_m2_comp_kernel.
-#ifdef NZ_CONV_MIN_BLOCKS
-#define NZ_CONV_BOUNDS __launch_bounds__(kConvRuns, NZ_CONV_MIN_BLOCKS)
-#else
-#define NZ_CONV_BOUNDS __launch_bounds__(kConvRuns)
-#endif
-enum class Layout { kBond, kSite, kTiled };  // n-major bond records, n-major site records, tiled bond records
+// statistics 2, 4, 5, 6 (one per z).
+enum class Layout { kBond, kSite, kTiled, kTiledSite };  // records of bonds or sites, n-major or tiled
 
-template <int PRECISION, Layout LAYOUT, bool MAXSET, int kConvPT>
-__global__ void NZ_CONV_BOUNDS conv_window_kernel(ConvParams p) {
-    using wtype = typename std::conditional<PRECISION == 0, double, float>::type;
-    constexpr bool SITE = LAYOUT == Layout::kSite, TILED = LAYOUT == Layout::kTiled;
-    __shared__ wtype s_w[kConvChunk + (TILED ? 8 : 0)][kConvPT];
+template <Layout LAYOUT, bool MAXSET>
+__global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
+    constexpr bool SITE = LAYOUT == Layout::kSite || LAYOUT == Layout::kTiledSite;
+    constexpr bool TILED = LAYOUT == Layout::kTiled || LAYOUT == Layout::kTiledSite;
+    __shared__ double s_w[kConvChunk + (TILED ? 8 : 0)][kConvPT];
     __shared__ uint32_t s_lo[kConvPT], s_len[kConvPT];
     __shared__ uint32_t s_range[2];
     const int r = blockIdx.x * kConvRuns + threadIdx.x;
     const int p0 = blockIdx.y * kConvPT;
-    // FP64: statistics 2, 4, 5, 6; FP32: 2, 5, 6 (m2 has its compensated kernel)
     constexpr int kOther[4] = {2, 4, 5, 6};
-    constexpr int kOther32[3] = {2, 5, 6};
-    const int s = MAXSET ? 1 : (PRECISION == 0 ? kOther[blockIdx.z] : kOther32[blockIdx.z]);
+    const int s = MAXSET ? 1 : kOther[blockIdx.z];
     if (threadIdx.x < kConvPT) {
         const int pi = p0 + threadIdx.x;
         s_lo[threadIdx.x] = pi < p.P ? p.band_lo[pi] : 0u;
@@ -542,7 +509,7 @@ __global__ void NZ_CONV_BOUNDS conv_window_kernel(ConvParams p) {
     __syncthreads();
     const uint32_t nlo = s_range[0], nhi = s_range[1];
     if (nlo >= nhi) return;
-    ConvAcc<PRECISION> acc[kConvPT], acc0[MAXSET ? kConvPT : 1], acc3[MAXSET ? kConvPT : 1];
+    double acc[kConvPT] = {}, acc0[MAXSET ? kConvPT : 1] = {}, acc3[MAXSET ? kConvPT : 1] = {};
     for (uint32_t c0 = nlo; c0 < nhi; c0 += kConvChunk) {
         const uint32_t cn = min((uint32_t)kConvChunk, nhi - c0);
         // tiled: rows of the 8-row group that holds c0 come first
@@ -551,10 +518,10 @@ __global__ void NZ_CONV_BOUNDS conv_window_kernel(ConvParams p) {
         for (int i = threadIdx.x; i < (kConvChunk + (TILED ? 8 : 0)) * kConvPT; i += kConvRuns) {
             const int row = i / kConvPT, j = i % kConvPT;
             const uint32_t n = c0 + row - lead;
-            wtype v = 0;
+            double v = 0;
             if ((uint32_t)row - lead < cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
                 const size_t widx = (size_t)(p0 + j) * p.cap + (n - s_lo[j]);
-                v = PRECISION == 0 ? (wtype)p.w64[widx] : (wtype)p.w32[widx];
+                v = p.w64[widx];
             }
             s_w[row][j] = v;
         }
@@ -563,37 +530,37 @@ __global__ void NZ_CONV_BOUNDS conv_window_kernel(ConvParams p) {
             if (r < p.n_runs) {
                 const uint32_t first = c0 - p.n_begin - lead, groups = (lead + cn + 7u) / 8u;
                 if (MAXSET) {
-                    conv_rows_max_tiled<PRECISION, kConvPT>(p, first, groups, r, s_w, acc0, acc, acc3);
+                    conv_rows_max_tiled<SITE>(p, first, groups, r, s_w, acc0, acc, acc3);
                 } else if (s == 2) {
-                    if (p.rec.narrow) conv_rows_tiled<PRECISION, 8, kConvPT>(p, first, groups, r, s_w, acc);
-                    else conv_rows_tiled<PRECISION, 2, kConvPT>(p, first, groups, r, s_w, acc);
+                    if (p.rec.narrow) conv_rows_tiled<8>(p, first, groups, r, s_w, acc);
+                    else conv_rows_tiled<2>(p, first, groups, r, s_w, acc);
                 } else if (s == 4) {
-                    if (p.rec.narrow) conv_rows_tiled<PRECISION, 9, kConvPT>(p, first, groups, r, s_w, acc);
-                    else conv_rows_tiled<PRECISION, 4, kConvPT>(p, first, groups, r, s_w, acc);
+                    if (p.rec.narrow) conv_rows_tiled<9>(p, first, groups, r, s_w, acc);
+                    else conv_rows_tiled<4>(p, first, groups, r, s_w, acc);
                 } else if (s == 5) {
-                    conv_rows_tiled<PRECISION, 5, kConvPT>(p, first, groups, r, s_w, acc);
+                    conv_rows_tiled<5>(p, first, groups, r, s_w, acc);
                 } else {
-                    if (p.rec.m4_hi) conv_rows_tiled<PRECISION, 6, kConvPT>(p, first, groups, r, s_w, acc);
-                    else conv_rows_tiled<PRECISION, 7, kConvPT>(p, first, groups, r, s_w, acc);
+                    if (p.rec.m4_hi) conv_rows_tiled<6>(p, first, groups, r, s_w, acc);
+                    else conv_rows_tiled<7>(p, first, groups, r, s_w, acc);
                 }
             }
         } else if (r < p.n_runs) {
             if (MAXSET) {
-                conv_rows_max<PRECISION, SITE, kConvPT>(p, c0, cn, r, s_w, acc0, acc, acc3);
+                conv_rows_max<SITE>(p, c0, cn, r, s_w, acc0, acc, acc3);
             } else {
                 switch (s) {
                     case 2:
-                        if (p.rec.narrow) conv_rows<PRECISION, 8, SITE, kConvPT>(p, c0, cn, r, s_w, acc);
-                        else conv_rows<PRECISION, 2, SITE, kConvPT>(p, c0, cn, r, s_w, acc);
+                        if (p.rec.narrow) conv_rows<8, SITE>(p, c0, cn, r, s_w, acc);
+                        else conv_rows<2, SITE>(p, c0, cn, r, s_w, acc);
                         break;
                     case 4:
-                        if (p.rec.narrow) conv_rows<PRECISION, 9, SITE, kConvPT>(p, c0, cn, r, s_w, acc);
-                        else conv_rows<PRECISION, 4, SITE, kConvPT>(p, c0, cn, r, s_w, acc);
+                        if (p.rec.narrow) conv_rows<9, SITE>(p, c0, cn, r, s_w, acc);
+                        else conv_rows<4, SITE>(p, c0, cn, r, s_w, acc);
                         break;
-                    case 5: conv_rows<PRECISION, 5, SITE, kConvPT>(p, c0, cn, r, s_w, acc); break;
+                    case 5: conv_rows<5, SITE>(p, c0, cn, r, s_w, acc); break;
                     default:
-                        if (p.rec.m4_hi) conv_rows<PRECISION, 6, SITE, kConvPT>(p, c0, cn, r, s_w, acc);
-                        else conv_rows<PRECISION, 7, SITE, kConvPT>(p, c0, cn, r, s_w, acc);
+                        if (p.rec.m4_hi) conv_rows<6, SITE>(p, c0, cn, r, s_w, acc);
+                        else conv_rows<7, SITE>(p, c0, cn, r, s_w, acc);
                         break;
                 }
             }
@@ -605,159 +572,12 @@ __global__ void NZ_CONV_BOUNDS conv_window_kernel(ConvParams p) {
             const int pi = p0 + j;
             if (pi >= p.P) continue;
             double *o = p.acc + ((size_t)r * p.P + pi) * 7;
-            o[s] += acc[j].value();
+            o[s] += acc[j];
             if (MAXSET) {
-                if (p.spanning) o[0] += acc0[j].value();
-                o[3] += acc3[j].value();
+                if (p.spanning) o[0] += acc0[j];
+                o[3] += acc3[j];
             }
         }
-    }
-}
-
-// ---------------------------------------------------------------------
-// m2 with compensated FP32 arithmetic
-// ---------------------------------------------------------------------
-// grid (run tiles, tiles of kM2PT probabilities): each thread the kM2PT m2
-// values of its run.  A chunk of rows that meets the core of any of the
-// tile's probabilities runs the compensated arithmetic on all its rows
-// (branch-free, so the kM2PT accumulator chains interleave); a chunk
-// entirely in the tails runs plain FP32 products.
-// record loads in flight per thread of the compensated m2 kernel: 32
-// against 16, 1092 against 1099 ms per 100,000-run L = 256 step (same box,
-// the convolution stream 801 against 838 ms)
-#ifndef NZ_M2_BATCH
-#define NZ_M2_BATCH 32
-#endif
-constexpr int kM2Batch = NZ_M2_BATCH;
-
-// kM2PT probabilities per CTA (the tuned m2_tile, 8 or 16; 8 by default:
-// on the same box 8 gave 1085.8 and 1204.7 ms per 100,000-run L = 256 step
-// against 1108.8 and 1224.7 ms for 16 (two boxes); 32 measured 1285 against
-// 1128 ms for 16)
-template <bool NARROW, int kM2PT>
-__global__ void NZ_CONV_BOUNDS conv_m2_comp_kernel(ConvParams p) {
-    __shared__ float s_wh[kConvChunk][kM2PT], s_wl[kConvChunk][kM2PT];
-    __shared__ uint32_t s_lo[kM2PT], s_len[kM2PT], s_clo[kM2PT], s_clen[kM2PT];
-    __shared__ uint32_t s_range[2];
-    const int r = blockIdx.x * kConvRuns + threadIdx.x;
-    const int p0 = blockIdx.y * kM2PT;
-    if (threadIdx.x < kM2PT) {
-        const int pi = p0 + threadIdx.x;
-        s_lo[threadIdx.x] = pi < p.P ? p.band_lo[pi] : 0u;
-        s_len[threadIdx.x] = pi < p.P ? p.band_len[pi] : 0u;
-        s_clo[threadIdx.x] = pi < p.P ? p.core_lo[pi] : 0u;
-        s_clen[threadIdx.x] = pi < p.P ? p.core_len[pi] : 0u;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t a = 0xffffffffu, b = 0;
-        for (int j = 0; j < kM2PT; ++j)
-            if (s_len[j]) { a = min(a, s_lo[j]); b = max(b, s_lo[j] + s_len[j]); }
-        s_range[0] = max(a, p.n_begin);
-        s_range[1] = min(b, p.n_end);
-    }
-    __syncthreads();
-    const uint32_t nlo = s_range[0], nhi = s_range[1];
-    if (nlo >= nhi) return;
-    Dot2Acc acc[kM2PT];
-    const uint32_t *m2n = reinterpret_cast<const uint32_t *>(p.rec.m2);
-    for (uint32_t c0 = nlo; c0 < nhi; c0 += kConvChunk) {
-        const uint32_t cn = min((uint32_t)kConvChunk, nhi - c0);
-        // does the chunk meet a core?  (uniform over the CTA)
-        bool core = false;
-#pragma unroll
-        for (int j = 0; j < kM2PT; ++j)
-            core |= s_clen[j] && s_clo[j] < c0 + cn && c0 < s_clo[j] + s_clen[j];
-        __syncthreads();
-        for (int i = threadIdx.x; i < kConvChunk * kM2PT; i += kConvRuns) {
-            const int rw = i / kM2PT, j = i % kM2PT;
-            const uint32_t n = c0 + rw;
-            float vh = 0.0f, vl = 0.0f;
-            if (rw < (int)cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
-                const size_t widx = (size_t)(p0 + j) * p.cap + (n - s_lo[j]);
-                vh = p.w32[widx];
-                vl = p.w32lo[widx];
-            }
-            s_wh[rw][j] = vh;
-            s_wl[rw][j] = vl;
-        }
-        __syncthreads();
-        if (r >= p.n_runs) continue;
-        const size_t base = (size_t)(c0 - p.n_begin) * p.rec.run_stride + r;
-        // raw m2 words of kM2Batch rows are loaded before any is split and
-        // used, so that many loads are in flight per thread
-        using raw_t = typename std::conditional<NARROW, uint32_t, uint64_t>::type;
-        const raw_t *plane = NARROW ? reinterpret_cast<const raw_t *>(m2n)
-                                    : reinterpret_cast<const raw_t *>(p.rec.m2);
-        auto split = [&](raw_t w, float &qh, float &ql) {
-            if constexpr (NARROW) split_u32(w, qh, ql);
-            else split_u64(w, qh, ql);
-        };
-        uint32_t i = 0;
-        if (core) {
-            for (; i + kM2Batch <= cn; i += kM2Batch) {
-                raw_t w[kM2Batch];
-#pragma unroll
-                for (int b = 0; b < kM2Batch; ++b) w[b] = plane[base + (size_t)(i + b) * p.rec.run_stride];
-#pragma unroll
-                for (int b = 0; b < kM2Batch; ++b) {
-                    float qh, ql;
-                    split(w[b], qh, ql);
-#pragma unroll
-                    for (int j = 0; j < kM2PT; ++j) acc[j].add(s_wh[i + b][j], s_wl[i + b][j], qh, ql);
-                }
-            }
-            for (; i < cn; ++i) {
-                float qh, ql;
-                split(plane[base + (size_t)i * p.rec.run_stride], qh, ql);
-#pragma unroll
-                for (int j = 0; j < kM2PT; ++j) acc[j].add(s_wh[i][j], s_wl[i][j], qh, ql);
-            }
-        } else {
-            for (; i + kM2Batch <= cn; i += kM2Batch) {
-                raw_t w[kM2Batch];
-#pragma unroll
-                for (int b = 0; b < kM2Batch; ++b) w[b] = plane[base + (size_t)(i + b) * p.rec.run_stride];
-#pragma unroll
-                for (int b = 0; b < kM2Batch; ++b) {
-                    float qh, ql;
-                    split(w[b], qh, ql);
-                    const float q = __fadd_rn(qh, ql);
-#pragma unroll
-                    for (int j = 0; j < kM2PT; ++j) acc[j].add_tail(s_wh[i + b][j], q);
-                }
-            }
-            for (; i < cn; ++i) {
-                float qh, ql;
-                split(plane[base + (size_t)i * p.rec.run_stride], qh, ql);
-                const float q = __fadd_rn(qh, ql);
-#pragma unroll
-                for (int j = 0; j < kM2PT; ++j) acc[j].add_tail(s_wh[i][j], q);
-            }
-#pragma unroll
-            for (int j = 0; j < kM2PT; ++j) acc[j].flush_tail();
-        }
-    }
-    if (r < p.n_runs) {
-#pragma unroll
-        for (int j = 0; j < kM2PT; ++j) {
-            const int pi = p0 + j;
-            if (pi >= p.P) continue;
-            p.acc[((size_t)r * p.P + pi) * 7 + 4] += acc[j].value();
-        }
-    }
-}
-
-void launch_conv_m2_comp(const ConvParams &p, cudaStream_t s) {
-    if (p.n_runs <= 0 || p.P <= 0) return;
-    const int pt = p.m2_tile == 16 ? 16 : 8;
-    dim3 g((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + pt - 1) / pt, 1);
-    if (pt == 8) {
-        if (p.rec.narrow) conv_m2_comp_kernel<true, 8><<<g, kConvRuns, 0, s>>>(p);
-        else conv_m2_comp_kernel<false, 8><<<g, kConvRuns, 0, s>>>(p);
-    } else {
-        if (p.rec.narrow) conv_m2_comp_kernel<true, 16><<<g, kConvRuns, 0, s>>>(p);
-        else conv_m2_comp_kernel<false, 16><<<g, kConvRuns, 0, s>>>(p);
     }
 }
 
@@ -766,48 +586,30 @@ bool conv_grid_fits(int32_t n_runs, int32_t P) {
     return n_runs > 0 && P > 0 && (P + kConvPT - 1) / kConvPT <= 65535;
 }
 
-// PT_OTHER: probabilities per CTA of the other statistics' kernel (m0, m3,
-// m4: 18 of the 26 record bytes at L = 256); the max-set kernel keeps 8 (16
-// takes it to 201 registers beside the union-find)
-template <int PT_OTHER>
-static void launch_conv_window_pt(const ConvParams &p, int precision, cudaStream_t s) {
+void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
+    if (p.n_runs <= 0 || p.P <= 0) return;
+    if (precision != 0) {  // ensembles only: tiled records
+        launch_conv_tiles(p, s);
+        return;
+    }
     // (run tiles, p tiles, statistics); launching the p tiles of one run tile
     // back to back (for L2 reuse of its records) measured slower
     dim3 gmax((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + kConvPT - 1) / kConvPT, 1);
-    dim3 gother(gmax.x, (p.P + PT_OTHER - 1) / PT_OTHER, precision == 0 ? 4 : 3);
+    dim3 gother(gmax.x, gmax.y, 4);
     // the record model is a template parameter: a run-time test in the row
-    // loop cost 17 % of the kernel's time.  (In FP32 only site ensembles come
-    // here: bond ensembles write tiles.)
-    if (precision != 0) {
-        conv_window_kernel<1, Layout::kSite, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-        conv_window_kernel<1, Layout::kSite, false, PT_OTHER><<<gother, kConvRuns, 0, s>>>(p);
-        launch_conv_m2_comp(p, s);
-    } else if (p.rec.site) {
-        conv_window_kernel<0, Layout::kSite, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-        conv_window_kernel<0, Layout::kSite, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
-    } else {
-        conv_window_kernel<0, Layout::kBond, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-        conv_window_kernel<0, Layout::kBond, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
-    }
-}
-
-void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
-    if (p.n_runs <= 0 || p.P <= 0) return;
-    if (p.tiled) {
-        if (precision != 0) {
-            launch_conv_tiles(p, s);
-        } else {
-            dim3 gmax((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + kConvPT - 1) / kConvPT, 1);
-            dim3 gother(gmax.x, gmax.y, 4);
-            conv_window_kernel<0, Layout::kTiled, true, kConvPT><<<gmax, kConvRuns, 0, s>>>(p);
-            conv_window_kernel<0, Layout::kTiled, false, kConvPT><<<gother, kConvRuns, 0, s>>>(p);
-        }
-        return;
-    }
-    // the FP64 path keeps 8 probabilities per CTA (its accumulators are
-    // twice as wide)
-    if (precision != 0 && p.conv_tile == 16) launch_conv_window_pt<16>(p, precision, s);
-    else launch_conv_window_pt<kConvPT>(p, precision, s);
+    // loop cost 17 % of the kernel's time
+    auto launch = [&](auto max_set, auto others) {
+        max_set<<<gmax, kConvRuns, 0, s>>>(p);
+        others<<<gother, kConvRuns, 0, s>>>(p);
+    };
+    if (p.tiled && p.rec.site)
+        launch(conv_window_kernel<Layout::kTiledSite, true>, conv_window_kernel<Layout::kTiledSite, false>);
+    else if (p.tiled)
+        launch(conv_window_kernel<Layout::kTiled, true>, conv_window_kernel<Layout::kTiled, false>);
+    else if (p.rec.site)
+        launch(conv_window_kernel<Layout::kSite, true>, conv_window_kernel<Layout::kSite, false>);
+    else
+        launch(conv_window_kernel<Layout::kBond, true>, conv_window_kernel<Layout::kBond, false>);
 }
 
 // Weights of the FP32 convolution: the part of each p's band whose weights
@@ -1331,7 +1133,7 @@ __global__ void __launch_bounds__(32 * kMicroWarps, 2) micro_tiled_kernel(MicroP
         return;
     }
     const uint64_t R = (uint64_t)p.n_runs;
-    const u128 held = (u128)p.N * R;
+    const u128 held = (u128)(rec.site ? n : p.N) * R;  // sites in clusters: all N (bond) or the n occupied (site)
     u128 sum = 0;
     U256 sq = {{0, 0, 0, 0}};
     switch (warp) {  // 0 max, 1 m0, 2 m1 (= N - max: same M2 as max), 3 m2, 4 m3, 5 m4

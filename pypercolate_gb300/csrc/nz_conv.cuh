@@ -9,19 +9,11 @@ namespace nz {
 
 constexpr int kConvChunk = 128;  // rows summed in FP32 before they are added into the running sum
 
-// Window accumulator of one canonical value.  FP64 path: an FP64 sum.  FP32
-// path: the FP32 partial sums of the row chunks are added into an FP32
-// (sum, compensation) pair by an error-free addition -- as accurate as an
-// FP64 sum of them, without the FP64 pipe, which runs at 1/64 of the FP32
-// rate on this chip.
-template <int PRECISION>
+// Window accumulator of one canonical value: the FP32 partial sums of the row
+// chunks are added into an FP32 (sum, compensation) pair by an error-free
+// addition -- as accurate as an FP64 sum of them, without the FP64 pipe, which
+// runs at 1/64 of the FP32 rate on this chip.
 struct ConvAcc {
-    double v = 0.0;
-    __device__ __forceinline__ void add(double x) { v += x; }
-    __device__ __forceinline__ double value() const { return v; }
-};
-template <>
-struct ConvAcc<1> {
     float s = 0.0f, c = 0.0f;
     // chunk sums and the running sum are >= 0: Fast2Sum on the operands
     // ordered by size is exact (3 additions and a max / min, not TwoSum's 6)

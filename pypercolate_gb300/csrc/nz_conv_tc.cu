@@ -176,19 +176,18 @@ __device__ __forceinline__ void load_pieces(const T *plane, int64_t stride, uint
 // (all in flight at once); rows past the end are zeroed on conversion.  m4 with
 // its high words takes pieces (200 runs at L = 512: 6.7 -> 4.8 ms); the others'
 // kernel is faster without (3.8 against 4.2 ms).
-template <int S, bool TILED>
+template <int S>
 __device__ __forceinline__ void load_chunk(const NzRecords &rec, uint32_t first, int32_t r, uint32_t k0, uint32_t last,
                                            raw_word<S> (&raw)[kTcK], uint32_t (&hi)[S == 6 ? kTcK : 1]) {
     const raw_word<S> *plane = raw_plane<S>(rec);
-    if constexpr (S == 6 && TILED) {
+    if constexpr (S == 6) {
         load_pieces(plane, rec.run_stride, first + k0, first + last, r, raw);
         load_pieces(rec.m4_hi, rec.run_stride, first + k0, first + last, r, hi);
     } else {
 #pragma unroll
         for (int k = 0; k < kTcK; ++k) {
             const uint32_t i = first + min(k0 + (uint32_t)k, last);
-            raw[k] = plane[record_off<sizeof(raw_word<S>)>(rec, TILED, i, r)];
-            if constexpr (S == 6) hi[k] = rec.m4_hi[record_off<4>(rec, TILED, i, r)];
+            raw[k] = plane[tile_off<sizeof(raw_word<S>)>(rec.run_stride, i, r)];
         }
     }
 }
@@ -252,7 +251,7 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
     };
     raw_word<S> raw[kTcK];
     uint32_t raw_hi[S == 6 ? kTcK : 1];
-    load_chunk<S, !SITE>(p.rec, first, run, 0, last, raw, raw_hi);
+    load_chunk<S>(p.rec, first, run, 0, last, raw, raw_hi);
     bool bad = false;
     uint32_t ch = 0;
     for (; ch < nchunks; ++ch) {
@@ -268,7 +267,7 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
             }
             // the next chunk's loads fly while this one is staged, multiplied
             // and drained
-            if (ch + 1 < nchunks) load_chunk<S, !SITE>(p.rec, first, run, (ch + 1) * kTcK, last, raw, raw_hi);
+            if (ch + 1 < nchunks) load_chunk<S>(p.rec, first, run, (ch + 1) * kTcK, last, raw, raw_hi);
             float *ah = sh.a[st][0] + a_off, *al = sh.a[st][1] + a_off;
 #pragma unroll
             for (int kb = 0; kb < kTcK / 4; ++kb) {
@@ -444,14 +443,12 @@ bool conv_tc_grid_fits(int32_t n_runs, int32_t P) {
 
 int launch_conv_window_tc(const ConvParams &p, cudaStream_t s) {
     if (p.n_runs <= 0 || p.P <= 0) return 0;
-    // site ensembles write n-major records, all others tiles
-    const cudaError_t e = p.tiled ? launch_tc<false>(p, s) : launch_tc<true>(p, s);
+    const cudaError_t e = p.rec.site ? launch_tc<true>(p, s) : launch_tc<false>(p, s);
     if (e != cudaSuccess) return -1;
     // m2 needs ~5e-11 relative per run (the susceptibility curve within 1e-6
     // absolute of FP64 at L = 1024), beyond FP32 tensor-core accumulation:
     // it runs on the compensated SIMT kernel
-    if (p.tiled) launch_conv_tiles_m2(p, s);
-    else launch_conv_m2_comp(p, s);
+    launch_conv_tiles_m2(p, s);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

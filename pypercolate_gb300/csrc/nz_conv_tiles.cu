@@ -1,10 +1,9 @@
 // nz_conv_tiles.cu -- FP32 convolution of tiled record windows.
 //
 // The products and sums of bond_canonical_statistics (percolate/hpc.py:443-515),
-// C[run][p] += sum_n w[p][n] Q[n][run], for the records of a bond ensemble
-// (nz_records.cuh, tiled), every sum in the order of conv_window_kernel and
-// conv_m2_comp_kernel: rows upwards, in chunks of 128 from the first row that a
-// tile of 8 probabilities shares with the window.
+// C[run][p] += sum_n w[p][n] Q[n][run], for the records of an ensemble
+// (nz_records.cuh, tiled), every sum in one order: rows upwards, in chunks of 128
+// from the first row that a tile of 8 probabilities shares with the window.
 //
 // One CTA takes 128 runs (thread = run) and 8 probabilities.  32 rows of the 128
 // runs are one contiguous piece of a tiled plane, so one thread fetches them with
@@ -101,7 +100,8 @@ __device__ __forceinline__ void read_rows(const T *tile, int run, int i, T (&q)[
 template <int S>
 constexpr int kPerSm = S == 1 ? 4 : sizeof(raw_t<S>) == 8 ? 3 : 5;
 
-template <int S>
+// SITE (S = 1 only): records of site percolation, m1 = n - max instead of N - max
+template <int S, bool SITE>
 __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams p) {
     constexpr bool kMax = S == 1, kM2 = TileShared<S>::kM2;
     // rows in straight-line code: more of m2's would not fit the instruction cache
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
     if (cb < b) load_weights(cb);
     bool core = kM2 && meets_core();
 
-    ConvAcc<1> acc[kM2 ? 1 : kSets][kM2 ? 1 : kPT];
+    ConvAcc acc[kM2 ? 1 : kSets][kM2 ? 1 : kPT];
     uint64_t part[kM2 ? 1 : kSets][kM2 ? 1 : kPT / 2];
     Dot2Acc dot[kM2 ? kPT : 1];
     auto clear = [&]() {
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
                                 const uint32_t mx = q[i] & ~kSpanBit;
                                 products(0, (q[i] & kSpanBit) ? 1.0f : 0.0f);
                                 products(1, (float)mx);
-                                products(2, (float)(p.N - mx));
+                                products(2, (float)((SITE ? p.n_begin + row + (uint32_t)(i0 + i) : p.N) - mx));
                             } else if constexpr (S == 6) {
                                 products(0, fmaf((float)hi[i], 18446744073709551616.0f, u64_to_f32(q[i])));
                             } else if constexpr (sizeof(raw_t<S>) == 8) {
@@ -334,13 +334,13 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
     }
 }
 
-template <int S>
+template <int S, bool SITE = false>
 void launch(const ConvParams &p, cudaStream_t s) {
     dim3 grid((p.n_runs + kRuns - 1) / kRuns, (p.P + kPT - 1) / kPT);
     if (sizeof(TileShared<S>) > 48 * 1024)
-        cudaFuncSetAttribute(conv_tiles_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(conv_tiles_kernel<S, SITE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(TileShared<S>));
-    conv_tiles_kernel<S><<<grid, kRuns, sizeof(TileShared<S>), s>>>(p);
+    conv_tiles_kernel<S, SITE><<<grid, kRuns, sizeof(TileShared<S>), s>>>(p);
 }
 
 }  // namespace
@@ -351,7 +351,8 @@ void launch_conv_tiles_m2(const ConvParams &p, cudaStream_t s) {
 }
 
 void launch_conv_tiles(const ConvParams &p, cudaStream_t s) {
-    launch<1>(p, s);
+    if (p.rec.site) launch<1, true>(p, s);
+    else launch<1>(p, s);
     if (p.rec.narrow) launch<8>(p, s);
     else launch<2>(p, s);
     launch<5>(p, s);

@@ -1,4 +1,4 @@
-// nz_group.cuh -- Newman-Ziff bond percolation, one run per thread block.
+// nz_group.cuh -- Newman-Ziff percolation, one run per thread block.
 //
 // Replaces the hot loop of percolate/hpc.py:249-307 (bond_sample_states).
 // The bonds of a run are added in batches of B = 64 W (W warps, two
@@ -25,6 +25,15 @@
 //
 // Integers are exact throughout, so the records equal those of adding one
 // bond at a time, whatever the shape of the trees.
+//
+// Site percolation (SITE) is the same with a site per thread (B = 32 W): the
+// batch's sites are marked with their positions in it, so that each thread links
+// its site to those neighbours that are occupied before it.  A site claims its
+// own node, at which later neighbours of the batch wait, and its neighbours'
+// roots; once it holds them all, it and the up to four clusters become one.
+// There is no G until a first cluster has formed.  (One thread per run took 6 to
+// 170 times as long: 4,000 runs of 256 x 256, 508 ms for the whole ensemble
+// against 39; 300 of 400 x 400, 1,186 against 11.)
 //
 // A run needs few rounds (CPU count of this scheme at L = 256: 1.8 rounds per
 // batch of 64, 2.6 per 256, 4.7 per 1024), so one run keeps a whole block
@@ -54,6 +63,12 @@ constexpr int kMaxHops = 4096;                // guards against corrupted node w
 constexpr uint32_t kTagBits = 11;             // position in the batch (B <= 2048)
 constexpr uint32_t kStampTop = (1u << (32 - kTagBits)) - 2u;
 
+// Site percolation: the word of a site that the current batch occupies has this
+// bit, and its position in the batch in the low 16 bits.
+constexpr uint32_t kNewSite = 1u << 28;
+__device__ __forceinline__ bool is_new(uint32_t w) { return (w & (kRoot | kNewSite)) == (kRoot | kNewSite); }
+__device__ __forceinline__ uint32_t new_at(uint32_t w) { return w & 0xffffu; }
+
 // Node words of one run.  load() gives the word format of nz_common.cuh
 // (root: bit 31, sides 29..30, size; else the parent), sizes less one in
 // shared memory.
@@ -75,6 +90,16 @@ struct Nodes<true, false> {
         flag[x] = (uint8_t)(0x80u | (sides << 5));
     }
     static __device__ __forceinline__ uint32_t size(uint32_t w) { return (w & kSizeMask) + 1u; }
+    // site percolation: an unoccupied site, and one that the batch occupies
+    __device__ __forceinline__ void set_empty(uint32_t x) const {
+        val[x] = 0;
+        flag[x] = 0x88u;
+    }
+    static __device__ __forceinline__ bool is_empty(uint32_t w) { return (w & 0x08000000u) != 0; }
+    __device__ __forceinline__ void set_new(uint32_t x, uint32_t at, uint32_t sides) const {
+        val[x] = (uint16_t)at;
+        flag[x] = (uint8_t)(0x90u | (sides << 5));
+    }
 };
 
 template <>
@@ -96,6 +121,11 @@ struct Nodes<false, false> {
         put(x, make_root(size, sides));
     }
     static __device__ __forceinline__ uint32_t size(uint32_t w) { return root_size(w); }
+    __device__ __forceinline__ void set_empty(uint32_t x) const { put(x, kRoot); }
+    static __device__ __forceinline__ bool is_empty(uint32_t w) { return w == kRoot; }
+    __device__ __forceinline__ void set_new(uint32_t x, uint32_t at, uint32_t sides) const {
+        put(x, kRoot | (sides << kSideShift) | kNewSite | at);
+    }
 };
 
 // Sum of a 64-bit value over the warp: its low 64 bits, and what carries over.
@@ -145,6 +175,11 @@ struct Nodes<false, true> {
         put(x, make_root(size, sides));
     }
     static __device__ __forceinline__ uint32_t size(uint32_t w) { return root_size(w); }
+    __device__ __forceinline__ void set_empty(uint32_t x) const { put(x, kRoot); }
+    static __device__ __forceinline__ bool is_empty(uint32_t w) { return w == kRoot; }
+    __device__ __forceinline__ void set_new(uint32_t x, uint32_t at, uint32_t sides) const {
+        put(x, kRoot | (sides << kSideShift) | kNewSite | at);
+    }
     __device__ __forceinline__ Disp disp(uint32_t x) const {
         Disp v;
         asm volatile("ld.global.s64 %0, [%1];" : "=l"(v) : "l"(&cell[x].z));
@@ -412,20 +447,23 @@ struct Run {
     bool spanning, init_both;
 };
 
-// Does the rows of `run` with the whole block of W warps, handing batches of
+// Does the rows of `run` (SITE: of site percolation) with the whole block of W warps, handing batches of
 // rows to `sink`: wants(base, B) says (for the whole block alike) whether rows
 // base .. base + B - 1 of the window are wanted, put(i0, ...) takes this
-// thread's rows i0 .. i0 + kE - 1 (rows past the window's end among them).
+// thread's rows i0 .. i0 + E - 1 (rows past the window's end among them).
 // `nodes`: shared memory for node_bytes of the run (SHARED only).  TORUS: the
 // flag of a row says that a cluster wraps (g.wrap); other lattices: that one
 // spans.
 // Every thread of the block calls it and may call it again at once.  Returns
 // whether the run is finished and was found corrupt.
-template <int W, bool SHARED, bool TORUS, class Sink>
+template <int W, bool SHARED, bool TORUS, bool SITE, class Sink>
 __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, GroupShared<W, SHARED> &sh,
                                           Claims<W> &claims, uint8_t *nodes, Sink &sink) {
     constexpr bool NARROW = SHARED;
-    constexpr uint32_t B = 32u * W * kE;
+    constexpr int E = SITE ? 1 : kE;  // steps per thread and batch
+    constexpr int C = 4;              // finds: both ends of two bonds, or a site's neighbours
+    constexpr uint32_t B = 32u * W * E;
+    constexpr uint32_t kNone = 0xffffffffu;
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     typedef Nodes<SHARED, TORUS> NodesT;
     NodesT nd;
@@ -443,7 +481,10 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
     bool span = false, init_both = false, corrupt = false;
     if (run.n_begin == 0) {
         if constexpr (SHARED) {
-            for (uint32_t i = t; i < g.N; i += 32u * W) nd.set_root(i, 1u, sides_any(g, i));
+            for (uint32_t i = t; i < g.N; i += 32u * W) {
+                if (SITE) nd.set_empty(i);
+                else nd.set_root(i, 1u, sides_any(g, i));
+            }
         } else {
             for (uint32_t j = t; j < node_count<SHARED, TORUS>(g); j += 32u * W) {
                 uint32_t i = j;
@@ -454,24 +495,27 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                     if (row >= g.L || col >= g.L) continue;  // a padding slot, never read
                     i = row * g.L + col;
                 }
-                nd.set_root(j, 1u, sides_any(g, i));
+                if (SITE) nd.set_empty(j);
+                else nd.set_root(j, 1u, sides_any(g, i));
             }
         }
-        init_both = run.init_both;
+        init_both = !SITE && run.init_both;
         if (t < 2) sh.wrap[t] = 0xffffffffu;
         if (t == 0) {
-            sh.g_root = 0;
-            sh.g_sides = sides_any(g, 0);
-            Sums<NARROW> c;  // N clusters of one node, one of them G
+            sh.g_root = SITE ? kNone : 0u;
+            sh.g_sides = SITE ? 0u : sides_any(g, 0);
+            Sums<NARROW> c;  // bonds: N clusters of one node, one of them G; sites: none
             c.zero();
             RunState all;
             all.t2 = all.t3 = all.t4_lo = g.N;
             all.t4_hi = 0;
-            c.load(all);
-            c.minus_powers(1u);
-            c.g = 1;
+            if (!SITE) {
+                c.load(all);
+                c.minus_powers(1u);
+                c.g = 1;
+            }
             sh.carry[0] = c;
-            sh.clusters[0] = g.N;
+            sh.clusters[0] = SITE ? 0u : g.N;
         }
     } else {
         const RunState st = *run.state;
@@ -506,52 +550,66 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
 
     const bool given = run.perm != nullptr;
     const uint32_t rows = run.n_end - run.n_begin;
-    uint32_t ahead[kE];  // keyed bonds of the next batch
+    uint32_t ahead[E];  // keyed bonds of the next batch
     bool have_ahead = false;
     // M well below its power of two: cycle walks are common (the domain is
     // 1.8 M at L = 97, within 1.01 M at L = 2^k)
     const bool walks = !given && (sh.fp.maskR + 1ull) * (sh.fp.maskL + 1ull) > g.M + g.M / 8ull;
 
-    // (dx, dy) of a bond of the torus
-    auto step = [](bool is_down) {
-        typedef typename DispOf<SHARED, TORUS>::type D;
-        return is_down ? (D)1 : (D)((D)1 << (SHARED ? 16 : 32));
+    // torus: (dx, dy) of a bond (0 to the right, 1 downwards), or from a site to
+    // its neighbour 0 right, 1 left, 2 below, 3 above
+    typedef typename DispOf<SHARED, TORUS>::type Disp;
+    auto step = [](int dir) {
+        constexpr Disp kDx = (Disp)1 << (SHARED ? 16 : 32);
+        if (SITE) return dir == 0 ? kDx : dir == 1 ? -kDx : dir == 2 ? (Disp)1 : (Disp)-1;
+        return dir ? (Disp)1 : kDx;
+    };
+    // a loop closed at window row `row` winds around the torus where the two
+    // ways around it differ by d
+    auto close_loop = [&](Disp d, uint32_t row) {
+        if constexpr (TORUS) {
+            if (d == 0) return;
+            if (NodesT::dx(d) != 0 && row < sh.wrap[0]) atomicMin(&sh.wrap[0], row);
+            if (NodesT::dy(d) != 0 && row < sh.wrap[1]) atomicMin(&sh.wrap[1], row);
+        }
     };
     (void)step;
+    (void)close_loop;
 
     for (uint32_t base = 0; base < rows; base += B) {
-        const uint32_t i0 = base + t * kE;
-        // ---- 1. the bonds of rows i0, i0 + 1 and the roots of their ends
-        uint32_t edge[kE];
+        const uint32_t i0 = base + t * E;
+        // ---- 1. the bonds of rows i0, i0 + 1 (the site of row i0) and the roots of
+        // their ends (of its neighbours)
+        uint32_t edge[E];
 #pragma unroll
-        for (int k = 0; k < kE; ++k) edge[k] = 0;
+        for (int k = 0; k < E; ++k) edge[k] = 0;
         if (!given && g.M > 0) {
             auto from = [&](uint32_t j) {
-                const uint32_t idx = run.n_begin + i0 + j % kE + (j / kE) * B - 1u;
+                const uint32_t idx = run.n_begin + i0 + j % E + (j / E) * B - 1u;
                 return idx < g.M ? idx : 0u;
             };
             if (!walks) {
                 const FeistelPerm fp = sh.fp;
 #pragma unroll
-                for (int k = 0; k < kE; ++k) edge[k] = fp.at(from(k));
+                for (int k = 0; k < E; ++k) edge[k] = fp.at(from(k));
             } else if (have_ahead) {
 #pragma unroll
-                for (int k = 0; k < kE; ++k) edge[k] = ahead[k];
+                for (int k = 0; k < E; ++k) edge[k] = ahead[k];
                 have_ahead = false;
             } else {
                 // this batch's bonds and the next one's in one loop: a lane
                 // goes on to its next bond when the cycle walk of one ends, so
-                // the warp waits for the longest sum of 2 kE walks, not 2 kE
+                // the warp waits for the longest sum of 2 E walks, not 2 E
                 // times for the longest walk
                 const FeistelPerm fp = sh.fp;
                 uint32_t j = 0, y = from(0);
-                while (j < 2 * kE) {
+                while (j < 2 * E) {
                     y = fp.encrypt(y);
                     if (y < g.M) {
 #pragma unroll
-                        for (int k = 0; k < kE; ++k) {
+                        for (int k = 0; k < E; ++k) {
                             if (j == (uint32_t)k) edge[k] = y;
-                            if (j == (uint32_t)(kE + k)) ahead[k] = y;
+                            if (j == (uint32_t)(E + k)) ahead[k] = y;
                         }
                         ++j;
                         y = from(j);
@@ -560,35 +618,92 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                 have_ahead = true;
             }
         }
-        uint32_t start[2 * kE], x[2 * kE], w[2 * kE], first_w[2 * kE];
-        bool open[kE], down[kE] = {};
-        typename DispOf<SHARED, TORUS>::type pos[2 * kE] = {};  // displacement of each end from x
+        uint32_t start[C], x[C], w[C], first_w[C];
+        bool open[E], down[E] = {}, linked[C] = {};
+        uint32_t self = 0, self_sides = 0;  // the site's own node
+        typename DispOf<SHARED, TORUS>::type pos[C] = {};  // displacement of each start node from x
 #pragma unroll
-        for (int k = 0; k < kE; ++k) {
+        for (int k = 0; k < E; ++k) {
             const uint32_t n = run.n_begin + i0 + k;
             open[k] = i0 + k < rows && n > 0;
-            start[2 * k] = start[2 * k + 1] = 0;
-            if (open[k]) {
-                if (given) edge[k] = __ldg(run.perm + (n - 1u));
-                const uint32_t e = edge[k];
-                if (given && e >= g.M) open[k] = false;  // caller-supplied index out of range: no bond
-                else if constexpr (TORUS) decode_torus(g, e, start[2 * k], start[2 * k + 1], down[k]);
-                else decode_any(g, SHARED, e, start[2 * k], start[2 * k + 1]);
-            } else {
-                edge[k] = 0;
-            }
+            if (open[k] && given) edge[k] = __ldg(run.perm + (n - 1u));
+            if (!open[k]) edge[k] = 0;
+            if (given && edge[k] >= g.M) open[k] = false;  // caller-supplied index out of range: nothing happens
         }
+        if constexpr (!SITE) {
 #pragma unroll
-        for (int c = 0; c < 2 * kE; ++c) {
-            x[c] = start[c];
-            w[c] = nd.load(x[c]);
-            first_w[c] = w[c];
+            for (int k = 0; k < E; ++k) {
+                start[2 * k] = start[2 * k + 1] = 0;
+                if (open[k]) {
+                    if constexpr (TORUS) decode_torus(g, edge[k], start[2 * k], start[2 * k + 1], down[k]);
+                    else decode_any(g, SHARED, edge[k], start[2 * k], start[2 * k + 1]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                x[c] = start[c];
+                w[c] = nd.load(x[c]);
+                first_w[c] = w[c];
+            }
+        } else {
+            // occupy the batch's sites: until its turn a new site's node says
+            // at which position of the batch it comes
+            const uint32_t site = edge[0];
+            const bool chain = !TORUS && g.kind == NZ_GRAPH_CHAIN1D;
+            const uint32_t width = chain ? g.N : g.L, height = chain ? 1u : g.L;
+            const uint32_t row = chain ? 0u : site / width, col = site - row * width;
+            auto slot = [&](uint32_t rr, uint32_t cc) {
+                if (!SHARED && !TORUS && g.kind == NZ_GRAPH_GRID2D && kGridTiled) return grid_slot(g.tile_cols, rr, cc);
+                return rr * width + cc;
+            };
+            self = slot(row, col);
+            if (open[0]) open[0] = nd.is_empty(nd.load(self));
+            self_sides = sides_any(g, site);
+            __syncthreads();
+            if (open[0]) nd.set_new(self, t, self_sides);
+            __syncthreads();
+            if (given) {
+                // a caller's order may name a site twice in a batch: its first
+                // time counts (each turn lowers some site's position)
+                for (;;) {
+                    const bool earlier = open[0] && new_at(nd.load(self)) > t;
+                    if (!__syncthreads_or(earlier)) break;
+                    if (earlier) nd.set_new(self, t, self_sides);
+                    __syncthreads();
+                }
+                open[0] = open[0] && new_at(nd.load(self)) == t;
+            }
+            // neighbours that are occupied by now: right, left, below, above
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                bool there = open[0];
+                uint32_t rr = row, cc = col;
+                if constexpr (TORUS) {
+                    if (c == 0) cc = col + 1u == width ? 0u : col + 1u;
+                    if (c == 1) cc = col == 0 ? width - 1u : col - 1u;
+                    if (c == 2) rr = row + 1u == height ? 0u : row + 1u;
+                    if (c == 3) rr = row == 0 ? height - 1u : row - 1u;
+                } else {
+                    if (c == 0) { there = there && col + 1u < width; cc = col + 1u; }
+                    if (c == 1) { there = there && col > 0; cc = col - 1u; }
+                    if (c == 2) { there = there && row + 1u < height; rr = row + 1u; }
+                    if (c == 3) { there = there && row > 0; rr = row - 1u; }
+                }
+                start[c] = x[c] = there ? slot(rr, cc) : self;
+                w[c] = kRoot;
+                if (there) {
+                    const uint32_t v = nd.load(x[c]);
+                    linked[c] = !nd.is_empty(v) && !(is_new(v) && new_at(v) > t);
+                    if (linked[c]) w[c] = v;
+                }
+                first_w[c] = w[c];
+            }
         }
         auto climb = [&]() {
             for (int hops = 0; hops < kMaxHops; ++hops) {
                 bool more = false;
 #pragma unroll
-                for (int c = 0; c < 2 * kE; ++c) {
+                for (int c = 0; c < C; ++c) {
                     if (!is_root(w[c])) {
                         if constexpr (TORUS) pos[c] += nd.disp(x[c]);
                         x[c] = w[c];
@@ -600,50 +715,62 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             }
             corrupt = true;
 #pragma unroll
-            for (int c = 0; c < 2 * kE; ++c)
-                if (!is_root(w[c])) x[c & ~1] = x[c | 1];  // a bond that cannot be placed joins nothing
+            for (int c = 0; c < C; ++c)
+                if (!is_root(w[c])) {  // what cannot be placed joins nothing
+                    if (SITE) linked[c] = false;
+                    else x[c & ~1] = x[c | 1];
+                }
         };
         climb();
         if constexpr (!TORUS) {
 #pragma unroll
-            for (int c = 0; c < 2 * kE; ++c)
+            for (int c = 0; c < C; ++c)
                 if (!is_root(first_w[c]) && first_w[c] != x[c]) nd.shorten(start[c], x[c]);
         }
 
         // ---- 2., 3. rounds of joins
-        Sums<NARROW> d[kE];
-        uint32_t formed[kE], sd[kE], kind[kE];  // kind: 0 no join, 1 two clusters, 2 with G
+        Sums<NARROW> d[E];
+        uint32_t formed[E], sd[E], kind[E];  // kind: 0 nothing, 1 a cluster other than G formed, 2 joined to G
+        uint32_t fewer[E];                   // clusters lost by the step (modulo 2^32)
 #pragma unroll
-        for (int k = 0; k < kE; ++k) {
+        for (int k = 0; k < E; ++k) {
             d[k].zero();
-            formed[k] = sd[k] = kind[k] = 0;
+            formed[k] = sd[k] = kind[k] = fewer[k] = 0;
         }
         bool any_join = false;
         for (uint32_t round = 0; round <= B; ++round) {
-            const uint32_t tag = (claims.stamp << kTagBits) | (t * kE);
+            const uint32_t tag = (claims.stamp << kTagBits) | (t * E);
             bool wants = false;
-            uint32_t h[2 * kE];
+            uint32_t h[C], h_self = 0;
+            auto hash = [&](uint32_t at) {
+                return node_count<SHARED, TORUS>(g) <= claims.mask + 1u ? at : (at * 0x9E3779B1u) >> claims.shift;
+            };
 #pragma unroll
-            for (int c = 0; c < 2 * kE; ++c) h[c] = node_count<SHARED, TORUS>(g) <= claims.mask + 1u ? x[c] : (x[c] * 0x9E3779B1u) >> claims.shift;
+            for (int c = 0; c < C; ++c) h[c] = hash(x[c]);
+            if constexpr (SITE) {
+                // a site claims its own node too: its later neighbours wait
+                h_self = hash(self);
+                if (open[0]) {
+                    wants = true;
+                    atomicMin(claims.at + h_self, tag);
 #pragma unroll
-            for (int k = 0; k < kE; ++k) {
-                if constexpr (TORUS) {
-                    // a bond inside one cluster closes a loop, which winds
-                    // around the torus where the two ways around it differ
-                    if (open[k] && x[2 * k] == x[2 * k + 1]) {
-                        const auto d = pos[2 * k] + step(down[k]) - pos[2 * k + 1];
-                        if (d != 0) {
-                            const uint32_t row = i0 + k;
-                            if (NodesT::dx(d) != 0 && row < sh.wrap[0]) atomicMin(&sh.wrap[0], row);
-                            if (NodesT::dy(d) != 0 && row < sh.wrap[1]) atomicMin(&sh.wrap[1], row);
-                        }
-                    }
+                    for (int c = 0; c < C; ++c)
+                        if (linked[c] && x[c] != G) atomicMin(claims.at + h[c], tag);
                 }
-                open[k] = open[k] && x[2 * k] != x[2 * k + 1];
-                if (!open[k]) continue;
-                wants = true;
-                if (x[2 * k] != G) atomicMin(claims.at + h[2 * k], tag + k);
-                if (x[2 * k + 1] != G) atomicMin(claims.at + h[2 * k + 1], tag + k);
+            } else {
+#pragma unroll
+                for (int k = 0; k < E; ++k) {
+                    if constexpr (TORUS) {
+                        // a bond inside one cluster closes a loop
+                        if (open[k] && x[2 * k] == x[2 * k + 1])
+                            close_loop(pos[2 * k] + step(down[k]) - pos[2 * k + 1], i0 + k);
+                    }
+                    open[k] = open[k] && x[2 * k] != x[2 * k + 1];
+                    if (!open[k]) continue;
+                    wants = true;
+                    if (x[2 * k] != G) atomicMin(claims.at + h[2 * k], tag + k);
+                    if (x[2 * k + 1] != G) atomicMin(claims.at + h[2 * k + 1], tag + k);
+                }
             }
             if (!__syncthreads_or(wants)) break;
             any_join = true;
@@ -652,47 +779,125 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             if constexpr (TORUS) {
                 if (round == 0) {
 #pragma unroll
-                    for (int c = 0; c < 2 * kE; ++c)
+                    for (int c = 0; c < C; ++c)
                         if (!is_root(first_w[c]) && first_w[c] != x[c]) {
                             nd.shorten(start[c], x[c]);
                             nd.set_disp(start[c], pos[c]);
                         }
                 }
             }
-            // (a warp with no bond left does without, but in shared memory the
-            // code is faster without the branch)
-            if (SHARED || __any_sync(0xffffffffu, wanted))
+            if constexpr (SITE) {
+                if (open[0]) {
+                    bool lost = claims.at[h_self] != tag;
 #pragma unroll
-            for (int k = 0; k < kE; ++k) {
-                if (!open[k]) continue;
-                const uint32_t xu = x[2 * k], xv = x[2 * k + 1];
-                const bool gu = xu == G, gv = xv == G;
-                if ((!gu && claims.at[h[2 * k]] != tag + k) || (!gv && claims.at[h[2 * k + 1]] != tag + k)) {
-                    wants = true;
-                    continue;
+                    for (int c = 0; c < C; ++c) lost |= linked[c] && x[c] != G && claims.at[h[c]] != tag;
+                    wants = lost;
+                    if (!lost) {
+                        open[0] = false;
+                        // the site (one node, so far in no total) and the
+                        // distinct clusters around it become one
+                        bool first_of[C], with_g = false;
+                        uint32_t total = 1, most = 1, big = self, held = 0;
+                        sd[0] = self_sides;
+                        typename DispOf<SHARED, TORUS>::type at_big = 0;  // the site's position in big's cluster
+#pragma unroll
+                        for (int c = 0; c < C; ++c) {
+                            first_of[c] = linked[c] && x[c] != self;
+                            if constexpr (TORUS) {
+                                pos[c] -= step(c);  // the site's position in x's cluster
+                                if (linked[c] && x[c] == self) close_loop(pos[c], i0);
+                            }
+#pragma unroll
+                            for (int q = 0; q < c; ++q)
+                                if (linked[c] && linked[q] && x[q] == x[c]) {
+                                    if constexpr (TORUS) {
+                                        if (first_of[q]) close_loop(pos[c] - pos[q], i0);
+                                    }
+                                    first_of[c] = false;
+                                }
+                            if (!first_of[c]) continue;
+                            ++held;
+                            if (x[c] == G) {
+                                with_g = true;
+                                if constexpr (TORUS) at_big = pos[c];
+                                continue;
+                            }
+                            const uint32_t size = nd.size(w[c]);
+                            total += size;
+                            d[0].minus_powers(size);
+                            sd[0] |= root_sides(w[c]);
+                        }
+                        if (with_g) {
+                            big = G;
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < C; ++c) {
+                                const uint32_t size = nd.size(w[c]);
+                                if (first_of[c] && (size > most || big == self)) {
+                                    most = size;
+                                    big = x[c];
+                                    if constexpr (TORUS) at_big = pos[c];
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int c = 0; c < C; ++c) {
+                            if (!first_of[c] || x[c] == big) continue;
+                            nd.link(x[c], big);
+                            if constexpr (TORUS) nd.set_disp(x[c], at_big - pos[c]);
+                        }
+                        if (self != big) {
+                            nd.link(self, big);
+                            if constexpr (TORUS) nd.set_disp(self, at_big);
+                        }
+                        kind[0] = with_g ? 2 : 1;
+                        fewer[0] = held - 1u;
+                        if (with_g) {
+                            d[0].g = total;
+                        } else {
+                            nd.set_root(big, total, sd[0]);
+                            d[0].plus_powers(total);
+                            formed[0] = total;
+                        }
+                    }
                 }
-                open[k] = false;
-                const uint32_t a = nd.size(w[2 * k]), b = nd.size(w[2 * k + 1]);
-                if constexpr (TORUS) {
-                    // position of v's root as seen from u's
-                    const auto d = pos[2 * k] + step(down[k]) - pos[2 * k + 1];
-                    const bool under_u = gu || (!gv && a >= b);
-                    nd.set_disp(under_u ? xv : xu, under_u ? d : -d);
-                }
-                if (gu || gv) {
-                    const uint32_t c = gu ? xv : xu, wc = gu ? w[2 * k + 1] : w[2 * k];
-                    nd.link(c, G);
-                    kind[k] = 2;
-                    d[k].absorb(gu ? b : a);
-                    sd[k] = root_sides(wc);
-                } else {
-                    const bool keep_u = a >= b;
-                    kind[k] = 1;
-                    sd[k] = root_sides(w[2 * k]) | root_sides(w[2 * k + 1]);
-                    nd.link(keep_u ? xv : xu, keep_u ? xu : xv);
-                    nd.set_root(keep_u ? xu : xv, a + b, sd[k]);
-                    d[k].join(a, b);
-                    formed[k] = a + b;
+            } else {
+                // (a warp with no bond left does without, but in shared memory the
+                // code is faster without the branch)
+                if (SHARED || __any_sync(0xffffffffu, wanted))
+#pragma unroll
+                for (int k = 0; k < E; ++k) {
+                    if (!open[k]) continue;
+                    const uint32_t xu = x[2 * k], xv = x[2 * k + 1];
+                    const bool gu = xu == G, gv = xv == G;
+                    if ((!gu && claims.at[h[2 * k]] != tag + k) || (!gv && claims.at[h[2 * k + 1]] != tag + k)) {
+                        wants = true;
+                        continue;
+                    }
+                    open[k] = false;
+                    fewer[k] = 1;
+                    const uint32_t a = nd.size(w[2 * k]), b = nd.size(w[2 * k + 1]);
+                    if constexpr (TORUS) {
+                        // position of v's root as seen from u's
+                        const auto d = pos[2 * k] + step(down[k]) - pos[2 * k + 1];
+                        const bool under_u = gu || (!gv && a >= b);
+                        nd.set_disp(under_u ? xv : xu, under_u ? d : -d);
+                    }
+                    if (gu || gv) {
+                        const uint32_t c = gu ? xv : xu, wc = gu ? w[2 * k + 1] : w[2 * k];
+                        nd.link(c, G);
+                        kind[k] = 2;
+                        d[k].absorb(gu ? b : a);
+                        sd[k] = root_sides(wc);
+                    } else {
+                        const bool keep_u = a >= b;
+                        kind[k] = 1;
+                        sd[k] = root_sides(w[2 * k]) | root_sides(w[2 * k + 1]);
+                        nd.link(keep_u ? xv : xu, keep_u ? xu : xv);
+                        nd.set_root(keep_u ? xu : xv, a + b, sd[k]);
+                        d[k].join(a, b);
+                        formed[k] = a + b;
+                    }
                 }
             }
             if (--claims.stamp == 0) {  // stamps used up: start over with a clean table
@@ -704,8 +909,8 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             // many warps, one with none goes straight on to the next barrier)
             if ((SHARED && W <= 4) || __any_sync(0xffffffffu, wants)) {
 #pragma unroll
-                for (int c = 0; c < 2 * kE; ++c)
-                    if (open[c >> 1]) w[c] = nd.load(x[c]);
+                for (int c = 0; c < C; ++c)
+                    if (SITE ? open[0] && linked[c] : open[(c >> 1) % E]) w[c] = nd.load(x[c]);
                 climb();
             }
         }
@@ -721,31 +926,31 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                 wrap_row = g.wrap == 0 ? min(rx, ry) : g.wrap == 1 ? rx : g.wrap == 2 ? ry : max(rx, ry);
             }
         }
-        uint32_t ms[kE], m0[kE];
-        Sums<NARROW> m[kE];
+        uint32_t ms[E], m0[E];
+        Sums<NARROW> m[E];
         if (!any_join) {
             const Sums<NARROW> c = sh.carry[cur];
-            const uint32_t cl = sh.clusters[cur] - 1u;
+            const uint32_t cl = sh.clusters[cur] - (SITE && sh.clusters[cur] == 0 ? 0u : 1u);
 #pragma unroll
-            for (int k = 0; k < kE; ++k) {
+            for (int k = 0; k < E; ++k) {
                 m[k] = c;
                 m0[k] = cl;
                 ms[k] = g_size | (span || i0 + k >= wrap_row ? kSpanBit : 0u);
             }
         } else {
             // prefix sums over the thread's bonds, then over the warp
-            uint32_t top[kE];
+            uint32_t top[E];
             top[0] = formed[0];
 #pragma unroll
-            for (int k = 1; k < kE; ++k) {
+            for (int k = 1; k < E; ++k) {
                 top[k] = formed[k];
                 d[k].add(d[k - 1]);
                 top[k] = max(top[k], top[k - 1]);
             }
-            Sums<NARROW> inc = d[kE - 1];
-            uint32_t tmax = top[kE - 1], joins = 0;
+            Sums<NARROW> inc = d[E - 1];
+            uint32_t tmax = top[E - 1], joins = 0;
 #pragma unroll
-            for (int k = 0; k < kE; ++k) joins += kind[k] != 0 ? 1u : 0u;
+            for (int k = 0; k < E; ++k) joins += fewer[k];
             uint32_t njoin = joins;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -759,7 +964,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             }
             uint32_t sall = 0;
 #pragma unroll
-            for (int k = 0; k < kE; ++k) sall |= sd[k];
+            for (int k = 0; k < E; ++k) sall |= sd[k];
             sall = __reduce_or_sync(0xffffffffu, sall);
             if (lane == 31) {
                 sh.warp[warp] = inc;
@@ -822,9 +1027,9 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             uint32_t span_row = span ? 0u : 0xffffffffu;
             if (!TORUS && run.spanning && !span && (sides_all == 3u || init_both)) {
 #pragma unroll
-                for (int k = 0; k < kE; ++k) {
+                for (int k = 0; k < E; ++k) {
                     if (kind[k] == 0) continue;
-                    const uint32_t row = t * kE + k;
+                    const uint32_t row = t * E + k;
                     if (init_both) atomicMin(&sh.first[3], row);
                     if (kind[k] == 1) {
                         if (sd[k] == 3u) atomicMin(&sh.first[0], row);
@@ -842,22 +1047,22 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
                 if (t < 4) sh.first[t] = 0xffffffffu;
             }
 #pragma unroll
-            for (int k = 0; k < kE; ++k) {
-                pj += kind[k] != 0 ? 1u : 0u;
+            for (int k = 0; k < E; ++k) {
+                pj += fewer[k];
                 if (!want) continue;
                 m[k] = pre;
                 m[k].add(d[k]);
-                m0[k] = cl - pj - 1u;
+                m0[k] = cl - pj - (SITE && cl == pj ? 0u : 1u);
                 const uint32_t gs = m[k].g, largest = max(gs, max(ptop, top[k]));
                 if (largest != gs) {  // moments leave out the largest cluster, which is not G here
                     m[k].plus_powers(gs);
                     m[k].minus_powers(largest);
                 }
-                ms[k] = largest | (t * kE + k >= span_row || i0 + k >= wrap_row ? kSpanBit : 0u);
+                ms[k] = largest | (t * E + k >= span_row || i0 + k >= wrap_row ? kSpanBit : 0u);
             }
             if (t == 32u * W - 1u) {
                 Sums<NARROW> c = pre;
-                c.add(d[kE - 1]);
+                c.add(d[E - 1]);
                 sh.carry[cur ^ 1u] = c;
                 sh.clusters[cur ^ 1u] = cl - pj;
             }
@@ -865,7 +1070,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             // sides that G has now: those of the clusters it took in
             uint32_t gsd = 0;
 #pragma unroll
-            for (int k = 0; k < kE; ++k) gsd |= kind[k] == 2 ? sd[k] : 0u;
+            for (int k = 0; k < E; ++k) gsd |= kind[k] == 2 ? sd[k] : 0u;
             g_size = grown;
             cur ^= 1u;
             if (sides_all != g_sides) {
@@ -875,21 +1080,21 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             if (top_all > g_size) {
                 // another cluster is the largest now: it becomes G
 #pragma unroll
-                for (int k = 0; k < kE; ++k)
-                    if (formed[k] == top_all) atomicMin(&sh.winner, t * kE + k);
+                for (int k = 0; k < E; ++k)
+                    if (formed[k] == top_all) atomicMin(&sh.winner, t * E + k);
                 __syncthreads();
                 const uint32_t win = sh.winner;
-                if (win / kE == t) {
-                    uint32_t root = x[0];
+                if (win / E == t) {
+                    uint32_t root = SITE ? self : x[0];
 #pragma unroll
-                    for (int k = 1; k < kE; ++k)
-                        if (win % kE == (uint32_t)k) root = x[2 * k];
+                    for (int k = 1; k < E; ++k)
+                        if (win % E == (uint32_t)k) root = x[2 * k];
                     uint32_t wr = nd.load(root);
                     for (int hops = 0; hops < kMaxHops && !is_root(wr); ++hops) {
                         root = wr;
                         wr = nd.load(root);
                     }
-                    nd.set_root(G, g_size, g_sides);
+                    if (!SITE || G != kNone) nd.set_root(G, g_size, g_sides);
                     sh.g_root = root;
                     sh.g_sides = root_sides(wr);
                     Sums<NARROW> c = sh.carry[cur];
@@ -912,7 +1117,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
     const bool last = run.n_end == g.M + 1u;
     __syncthreads();
     if (!last) {
-        if (t == 0) nd.set_root(G, g_size, g_sides);
+        if (t == 0 && (!SITE || G != kNone)) nd.set_root(G, g_size, g_sides);
         __syncthreads();
         if constexpr (SHARED) {
             const uint32_t words = node_bytes<TORUS>(g.N) / 4u;

@@ -30,7 +30,7 @@ struct UfParams {
 // UfParams::init_flag
 const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
                                  uint32_t *flag_scratch, cudaStream_t s);
-void launch_uf_window(const UfParams &p, int perm_mode, bool span, int block, cudaStream_t s);
+void launch_uf_window(const UfParams &p, int perm_mode, bool span, cudaStream_t s);
 void launch_philox_perms(uint32_t M, int32_t n_runs, uint64_t key, uint64_t run0, uint32_t *out,
                          cudaStream_t s);
 void launch_pack_rows(const NzRecords &rec, int32_t run, uint32_t N, uint32_t M, int32_t spanning,
@@ -46,10 +46,8 @@ void launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t n_runs
 // the run in the window that begins at row 0)
 void launch_uf_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
 
-// nz_lattice.cu: site percolation (dispatched from nz_uf.cu)
-void launch_init_lattice_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
-                              cudaStream_t s);
-void launch_lattice_window(const UfParams &p, int perm_mode, bool span, int block, cudaStream_t s);
+// nz_lattice.cu: the same for site percolation
+void launch_site_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
 
 // nz_canonical.cu
 void launch_binomial_weights(uint32_t M, const double *ps, int32_t P, double cutoff, int32_t cap,
@@ -75,8 +73,6 @@ struct ConvParams {
     const float *w32;        // [P][cap] (FP32 path, its own narrower bands)
     const float *w32lo;      // [P][cap] w64 - w32 as FP32 (the compensated m2 products)
     const uint32_t *core_lo, *core_len;  // rows whose weight is >= e^-8 of the mode (m2 compensated)
-    int32_t m2_tile;         // probabilities per CTA of the compensated m2 kernel (8 or 16)
-    int32_t conv_tile;       // probabilities per CTA of the FP32 window kernels (8 or 16)
     double *acc;             // [n_runs][P][7], accumulated (+=)
     uint32_t *errors;        // tensor-core path: counts CTAs whose waits gave up (or null)
 };
@@ -95,8 +91,6 @@ void launch_narrow_weights_f32(const double *w64, const uint32_t *band_lo, const
 // nz_conv_tiles.cu: the FP32 convolution of tiled records (all statistics, or m2 alone)
 void launch_conv_tiles(const ConvParams &p, cudaStream_t s);
 void launch_conv_tiles_m2(const ConvParams &p, cudaStream_t s);
-// m2 (statistic 4) of the FP32 paths with compensated products and sums
-void launch_conv_m2_comp(const ConvParams &p, cudaStream_t s);
 // part: scratch [slices][P*7][3] doubles
 void launch_reduce_runs(const double *stats, int32_t n_runs, int32_t P, uint64_t *acc_count,
                         double *acc_mean, double *acc_m2, double *part, int32_t slices, cudaStream_t s);

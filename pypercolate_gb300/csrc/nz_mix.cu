@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(32 * W, 24 / W) mix_group_kernel(MixLaunch p, 
         sink.F = (uint32_t)p.m.F;
         sink.M = M;
         sink.start();
-        const bool bad = group::group_run<W, SHARED, false>(g, run, sh, claims, smem + (size_t)claim_count * 4u, sink);
+        const bool bad = group::group_run<W, SHARED, false, false>(g, run, sh, claims, smem + (size_t)claim_count * 4u, sink);
         if (bad && threadIdx.x == 0) atomicAdd(p.acc.errors, 1u);
         __syncthreads();
     }

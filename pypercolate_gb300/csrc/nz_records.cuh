@@ -30,20 +30,6 @@ __device__ __forceinline__ float u64_to_f32(uint64_t x) {
     return fmaf((float)(uint32_t)(x >> 32), 4294967296.0f, (float)(uint32_t)x);
 }
 
-template <int S>
-__device__ __forceinline__ float record_value_f(const NzRecords &rec, size_t off, uint32_t N) {
-    if (S == 0) return (rec.max_span[off] & kSpanBit) ? 1.0f : 0.0f;
-    if (S == 1) return (float)(rec.max_span[off] & ~kSpanBit);
-    if (S == 2) return (float)rec.m0[off];
-    if (S == 3) return (float)(N - (rec.max_span[off] & ~kSpanBit));
-    if (S == 4) return u64_to_f32(rec.m2[off]);
-    if (S == 5) return u64_to_f32(rec.m3[off]);
-    if (S == 7) return u64_to_f32(rec.m4_lo[off]);
-    if (S == 8) return (float)reinterpret_cast<const uint16_t *>(rec.m0)[off];
-    if (S == 9) return (float)reinterpret_cast<const uint32_t *>(rec.m2)[off];
-    return fmaf((float)rec.m4_hi[off], 18446744073709551616.0f, u64_to_f32(rec.m4_lo[off]));
-}
-
 // m0 and m2 of a record in either layout (narrow: uint16 / uint32)
 __device__ __forceinline__ uint32_t record_m0(const NzRecords &rec, size_t off) {
     return rec.narrow ? (uint32_t)reinterpret_cast<const uint16_t *>(rec.m0)[off] : rec.m0[off];
@@ -65,12 +51,6 @@ __device__ __forceinline__ size_t tile_off(int64_t run_stride, uint32_t i, int32
     const uint32_t turn = BYTES == 2 ? (uint32_t)(r >> 1) & 3u : (uint32_t)r & 7u;
     const size_t line = ((size_t)(i >> 5) * run_stride + r) * 32;
     return line + (((((i & 31u) / kPer) ^ turn) * kPer) | (i & (kPer - 1u)));
-}
-
-// the same, or n-major (runs next to each other)
-template <int BYTES>
-__device__ __forceinline__ size_t record_off(const NzRecords &rec, bool tiled, uint32_t i, int32_t r) {
-    return tiled ? tile_off<BYTES>(rec.run_stride, i, r) : (size_t)i * rec.run_stride + r;
 }
 
 // The raw words of rows i .. i + 7 (i a multiple of 8) of one run in a tiled

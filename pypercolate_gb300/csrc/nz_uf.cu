@@ -60,20 +60,17 @@ __global__ void pack_rows_kernel(NzRecords rec, int32_t run, uint32_t N, uint32_
 // ------------------------------------------------------------ launchers
 const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
                                  uint32_t *flag_scratch, cudaStream_t s) {
-    if (g.site) {
-        launch_init_lattice_runs(g, n_runs, nodes, state, s);
-        return nullptr;
-    }
-    // bond percolation: the union-find kernel initialises its runs itself
+    // the union-find kernel initialises its runs itself
     if (g.kind != NZ_GRAPH_EDGES) return nullptr;
     cudaMemsetAsync(flag_scratch, 0, sizeof(uint32_t), s);
     any_both_sides_kernel<<<(g.N + 255) / 256 < 1024 ? (g.N + 255) / 256 : 1024, 256, 0, s>>>(g, flag_scratch);
     return flag_scratch;
 }
 
-void launch_uf_window(const UfParams &p, int perm_mode, bool span, int block, cudaStream_t s) {
-    if (p.g.site) launch_lattice_window(p, perm_mode, span, block, s);
-    else launch_uf_groups(p, perm_mode != NZ_PERM_PHILOX, span, s);
+void launch_uf_window(const UfParams &p, int perm_mode, bool span, cudaStream_t s) {
+    const bool given = perm_mode != NZ_PERM_PHILOX;
+    if (p.g.site) launch_site_groups(p, given, span, s);
+    else launch_uf_groups(p, given, span, s);
 }
 
 void launch_philox_perms(uint32_t M, int32_t n_runs, uint64_t key, uint64_t run0, uint32_t *out,

@@ -158,3 +158,110 @@ def test_torus_windows(gpu):
             got.append(e.micro_sums())
         assert np.array_equal(got[0]['span_count'], got[1]['span_count'])
         assert (got[0]['sums'] == got[1]['sums']).all()
+
+
+def _site_run(kind, L, perm, wrap):
+    """Site percolation, one site at a time: max, flag, m0 and sums of powers."""
+    N = L if kind == 'chain' else L * L
+    height, width = (1, L) if kind == 'chain' else (L, L)
+    parent, off, size, sides = list(range(N)), [(0, 0)] * N, [0] * N, [0] * N
+    wx = wy = span = False
+    total, clusters, most = [0, 0, 0], 0, 0
+    out = [(0, False, 0, 0, 0, 0)]
+    for s in perm:
+        if s < N and size[s] == 0 and parent[s] == s:
+            row, col = s // width, s % width
+            size[s] = 1
+            if kind != 'torus':
+                at, end = (row, height) if kind == 'grid' else (col, width)
+                sides[s] = (1 if at == 0 else 0) | (2 if at == end - 1 else 0)
+            total = [t + 1 for t in total]
+            clusters += 1
+            most = max(most, 1)
+            span = span or sides[s] == 3
+            for dx, dy in ((1, 0), (-1, 0), (0, 1), (0, -1)):
+                r, c = row + dy, col + dx
+                if kind == 'torus':
+                    r, c = r % L, c % L
+                elif not (0 <= r < height and 0 <= c < width):
+                    continue
+                v = r * width + c
+                if size[v] == 0 and parent[v] == v:
+                    continue
+                pos = []
+                for x in (s, v):
+                    px = py = 0
+                    while parent[x] != x:
+                        px, py, x = px + off[x][0], py + off[x][1], parent[x]
+                    pos.append((x, px, py))
+                (a, ax, ay), (b, bx, by) = pos
+                ox, oy = ax + dx - bx, ay + dy - by
+                if a == b:
+                    wx, wy = wx or ox != 0, wy or oy != 0
+                    continue
+                if size[a] < size[b]:
+                    a, b, ox, oy = b, a, -ox, -oy
+                total = [t + (size[a] + size[b]) ** k - size[a] ** k - size[b] ** k
+                         for t, k in zip(total, (2, 3, 4))]
+                parent[b], off[b] = a, (ox, oy)
+                size[a] += size[b]
+                sides[a] |= sides[b]
+                clusters -= 1
+                most = max(most, size[a])
+                span = span or sides[a] == 3
+        flag = {'either': wx or wy, 'x': wx, 'y': wy, 'both': wx and wy}[wrap] if kind == 'torus' else span
+        out.append((most, flag, max(clusters - 1, 0)) + tuple(t - most ** k for t, k in zip(total, (2, 3, 4))))
+    return out
+
+
+@pytest.mark.parametrize('kind,L,runs', [
+    ('grid', 2, 3), ('grid', 3, 700), ('grid', 9, 5000), ('grid', 23, 40), ('grid', 100, 3), ('grid', 256, 1),
+    ('grid', 257, 1), ('chain', 3, 900), ('chain', 65536, 1), ('chain', 65537, 1), ('torus', 3, 2000),
+    ('torus', 24, 60), ('torus', 128, 2), ('torus', 129, 1)])
+@pytest.mark.parametrize('order', ['keyed', 'given'])
+def test_site_records(gpu, oracle, kind, L, runs, order):
+    """Occupied sites claim themselves and their neighbours' clusters; a
+    caller's order may name sites twice or none at all."""
+    from pypercolate_gb300 import lattice
+    N = L if kind == 'chain' else L * L
+    wrap = 'both' if kind == 'torus' else 'either'
+    runs = runs if order == 'keyed' else 2
+    if order == 'keyed':
+        host = lattice.sample_records(kind, L, 'site', wrap, n_runs=runs, key=41, run0=7)
+        perm = oracle.philox_permutation(41, 7 + runs - 1, N)
+    else:
+        rng = np.random.default_rng(L)
+        perms = np.stack([rng.permutation(N) for _ in range(runs)]).astype(np.uint32)
+        perms[:, N // 3:2 * N // 3] = rng.integers(0, N + 2, (runs, 2 * N // 3 - N // 3))
+        host = lattice.sample_records(kind, L, 'site', wrap, perms=perms)
+        perm = perms[-1]
+    want = _site_run(kind, L, perm.tolist(), wrap)
+    r = runs - 1
+    assert np.array_equal(host['edge'][1:, r], perm)
+    assert np.array_equal(host['max_span'][:, r] & 0x7fffffff, [w[0] for w in want])
+    assert np.array_equal((host['max_span'][:, r] >> 31).astype(bool), [w[1] for w in want])
+    assert np.array_equal(host['m0'][:, r], [w[2] for w in want])
+    assert host['m2'][:, r].tolist() == [w[3] for w in want]
+    assert host['m3'][:, r].tolist() == [w[4] for w in want]
+    m4 = [int(a) | int(b) << 64 for a, b in zip(host['m4_lo'][:, r], host['m4_hi'][:, r])]
+    assert m4 == [w[5] for w in want]
+
+
+@pytest.mark.parametrize('kind,L,window', [('grid', 30, 70), ('chain', 900, 256), ('grid', 258, 40000), ('torus', 24, 100),
+                                           ('torus', 130, 9000)])
+@pytest.mark.parametrize('precision', ['fp64', 'fp32'])
+def test_site_windows(gpu, kind, L, window, precision):
+    from pypercolate_gb300.ensemble import Ensemble
+    ps = np.array([0.3, 0.55, 0.6, 0.9])
+    got = []
+    for w in (0, window):
+        e = Ensemble(kind, L, ps, precision=precision, model='site', window=w)
+        e.run(40, key=3)
+        assert e.errors() == 0
+        got.append((e.micro_sums(), e.mean.cpu().numpy()))
+    (a, ma), (b, mb) = got
+    assert np.array_equal(a['span_count'], b['span_count'])
+    assert (a['sums'] == b['sums']).all()
+    # FP64: sums of < 2^17 terms in another order; FP32: partial sums of 128 rows
+    # cut elsewhere, each within 128 * 2^-24 of exact
+    np.testing.assert_allclose(ma, mb, rtol=1e-12 if precision == 'fp64' else 2e-5)
