@@ -407,32 +407,41 @@ __host__ __device__ __forceinline__ uint32_t node_count(const GraphDev &g) {
     return SHARED || TORUS ? g.N : g.slots;
 }
 
-// claims: one word per node where that is few, else enough that bonds of one
-// batch seldom share a word
+// Claims: one word per node where that is few, else enough that bonds of one
+// batch seldom share a word (a bond that loses a word to a stranger waits a round
+// for nothing), as far as they fit beside `nodes` bytes of a run with `blocks`
+// blocks to an SM (228 KB, of which 1 KB is each block's own and 256 B are left
+// for the caller).  Filling the SM beats 4,096 words whatever the nodes, which
+// kept a block out where they were too many and gave up room where they were
+// few: 1,000 runs of 97 x 97 1.07 -> 0.95 ms, 3,000 of 150 x 150 6.95 -> 5.77,
+// 1,000 of 256 x 256 7.02 -> 6.57, of chains of 6,000 0.37 -> 0.27, of the torus
+// 120 3.10 -> 1.83.  Powers of two need a cheaper hash (2 % less at L = 97), but
+// leave up to half of the room (7 % more at L = 128, 18 % on the torus 120).
 template <int W, bool SHARED>
-__host__ __device__ __forceinline__ uint32_t claim_words(uint32_t slots) {
-    constexpr uint32_t kMost = SHARED ? 4096u : 16384u;
-    constexpr uint32_t kEnough = 32u * W * kE * 16u < kMost ? 32u * W * kE * 16u : kMost;
-    uint32_t claims = 32;
-    while (claims < slots && claims < kEnough) claims <<= 1;
-    return claims;
+__host__ __device__ __forceinline__ uint32_t claim_words(uint32_t slots, uint32_t nodes, uint32_t blocks) {
+    constexpr uint32_t kMost = 16384u, kAsked = 32u * W * kE * 16u;
+    constexpr uint32_t kEnough = SHARED && kAsked < kMost ? kAsked : kMost;
+    const uint32_t left = 228u * 1024u / blocks - 1280u - (uint32_t)sizeof(GroupShared<W, SHARED>);
+    const uint32_t room = nodes + 1024u < left ? (left - nodes) / 4u & ~31u : 256u;
+    const uint32_t all = (slots + 31u) & ~31u;
+    const uint32_t claims = room < kEnough ? room : kEnough;
+    return claims < all ? claims : all;
 }
 
-// The claims of a block, for all the runs it takes.  `words`: a power of two
-// of them, at the start of the block's dynamic shared memory.
+// The claims of a block, for all the runs it takes, at the start of its dynamic
+// shared memory (a multiple of 32 words).
 template <int W>
 struct Claims {
     uint32_t *at;
-    uint32_t mask, shift;
+    uint32_t count;
     uint32_t stamp;  // counts the rounds down: a new round's claims beat all older ones
-    __device__ __forceinline__ void init(uint32_t *words, uint32_t count) {
+    __device__ __forceinline__ void init(uint32_t *words, uint32_t n) {
         at = words;
-        mask = count - 1u;
-        shift = __clz(mask);  // as many top bits of a multiplicative hash as the mask has
+        count = n;
         clear();
     }
     __device__ __forceinline__ void clear() {
-        for (uint32_t i = threadIdx.x; i <= mask; i += 32u * W) at[i] = 0xffffffffu;
+        for (uint32_t i = threadIdx.x; i < count; i += 32u * W) at[i] = 0xffffffffu;
         stamp = kStampTop;
     }
 };
@@ -743,7 +752,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
             bool wants = false;
             uint32_t h[C], h_self = 0;
             auto hash = [&](uint32_t at) {
-                return node_count<SHARED, TORUS>(g) <= claims.mask + 1u ? at : (at * 0x9E3779B1u) >> claims.shift;
+                return node_count<SHARED, TORUS>(g) <= claims.count ? at : __umulhi(at * 0x9E3779B1u, claims.count);
             };
 #pragma unroll
             for (int c = 0; c < C; ++c) h[c] = hash(x[c]);

@@ -101,11 +101,25 @@ __global__ void __launch_bounds__(32 * W, 24 / W) uf_group_kernel(UfParams p, ui
     if (bad && p.errors && threadIdx.x == 0) atomicAdd(p.errors, 1u);
 }
 
+// Runs that an SM has room and work for at a time: as many as fit with some 1,100
+// words of claims each, spread evenly over the waves that takes (3,000 chains of
+// 6,000, 20 to an SM: 9, 9 and 2 at a time 0.86 ms, 7, 7 and 6 0.72).
+inline int runs_per_sm(const UfParams &p) {
+    const uint32_t N = p.g.N;
+    const bool torus = p.g.kind == NZ_GRAPH_TORUS2D;
+    const int runs = (p.n_runs + 151) / 152;
+    if (N > (torus ? kSharedTorus : kSharedNodes)) return runs < 2 ? runs : 2;
+    const int fit = (int)(226u * 1024u / ((torus ? node_bytes<true>(N) : node_bytes<false>(N)) + 6144u));
+    const int waves = (runs + fit - 1) / fit;
+    return (runs + waves - 1) / waves;
+}
+
 template <int W, bool SHARED, bool TORUS, bool SITE>
 void launch_group(const UfParams &p, bool given, bool span, cudaStream_t s) {
-    const uint32_t claims = claim_words<W, SHARED>(node_count<SHARED, TORUS>(p.g));
-    size_t smem = (size_t)claims * 4u;
-    if (SHARED) smem += node_bytes<TORUS>(p.g.N);
+    const uint32_t nodes = SHARED ? node_bytes<TORUS>(p.g.N) : 0u;
+    const int blocks = min(24 / W, runs_per_sm(p));
+    const uint32_t claims = claim_words<W, SHARED>(node_count<SHARED, TORUS>(p.g), nodes, (uint32_t)blocks);
+    const size_t smem = (size_t)claims * 4u + nodes;
     if (smem > 40 * 1024)
         cudaFuncSetAttribute(uf_group_kernel<W, SHARED, TORUS, SITE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
@@ -116,7 +130,7 @@ void launch_group(const UfParams &p, bool given, bool span, cudaStream_t s) {
 // a thread) with the runs that are there and that fit, and batches of at most
 // an eighth of a run.  More warps per SM beat smaller batches until there are
 // about 24 (ms by warps per run 1, 2, 4, 8: 4,000 runs of 97 x 97, 6 to an SM,
-// 6.5, 4.1, 3.3, 3.6; 20,000 runs of 32 x 32, 24 to an SM, 1.1, 1.4, 1.9, 3.0).
+// 6.5, 4.1, 3.3, 3.6 with 4,096 words of claims; 20,000 runs of 32 x 32, 24 to an SM, 1.1, 1.4, 1.9, 3.0).
 // In global memory: 12 warps, two runs to an SM, so that the nodes of the
 // resident runs stay near L2's size (200 runs of 512 x 512: 18.6, 11.1, 9.3,
 // 10.7 ms with 4, 8, 12, 24), 24 where there are no more runs than SMs.  Sites
@@ -126,11 +140,8 @@ constexpr int kWarpsPerSm = 24;
 constexpr int kWarpChoices[8] = {1, 2, 3, 4, 6, 8, 12, 24};
 inline int group_warps(const UfParams &p, bool site) {
     const uint32_t N = p.g.N;
-    const bool torus = p.g.kind == NZ_GRAPH_TORUS2D;
-    if (N > (torus ? kSharedTorus : kSharedNodes)) return p.n_runs <= 152 ? 24 : 12;
-    int runs = (p.n_runs + 151) / 152;
-    const int fit = (int)(226u * 1024u / ((torus ? node_bytes<true>(N) : node_bytes<false>(N)) + 6144u));
-    runs = runs < fit ? runs : fit;
+    if (N > (p.g.kind == NZ_GRAPH_TORUS2D ? kSharedTorus : kSharedNodes)) return p.n_runs <= 152 ? 24 : 12;
+    const int runs = runs_per_sm(p);
     int w = 1;
     for (int c : kWarpChoices)
         if (c * runs <= kWarpsPerSm && (site ? 32u : 64u) * c * 8u <= p.g.M) w = c;

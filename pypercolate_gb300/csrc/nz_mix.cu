@@ -476,8 +476,9 @@ __global__ void mix_finalize_kernel(MixDev m, const uint32_t *counts, const uint
 // its runs needs; per_sm: blocks that fit on an SM.
 template <int W, bool SHARED, bool FUSED>
 static int launch_segment(const MixLaunch &p, int segment, uint32_t words, int per_sm, cudaStream_t s) {
-    const uint32_t claims = group::claim_words<W, SHARED>(words);
-    const size_t smem = (size_t)claims * 4u + (SHARED ? group::val_bytes(words) + group::flag_bytes(words) : 0u);
+    const uint32_t nodes = SHARED ? group::val_bytes(words) + group::flag_bytes(words) : 0u;
+    const uint32_t claims = group::claim_words<W, SHARED>(words, nodes, (uint32_t)per_sm);
+    const size_t smem = (size_t)claims * 4u + nodes;
     if (smem > 40 * 1024 &&
         cudaFuncSetAttribute(mix_group_kernel<W, SHARED, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
