@@ -25,6 +25,28 @@ __device__ __forceinline__ float gelu_grad(float z) {
     return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
+// The kernels of a step run one after the other, each for a few microseconds.
+// Each lets the next one start at once (its blocks take their places, set up
+// their barriers and TMEM) and waits itself, before its first access to global
+// memory, until the one before it is complete (programmatic dependent launch).
+__device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+static void launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute overlap;
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // ---------------------------------------------------------------------
 // GEMM on the tensor cores: tcgen05.mma kind::f16 with BF16 operands and an
 // FP32 accumulator in TMEM
@@ -184,7 +206,7 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
     float *C = out.C + blockIdx.z * out.slice;
     const float *A = in.A + (int64_t)kb * in.sak;
     const uint32_t cols = ntile <= 32 ? 32u : 64u;  // TMEM: power of two >= 32
-    if (t < ntile) sh.bias[t] = out.bias && n0 + t < N ? out.bias[n0 + t] : 0.0f;
+    start_next();
     // rows t % 128 of C; threads 128 .. 255 take columns 32 .. 63
     const int m = m0 + (t & 127), j0 = (t >> 7) * 32;
     const int64_t row = (int64_t)m * out.ldc + n0 + j0;
@@ -200,6 +222,8 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = sh.tmem;
+    wait_previous();
+    if (t < ntile) sh.bias[t] = out.bias && n0 + t < N ? out.bias[n0 + t] : 0.0f;
     const int nch = (K + kGK - 1) / kGK;
     constexpr bool kSums = sizeof(T) == 4;  // FP32 B: the gradient of the pre-activations
     float colsum = 0.0f, none = 0.0f;
@@ -308,6 +332,8 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
 // slices of `count` values, `stride` floats apart, summed in order into out
 // (deterministic split-K): the weight gradient and, after it, the bias gradient
 __global__ void splitk_sum_kernel(const float *slices, int splits, int64_t stride, int64_t count, float *out) {
+    start_next();
+    wait_previous();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
         float acc = 0.0f;
 #pragma unroll 8
@@ -331,7 +357,7 @@ static void gemm(int M, int N, int K, const GemmIn<T> &in, const GemmOut &out, i
         // which belongs to the function in the current device's context
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GemmSmem));
         dim3 grid((N + ntile - 1) / ntile, (M + kGM - 1) / kGM, splits);
-        kernel<<<grid, kGThreads, sizeof(GemmSmem), s>>>(M, N, K, in, out, ntile, k_split);
+        launch_chained(kernel, grid, kGThreads, sizeof(GemmSmem), s, M, N, K, in, out, ntile, k_split);
     };
     if constexpr (sizeof(T) == 2) {
         if (a_wide && b_wide) launch(mlp_gemm_kernel<true, true, T>);
@@ -350,6 +376,8 @@ __global__ void to_bf16_kernel(const float *a, __nv_bfloat16 *b, int64_t n) {
 // Weighted squared error: loss = sum_{b,o} w[b][o] (y - t)^2 / B ; dY = 2 w (y - t) / B
 __global__ void mse_kernel(const float *Y, const float *T, const float *Wt, int B, int N, float *dY,
                            float *loss_parts) {
+    start_next();
+    wait_previous();
     float s = 0.0f;
     const int64_t n = (int64_t)B * N;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -370,6 +398,8 @@ __global__ void mse_kernel(const float *Y, const float *T, const float *Wt, int 
 
 __global__ void adam_kernel(float *p, const float *g, float *m, float *v, __nv_bfloat16 *pb, int64_t n, float lr,
                             float b1, float b2, float eps, float c1, float c2) {
+    start_next();
+    wait_previous();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.0f - b1) * gi;
@@ -451,8 +481,8 @@ int nz_mlp_forward(const int32_t *widths, int32_t n_layers, int32_t batch, const
 int nz_mlp_loss(const float *y, const float *target, const float *weight, int32_t batch, int32_t n_out,
                 float *dy, float *loss_parts, int32_t n_parts, void *stream) {
     if (!y || !target || !dy || !loss_parts || batch <= 0 || n_out <= 0 || n_parts <= 0) return NZ_ERR_INVALID;
-    mse_kernel<<<n_parts, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(y, target, weight, batch, n_out, dy,
-                                                                            loss_parts);
+    launch_chained(mse_kernel, dim3(n_parts), 256, 0, reinterpret_cast<cudaStream_t>(stream), y, target, weight, batch,
+                   n_out, dy, loss_parts);
     return cudaGetLastError() == cudaSuccess ? NZ_OK : NZ_ERR_CUDA;
 }
 
@@ -497,8 +527,8 @@ int nz_mlp_backward(const int32_t *widths, int32_t n_layers, int32_t batch, cons
         gemm(K, N, batch, g, GemmOut{Epi::kPlain, nullptr, nullptr, dst, N, per_slice, dst + (int64_t)K * N}, splits,
              k_split, s);
         if (splits > 1)
-            splitk_sum_kernel<<<blocks_for(per_slice), 256, 0, s>>>(spare, splits, per_slice, per_slice,
-                                                                   grads + wo[l]);
+            launch_chained(splitk_sum_kernel, dim3(blocks_for(per_slice)), 256, 0, s, spare, splits, per_slice,
+                           per_slice, grads + wo[l]);
         if (l == 0) break;
         // dZ of layer l - 1 = (dZ W^T) * GELU'(z)  (W[K][N]: B(k=n, n=k) = W[k][n])
         const GemmIn<__nv_bfloat16> b{dZ, N, 1, pb + wo[l], 1, N};
@@ -523,8 +553,8 @@ int nz_mlp_adam(float *params, const float *grads, float *m, float *v, void *par
                 float lr, float beta1, float beta2, float eps, int32_t step, void *stream) {
     if (!params || !grads || !m || !v || !params_bf16 || count <= 0 || step <= 0) return NZ_ERR_INVALID;
     const float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
-    adam_kernel<<<blocks_for(count), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        params, grads, m, v, reinterpret_cast<__nv_bfloat16 *>(params_bf16), count, lr, beta1, beta2, eps, c1, c2);
+    launch_chained(adam_kernel, dim3(blocks_for(count)), 256, 0, reinterpret_cast<cudaStream_t>(stream), params, grads, m,
+                   v, reinterpret_cast<__nv_bfloat16 *>(params_bf16), count, lr, beta1, beta2, eps, c1, c2);
     return cudaGetLastError() == cudaSuccess ? NZ_OK : NZ_ERR_CUDA;
 }
 
