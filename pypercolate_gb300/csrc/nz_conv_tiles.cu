@@ -5,7 +5,7 @@
 // (nz_records.cuh, tiled), every sum in one order: rows upwards, in chunks of 128
 // from the first row that a tile of 8 probabilities shares with the window.
 //
-// One CTA takes 128 runs (thread = run) and 8 probabilities.  32 rows of the 128
+// One CTA takes 128 runs (thread = run) and Q of the tile's 8 probabilities.  32 rows of the 128
 // runs are one contiguous piece of a tiled plane, so one thread fetches them with
 // one bulk copy per plane (cp.async.bulk), two pieces in flight, and the threads
 // read their run's rows from shared memory in 16-byte loads without bank
@@ -13,7 +13,7 @@
 // chunk's are loaded while this one is summed.  FP32 products go two to an
 // instruction (fma.rn.f32x2, each half rounded like a single one).
 //
-// 4,000 runs at L = 97, 501 p: 0.37 ms for max, 0.20 for m0, 0.31 each for m3
+// 4,000 runs at L = 97, 501 p: 0.39 ms for max, 0.19 for m0, 0.31 each for m3
 // and m4, 0.86 for m2.  Reading the rows of one run straight from global memory,
 // 16 bytes per thread and 128 bytes apart, kept the load pipe busy 80 % of the
 // time and took 0.48, 2.0 (m0, m3 and m4) and 0.92 ms; 16 probabilities per CTA
@@ -32,10 +32,9 @@ namespace nz {
 namespace {
 
 constexpr int kRuns = 128;    // runs per CTA
-constexpr int kPT = 8;        // probabilities per CTA
+constexpr int kPT = 8;        // probabilities per tile
 constexpr int kRows = 32;     // rows per tile
 constexpr int kWRows = kConvChunk + 8;  // weights staged: a chunk, from the 8-row group of its first row
-constexpr int kWPer = (kWRows * kPT + kRuns - 1) / kRuns;
 
 // S: 1 the max_span plane (statistics 0, 1 and 3), 2 / 8 m0 (uint32 / uint16),
 // 4 / 9 m2 (uint64 / uint32), 5 m3, 6 / 7 m4 with / without its high words
@@ -54,15 +53,15 @@ __device__ __forceinline__ const raw_t<S> *plane_of(const NzRecords &rec) {
     else return rec.m4_lo;
 }
 
-template <int S>
+template <int S, int Q>
 struct TileShared {
     static constexpr bool kM2 = S == 4 || S == 9;
     raw_t<S> q[2][kRuns * kRows];
     uint32_t hi[S == 6 ? 2 : 1][S == 6 ? kRuns * kRows : 4];
-    float w[kM2 ? 2 : 1][kWRows][kPT];  // [hi, lo]
+    float w[kM2 ? 2 : 1][kWRows][Q];  // [hi, lo]
     uint64_t full[2];
     uint32_t lo[kPT], len[kPT], clo[kPT], clen[kPT];
-    uint32_t range[2];  // window rows of the CTA
+    uint32_t range[4];  // window rows of the CTA; of the tile's probabilities
 };
 
 __device__ __forceinline__ uint64_t pair(float a, float b) {
@@ -101,15 +100,18 @@ template <int S>
 constexpr int kPerSm = S == 1 ? 4 : sizeof(raw_t<S>) == 8 ? 3 : 5;
 
 // SITE (S = 1 only): records of site percolation, m1 = n - max instead of N - max
-template <int S, bool SITE>
+template <int S, int Q, bool SITE>
 __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams p) {
-    constexpr bool kMax = S == 1, kM2 = TileShared<S>::kM2;
+    constexpr bool kMax = S == 1, kM2 = TileShared<S, Q>::kM2;
     // rows in straight-line code: more of m2's would not fit the instruction cache
     constexpr int kStep = kM2 ? 4 : 8;
     constexpr int kSets = kMax ? 3 : 1, kOut = S == 8 ? 2 : S == 9 ? 4 : S == 7 ? 6 : S;
     extern __shared__ __align__(128) uint8_t smem[];
-    TileShared<S> &sh = *reinterpret_cast<TileShared<S> *>(smem);
-    const int run = threadIdx.x, r = blockIdx.x * kRuns + run, p0 = blockIdx.y * kPT;
+    TileShared<S, Q> &sh = *reinterpret_cast<TileShared<S, Q> *>(smem);
+    constexpr int kWPer = (kWRows * Q + kRuns - 1) / kRuns;
+    // the tile's first probability, and which of its kPT are this CTA's
+    const int run = threadIdx.x, r = blockIdx.x * kRuns + run, p0 = (int)blockIdx.y / (kPT / Q) * kPT;
+    const int q0 = Q == kPT ? 0 : (int)blockIdx.y % (kPT / Q) * Q;
     if (run < kPT) {
         const bool in = p0 + run < p.P;
         sh.lo[run] = in ? p.band_lo[p0 + run] : 0u;
@@ -123,21 +125,24 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
         tc::mbar_init_fence();
     }
     __syncthreads();
-    if (run == 0) {
+    if (run < 2) {  // the CTA's probabilities; all of the tile's
         uint32_t lo = 0xffffffffu, hi = 0;
-        for (int j = 0; j < kPT; ++j)
+        for (int j = run == 0 ? q0 : 0; j < (run == 0 ? q0 + Q : kPT); ++j)
             if (sh.len[j]) {
                 lo = min(lo, sh.lo[j]);
                 hi = max(hi, sh.lo[j] + sh.len[j]);
             }
         lo = max(lo, p.n_begin);
         hi = min(hi, p.n_end);
-        sh.range[0] = lo < hi ? lo - p.n_begin : 0u;
-        sh.range[1] = lo < hi ? hi - p.n_begin : 0u;
+        sh.range[2 * run] = lo < hi ? lo - p.n_begin : 0u;
+        sh.range[2 * run + 1] = lo < hi ? hi - p.n_begin : 0u;
     }
     __syncthreads();
     const uint32_t a = sh.range[0], b = sh.range[1];  // window rows
     if (a >= b) return;
+    // chunks are counted from the tile's first row, whichever probabilities are
+    // the CTA's, so that their sums do not depend on Q
+    const uint32_t a8 = Q == kPT ? a : sh.range[2], b8 = Q == kPT ? b : sh.range[3];
     const uint32_t tile0 = a / kRows, tiles = (b + kRows - 1) / kRows - tile0;
     const int runs = min(kRuns, p.n_runs - (int)blockIdx.x * kRuns);
     auto fetch = [&](uint32_t k) {  // one thread: tile tile0 + k into stage k % 2
@@ -155,7 +160,7 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
     }
 
     // the chunk [ca, cb) of the rows
-    uint32_t ca = a, cb = min(a + (uint32_t)kConvChunk, b);
+    uint32_t ca = a8 + (a - a8) / kConvChunk * kConvChunk, cb = min(ca + (uint32_t)kConvChunk, b8);
     // weights of the chunk that begins at row c, zero outside it
     float wreg[kWPer], wreg_lo[kM2 ? kWPer : 1];
     auto load_weights = [&](uint32_t c) {
@@ -165,8 +170,8 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
             const int i = run + q * kRuns, j = i / kWRows;
             const uint32_t row = base + (uint32_t)(i % kWRows), n = p.n_begin + row;
             float v = 0.0f, vl = 0.0f;
-            if (j < kPT && row >= c && row < end && n >= sh.lo[j] && n < sh.lo[j] + sh.len[j]) {
-                const size_t at = (size_t)(p0 + j) * p.cap + (n - sh.lo[j]);
+            if (j < Q && row >= c && row < end && n >= sh.lo[q0 + j] && n < sh.lo[q0 + j] + sh.len[q0 + j]) {
+                const size_t at = (size_t)(p0 + q0 + j) * p.cap + (n - sh.lo[q0 + j]);
                 v = p.w32[at];
                 if (kM2) vl = p.w32lo[at];
             }
@@ -178,7 +183,7 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
 #pragma unroll
         for (int q = 0; q < kWPer; ++q) {
             const int i = run + q * kRuns, j = i / kWRows, row = i % kWRows;
-            if (j < kPT) {
+            if (j < Q) {
                 sh.w[0][row][j] = wreg[q];
                 if (kM2) sh.w[kM2 ? 1 : 0][row][j] = wreg_lo[q];
             }
@@ -200,28 +205,28 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
     if (cb < b) load_weights(cb);
     bool core = kM2 && meets_core();
 
-    ConvAcc acc[kM2 ? 1 : kSets][kM2 ? 1 : kPT];
-    uint64_t part[kM2 ? 1 : kSets][kM2 ? 1 : kPT / 2];
-    Dot2Acc dot[kM2 ? kPT : 1];
+    ConvAcc acc[kM2 ? 1 : kSets][kM2 ? 1 : Q];
+    uint64_t part[kM2 ? 1 : kSets][kM2 ? 1 : Q / 2];
+    Dot2Acc dot[kM2 ? Q : 1];
     auto clear = [&]() {
         if constexpr (!kM2) {
 #pragma unroll
             for (int s = 0; s < kSets; ++s)
 #pragma unroll
-                for (int j = 0; j < kPT / 2; ++j) part[s][j] = 0;
+                for (int j = 0; j < Q / 2; ++j) part[s][j] = 0;
         }
     };
     auto flush = [&]() {
         if constexpr (kM2) {
             if (!core) {
 #pragma unroll
-                for (int j = 0; j < kPT; ++j) dot[j].flush_tail();
+                for (int j = 0; j < Q; ++j) dot[j].flush_tail();
             }
         } else {
 #pragma unroll
             for (int s = 0; s < kSets; ++s)
 #pragma unroll
-                for (int j = 0; j < kPT / 2; ++j) {
+                for (int j = 0; j < Q / 2; ++j) {
                     float x, y;
                     unpair(part[s][j], x, y);
                     acc[s][2 * j].add(x);
@@ -265,21 +270,28 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
                             if (core) {
                                 const float *wl = sh.w[1][w0 + i0 + i];
 #pragma unroll
-                                for (int j = 0; j < kPT; ++j) dot[j].add(w[j], wl[j], qh, ql);
+                                for (int j = 0; j < Q; ++j) dot[j].add(w[j], wl[j], qh, ql);
                             } else {
                                 const float v = __fadd_rn(qh, ql);
 #pragma unroll
-                                for (int j = 0; j < kPT; ++j) dot[j].add_tail(w[j], v);
+                                for (int j = 0; j < Q; ++j) dot[j].add_tail(w[j], v);
                             }
                         } else {
-                            const ulonglong2 *w2 = reinterpret_cast<const ulonglong2 *>(w);
-                            const ulonglong2 wa = w2[0], wb = w2[1];
+                            uint64_t ww[Q / 2];
+                            if constexpr (Q == 2) {
+                                ww[0] = *reinterpret_cast<const uint64_t *>(w);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < Q / 4; ++j) {
+                                    const ulonglong2 two = reinterpret_cast<const ulonglong2 *>(w)[j];
+                                    ww[2 * j] = two.x;
+                                    ww[2 * j + 1] = two.y;
+                                }
+                            }
                             auto products = [&](int s, float v) {
                                 const uint64_t vv = pair(v, v);
-                                fma2(part[s][0], wa.x, vv);
-                                fma2(part[s][1], wa.y, vv);
-                                fma2(part[s][2], wb.x, vv);
-                                fma2(part[s][3], wb.y, vv);
+#pragma unroll
+                                for (int j = 0; j < Q / 2; ++j) fma2(part[s][j], ww[j], vv);
                             };
                             if constexpr (kMax) {
                                 const uint32_t mx = q[i] & ~kSpanBit;
@@ -303,7 +315,7 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
                 __syncthreads();
                 store_weights();
                 ca = cb;
-                cb = min(ca + (uint32_t)kConvChunk, b);
+                cb = min(ca + (uint32_t)kConvChunk, b8);
                 __syncthreads();
                 if (cb < b) load_weights(cb);
                 if (kM2) core = meets_core();
@@ -318,9 +330,9 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
     flush();
     if (r < p.n_runs) {
 #pragma unroll
-        for (int j = 0; j < kPT; ++j) {
-            if (p0 + j >= p.P) continue;
-            double *o = p.acc + ((size_t)r * p.P + p0 + j) * 7;
+        for (int j = 0; j < Q; ++j) {
+            if (p0 + q0 + j >= p.P) continue;
+            double *o = p.acc + ((size_t)r * p.P + p0 + q0 + j) * 7;
             if constexpr (kM2) {
                 o[4] += dot[j].value();
             } else if constexpr (kMax) {
@@ -334,13 +346,32 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
     }
 }
 
+template <int S, int Q, bool SITE>
+void launch_q(const ConvParams &p, cudaStream_t s) {
+    dim3 grid((p.n_runs + kRuns - 1) / kRuns, (p.P + kPT - 1) / kPT * (kPT / Q));
+    if (sizeof(TileShared<S, Q>) > 48 * 1024)
+        cudaFuncSetAttribute(conv_tiles_kernel<S, Q, SITE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(TileShared<S, Q>));
+    conv_tiles_kernel<S, Q, SITE><<<grid, kRuns, sizeof(TileShared<S, Q>), s>>>(p);
+}
+
+// Probabilities per CTA.  Fewer make more CTAs, whose rows are fewer where the
+// bands lie apart, but load the records more often: 2 where a tile of 8 each
+// would leave SMs idle (1,000 runs of 300 x 300 at 50 p, 56 tiles: 9.8 ms with
+// 8, 4.1 with 4, 2.2 with 2), else 4 for max and m0 (11,000 us of all kernels at
+// L = 256 are 250 less), for m2 up to 8 tiles per SM (2,000 runs of 200 x 200 at
+// 301 p, 608 tiles: 911 us with 8, 755 with 4; 4,000 of 97 x 97, 2,016 tiles:
+// 853 and 891), and for m3 and m4 up to 2 (1,000 of 64 x 64, 304 tiles: 44 and
+// 45; 1,000 of 32 x 32, 208 tiles: 22 and 18).
 template <int S, bool SITE = false>
 void launch(const ConvParams &p, cudaStream_t s) {
-    dim3 grid((p.n_runs + kRuns - 1) / kRuns, (p.P + kPT - 1) / kPT);
-    if (sizeof(TileShared<S>) > 48 * 1024)
-        cudaFuncSetAttribute(conv_tiles_kernel<S, SITE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(TileShared<S>));
-    conv_tiles_kernel<S, SITE><<<grid, kRuns, sizeof(TileShared<S>), s>>>(p);
+    constexpr bool kWide = S == 5 || S == 6 || S == 7;
+    const int64_t tiles = (int64_t)((p.n_runs + kRuns - 1) / kRuns) * ((p.P + kPT - 1) / kPT);
+    if (tiles < 152) return launch_q<S, 2, SITE>(p, s);
+    if constexpr (kWide || TileShared<S, kPT>::kM2) {
+        if (tiles >= (kWide ? 2 : 8) * 152) return launch_q<S, kPT, SITE>(p, s);
+    }
+    launch_q<S, 4, SITE>(p, s);
 }
 
 }  // namespace
