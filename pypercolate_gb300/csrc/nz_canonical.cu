@@ -276,20 +276,20 @@ void launch_band_dot(const uint32_t *band_lo, const uint32_t *band_len, const do
 // =====================================================================
 // FP64 (the FP32 convolution of an ensemble's tiled records: nz_conv_tiles.cu)
 constexpr int kConvRuns = 128;  // runs per CTA (one per thread)
-constexpr int kConvPT = 8;      // probabilities per CTA
+constexpr int kConvPT = 8;      // most probabilities per CTA
 constexpr int kConvBatch = 16;  // record loads in flight per thread
 
 // grid: (run tiles, p tiles, 7 statistics).  Each thread accumulates the
-// kConvPT canonical values of its run for one statistic over the window's
+// PT canonical values of its run for one statistic over the window's
 // rows, with the tile's weights staged in shared memory (zero outside each
 // p's band), with FP64 products and sums.
-template <int S, bool SITE>
+template <int S, bool SITE, int PT>
 __device__ __forceinline__ void conv_rows(const ConvParams &p, uint32_t c0, uint32_t cn, int r,
-                                          const double (*s_w)[kConvPT],
+                                          const double (*s_w)[PT],
                                           double *acc) {
-    double part[kConvPT];
+    double part[PT];
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) part[j] = 0;
+    for (int j = 0; j < PT; ++j) part[j] = 0;
     const size_t base = (size_t)(c0 - p.n_begin) * p.rec.run_stride + r;
     // m1 = (sites in clusters) - max: N for bond records, n for site records
     auto value = [&](uint32_t i) -> double {
@@ -308,29 +308,29 @@ __device__ __forceinline__ void conv_rows(const ConvParams &p, uint32_t c0, uint
 #pragma unroll
         for (int b = 0; b < kConvBatch; ++b)
 #pragma unroll
-            for (int j = 0; j < kConvPT; ++j) part[j] = fma(s_w[i + b][j], q[b], part[j]);
+            for (int j = 0; j < PT; ++j) part[j] = fma(s_w[i + b][j], q[b], part[j]);
     }
     for (; i < cn; ++i) {
         const double q = value(i);
 #pragma unroll
-        for (int j = 0; j < kConvPT; ++j) part[j] = fma(s_w[i][j], q, part[j]);
+        for (int j = 0; j < PT; ++j) part[j] = fma(s_w[i][j], q, part[j]);
     }
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) acc[j] += part[j];
+    for (int j = 0; j < PT; ++j) acc[j] += part[j];
 }
 
 // Statistics 0 (spanning), 1 (max) and 3 (m1 = held - max) all come from the
 // max_span plane: one pass loads each word once and feeds the three sets of
 // products (each accumulator adds the same values in the same order as a
 // pass per statistic would).
-template <bool SITE>
+template <bool SITE, int PT>
 __device__ __forceinline__ void conv_rows_max(const ConvParams &p, uint32_t c0, uint32_t cn, int r,
-                                              const double (*s_w)[kConvPT],
+                                              const double (*s_w)[PT],
                                               double *acc0, double *acc1,
                                               double *acc3) {
-    double p0[kConvPT], p1[kConvPT], p3[kConvPT];
+    double p0[PT], p1[PT], p3[PT];
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) p0[j] = p1[j] = p3[j] = 0;
+    for (int j = 0; j < PT; ++j) p0[j] = p1[j] = p3[j] = 0;
     const size_t base = (size_t)(c0 - p.n_begin) * p.rec.run_stride + r;
     auto step = [&](uint32_t i, uint32_t ms) {
         const uint32_t held = SITE ? c0 + i : p.N;
@@ -338,7 +338,7 @@ __device__ __forceinline__ void conv_rows_max(const ConvParams &p, uint32_t c0, 
         const double q0 = (ms & kSpanBit) ? (double)1 : (double)0;
         const double q1 = (double)mx, q3 = (double)(held - mx);
 #pragma unroll
-        for (int j = 0; j < kConvPT; ++j) {
+        for (int j = 0; j < PT; ++j) {
             const double w = s_w[i][j];
             p0[j] = fma(w, q0, p0[j]);  // (dropped at the end without a spanning statistic)
             p1[j] = fma(w, q1, p1[j]);
@@ -355,7 +355,7 @@ __device__ __forceinline__ void conv_rows_max(const ConvParams &p, uint32_t c0, 
     }
     for (; i < cn; ++i) step(i, p.rec.max_span[base + (size_t)i * p.rec.run_stride]);
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) {
+    for (int j = 0; j < PT; ++j) {
         acc0[j] += p0[j];
         acc1[j] += p1[j];
         acc3[j] += p3[j];
@@ -409,27 +409,28 @@ __device__ __forceinline__ void for_groups(uint32_t groups, Load load, Step step
 
 // part[j] += the products of 8 rows, for the probabilities whose bands meet them
 // (bit j of `in`, the same for the whole block)
-__device__ __forceinline__ void add_group(const double (*w)[kConvPT], uint32_t in, const double (&v)[8],
-                                          double (&part)[kConvPT]) {
+template <int PT>
+__device__ __forceinline__ void add_group(const double (*w)[PT], uint32_t in, const double (&v)[8],
+                                          double (&part)[PT]) {
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) {
+    for (int j = 0; j < PT; ++j) {
         if (!(in >> j & 1u)) continue;
 #pragma unroll
         for (int b = 0; b < 8; ++b) part[j] = fma(w[b][j], v[b], part[j]);
     }
 }
 
-template <int S>
+template <int S, int PT>
 __device__ __forceinline__ void conv_rows_tiled(const ConvParams &p, uint32_t first, uint32_t groups, int r,
-                                                const double (*s_w)[kConvPT], const uint32_t *s_in,
+                                                const double (*s_w)[PT], const uint32_t *s_in,
                                                 double *acc) {
     struct Raw {
         tile_raw<S> q[8];
         uint32_t hi[S == 6 ? 8 : 1];
     };
-    double part[kConvPT];
+    double part[PT];
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) part[j] = 0;
+    for (int j = 0; j < PT; ++j) part[j] = 0;
     for_groups<Raw>(
         groups,
         [&](uint32_t k, Raw &q) {
@@ -440,23 +441,23 @@ __device__ __forceinline__ void conv_rows_tiled(const ConvParams &p, uint32_t fi
             double v[8];
 #pragma unroll
             for (int b = 0; b < 8; ++b) v[b] = tile_value<S>(q.q[b], S == 6 ? q.hi[S == 6 ? b : 0] : 0u);
-            add_group(s_w + 8 * k, s_in[k], v, part);
+            add_group<PT>(s_w + 8 * k, s_in[k], v, part);
         });
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) acc[j] += part[j];
+    for (int j = 0; j < PT; ++j) acc[j] += part[j];
 }
 
-template <bool SITE>
+template <bool SITE, int PT>
 __device__ __forceinline__ void conv_rows_max_tiled(const ConvParams &p, uint32_t first, uint32_t groups, int r,
-                                                    const double (*s_w)[kConvPT], const uint32_t *s_in,
+                                                    const double (*s_w)[PT], const uint32_t *s_in,
                                                     double *acc0, double *acc1,
                                                     double *acc3) {
     struct Raw {
         uint32_t q[8];
     };
-    double p0[kConvPT], p1[kConvPT], p3[kConvPT];
+    double p0[PT], p1[PT], p3[PT];
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) p0[j] = p1[j] = p3[j] = 0;
+    for (int j = 0; j < PT; ++j) p0[j] = p1[j] = p3[j] = 0;
     for_groups<Raw>(
         groups, [&](uint32_t k, Raw &q) { load_rows8(p.rec.max_span, p.rec.run_stride, first + 8 * k, r, q.q); },
         [&](uint32_t k, const Raw &q) {
@@ -467,27 +468,27 @@ __device__ __forceinline__ void conv_rows_max_tiled(const ConvParams &p, uint32_
                 flags |= q.q[b];
                 v[b] = (double)(q.q[b] & ~kSpanBit);
             }
-            add_group(s_w + 8 * k, s_in[k], v, p1);
+            add_group<PT>(s_w + 8 * k, s_in[k], v, p1);
 #pragma unroll
             for (int b = 0; b < 8; ++b)
                 v[b] = (double)((SITE ? p.n_begin + first + 8 * k + b : p.N) - (q.q[b] & ~kSpanBit));
-            add_group(s_w + 8 * k, s_in[k], v, p3);
+            add_group<PT>(s_w + 8 * k, s_in[k], v, p3);
             // spanning: rows without it add nothing (a third of the work below
             // the threshold)
             if (!p.spanning || !(flags & kSpanBit)) return;
 #pragma unroll
             for (int b = 0; b < 8; ++b) v[b] = (q.q[b] & kSpanBit) ? 1.0 : 0.0;
-            add_group(s_w + 8 * k, s_in[k], v, p0);
+            add_group<PT>(s_w + 8 * k, s_in[k], v, p0);
         });
 #pragma unroll
-    for (int j = 0; j < kConvPT; ++j) {
+    for (int j = 0; j < PT; ++j) {
         acc0[j] += p0[j];
         acc1[j] += p1[j];
         acc3[j] += p3[j];
     }
 }
 
-// Each thread accumulates the kConvPT canonical values of its run over the
+// Each thread accumulates the PT canonical values of its run over the
 // window's rows, with the tile's weights staged in shared memory (zero
 // outside each p's band), in FP64.
 // MAXSET: grid (run tiles, p tiles, 1), statistics 0, 1 and 3 from the
@@ -495,19 +496,19 @@ __device__ __forceinline__ void conv_rows_max_tiled(const ConvParams &p, uint32_
 // statistics 2, 4, 5, 6 (one per z).
 enum class Layout { kBond, kSite, kTiled, kTiledSite };  // records of bonds or sites, n-major or tiled
 
-template <Layout LAYOUT, bool MAXSET>
+template <Layout LAYOUT, bool MAXSET, int PT>
 __global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
     constexpr bool SITE = LAYOUT == Layout::kSite || LAYOUT == Layout::kTiledSite;
     constexpr bool TILED = LAYOUT == Layout::kTiled || LAYOUT == Layout::kTiledSite;
-    __shared__ double s_w[kConvChunk + (TILED ? 8 : 0)][kConvPT];
-    __shared__ uint32_t s_lo[kConvPT], s_len[kConvPT];
+    __shared__ double s_w[kConvChunk + (TILED ? 8 : 0)][PT];
+    __shared__ uint32_t s_lo[PT], s_len[PT];
     __shared__ uint32_t s_range[2];
     __shared__ uint32_t s_in[TILED ? kConvChunk / 8 + 1 : 1];  // probabilities whose bands meet the 8-row group
     const int r = blockIdx.x * kConvRuns + threadIdx.x;
-    const int p0 = blockIdx.y * kConvPT;
+    const int p0 = blockIdx.y * PT;
     constexpr int kOther[4] = {2, 4, 5, 6};
     const int s = MAXSET ? 1 : kOther[blockIdx.z];
-    if (threadIdx.x < kConvPT) {
+    if (threadIdx.x < PT) {
         const int pi = p0 + threadIdx.x;
         s_lo[threadIdx.x] = pi < p.P ? p.band_lo[pi] : 0u;
         s_len[threadIdx.x] = pi < p.P ? p.band_len[pi] : 0u;
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t a = 0xffffffffu, b = 0;
-        for (int j = 0; j < kConvPT; ++j)
+        for (int j = 0; j < PT; ++j)
             if (s_len[j]) { a = min(a, s_lo[j]); b = max(b, s_lo[j] + s_len[j]); }
         a = max(a, p.n_begin);
         b = min(b, p.n_end);
@@ -524,14 +525,14 @@ __global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
     __syncthreads();
     const uint32_t nlo = s_range[0], nhi = s_range[1];
     if (nlo >= nhi) return;
-    double acc[kConvPT] = {}, acc0[MAXSET ? kConvPT : 1] = {}, acc3[MAXSET ? kConvPT : 1] = {};
+    double acc[PT] = {}, acc0[MAXSET ? PT : 1] = {}, acc3[MAXSET ? PT : 1] = {};
     for (uint32_t c0 = nlo; c0 < nhi; c0 += kConvChunk) {
         const uint32_t cn = min((uint32_t)kConvChunk, nhi - c0);
         // tiled: rows of the 8-row group that holds c0 come first
         const uint32_t lead = TILED ? (c0 - p.n_begin) & 7u : 0u;
         __syncthreads();
-        for (int i = threadIdx.x; i < (kConvChunk + (TILED ? 8 : 0)) * kConvPT; i += kConvRuns) {
-            const int row = i / kConvPT, j = i % kConvPT;
+        for (int i = threadIdx.x; i < (kConvChunk + (TILED ? 8 : 0)) * PT; i += kConvRuns) {
+            const int row = i / PT, j = i % PT;
             const uint32_t n = c0 + row - lead;
             double v = 0;
             if ((uint32_t)row - lead < cn && n >= s_lo[j] && n < s_lo[j] + s_len[j]) {
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
             // window rows and chunk rows of the group, then of each band
             const uint32_t a = max(c0, c0 - lead + 8u * threadIdx.x), b = min(c0 + cn, c0 - lead + 8u * threadIdx.x + 8u);
             uint32_t in = 0;
-            for (int j = 0; j < kConvPT; ++j)
+            for (int j = 0; j < PT; ++j)
                 if (s_len[j] && a < b && s_lo[j] < b && a < s_lo[j] + s_len[j]) in |= 1u << j;
             s_in[threadIdx.x] = in;
         }
@@ -553,37 +554,37 @@ __global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
             if (r < p.n_runs) {
                 const uint32_t first = c0 - p.n_begin - lead, groups = (lead + cn + 7u) / 8u;
                 if (MAXSET) {
-                    conv_rows_max_tiled<SITE>(p, first, groups, r, s_w, s_in, acc0, acc, acc3);
+                    conv_rows_max_tiled<SITE, PT>(p, first, groups, r, s_w, s_in, acc0, acc, acc3);
                 } else if (s == 2) {
-                    if (p.rec.narrow) conv_rows_tiled<8>(p, first, groups, r, s_w, s_in, acc);
-                    else conv_rows_tiled<2>(p, first, groups, r, s_w, s_in, acc);
+                    if (p.rec.narrow) conv_rows_tiled<8, PT>(p, first, groups, r, s_w, s_in, acc);
+                    else conv_rows_tiled<2, PT>(p, first, groups, r, s_w, s_in, acc);
                 } else if (s == 4) {
-                    if (p.rec.narrow) conv_rows_tiled<9>(p, first, groups, r, s_w, s_in, acc);
-                    else conv_rows_tiled<4>(p, first, groups, r, s_w, s_in, acc);
+                    if (p.rec.narrow) conv_rows_tiled<9, PT>(p, first, groups, r, s_w, s_in, acc);
+                    else conv_rows_tiled<4, PT>(p, first, groups, r, s_w, s_in, acc);
                 } else if (s == 5) {
-                    conv_rows_tiled<5>(p, first, groups, r, s_w, s_in, acc);
+                    conv_rows_tiled<5, PT>(p, first, groups, r, s_w, s_in, acc);
                 } else {
-                    if (p.rec.m4_hi) conv_rows_tiled<6>(p, first, groups, r, s_w, s_in, acc);
-                    else conv_rows_tiled<7>(p, first, groups, r, s_w, s_in, acc);
+                    if (p.rec.m4_hi) conv_rows_tiled<6, PT>(p, first, groups, r, s_w, s_in, acc);
+                    else conv_rows_tiled<7, PT>(p, first, groups, r, s_w, s_in, acc);
                 }
             }
         } else if (r < p.n_runs) {
             if (MAXSET) {
-                conv_rows_max<SITE>(p, c0, cn, r, s_w, acc0, acc, acc3);
+                conv_rows_max<SITE, PT>(p, c0, cn, r, s_w, acc0, acc, acc3);
             } else {
                 switch (s) {
                     case 2:
-                        if (p.rec.narrow) conv_rows<8, SITE>(p, c0, cn, r, s_w, acc);
-                        else conv_rows<2, SITE>(p, c0, cn, r, s_w, acc);
+                        if (p.rec.narrow) conv_rows<8, SITE, PT>(p, c0, cn, r, s_w, acc);
+                        else conv_rows<2, SITE, PT>(p, c0, cn, r, s_w, acc);
                         break;
                     case 4:
-                        if (p.rec.narrow) conv_rows<9, SITE>(p, c0, cn, r, s_w, acc);
-                        else conv_rows<4, SITE>(p, c0, cn, r, s_w, acc);
+                        if (p.rec.narrow) conv_rows<9, SITE, PT>(p, c0, cn, r, s_w, acc);
+                        else conv_rows<4, SITE, PT>(p, c0, cn, r, s_w, acc);
                         break;
-                    case 5: conv_rows<5, SITE>(p, c0, cn, r, s_w, acc); break;
+                    case 5: conv_rows<5, SITE, PT>(p, c0, cn, r, s_w, acc); break;
                     default:
-                        if (p.rec.m4_hi) conv_rows<6, SITE>(p, c0, cn, r, s_w, acc);
-                        else conv_rows<7, SITE>(p, c0, cn, r, s_w, acc);
+                        if (p.rec.m4_hi) conv_rows<6, SITE, PT>(p, c0, cn, r, s_w, acc);
+                        else conv_rows<7, SITE, PT>(p, c0, cn, r, s_w, acc);
                         break;
                 }
             }
@@ -591,7 +592,7 @@ __global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
     }
     if (r < p.n_runs) {
 #pragma unroll
-        for (int j = 0; j < kConvPT; ++j) {
+        for (int j = 0; j < PT; ++j) {
             const int pi = p0 + j;
             if (pi >= p.P) continue;
             double *o = p.acc + ((size_t)r * p.P + pi) * 7;
@@ -610,15 +611,11 @@ bool conv_grid_fits(int32_t n_runs, int32_t P) {
     return n_runs > 0 && P > 0 && (P + kConvPT - 1) / kConvPT <= 65535;
 }
 
-void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
-    if (p.n_runs <= 0 || p.P <= 0) return;
-    if (precision != 0) {  // ensembles only: tiled records
-        launch_conv_tiles(p, s);
-        return;
-    }
+template <int PT>
+static void launch_conv_fp64(const ConvParams &p, cudaStream_t s) {
     // (run tiles, p tiles, statistics); launching the p tiles of one run tile
     // back to back (for L2 reuse of its records) measured slower
-    dim3 gmax((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + kConvPT - 1) / kConvPT, 1);
+    dim3 gmax((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + PT - 1) / PT, 1);
     dim3 gother(gmax.x, gmax.y, 4);
     // the record model is a template parameter: a run-time test in the row
     // loop cost 17 % of the kernel's time
@@ -627,13 +624,29 @@ void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
         others<<<gother, kConvRuns, 0, s>>>(p);
     };
     if (p.tiled && p.rec.site)
-        launch(conv_window_kernel<Layout::kTiledSite, true>, conv_window_kernel<Layout::kTiledSite, false>);
+        launch(conv_window_kernel<Layout::kTiledSite, true, PT>, conv_window_kernel<Layout::kTiledSite, false, PT>);
     else if (p.tiled)
-        launch(conv_window_kernel<Layout::kTiled, true>, conv_window_kernel<Layout::kTiled, false>);
+        launch(conv_window_kernel<Layout::kTiled, true, PT>, conv_window_kernel<Layout::kTiled, false, PT>);
     else if (p.rec.site)
-        launch(conv_window_kernel<Layout::kSite, true>, conv_window_kernel<Layout::kSite, false>);
+        launch(conv_window_kernel<Layout::kSite, true, PT>, conv_window_kernel<Layout::kSite, false, PT>);
     else
-        launch(conv_window_kernel<Layout::kBond, true>, conv_window_kernel<Layout::kBond, false>);
+        launch(conv_window_kernel<Layout::kBond, true, PT>, conv_window_kernel<Layout::kBond, false, PT>);
+}
+
+void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
+    if (p.n_runs <= 0 || p.P <= 0) return;
+    if (precision != 0) {  // ensembles only: tiled records
+        launch_conv_tiles(p, s);
+        return;
+    }
+    // Fewer probabilities per CTA, so more CTAs, where tiles of 8 leave SMs idle
+    // (whole ensembles in ms with 8, 4, 2: 200 runs of 200 x 200 at 100 p, 26
+    // tiles, 8.4, 5.5, 4.2; 1,000 toruses of 64 x 64 at 101 p, 104 tiles, 3.0,
+    // 2.6, 2.6; 1,000 grids of 128 x 128 at 201 p, 208 tiles, 8.6, 8.5, 8.8).
+    const int64_t tiles = (int64_t)((p.n_runs + kConvRuns - 1) / kConvRuns) * ((p.P + kConvPT - 1) / kConvPT);
+    if (tiles < 64) launch_conv_fp64<2>(p, s);
+    else if (tiles < 152) launch_conv_fp64<4>(p, s);
+    else launch_conv_fp64<kConvPT>(p, s);
 }
 
 // Weights of the FP32 convolution: the part of each p's band whose weights

@@ -281,3 +281,19 @@ def test_convolution_of_many_and_few_probabilities(gpu, kind, L, model):
         got.append(e.mean.cpu().numpy().reshape(P, -1)[:16])
     assert np.isfinite(got[0]).all()
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+@pytest.mark.parametrize('kind,L,model,runs', [('grid', 24, 'bond', 130), ('torus', 20, 'site', 300),
+                                               ('chain', 3000, 'bond', 5)])
+def test_fp64_convolution_of_many_and_few_probabilities(gpu, kind, L, model, runs):
+    from pypercolate_gb300.ensemble import Ensemble
+    got = []
+    for P in (16, 300, 5000):  # 2, 2 or 4, 8 probabilities per thread block
+        ps = np.concatenate([np.linspace(0.02, 0.97, 16), np.linspace(0.4, 0.6, P - 16)])
+        e = Ensemble(kind, L, ps, precision='fp64', model=model)
+        e.run(runs, key=3)
+        assert e.errors() == 0
+        got.append(e.mean.cpu().numpy().reshape(P, -1)[:16])
+    # FP64 sums of < 2^12 non-negative terms in another order
+    np.testing.assert_allclose(got[1], got[0], rtol=1e-12)
+    np.testing.assert_allclose(got[2], got[0], rtol=1e-12)
