@@ -19,7 +19,7 @@
 // band keep ~2^-44 relative accuracy without FP64, whose rate on this chip is
 // 1/64 of FP32).  Shared memory and TMEM accumulators are double-buffered.
 // m2 (the susceptibility, which needs ~5e-11 relative per run) is not done
-// here: the launcher adds the compensated SIMT kernel of nz_canonical.cu.
+// here: the launcher adds the compensated kernel of nz_conv_tiles.cu.
 //
 // Reference: the products and sums of bond_canonical_statistics
 // (percolate/hpc.py:443-515), sum_n B(M, n, p) Q_n per statistic.
@@ -68,7 +68,7 @@ struct TcShared {
     uint64_t mbar[2];               // MMAs of the chunk in each stage done
     uint32_t tmem;                  // TMEM base address
     uint32_t lo[kTcP], len[kTcP];   // FP32 bands of the CTA's probabilities
-    uint32_t range[2];
+    uint32_t range[2];              // rows of the CTA
 };
 
 // Instruction descriptor of tcgen05.mma kind::tf32: D FP32 (bits 4-5 = 1),
@@ -203,8 +203,9 @@ __device__ __forceinline__ float raw_value(raw_word<S> w, uint32_t hi, uint32_t 
 }
 
 // One CTA's tile for statistic S (7 = m4 without its high-word plane).
-template <int S, bool SITE>
-__device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, int p0, uint32_t nlo, uint32_t nhi) {
+template <int S, bool SITE, bool SPLIT>
+__device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, int p0, uint32_t nlo, uint32_t nhi, int j0,
+                                             int own) {
     const int t = threadIdx.x, warp = t >> 5;
     const int r = blockIdx.x * kTcRuns + t;
     const bool live = r < p.n_runs;
@@ -361,7 +362,7 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
         double *o = p.acc + (size_t)r * p.P * 7;
 #pragma unroll
         for (int j = 0; j < kTcP; ++j)
-            if (p0 + j < p.P) o[(size_t)(p0 + j) * 7 + out] += (double)acc_s[j] + (double)acc_c[j];
+            if ((!SPLIT || (j >= j0 && j < j0 + own)) && p0 + j < p.P) o[(size_t)(p0 + j) * 7 + out] += (double)acc_s[j] + (double)acc_c[j];
     }
 }
 
@@ -370,8 +371,8 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
 // high words; HI = true: m4 with its high words alone (its wider loads would
 // otherwise set the register count of every statistic's code).  m2 (4) runs
 // on the compensated SIMT kernel.
-template <bool SITE, bool HI>
-__global__ void __launch_bounds__(kTcRuns) conv_tc_kernel(ConvParams p) {
+template <bool SITE, bool HI, bool SPLIT>
+__global__ void __launch_bounds__(kTcRuns) conv_tc_kernel(ConvParams p, int split) {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     TcShared &sh = *reinterpret_cast<TcShared *>(tc_smem);
     // statistic of this z: m2 (4) runs on the compensated SIMT kernel
@@ -379,7 +380,8 @@ __global__ void __launch_bounds__(kTcRuns) conv_tc_kernel(ConvParams p) {
     constexpr int kStat[6] = {0, 1, 2, 3, 5, 6};
     const int z = kStat[blockIdx.z];
     if (!HI && z == 0 && !p.spanning) return;
-    const int p0 = blockIdx.y * kTcP;
+    const int p0 = SPLIT ? (int)blockIdx.y / split * kTcP : (int)blockIdx.y * kTcP;
+    const int own = SPLIT ? kTcP / split : kTcP, j0 = SPLIT ? (int)blockIdx.y % split * own : 0;  // of its tile
     if (threadIdx.x < kTcP) {
         const int pi = p0 + threadIdx.x;
         sh.lo[threadIdx.x] = pi < p.P ? p.band_lo[pi] : 0u;
@@ -387,52 +389,76 @@ __global__ void __launch_bounds__(kTcRuns) conv_tc_kernel(ConvParams p) {
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t a = 0xffffffffu, b = 0;
+        uint32_t a = 0xffffffffu, b = 0, first = 0xffffffffu;
         for (int j = 0; j < kTcP; ++j)
-            if (sh.len[j]) { a = min(a, sh.lo[j]); b = max(b, sh.lo[j] + sh.len[j]); }
-        sh.range[0] = max(a, p.n_begin);
-        sh.range[1] = min(b, p.n_end);
+            if (sh.len[j]) {
+                first = min(first, sh.lo[j]);
+                if (SPLIT && (j < j0 || j >= j0 + own)) sh.len[j] = 0;  // another CTA's: no weights here
+                else { a = min(a, sh.lo[j]); b = max(b, sh.lo[j] + sh.len[j]); }
+            }
+        first = max(first, p.n_begin);
+        a = max(a, p.n_begin);
+        b = min(b, p.n_end);
+        // chunks and drains are counted from the tile's first row, so that the
+        // sums do not depend on the split
+        if (SPLIT && a < b) a = first + (a - first) / (kTcK * kTcDrain) * (kTcK * kTcDrain);
+        sh.range[0] = a;
+        sh.range[1] = b;
     }
     __syncthreads();
     const uint32_t nlo = sh.range[0], nhi = sh.range[1];
     if (nlo >= nhi) return;
     if (HI) {
-        conv_tc_tile<6, SITE>(p, sh, p0, nlo, nhi);
+        conv_tc_tile<6, SITE, SPLIT>(p, sh, p0, nlo, nhi, j0, own);
         return;
     }
     switch (z) {
-        case 0: conv_tc_tile<0, SITE>(p, sh, p0, nlo, nhi); break;
-        case 1: conv_tc_tile<1, SITE>(p, sh, p0, nlo, nhi); break;
+        case 0: conv_tc_tile<0, SITE, SPLIT>(p, sh, p0, nlo, nhi, j0, own); break;
+        case 1: conv_tc_tile<1, SITE, SPLIT>(p, sh, p0, nlo, nhi, j0, own); break;
         case 2:
-            if (p.rec.narrow) conv_tc_tile<8, SITE>(p, sh, p0, nlo, nhi);
-            else conv_tc_tile<2, SITE>(p, sh, p0, nlo, nhi);
+            if (p.rec.narrow) conv_tc_tile<8, SITE, SPLIT>(p, sh, p0, nlo, nhi, j0, own);
+            else conv_tc_tile<2, SITE, SPLIT>(p, sh, p0, nlo, nhi, j0, own);
             break;
-        case 3: conv_tc_tile<3, SITE>(p, sh, p0, nlo, nhi); break;
-        case 5: conv_tc_tile<5, SITE>(p, sh, p0, nlo, nhi); break;
-        default: conv_tc_tile<7, SITE>(p, sh, p0, nlo, nhi); break;
+        case 3: conv_tc_tile<3, SITE, SPLIT>(p, sh, p0, nlo, nhi, j0, own); break;
+        case 5: conv_tc_tile<5, SITE, SPLIT>(p, sh, p0, nlo, nhi, j0, own); break;
+        default: conv_tc_tile<7, SITE, SPLIT>(p, sh, p0, nlo, nhi, j0, own); break;
     }
 }
 
-template <bool SITE, bool HI>
-cudaError_t launch_tc_k(const ConvParams &p, unsigned stats, cudaStream_t s) {
+template <bool SITE, bool HI, bool SPLIT>
+cudaError_t launch_tc_k(const ConvParams &p, unsigned stats, int split, cudaStream_t s) {
     // above 48 KB of dynamic shared memory (32-row chunks) the launch needs
     // the attribute, which belongs to the function in the current device's
     // context: set it before every such launch
     if constexpr (sizeof(TcShared) > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(conv_tc_kernel<SITE, HI>,
+        const cudaError_t e = cudaFuncSetAttribute(conv_tc_kernel<SITE, HI, SPLIT>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcShared));
         if (e != cudaSuccess) return e;
     }
-    dim3 grid((p.n_runs + kTcRuns - 1) / kTcRuns, (p.P + kTcP - 1) / kTcP, stats);
-    conv_tc_kernel<SITE, HI><<<grid, kTcRuns, sizeof(TcShared), s>>>(p);
+    const int runs = (p.n_runs + kTcRuns - 1) / kTcRuns, tiles = (p.P + kTcP - 1) / kTcP;
+    conv_tc_kernel<SITE, HI, SPLIT><<<dim3(runs, tiles * split, stats), kTcRuns, sizeof(TcShared), s>>>(p, split);
     return cudaGetLastError();
+}
+
+// Few tiles (of 128 runs x 32 probabilities) leave SMs idle while each walks
+// through the rows of 32 bands: a tile's probabilities are then shared out over
+// `split` CTAs, which need not read the rows of the others' bands.  (us with split
+// 1, 2, 4, 8: m4 with its high words, 200 runs of 512 x 512 at 501 p, 32 tiles,
+// 4,830, 2,710, 1,660, 1,290, 1,000 of 400 x 400 at 200 p, 56 tiles, 6,670, 3,550,
+// 2,130, 2,000; the others together 3,760, 3,400, 2,930, 3,310 and 5,480, 5,860,
+// 5,730, 5,690; at 50 p, 4 tiles, 25,400, 17,100, 8,250, 3,840.)
+template <bool SITE, bool HI>
+cudaError_t launch_tc_s(const ConvParams &p, unsigned stats, cudaStream_t s) {
+    const int64_t tiles = (int64_t)((p.n_runs + kTcRuns - 1) / kTcRuns) * ((p.P + kTcP - 1) / kTcP);
+    const int split = HI ? (tiles <= 64 ? 8 : tiles <= 128 ? 4 : 1) : (tiles <= 16 ? 8 : tiles <= 32 ? 4 : 1);
+    return split > 1 ? launch_tc_k<SITE, HI, true>(p, stats, split, s) : launch_tc_k<SITE, HI, false>(p, stats, 1, s);
 }
 
 template <bool SITE>
 cudaError_t launch_tc(const ConvParams &p, cudaStream_t s) {
-    if (!p.rec.m4_hi) return launch_tc_k<SITE, false>(p, 6, s);
-    const cudaError_t e = launch_tc_k<SITE, false>(p, 5, s);
-    return e != cudaSuccess ? e : launch_tc_k<SITE, true>(p, 1, s);
+    if (!p.rec.m4_hi) return launch_tc_s<SITE, false>(p, 6, s);
+    const cudaError_t e = launch_tc_s<SITE, false>(p, 5, s);
+    return e != cudaSuccess ? e : launch_tc_s<SITE, true>(p, 1, s);
 }
 
 }  // namespace

@@ -267,18 +267,20 @@ def test_site_windows(gpu, kind, L, window, precision):
     np.testing.assert_allclose(ma, mb, rtol=1e-12 if precision == 'fp64' else 2e-5)
 
 
+@pytest.mark.parametrize('precision', ['fp32', 'tf32x3'])
 @pytest.mark.parametrize('kind,L,model', [('grid', 24, 'bond'), ('grid', 90, 'site'), ('grid', 345, 'bond'),
                                           ('chain', 3000, 'bond')])
-def test_convolution_of_many_and_few_probabilities(gpu, kind, L, model):
-    """2, 4 or 8 probabilities per thread block: the same bits."""
+def test_convolution_of_many_and_few_probabilities(gpu, kind, L, model, precision):
+    """2, 4 or 8 (on the tensor cores 4, 8 or 32) probabilities per thread
+    block: the same bits."""
     from pypercolate_gb300.ensemble import Ensemble
     got = []
-    for P in (16, 1000, 5000):
-        ps = np.concatenate([np.linspace(0.02, 0.97, 16), np.linspace(0.4, 0.6, P - 16)])
-        e = Ensemble(kind, L, ps, precision='fp32', model=model, window=0 if L != 24 else 200)
+    for P in (32, 1000, 5000):
+        ps = np.concatenate([np.linspace(0.02, 0.97, 32), np.linspace(0.4, 0.6, P - 32)])
+        e = Ensemble(kind, L, ps, precision=precision, model=model, window=0 if L != 24 else 200)
         e.run(130, key=3)
         assert e.errors() == 0
-        got.append(e.mean.cpu().numpy().reshape(P, -1)[:16])
+        got.append(e.mean.cpu().numpy().reshape(P, -1)[:32])
     assert np.isfinite(got[0]).all()
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
 
