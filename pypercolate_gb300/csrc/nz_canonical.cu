@@ -39,7 +39,7 @@ __device__ __forceinline__ double log_binom_shape(uint32_t M, uint32_t n, double
 template <int BLOCK>
 __device__ void band_weights_block(uint32_t M, double p, double cutoff, int32_t cap, double *wp, uint32_t &lo_out,
                                    uint32_t &len_out, bool &overflow) {
-    __shared__ double s_scan[BLOCK / 32];
+    __shared__ double s_scan[2][BLOCK];
     __shared__ double s_red[BLOCK];
     __shared__ uint32_t s_lo, s_hi;
     if (threadIdx.x == 0) {
@@ -76,37 +76,31 @@ __device__ void band_weights_block(uint32_t M, double p, double cutoff, int32_t 
         __syncthreads();
         return;
     }
-    const double odds = p / (1.0 - p), lpq = log(p) - log1p(-p);
-    const bool direct = odds > 1e-290;  // (below, odds or its product may lose bits)
-    // pass 1: log weights relative to the low edge (prefix scan of log ratios)
-    // -- one logarithm of the ratio itself, within 2^-53 of it, instead of three
-    // whose sum keeps the rounding of terms near 10
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double lpq = log(p) - log1p(-p);
+    // pass 1: log weights relative to the low edge (prefix scan of log ratios, in
+    // two buffers by turns: a barrier a step)
     double carry = 0.0;
     double vmax = -INFINITY;
+    int buf = 0;
     for (uint32_t base = 0; base < len; base += BLOCK) {
         const uint32_t j = base + threadIdx.x;
         double x = 0.0;
         if (j > 0 && j < len) {
             const double n = (double)(lo + j);
-            const double ratio = ((double)M - n + 1.0) / n;
-            x = direct ? log(ratio * odds) : log(ratio) + lpq;
+            x = log((double)M - n + 1.0) - log(n) + lpq;
         }
-        for (int off = 1; off < 32; off <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
+        for (int off = 1; off < BLOCK; off <<= 1) {  // Hillis-Steele inclusive scan
+            s_scan[buf][threadIdx.x] = x;
+            __syncthreads();
+            if (threadIdx.x >= (unsigned)off) x += s_scan[buf][threadIdx.x - off];
+            buf ^= 1;
         }
-        if (lane == 31) s_scan[warp] = x;
+        s_scan[buf][threadIdx.x] = x;
         __syncthreads();
-        double before = 0.0, all = 0.0;  // the earlier warps' sums, and all of them
-        for (int q = 0; q < BLOCK / 32; ++q) {
-            if (q == warp) before = all;
-            all += s_scan[q];
-        }
-        const double lv = carry + before + x;
+        const double lv = carry + x;
         if (j < len) { wp[j] = lv; vmax = fmax(vmax, lv); }
-        carry += all;
-        __syncthreads();
+        carry += s_scan[buf][BLOCK - 1];
+        buf ^= 1;
     }
     s_red[threadIdx.x] = vmax;
     __syncthreads();
@@ -520,6 +514,15 @@ __global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
             if (s_len[j]) { a = min(a, s_lo[j]); b = max(b, s_lo[j] + s_len[j]); }
         a = max(a, p.n_begin);
         b = min(b, p.n_end);
+        // chunks are counted from the first row of kConvPT probabilities, so
+        // that the sums do not depend on PT
+        if (PT < kConvPT && a < b) {
+            uint32_t first = a;
+            for (int pi = p0 / kConvPT * kConvPT; pi < min(p.P, p0 / kConvPT * kConvPT + kConvPT); ++pi)
+                if (p.band_len[pi]) first = min(first, p.band_lo[pi]);
+            first = max(first, p.n_begin);
+            a = first + (a - first) / kConvChunk * kConvChunk;
+        }
         s_range[0] = a; s_range[1] = b;
     }
     __syncthreads();

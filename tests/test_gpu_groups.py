@@ -296,6 +296,4 @@ def test_fp64_convolution_of_many_and_few_probabilities(gpu, kind, L, model, run
         e.run(runs, key=3)
         assert e.errors() == 0
         got.append(e.mean.cpu().numpy().reshape(P, -1)[:16])
-    # FP64 sums of < 2^12 non-negative terms in another order
-    np.testing.assert_allclose(got[1], got[0], rtol=1e-12)
-    np.testing.assert_allclose(got[2], got[0], rtol=1e-12)
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
