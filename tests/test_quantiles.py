@@ -79,3 +79,19 @@ def test_t_quantiles(fns):
     q, v = (w.ravel() for w in np.meshgrid([0.025, 0.975, 0.15865, 0.51, 1e-7], v))
     out = fns('tq', q, v, np.empty(q.size))[-1]
     np.testing.assert_allclose(out, st.t.ppf(q, v), rtol=1e-8)
+
+
+@pytest.mark.parametrize('tail', [0.4, 0.15865, 0.025, 0.0005])
+@pytest.mark.parametrize('v', [400, 700, 2000, 9999])
+def test_t_expansion_where_it_applies(fns, tail, v):
+    """Five terms leave < 1e-15; some ten roundings of 2^-53 and the normal
+    quantile's own on top: < 1e-14.  (Tails of 0.0005 at v = 400 and 700 are
+    iterated, with lgamma's 1e-13 of the prefactor.)"""
+    mp = pytest.importorskip('mpmath')
+    got = fns('tq', [1.0 - tail], [v], np.empty(1))[-1][0]
+    with mp.workdps(30):
+        tail = mp.mpf(1.0) - mp.mpf(1.0 - tail)
+        z = mp.sqrt(2) * mp.erfinv(1 - 2 * tail)
+        want = mp.findroot(lambda t: mp.betainc(mp.mpf(v) / 2, mp.mpf(1) / 2, 0, v / (v + t * t),
+                                                regularized=True) / 2 - tail, z * (1 + (z * z + 1) / (4 * v)))
+        assert abs(got / want - 1) < (1e-14 if tail > 0.001 or v >= 2000 else 1e-12)
