@@ -28,22 +28,20 @@ sys.path.insert(0, REPO)
 L_DEFAULT = 256
 P_DEFAULT = 1001
 KEY = 1234
-# algorithmic DRAM bytes per bond addition of the union-find kernel: four
-# random 32-byte sectors (find(u), find(v), the child pointer and the root
-# word written on a union) plus the per-step record it streams
+# algorithmic DRAM bytes per bond addition of the union-find kernel: the
+# per-step record it streams.  Up to N = 65,536 nodes the node words of a run
+# live in shared memory; beyond, in global memory, near L2's size for the runs
+# that are resident
 
 
 def uf_bytes_per_add(N):
-    """4 x 32 B plus the record the ensemble writes per step: 26 B up to
-    N = 65,536 nodes (m0 and m2 narrow), 32 B up to 115,000 (no m4 high
-    words), 36 B above."""
-    return 4 * 32 + (26 if N <= 65536 else 32 if N <= 115000 else 36)
-# measured DRAM bytes (read + write) per bond addition of uf_window_kernel:
-# ncu capture of spanning_2d_grid(256), 12,288 runs, one 1,024-row window at
-# p ~ 0.5; a full launch's traffic is this figure times the additions it
-# makes
-UF_TRAFFIC_PER_ADD = 177.3
-UF_READ_PER_ADD = 90.6  # of which read (the scattered finds)
+    """The record the ensemble writes per step: 26 B up to N = 65,536 nodes
+    (m0 and m2 narrow), 32 B up to 115,000 (no m4 high words), 36 B above."""
+    return 26 if N <= 65536 else 32 if N <= 115000 else 36
+# measured DRAM bytes (read + write) per bond addition of uf_group_kernel:
+# ncu capture of spanning_2d_grid(256), 608 runs in one window of all rows; a
+# full launch's traffic is this figure times the additions it makes
+UF_TRAFFIC_PER_ADD = 25.3
 
 
 def bench_window(M, R, window):
@@ -204,34 +202,6 @@ def peaks():
         d = json.load(open(path))
         return float(d['hbm_gbs']), 'measured'
     return 6800.0, 'fallback'
-
-
-def random_gather_rate(gib=16, k=1 << 28, reps=3):
-    """Random-access ceiling of this GPU's HBM: 4-byte gathers at uniformly
-    random positions of a `gib` GiB array (far larger than L2), each touching
-    its own 32-byte sector; returns sectors (gathers) per second, best of
-    `reps` (CUDA events).  The union-find's finds are such accesses."""
-    import torch
-    n = (gib << 30) // 4
-    a = torch.zeros(n, dtype=torch.int32, device='cuda')
-    gen = torch.Generator(device='cuda')
-    gen.manual_seed(7)
-    idx = torch.randint(0, n, (k,), device='cuda', generator=gen)
-    out = torch.empty(k, dtype=torch.int32, device='cuda')
-    torch.index_select(a, 0, idx, out=out)
-    best = None
-    for _ in range(reps):
-        e0 = torch.cuda.Event(enable_timing=True)
-        e1 = torch.cuda.Event(enable_timing=True)
-        e0.record()
-        torch.index_select(a, 0, idx, out=out)
-        e1.record()
-        torch.cuda.synchronize()
-        t = e0.elapsed_time(e1) * 1e-3
-        best = t if best is None else min(best, t)
-    del a, idx, out
-    torch.cuda.empty_cache()
-    return k / best
 
 
 class ClockSampler:
@@ -591,16 +561,15 @@ def main():
     achieved = uf_bytes * adds_per_launch / uf_avg_s / 1e9
     peak, peak_kind = peaks()
     launches = {k: v[0] for k, v in prof.items()}
-    # second ceiling for the union-find: HBM's rate of scattered sector reads
-    gather_rate = random_gather_rate()
     uf_adds_per_s = adds_per_launch / uf_avg_s
-    # kernels per profiled launch sequence: set-up (band weights, FP32
-    # weights, node and state initialisation), union-find, micro reductions,
-    # convolution (FP32: max-set, other statistics, compensated m2; tf32x3:
-    # tcgen05 kernel, compensated m2; FP64: max-set, other statistics),
-    # reduction (micro count, two run-reduction passes, count)
-    kernels_per_seq = {'setup': 3 if args.precision == 'fp64' else 4, 'union_find': 1, 'micro': 1,
-                       'conv': {'fp32': 3, 'tf32x3': 2, 'fp64': 2}[args.precision], 'reduce': 4}
+    # kernels per profiled launch sequence: set-up (counted on two streams:
+    # band weights, FP32 weights), union-find, micro reductions, convolution
+    # (FP32: max-set, m0, m3, m4, m2; tf32x3: tcgen05 kernel, twice with m4
+    # high words, m2; FP64: max-set, other statistics), reduction (micro count,
+    # two run-reduction passes, count)
+    kernels_per_seq = {'setup': 0.5 if args.precision == 'fp64' else 1, 'union_find': 1, 'micro': 1,
+                       'conv': {'fp32': 5, 'tf32x3': 2 if N <= 115000 else 3, 'fp64': 2}[args.precision],
+                       'reduce': 4}
     gpu_launches = int(sum(launches[k] * kernels_per_seq[k] for k in launches))
 
     # per-curve error of the timed arithmetic against FP64, on a sample of
@@ -646,7 +615,7 @@ def main():
 
     # batched uneven workload: 10^6 runs, 2D L log-uniform in [8, 512] and
     # chains l log-uniform in [1024, 65536], 50/50, one persistent launch per
-    # ensemble replayed as a CUDA graph; launch shape from the autotuner
+    # ensemble replayed as a CUDA graph; reduction from the autotuner
     mix = None
     if args.mix_runs > 0:
         from pypercolate_gb300.autotune import tune_mix
@@ -721,21 +690,15 @@ def main():
                    'precision': args.precision, 'l2_fetch_bytes': l2_fetch,
                    'l2': 'inputs larger than L2 (%.1f GB of union-find state per step)'
                          % (R * N * 4 / 1e9)},
-        'roofline': {'bound': 'hbm', 'achieved': achieved, 'peak': peak, 'unit': 'GB/s',
+        'roofline': {'bound': 'instruction latency (node words in shared memory; HBM carries the records only)',
+                     'achieved': achieved, 'peak': peak, 'unit': 'GB/s',
                      'frac': achieved / peak, 'traffic': UF_TRAFFIC_PER_ADD * adds_per_launch,
                      'traffic_source': 'ncu dram__bytes_read.sum + dram__bytes_write.sum per '
-                                       'addition on a 12,288-run capture, scaled to the '
+                                       'addition on a 608-run capture, scaled to the '
                                        'launch by its additions',
-                     'kernel': 'uf_window_kernel', 'peak_source': peak_kind,
+                     'kernel': 'uf_group_kernel', 'peak_source': peak_kind,
                      'bytes_per_addition': uf_bytes,
-                     'avg_launch_ms': uf_avg_s * 1e3,
-                     'random_access': {
-                         'gather_sectors_per_s': gather_rate,
-                         'uf_read_sectors_per_s': uf_adds_per_s * UF_READ_PER_ADD / 32.0,
-                         'frac': uf_adds_per_s * UF_READ_PER_ADD / 32.0 / gather_rate,
-                         'note': 'ceiling = 4-B torch.index_select gathers at random positions of '
-                                 'a 16 GiB array; union-find sector reads from the measured '
-                                 '%.1f B read per addition' % UF_READ_PER_ADD}},
+                     'avg_launch_ms': uf_avg_s * 1e3},
         'kernel_ms_per_step': {k: v[1] / args.steps for k, v in prof.items()},
         'plain_gpu': plain,
         'batched_uneven': mix,
@@ -757,10 +720,7 @@ def main():
     }
     if not default_leg:
         # the traffic figure and the CPU oracle pipeline are for the bond grid
-        line['roofline']['kernel'] = ('torus_window_kernel' if args.lattice == 'torus'
-                                      else 'site_window_kernel')
         line['roofline']['traffic'] = None
-        line['roofline'].pop('random_access', None)
     if rank == 0:
         if default_leg:
             try:

@@ -360,15 +360,14 @@ int nz_ensemble(const NzGraph *graph, int32_t spanning, int32_t n_runs,
 
 /* Launch shapes of the ensemble pipeline, chosen by an autotuner (the Python
  * package's autotune.tune_ensemble) rather than fixed; a field of 0 takes the
- * default.  uf_block: runs per CTA of the union-find (32, 64 or 128; 128);
- * m2_tile: probabilities per CTA of the compensated m2 convolution (8 or 16;
- * 8); reduce_slices: slices of runs of the canonical run reduction (1 ..
- * 256; 1, 16 or 64 by run count); conv_tile: probabilities per CTA of the
- * FP32 convolution kernel of m0, m3 and m4 (8 or 16; 8); taper: 1 =
- * the first and the last record window a quarter window long (the first
- * window's union-find and the last window's reductions run alone), 0 = all
- * windows full (0).  The record window is nz_ensemble's `window`.  No
- * counterpart in the reference (its runs are Python calls). */
+ * default.  reduce_slices: slices of runs of the canonical run reduction (1 ..
+ * 256; 1, 16 or 64 by run count); taper: 1 = the first and the last record
+ * window a quarter window long (the first window's union-find and the last
+ * window's reductions run alone), 0 = all windows full (0).  uf_block (32, 64
+ * or 128), m2_tile and conv_tile (8 or 16) are checked and have no effect: the
+ * union-find and the convolutions choose their blocks by the sizes.  The record
+ * window is nz_ensemble's `window`.  No counterpart in the reference (its runs
+ * are Python calls). */
 typedef struct NzTuning {
     int32_t uf_block;
     int32_t m2_tile;
@@ -427,17 +426,18 @@ typedef struct NzMixAccum {
     uint32_t *errors;  /* [1] runs skipped by a failed internal check (0)    */
 } NzMixAccum;
 
-/* Workspace for n_runs runs and `threads` persistent threads; each thread's
- * node slot is sized for the largest lattice of the spec.  Beside the node
- * slots: per-run checkpoint records (36 B per run and checkpoint) for
- * NZ_MIX_REDUCE_RECORDS, per-class sums (216 B per class and checkpoint)
- * for NZ_MIX_REDUCE_FUSED. */
+/* Workspace for n_runs runs with `threads` node slots in global memory, each
+ * sized for the largest lattice of the spec (only lattices beyond 65,536 node
+ * words use them, one per resident run).  Beside the node slots: per-run
+ * checkpoint records (36 B per run and checkpoint) for NZ_MIX_REDUCE_RECORDS,
+ * per-class sums (216 B per class and checkpoint) for NZ_MIX_REDUCE_FUSED. */
 size_t nz_mix_workspace_bytes(const NzMixSpec *spec, int32_t n_runs,
                               int32_t threads);
 /* key_dev: device pointer to the Philox key (read by the kernels, so a
  * captured CUDA graph of this call can be replayed with another key).
- * threads: persistent threads; block: threads per CTA; smem_words: per-thread
- * shared-memory node slot (0 = none) -- runs with N <= smem_words use it.
+ * threads: node slots (at most that many of the largest lattices run at a
+ * time); block and smem_words are checked and have no effect: a thread block
+ * takes a run, its size and memory chosen by the lattice's.
  * Output arrays are overwritten (not accumulated). */
 int nz_mix(const NzMixSpec *spec, const uint32_t *thr_grid,
            const uint32_t *thr_chain, const uint64_t *key_dev, int32_t n_runs,
@@ -498,7 +498,7 @@ int nz_get_l2_fetch_granularity(int32_t *bytes);
  * sequences and their summed elapsed milliseconds, and clears the record.
  * (The project's own instrumentation; no counterpart in the reference.) */
 #define NZ_PROF_SETUP 0      /* weights, run initialisation                 */
-#define NZ_PROF_UNION_FIND 1 /* uf_window_kernel                            */
+#define NZ_PROF_UNION_FIND 1 /* uf_group_kernel                             */
 #define NZ_PROF_MICRO 2      /* fused microcanonical reductions             */
 #define NZ_PROF_CONV 3       /* banded canonical convolution                */
 #define NZ_PROF_REDUCE 4     /* merge over runs                             */

@@ -1,17 +1,17 @@
 """Autotuners for the two ensemble paths.
 
-tune_mix       batched uneven ensembles (``nz_mix``): persistent threads
-               (runs in flight), threads per CTA (runs per CTA), the
-               shared-memory node slot per thread (placement: small lattices
-               in shared memory, the rest in HBM / L2) and the reduction
-               (per-run checkpoint records reduced by a second kernel, or
-               fused into the union-find as exact integer atomics).
-tune_ensemble  one lattice per ensemble (``nz_ensemble_tuned``): runs per
-               CTA of the union-find, the probability tiles of the compensated
-               m2 convolution and of the other statistics' convolution, the
-               record window (rows reduced and convolved
-               per pass: the reduction tiling over n) and the slices of runs
-               of the canonical run reduction (its tiling over runs).
+tune_mix       batched uneven ensembles (``nz_mix``): the reduction (per-run
+               checkpoint records reduced by a second kernel, or fused into
+               the union-find as exact integer atomics) and the node slots of
+               the lattices too large for shared memory.
+tune_ensemble  one lattice per ensemble (``nz_ensemble_tuned``): the record
+               window (rows reduced and convolved per pass: the reduction
+               tiling over n), its schedule and the slices of runs of the
+               canonical run reduction (its tiling over runs).
+
+Both also time arguments that the kernels no longer depend on (threads per
+CTA, probability tiles, node slots in shared memory), which callers and cached
+results may name.
 
 Each candidate runs the same workload, timed with CUDA events on the
 launching stream; the fastest wins.  Results are cached in a JSON file keyed
@@ -29,9 +29,7 @@ DEFAULT_CACHE = os.path.join(os.path.expanduser('~'), '.cache', 'pypercolate_gb3
 
 
 def _candidates(nmax, free_bytes):
-    """A compact grid: runs in flight x runs per CTA x shared-memory slot
-    (64 words hold the grids up to L = 8, 128 words up to L = 10: the
-    smallest lattices of the mix run out of shared memory)."""
+    """(node slots, threads per CTA, shared-memory words) to try."""
     out = []
     for threads, block, smem in ((49152, 128, 0), (65536, 128, 0), (98304, 128, 0),
                                  (131072, 128, 0), (65536, 64, 0), (98304, 64, 0),
@@ -108,7 +106,9 @@ def default_window(M, n_runs):
 
 
 def ensemble_candidates(M, n_runs):
-    """The library's defaults, then one launch-shape change at a time."""
+    """The library's defaults, then one launch-shape change at a time.
+    (uf_block, m2_tile and conv_tile have no effect: the library's kernels
+    choose their blocks by the sizes.)"""
     w = default_window(M, n_runs)
     base = {'uf_block': 128, 'm2_tile': 8, 'conv_tile': 8, 'taper': 0,
             'reduce_slices': 64 if n_runs >= 65536 else 16, 'window': w}

@@ -426,10 +426,7 @@ constexpr uint64_t kM4HighFreeNodes = 115001;  // max_s s^3 (N - s) < 2^64 for N
 // union-find on s1, at the device's greatest stream priority, and the
 // consumers of each window (micro reductions, convolution, final reduction)
 // on s2, with the events that order them; both fork from and join back into
-// the caller's stream.  With the union-find's blocks dispatched first, a
-// 100,000-run L = 256 step took 1187.2 against 1197.1 ms on the caller's
-// (default-priority) stream, same box: the union-find 1038 against 1082 ms,
-// the consumers beside it slower.  Slots are created on first use and kept
+// the caller's stream.  Slots are created on first use and kept
 // for the life of the process; a call holds one for as long as it enqueues
 // work, so concurrent calls never share events.
 struct AuxSlot {
@@ -494,9 +491,7 @@ struct JoinGuard {
 
 int32_t pick_window(uint32_t M, int32_t n_runs, int32_t window) {
     if (window > 0) return window > (int32_t)(M + 1) ? (int32_t)(M + 1) : window;
-    // records of one window at most ~32 GiB (two windows in flight): at
-    // 100,000 runs windows of ~9,500 rows measured 0.8 % faster than ~4,800
-    // (16 GiB; 1.4 % faster than ~2,700) and ~19,000 no faster again
+    // records of one window at most ~32 GiB (two windows in flight)
     double w = 32.0 * (1ull << 30) / ((double)n_runs * kRecordBytes);
     if (w < 256) w = 256;
     if (w > M + 1) w = M + 1;

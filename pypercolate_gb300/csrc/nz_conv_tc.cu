@@ -370,13 +370,14 @@ __device__ __forceinline__ void conv_tc_tile(const ConvParams &p, TcShared &sh, 
 // statistics 0, 1, 2, 3, 5, 6, or 0, 1, 2, 3, 5 when the records carry m4
 // high words; HI = true: m4 with its high words alone (its wider loads would
 // otherwise set the register count of every statistic's code).  m2 (4) runs
-// on the compensated SIMT kernel.
+// on the compensated SIMT kernel.  SPLIT: `split` CTAs share a tile's
+// probabilities.
 template <bool SITE, bool HI, bool SPLIT>
 __global__ void __launch_bounds__(kTcRuns) conv_tc_kernel(ConvParams p, int split) {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     TcShared &sh = *reinterpret_cast<TcShared *>(tc_smem);
-    // statistic of this z: m2 (4) runs on the compensated SIMT kernel
-    // (conv_m2_comp_kernel) instead
+    // statistic of this z: m2 (4) runs on the compensated kernel of
+    // nz_conv_tiles.cu instead
     constexpr int kStat[6] = {0, 1, 2, 3, 5, 6};
     const int z = kStat[blockIdx.z];
     if (!HI && z == 0 && !p.spanning) return;

@@ -1,7 +1,7 @@
 // nz_uf.cu -- permutations, reference rows and the union-find's dispatch.
 //
-// Bond percolation (percolate/hpc.py:249-307, bond_sample_states) runs in
-// nz_ufg.cu, site percolation in nz_lattice.cu; both write the per-step records
+// Bond percolation (percolate/hpc.py:249-307, bond_sample_states) is launched by
+// nz_ufg.cu, site percolation by nz_lattice.cu; both write the per-step records
 // that the consumers share.
 #include <cstdint>
 

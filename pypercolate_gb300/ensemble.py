@@ -49,9 +49,10 @@ class Ensemble:
     model     'bond' (the reference's model) or 'site' percolation; for site
               percolation M = N steps, and p is the site occupation probability
     ps        occupation probabilities of the canonical curves
-    precision 'fp32' (FP32 SIMT products, FP64 accumulation over row chunks),
-              'tf32x3' (tensor cores: three split TF32 products per term, FP32
-              sums per 32-row chunk added into TwoSum pairs) or 'fp64'
+    precision 'fp32' (FP32 SIMT products, sums of 128 rows added into
+              (sum, compensation) pairs), 'tf32x3' (tensor cores: three split
+              TF32 products per term, sums of 64 rows added into such pairs)
+              or 'fp64'
     micro     also accumulate microcanonical run-reductions for every n
     window    rows per union-find launch (0: sized to ~32 GiB of records per window)
     tuning    launch shapes {'uf_block', 'm2_tile', 'reduce_slices', 'conv_tile', 'taper'}
