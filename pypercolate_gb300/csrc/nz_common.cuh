@@ -135,7 +135,7 @@ struct GraphDev {
     uint32_t site;        // NZ_MODEL_SITE given: M = N steps occupy sites
     uint32_t wrap;        // torus: NZ_WRAP_* >> 9 (0 either, 1 x, 2 y, 3 both)
     uint32_t L, N, M;
-    uint32_t slots;       // union-find words per run (>= N: layout padding, torus cells)
+    uint32_t slots;       // union-find words per run (>= N, 2: layout padding, torus cells)
     uint32_t tile_cols;   // grid: 4 x 2 site blocks per block row, (L+3)/4
     uint32_t row_edges;   // grid: (L-1)*(2L-1) edges in rows 0..L-2
     uint32_t two_l_m1;    // grid: 2L-1
@@ -220,7 +220,7 @@ inline GraphDev make_graph_dev(const NzGraph &g, uint32_t N, uint32_t M) {
     d.two_l_m1 = 1;
     d.inv_two_l_m1 = 1.0f;
     d.tile_cols = 0;
-    d.slots = N;
+    d.slots = N < 2 ? 2u : N;  // (one node's 16-bit value and flag are a word each between windows)
     if (d.kind == NZ_GRAPH_GRID2D) {
         d.two_l_m1 = 2u * g.length - 1u;
         d.row_edges = (g.length - 1u) * d.two_l_m1;

@@ -248,7 +248,8 @@ def test_site_records(gpu, oracle, kind, L, runs, order):
 
 
 @pytest.mark.parametrize('kind,L,window', [('grid', 30, 70), ('chain', 900, 256), ('grid', 258, 40000), ('torus', 24, 100),
-                                           ('torus', 130, 9000)])
+                                           ('torus', 130, 9000), ('chain', 1, 1), ('grid', 1, 1), ('torus', 1, 1),
+                                           ('chain', 2, 1)])
 @pytest.mark.parametrize('precision', ['fp64', 'fp32'])
 def test_site_windows(gpu, kind, L, window, precision):
     from pypercolate_gb300.ensemble import Ensemble
