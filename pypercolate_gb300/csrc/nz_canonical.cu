@@ -1428,10 +1428,13 @@ void launch_finalize(const uint8_t *avg, int32_t P, int32_t spanning, double N, 
 // Beta quantiles (iterative, FP64) are most of the work, and rows where some
 // but not all runs span are contiguous, so splitting them doubles the
 // threads working on those rows.
+// Of each warp LANES threads have one of these, the others none.
+template <int LANES>
 __global__ void micro_finalize_kernel(NzMicroAccum acc, uint32_t N, uint32_t M, int32_t spanning, double alpha,
                                       int32_t normalize, double *out) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n = t >> 1, half = t & 1u;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / 32u * LANES + lane;
+    const uint32_t n = lane < (uint32_t)LANES ? t >> 1 : M + 1u, half = t & 1u;
     const double R = (double)*acc.count;
     // every row has R runs: one pair of t quantiles per block
     const TPair tq = t_pair_block(1.0 - alpha, R - 1.0, R - 1.0, n <= M);
@@ -1488,9 +1491,17 @@ void launch_micro_finalize(const NzMicroAccum &acc, uint32_t N, uint32_t M, int3
     // figure).  Every block works out its own t quantiles, which the 32,700
     // one-warp blocks of a 512 x 512 grid pay for (4.5 against 1.7 ms).
     const uint64_t threads = 2ull * ((uint64_t)M + 1);
+    // Where warps of 8 rows' halves still find a quarter of an SM each, they
+    // are shorter than full ones, in which the slowest of 32 quantiles counts
+    // (10^4 runs of 32 x 32 346 -> 256 us, 6 10^4 556 -> 384; 1,000 of 48 x 48,
+    // beyond, 203 and 219).
+    if (threads <= 8u * 4u * 152u) {
+        micro_finalize_kernel<8><<<(unsigned)((threads + 7) / 8), 32, 0, s>>>(acc, N, M, spanning, alpha, normalize, out);
+        return;
+    }
     const unsigned block = threads <= 80000 ? 32 : 128;
-    micro_finalize_kernel<<<(unsigned)((threads + block - 1) / block), block, 0, s>>>(acc, N, M, spanning, alpha,
-                                                                                     normalize, out);
+    micro_finalize_kernel<32><<<(unsigned)((threads + block - 1) / block), block, 0, s>>>(acc, N, M, spanning, alpha,
+                                                                                         normalize, out);
 }
 
 __global__ void t_quantile_kernel(const double *q, const double *df, int32_t count, double *out) {
