@@ -366,8 +366,11 @@ void launch_q(const ConvParams &p, cudaStream_t s) {
 template <int S, bool SITE = false>
 void launch(const ConvParams &p, cudaStream_t s) {
     constexpr bool kWide = S == 5 || S == 6 || S == 7;
-    const int64_t tiles = (int64_t)((p.n_runs + kRuns - 1) / kRuns) * ((p.P + kPT - 1) / kPT);
+    const int64_t p_tiles = (p.P + kPT - 1) / kPT, tiles = (int64_t)((p.n_runs + kRuns - 1) / kRuns) * p_tiles;
     if (tiles < 152) return launch_q<S, 2, SITE>(p, s);
+    // (the grid's y, of p_tiles kPT / Q, has 16 bits: conv_grid_fits admits kPT
+    // to a block)
+    if (p_tiles * (kPT / 4) > 65535) return launch_q<S, kPT, SITE>(p, s);
     if constexpr (kWide || TileShared<S, kPT>::kM2) {
         if (tiles >= (kWide ? 2 : 8) * 152) return launch_q<S, kPT, SITE>(p, s);
     }
