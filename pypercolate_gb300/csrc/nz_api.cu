@@ -155,7 +155,8 @@ int nz_microcanonical(const NzGraph *graph, int32_t spanning, int32_t n_runs, in
     const uint32_t *perm_src = perms;
     int mode = perm_mode;
     if (perm_mode == NZ_PERM_MT19937) {
-        launch_mt_perms(M, n_runs, mt_seed_words, mt_seed_len, mt_words_stride, mt_perms, s);
+        if (launch_mt_perms(M, n_runs, mt_seed_words, mt_seed_len, mt_words_stride, mt_perms, s) != cudaSuccess)
+            return NZ_ERR_CUDA;
         perm_src = mt_perms;
         mode = NZ_PERM_GIVEN;
     }
@@ -175,7 +176,7 @@ int nz_microcanonical(const NzGraph *graph, int32_t spanning, int32_t n_runs, in
     p.tiled = false;
     {
         ProfScope prof(NZ_PROF_UNION_FIND, s);
-        launch_uf_window(p, mode, spanning != 0, s);
+        if (launch_uf_window(p, mode, spanning != 0, s) != cudaSuccess) return NZ_ERR_CUDA;
     }
     return check_launch();
 }
@@ -223,7 +224,8 @@ int nz_permutations(uint32_t num_edges, int32_t n_runs, int32_t perm_mode, uint6
     if (perm_mode == NZ_PERM_PHILOX) launch_philox_perms(num_edges, n_runs, key, run0, out, s);
     else if (perm_mode == NZ_PERM_MT19937) {
         if (!mt_seed_words || !mt_seed_len) return NZ_ERR_INVALID;
-        launch_mt_perms(num_edges, n_runs, mt_seed_words, mt_seed_len, mt_words_stride, out, s);
+        if (launch_mt_perms(num_edges, n_runs, mt_seed_words, mt_seed_len, mt_words_stride, out, s) != cudaSuccess)
+            return NZ_ERR_CUDA;
     } else return NZ_ERR_INVALID;
     return check_launch();
 }
@@ -303,7 +305,7 @@ int nz_canonical_statistics_records(const NzRecords *rec, uint32_t num_nodes, ui
     p.acc = out;
     p.errors = nullptr;
     p.tiled = false;
-    launch_conv_window(p, 0, s);
+    if (launch_conv_window(p, 0, s) != cudaSuccess) return NZ_ERR_CUDA;
     return check_launch();
 }
 
@@ -381,7 +383,8 @@ int nz_micro_merge(const NzMicroAccum *dst, const NzMicroAccum *src, uint32_t nu
 int nz_mt_stream_permutations(const uint32_t *state_in, uint32_t num_edges, int32_t n_runs, uint32_t *out,
                               uint32_t *state_out, void *stream) {
     if (!state_in || !state_out || n_runs <= 0 || (num_edges > 0 && !out)) return NZ_ERR_INVALID;
-    launch_mt_stream_perms(state_in, num_edges, n_runs, out, state_out, as_stream(stream));
+    if (launch_mt_stream_perms(state_in, num_edges, n_runs, out, state_out, as_stream(stream)) != cudaSuccess)
+        return NZ_ERR_CUDA;
     return check_launch();
 }
 
@@ -698,7 +701,8 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
         up.n_begin = w0; up.n_end = w1;
         {
             ProfScope prof(NZ_PROF_UNION_FIND, s1);
-            launch_uf_window(up, NZ_PERM_PHILOX, spanning != 0, s1);
+            // (without it there are no records to reduce)
+            if (launch_uf_window(up, NZ_PERM_PHILOX, spanning != 0, s1) != cudaSuccess) return NZ_ERR_CUDA;
         }
         if (cudaEventRecord(aux.a->produced[b], s1) != cudaSuccess ||
             cudaStreamWaitEvent(s2, aux.a->produced[b], 0) != cudaSuccess)
@@ -713,11 +717,9 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
             ProfScope prof(NZ_PROF_CONV, s2);
             cp.rec = L.rec[b];
             cp.n_begin = w0; cp.n_end = w1;
-            if (conv_precision == 2) {
-                if (launch_conv_window_tc(cp, s2) != 0) return NZ_ERR_CUDA;
-            } else {
-                launch_conv_window(cp, conv_precision, s2);
-            }
+            if (conv_precision == 2 ? launch_conv_window_tc(cp, s2) != 0
+                                    : launch_conv_window(cp, conv_precision, s2) != cudaSuccess)
+                return NZ_ERR_CUDA;
         }
         if (cudaEventRecord(aux.a->consumed[b], s2) != cudaSuccess) return NZ_ERR_CUDA;
     }

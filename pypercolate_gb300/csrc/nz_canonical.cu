@@ -615,7 +615,7 @@ bool conv_grid_fits(int32_t n_runs, int32_t P) {
 }
 
 template <int PT>
-static void launch_conv_fp64(const ConvParams &p, cudaStream_t s) {
+static cudaError_t launch_conv_fp64(const ConvParams &p, cudaStream_t s) {
     // (run tiles, p tiles, statistics); launching the p tiles of one run tile
     // back to back (for L2 reuse of its records) measured slower
     dim3 gmax((p.n_runs + kConvRuns - 1) / kConvRuns, (p.P + PT - 1) / PT, 1);
@@ -623,33 +623,25 @@ static void launch_conv_fp64(const ConvParams &p, cudaStream_t s) {
     // the record model is a template parameter: a run-time test in the row
     // loop cost 17 % of the kernel's time
     auto launch = [&](auto max_set, auto others) {
-        max_set<<<gmax, kConvRuns, 0, s>>>(p);
-        others<<<gother, kConvRuns, 0, s>>>(p);
+        const cudaError_t e = launch_kernel(max_set, gmax, kConvRuns, 0, 0, s, p);
+        return e == cudaSuccess ? launch_kernel(others, gother, kConvRuns, 0, 0, s, p) : e;
     };
     if (p.tiled && p.rec.site)
-        launch(conv_window_kernel<Layout::kTiledSite, true, PT>, conv_window_kernel<Layout::kTiledSite, false, PT>);
-    else if (p.tiled)
-        launch(conv_window_kernel<Layout::kTiled, true, PT>, conv_window_kernel<Layout::kTiled, false, PT>);
-    else if (p.rec.site)
-        launch(conv_window_kernel<Layout::kSite, true, PT>, conv_window_kernel<Layout::kSite, false, PT>);
-    else
-        launch(conv_window_kernel<Layout::kBond, true, PT>, conv_window_kernel<Layout::kBond, false, PT>);
+        return launch(conv_window_kernel<Layout::kTiledSite, true, PT>, conv_window_kernel<Layout::kTiledSite, false, PT>);
+    if (p.tiled) return launch(conv_window_kernel<Layout::kTiled, true, PT>, conv_window_kernel<Layout::kTiled, false, PT>);
+    if (p.rec.site) return launch(conv_window_kernel<Layout::kSite, true, PT>, conv_window_kernel<Layout::kSite, false, PT>);
+    return launch(conv_window_kernel<Layout::kBond, true, PT>, conv_window_kernel<Layout::kBond, false, PT>);
 }
 
-void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
-    if (p.n_runs <= 0 || p.P <= 0) return;
-    if (precision != 0) {  // ensembles only: tiled records
-        launch_conv_tiles(p, s);
-        return;
-    }
+cudaError_t launch_conv_window(const ConvParams &p, int precision, cudaStream_t s) {
+    if (p.n_runs <= 0 || p.P <= 0) return cudaSuccess;
+    if (precision != 0) return launch_conv_tiles(p, s);  // ensembles only: tiled records
     // Fewer probabilities per CTA, so more CTAs, where tiles of 8 leave SMs idle
     // (whole ensembles in ms with 8, 4, 2: 200 runs of 200 x 200 at 100 p, 26
     // tiles, 8.4, 5.5, 4.2; 1,000 toruses of 64 x 64 at 101 p, 104 tiles, 3.0,
     // 2.6, 2.6; 1,000 grids of 128 x 128 at 201 p, 208 tiles, 8.6, 8.5, 8.8).
     const int64_t tiles = (int64_t)((p.n_runs + kConvRuns - 1) / kConvRuns) * ((p.P + kConvPT - 1) / kConvPT);
-    if (tiles < 64) launch_conv_fp64<2>(p, s);
-    else if (tiles < 152) launch_conv_fp64<4>(p, s);
-    else launch_conv_fp64<kConvPT>(p, s);
+    return tiles < 64 ? launch_conv_fp64<2>(p, s) : tiles < 152 ? launch_conv_fp64<4>(p, s) : launch_conv_fp64<kConvPT>(p, s);
 }
 
 // Weights of the FP32 convolution: the part of each p's band whose weights

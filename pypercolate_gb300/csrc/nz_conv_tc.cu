@@ -475,8 +475,7 @@ int launch_conv_window_tc(const ConvParams &p, cudaStream_t s) {
     // m2 needs ~5e-11 relative per run (the susceptibility curve within 1e-6
     // absolute of FP64 at L = 1024), beyond FP32 tensor-core accumulation:
     // it runs on the compensated SIMT kernel
-    launch_conv_tiles_m2(p, s);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_conv_tiles_m2(p, s) == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace nz

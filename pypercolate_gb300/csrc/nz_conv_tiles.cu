@@ -347,12 +347,10 @@ __global__ void __launch_bounds__(kRuns, kPerSm<S>) conv_tiles_kernel(ConvParams
 }
 
 template <int S, int Q, bool SITE>
-void launch_q(const ConvParams &p, cudaStream_t s) {
+cudaError_t launch_q(const ConvParams &p, cudaStream_t s) {
     dim3 grid((p.n_runs + kRuns - 1) / kRuns, (p.P + kPT - 1) / kPT * (kPT / Q));
-    if (sizeof(TileShared<S, Q>) > 48 * 1024)
-        cudaFuncSetAttribute(conv_tiles_kernel<S, Q, SITE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(TileShared<S, Q>));
-    conv_tiles_kernel<S, Q, SITE><<<grid, kRuns, sizeof(TileShared<S, Q>), s>>>(p);
+    constexpr size_t kSmem = sizeof(TileShared<S, Q>);
+    return launch_kernel(conv_tiles_kernel<S, Q, SITE>, grid, kRuns, kSmem, kSmem, s, p);
 }
 
 // Probabilities per CTA.  Fewer make more CTAs, whose rows are fewer where the
@@ -364,7 +362,7 @@ void launch_q(const ConvParams &p, cudaStream_t s) {
 // 853 and 891), and for m3 and m4 up to 2 (1,000 of 64 x 64, 304 tiles: 44 and
 // 45; 1,000 of 32 x 32, 208 tiles: 22 and 18).
 template <int S, bool SITE = false>
-void launch(const ConvParams &p, cudaStream_t s) {
+cudaError_t launch(const ConvParams &p, cudaStream_t s) {
     constexpr bool kWide = S == 5 || S == 6 || S == 7;
     const int64_t p_tiles = (p.P + kPT - 1) / kPT, tiles = (int64_t)((p.n_runs + kRuns - 1) / kRuns) * p_tiles;
     if (tiles < 152) return launch_q<S, 2, SITE>(p, s);
@@ -374,25 +372,21 @@ void launch(const ConvParams &p, cudaStream_t s) {
     if constexpr (kWide || TileShared<S, kPT>::kM2) {
         if (tiles >= (kWide ? 2 : 8) * 152) return launch_q<S, kPT, SITE>(p, s);
     }
-    launch_q<S, 4, SITE>(p, s);
+    return launch_q<S, 4, SITE>(p, s);
 }
 
 }  // namespace
 
-void launch_conv_tiles_m2(const ConvParams &p, cudaStream_t s) {
-    if (p.rec.narrow) launch<9>(p, s);
-    else launch<4>(p, s);
+cudaError_t launch_conv_tiles_m2(const ConvParams &p, cudaStream_t s) {
+    return p.rec.narrow ? launch<9>(p, s) : launch<4>(p, s);
 }
 
-void launch_conv_tiles(const ConvParams &p, cudaStream_t s) {
-    if (p.rec.site) launch<1, true>(p, s);
-    else launch<1>(p, s);
-    if (p.rec.narrow) launch<8>(p, s);
-    else launch<2>(p, s);
-    launch<5>(p, s);
-    if (p.rec.m4_hi) launch<6>(p, s);
-    else launch<7>(p, s);
-    launch_conv_tiles_m2(p, s);
+cudaError_t launch_conv_tiles(const ConvParams &p, cudaStream_t s) {
+    cudaError_t e = p.rec.site ? launch<1, true>(p, s) : launch<1>(p, s);
+    if (e == cudaSuccess) e = p.rec.narrow ? launch<8>(p, s) : launch<2>(p, s);
+    if (e == cudaSuccess) e = launch<5>(p, s);
+    if (e == cudaSuccess) e = p.rec.m4_hi ? launch<6>(p, s) : launch<7>(p, s);
+    return e == cudaSuccess ? launch_conv_tiles_m2(p, s) : e;
 }
 
 }  // namespace nz

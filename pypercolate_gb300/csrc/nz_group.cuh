@@ -428,6 +428,10 @@ __host__ __device__ __forceinline__ uint32_t claim_words(uint32_t slots, uint32_
     return claims < all ? claims : all;
 }
 
+// The most shared memory that a block's claims and nodes take: one block to an SM.
+template <int W, bool SHARED>
+constexpr size_t most_shared() { return 228u * 1024u - 1280u - sizeof(GroupShared<W, SHARED>); }
+
 // The claims of a block, for all the runs it takes, at the start of its dynamic
 // shared memory (a multiple of 32 words).
 template <int W>

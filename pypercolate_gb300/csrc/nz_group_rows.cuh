@@ -115,15 +115,13 @@ inline int runs_per_sm(const UfParams &p) {
 }
 
 template <int W, bool SHARED, bool TORUS, bool SITE>
-void launch_group(const UfParams &p, bool given, bool span, cudaStream_t s) {
+cudaError_t launch_group(const UfParams &p, bool given, bool span, cudaStream_t s) {
     const uint32_t nodes = SHARED ? node_bytes<TORUS>(p.g.N) : 0u;
     const int blocks = min(24 / W, runs_per_sm(p));
     const uint32_t claims = claim_words<W, SHARED>(node_count<SHARED, TORUS>(p.g), nodes, (uint32_t)blocks);
     const size_t smem = (size_t)claims * 4u + nodes;
-    if (smem > 40 * 1024)
-        cudaFuncSetAttribute(uf_group_kernel<W, SHARED, TORUS, SITE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    uf_group_kernel<W, SHARED, TORUS, SITE><<<p.n_runs, 32 * W, smem, s>>>(p, claims, given, span);
+    return launch_kernel(uf_group_kernel<W, SHARED, TORUS, SITE>, dim3(p.n_runs), 32 * W, smem, most_shared<W, SHARED>(), s, p,
+                         claims, given, span);
 }
 
 // Warps per run.  In shared memory: kWarpsPerSm warps on every SM (80 registers
@@ -149,26 +147,23 @@ inline int group_warps(const UfParams &p, bool site) {
 }
 
 template <bool TORUS, bool SITE>
-void launch_groups(const UfParams &p, bool given, bool span, cudaStream_t s) {
+cudaError_t launch_groups(const UfParams &p, bool given, bool span, cudaStream_t s) {
     const int warps = group_warps(p, SITE);
     if (p.g.N <= (TORUS ? kSharedTorus : kSharedNodes)) {
         switch (warps) {
-            case 1: launch_group<1, true, TORUS, SITE>(p, given, span, s); break;
-            case 2: launch_group<2, true, TORUS, SITE>(p, given, span, s); break;
-            case 3: launch_group<3, true, TORUS, SITE>(p, given, span, s); break;
-            case 4: launch_group<4, true, TORUS, SITE>(p, given, span, s); break;
-            case 6: launch_group<6, true, TORUS, SITE>(p, given, span, s); break;
-            case 8: launch_group<8, true, TORUS, SITE>(p, given, span, s); break;
-            case 12: launch_group<12, true, TORUS, SITE>(p, given, span, s); break;
-            default: launch_group<24, true, TORUS, SITE>(p, given, span, s); break;
+            case 1: return launch_group<1, true, TORUS, SITE>(p, given, span, s);
+            case 2: return launch_group<2, true, TORUS, SITE>(p, given, span, s);
+            case 3: return launch_group<3, true, TORUS, SITE>(p, given, span, s);
+            case 4: return launch_group<4, true, TORUS, SITE>(p, given, span, s);
+            case 6: return launch_group<6, true, TORUS, SITE>(p, given, span, s);
+            case 8: return launch_group<8, true, TORUS, SITE>(p, given, span, s);
+            case 12: return launch_group<12, true, TORUS, SITE>(p, given, span, s);
+            default: return launch_group<24, true, TORUS, SITE>(p, given, span, s);
         }
-    } else if (warps == 12) {
-        launch_group<12, false, TORUS, SITE>(p, given, span, s);
-    } else {
-        launch_group<24, false, TORUS, SITE>(p, given, span, s);
     }
+    if (warps == 12) return launch_group<12, false, TORUS, SITE>(p, given, span, s);
+    return launch_group<24, false, TORUS, SITE>(p, given, span, s);
 }
-
 
 }  // namespace group
 }  // namespace nz

@@ -10,6 +10,25 @@
 
 namespace nz {
 
+// Launches with `smem` bytes of dynamic shared memory.  How much a kernel may be
+// given is a property of the kernel, for all host threads of the context alike: it
+// is set to `most`, the most that any call gives it, and so never taken from under
+// another thread's launch.
+template <class... P, class... A>
+cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, size_t most, cudaStream_t s,
+                          A... args) {
+    if (most > 40 * 1024) {  // (with the static shared memory, beyond what is given unasked)
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 struct UfParams {
     GraphDev g;
     int32_t n_runs;
@@ -30,24 +49,24 @@ struct UfParams {
 // UfParams::init_flag
 const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
                                  uint32_t *flag_scratch, cudaStream_t s);
-void launch_uf_window(const UfParams &p, int perm_mode, bool span, cudaStream_t s);
+cudaError_t launch_uf_window(const UfParams &p, int perm_mode, bool span, cudaStream_t s);
 void launch_philox_perms(uint32_t M, int32_t n_runs, uint64_t key, uint64_t run0, uint32_t *out,
                          cudaStream_t s);
 void launch_pack_rows(const NzRecords &rec, int32_t run, uint32_t N, uint32_t M, int32_t spanning,
                       uint8_t *rows, cudaStream_t s);
 
 // nz_mt.cu: numpy's permutations
-void launch_mt_perms(uint32_t M, int32_t n_runs, const uint32_t *seed_words, const int32_t *seed_len,
-                     int32_t stride, uint32_t *out, cudaStream_t s);
-void launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t n_runs, uint32_t *out,
-                            uint32_t *state_out, cudaStream_t s);
+cudaError_t launch_mt_perms(uint32_t M, int32_t n_runs, const uint32_t *seed_words, const int32_t *seed_len,
+                            int32_t stride, uint32_t *out, cudaStream_t s);
+cudaError_t launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t n_runs, uint32_t *out,
+                                   uint32_t *state_out, cudaStream_t s);
 
 // nz_ufg.cu: bond percolation with a thread block per run (which initialises
 // the run in the window that begins at row 0)
-void launch_uf_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
+cudaError_t launch_uf_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
 
 // nz_lattice.cu: the same for site percolation
-void launch_site_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
+cudaError_t launch_site_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
 
 // nz_canonical.cu
 void launch_binomial_weights(uint32_t M, const double *ps, int32_t P, double cutoff, int32_t cap,
@@ -77,7 +96,7 @@ struct ConvParams {
     uint32_t *errors;        // tensor-core path: counts CTAs whose waits gave up (or null)
 };
 bool conv_grid_fits(int32_t n_runs, int32_t P);  // grid of launch_conv_window within CUDA's limits
-void launch_conv_window(const ConvParams &p, int precision, cudaStream_t s);
+cudaError_t launch_conv_window(const ConvParams &p, int precision, cudaStream_t s);
 // 3xTF32 tensor-core convolution (tcgen05) of the FP32 bands; 0 or -1 (launch error)
 bool conv_tc_grid_fits(int32_t n_runs, int32_t P);
 int launch_conv_window_tc(const ConvParams &p, cudaStream_t s);
@@ -89,8 +108,8 @@ void launch_narrow_weights_f32(const double *w64, const uint32_t *band_lo, const
                                int32_t cap, double rel, double rel_core, float *w32, float *w32lo, uint32_t *lo32,
                                uint32_t *len32, uint32_t *core_lo, uint32_t *core_len, cudaStream_t s);
 // nz_conv_tiles.cu: the FP32 convolution of tiled records (all statistics, or m2 alone)
-void launch_conv_tiles(const ConvParams &p, cudaStream_t s);
-void launch_conv_tiles_m2(const ConvParams &p, cudaStream_t s);
+cudaError_t launch_conv_tiles(const ConvParams &p, cudaStream_t s);
+cudaError_t launch_conv_tiles_m2(const ConvParams &p, cudaStream_t s);
 // part: scratch [slices][P*7][3] doubles
 void launch_reduce_runs(const double *stats, int32_t n_runs, int32_t P, uint64_t *acc_count,
                         double *acc_mean, double *acc_m2, double *part, int32_t slices, cudaStream_t s);

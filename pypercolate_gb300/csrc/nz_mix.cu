@@ -479,15 +479,13 @@ static int launch_segment(const MixLaunch &p, int segment, uint32_t words, int p
     const uint32_t nodes = SHARED ? group::val_bytes(words) + group::flag_bytes(words) : 0u;
     const uint32_t claims = group::claim_words<W, SHARED>(words, nodes, (uint32_t)per_sm);
     const size_t smem = (size_t)claims * 4u + nodes;
-    if (smem > 40 * 1024 &&
-        cudaFuncSetAttribute(mix_group_kernel<W, SHARED, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-        return NZ_ERR_INVALID;
     int blocks = 152 * per_sm;
     if (blocks > p.m.n_runs) blocks = p.m.n_runs;
     if (!SHARED && blocks > p.T) blocks = p.T;  // one node array each
-    mix_group_kernel<W, SHARED, FUSED><<<blocks, 32 * W, smem, s>>>(p, segment, claims, p.home_words);
-    return NZ_OK;
+    return launch_kernel(mix_group_kernel<W, SHARED, FUSED>, dim3(blocks), 32 * W, smem, group::most_shared<W, SHARED>(), s, p,
+                         segment, claims, p.home_words) == cudaSuccess
+               ? NZ_OK
+               : NZ_ERR_CUDA;
 }
 
 template <bool FUSED>

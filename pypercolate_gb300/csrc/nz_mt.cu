@@ -247,35 +247,29 @@ __global__ void __launch_bounds__(kThreads) mt_perm_kernel(uint32_t M, uint32_t 
     }
 }
 
-void launch(uint32_t M, uint32_t blocks, uint32_t runs, const uint32_t *seed_words, const int32_t *seed_len,
-            int32_t stride, const uint32_t *state_in, uint32_t *state_out, uint32_t *out, cudaStream_t s) {
-    if (M <= kSmallM) {
-        const size_t smem = (2 * (size_t)M + 15) & ~(size_t)15;
-        if (smem + sizeof(MtShared) > 48 * 1024)
-            cudaFuncSetAttribute(mt_perm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        mt_perm_kernel<true><<<blocks, kThreads, smem, s>>>(M, runs, seed_words, seed_len, stride, state_in, state_out,
-                                                            out);
-    } else {
-        mt_perm_kernel<false><<<blocks, kThreads, 0, s>>>(M, runs, seed_words, seed_len, stride, state_in, state_out,
-                                                          out);
-    }
+cudaError_t launch(uint32_t M, uint32_t blocks, uint32_t runs, const uint32_t *seed_words, const int32_t *seed_len,
+                   int32_t stride, const uint32_t *state_in, uint32_t *state_out, uint32_t *out, cudaStream_t s) {
+    const bool small = M <= kSmallM;
+    return launch_kernel(small ? mt_perm_kernel<true> : mt_perm_kernel<false>, dim3(blocks), kThreads,
+                         small ? (2 * (size_t)M + 15) & ~(size_t)15 : 0, small ? 2 * (size_t)kSmallM : 0, s, M, runs,
+                         seed_words, seed_len, stride, state_in, state_out, out);
 }
 
 }  // namespace
 
-void launch_mt_perms(uint32_t M, int32_t n_runs, const uint32_t *seed_words, const int32_t *seed_len, int32_t stride,
-                     uint32_t *out, cudaStream_t s) {
-    if (n_runs <= 0 || M == 0) return;
-    launch(M, (uint32_t)n_runs, 1u, seed_words, seed_len, stride, nullptr, nullptr, out, s);
+cudaError_t launch_mt_perms(uint32_t M, int32_t n_runs, const uint32_t *seed_words, const int32_t *seed_len,
+                            int32_t stride, uint32_t *out, cudaStream_t s) {
+    if (n_runs <= 0 || M == 0) return cudaSuccess;
+    return launch(M, (uint32_t)n_runs, 1u, seed_words, seed_len, stride, nullptr, nullptr, out, s);
 }
 
 // Continuation of one MT19937 stream (numpy's global RandomState): n_runs
 // permutations of range(M) are drawn one after another exactly as
 // np.random.permutation(M) would draw them (percolate/percolate.py:270, once
 // per run in run order), and the advanced state is stored.
-void launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t n_runs, uint32_t *out, uint32_t *state_out,
-                            cudaStream_t s) {
-    launch(M, 1u, (uint32_t)n_runs, nullptr, nullptr, 0, state_in, state_out, out, s);
+cudaError_t launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t n_runs, uint32_t *out,
+                                   uint32_t *state_out, cudaStream_t s) {
+    return launch(M, 1u, (uint32_t)n_runs, nullptr, nullptr, 0, state_in, state_out, out, s);
 }
 
 }  // namespace nz

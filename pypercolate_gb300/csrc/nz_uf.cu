@@ -67,10 +67,9 @@ const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *no
     return flag_scratch;
 }
 
-void launch_uf_window(const UfParams &p, int perm_mode, bool span, cudaStream_t s) {
+cudaError_t launch_uf_window(const UfParams &p, int perm_mode, bool span, cudaStream_t s) {
     const bool given = perm_mode != NZ_PERM_PHILOX;
-    if (p.g.site) launch_site_groups(p, given, span, s);
-    else launch_uf_groups(p, given, span, s);
+    return p.g.site ? launch_site_groups(p, given, span, s) : launch_uf_groups(p, given, span, s);
 }
 
 void launch_philox_perms(uint32_t M, int32_t n_runs, uint64_t key, uint64_t run0, uint32_t *out,

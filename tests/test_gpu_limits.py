@@ -33,3 +33,44 @@ def test_many_probabilities(gpu, P, model):
         few.run(130, key=3)
         for a, b in ((mean, few.mean), (m2, few.m2)):
             assert np.array_equal(a[first:first + 16], b.cpu().numpy().reshape(16, 7))
+
+
+@pytest.mark.parametrize('what', ['runs', 'permutations'])
+def test_threads_with_blocks_of_different_memory(gpu, what):
+    """Two host threads on streams of their own launch one kernel with much and
+    with little shared memory per block: neither takes the other's away."""
+    import threading
+
+    import torch
+    from pypercolate_gb300 import hpc
+    lib = gpu.lib_handle()
+    failed = []
+
+    def runs(L, stream, times):
+        spec = hpc.GraphSpec(gpu.GRAPH_GRID2D, L)
+        g, rec = spec.struct(), gpu.Records(spec.M + 1, 1, with_edge=False)
+        need = lib.nz_microcanonical_workspace_bytes(g, 1, gpu.PERM_PHILOX)
+        ws = gpu.device_empty(need)
+        for _ in range(times):
+            if lib.nz_microcanonical(g, 1, 1, gpu.PERM_PHILOX, 1, 0, None, None, None, 1, gpu.ptr(ws), need,
+                                     rec.struct(), stream.cuda_stream):
+                failed.append(L)
+        stream.synchronize()
+
+    def permutations(M, stream, times):
+        words, lens = (torch.zeros(1, dtype=torch.int32, device='cuda') for _ in range(2))
+        out = torch.empty(M, dtype=torch.int32, device='cuda')
+        torch.cuda.synchronize()
+        for _ in range(times):
+            if lib.nz_permutations(M, 1, gpu.PERM_MT19937, 0, 0, gpu.ptr(words), gpu.ptr(lens), 1, gpu.ptr(out),
+                                   stream.cuda_stream):
+                failed.append(M)
+        stream.synchronize()
+
+    work, sizes = {'runs': (runs, (256, 181)), 'permutations': (permutations, (65160, 30000))}[what]
+    threads = [threading.Thread(target=work, args=(size, torch.cuda.Stream(), 1500)) for size in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
