@@ -1067,8 +1067,8 @@ constexpr int kMicroWarps = 16;
 template <bool NARROW>
 struct MicroSums {
     uint32_t span;
-    uint64_t s_max, s_m0, s_m2;  // max, m0 < 2^21 and m2 < 2^42, of at most 2^24 runs
-    u128 s_m3, s_m4;
+    uint64_t s_max, s_m0;  // < 2^21, of at most 2^24 runs
+    u128 s_m2, s_m3, s_m4;  // (m2 < 2^42: 2^66)
     u128 q_max, q_m0, q_m2;
     typename std::conditional<NARROW, u128, U192>::type q_m3;  // m3 < 2^48 (narrow) or 2^63
     U192 q_m4;                                                 // m4 < 2^64 (narrow) or 2^84
@@ -1102,7 +1102,7 @@ __global__ void __launch_bounds__(32 * kMicroWarps, 2) micro_tiled_kernel(MicroP
     const uint32_t i = blockIdx.x * 32u + lane, n = p.n_begin + i;
     const NzRecords &rec = p.rec;
     MicroSums<NARROW> a = {};
-    uint64_t q_max = 0, q_m0 = 0;  // per thread: at most 2^20 runs' squares < 2^42
+    uint64_t q_max = 0, q_m0 = 0, s_m2 = 0;  // per thread: at most 2^20 runs' values < 2^42
     struct Rec {
         uint32_t ms, m0, m4_hi;
         uint64_t m2, m3, m4;
@@ -1124,7 +1124,7 @@ __global__ void __launch_bounds__(32 * kMicroWarps, 2) micro_tiled_kernel(MicroP
         a.span += q.ms >> 31;
         a.s_max += mx;
         a.s_m0 += q.m0;
-        a.s_m2 += q.m2;
+        s_m2 += q.m2;
         a.s_m3 += q.m3;
         a.s_m4 += ((u128)q.m4_hi << 64) | q.m4;
         q_max += (uint64_t)mx * mx;
@@ -1148,6 +1148,7 @@ __global__ void __launch_bounds__(32 * kMicroWarps, 2) micro_tiled_kernel(MicroP
         for (int k = 0; k < kAhead; ++k) add(q[k]);
     }
     for (; r < p.n_runs; r += kMicroWarps) add(load(r));
+    a.s_m2 = s_m2;
     a.q_max = q_max;
     a.q_m0 = q_m0;
     for (uint32_t w = 0; w < (uint32_t)kMicroWarps; ++w) {
