@@ -349,6 +349,7 @@ int nz_microcanonical_reduce(const NzRecords *rec, uint32_t num_nodes, uint32_t 
     MicroParams mp;
     mp.rec = *rec;
     mp.tiled = false;
+    mp.part = nullptr;
     mp.n_begin = n_begin;
     mp.n_end = n_end;
     mp.N = num_nodes;
@@ -547,8 +548,9 @@ size_t ensemble_layout(Carver &c, const GraphDev &g, int32_t n_runs, int32_t P, 
     // enough slices to occupy the SMs whatever the run count (1,000 runs, 201 p:
     // one slice 150 us, 16 slices 20)
     L.slices = n_runs < 256 ? 1 : (n_runs < 65536 ? 16 : 64);
-    // room for the largest tuned slice count
-    L.part = c.take<double>((size_t)kMaxSlices * P * 7 * 3);
+    // room for the largest tuned slice count, and (before) for the slices of
+    // the microcanonical reductions
+    L.part = c.take<double>(std::max((size_t)kMaxSlices * P * 7 * 3, micro_part_bytes() / sizeof(double)));
     return c.used;
 }
 
@@ -665,6 +667,7 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
     MicroParams mp;
     if (micro) {
         mp.tiled = up.tiled;
+        mp.part = L.part;
         mp.N = N;
         mp.n_runs = n_runs;
         mp.acc = *micro;

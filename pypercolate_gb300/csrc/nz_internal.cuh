@@ -117,6 +117,7 @@ void launch_reduce_runs(const double *stats, int32_t n_runs, int32_t P, uint64_t
 struct MicroParams {
     NzRecords rec;
     bool tiled;  // as UfParams::tiled
+    void *part;  // tiled: micro_part_bytes() of scratch
     uint32_t n_begin, n_end;
     uint32_t N;
     int32_t n_runs;
@@ -124,6 +125,7 @@ struct MicroParams {
     uint32_t M;
     const uint64_t *count_before;  // device: runs already in acc
 };
+size_t micro_part_bytes();
 void launch_micro_window(const MicroParams &p, cudaStream_t s);
 void launch_micro_count(uint64_t *count, int32_t n_runs, cudaStream_t s);
 void launch_canonical_merge(uint64_t *dst_count, double *dst_mean, double *dst_m2, const uint64_t *src_count,
