@@ -65,7 +65,11 @@ cudaError_t launch_mt_stream_perms(const uint32_t *state_in, uint32_t M, int32_t
 // the run in the window that begins at row 0)
 cudaError_t launch_uf_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
 
-// nz_lattice.cu: the same for site percolation
+// nz_uft.cu: bonds and sites with a thread per run, and where that is the better one
+bool run_per_thread(const UfParams &p);
+cudaError_t launch_uf_threads(const UfParams &p, bool given, bool span, cudaStream_t s);
+
+// nz_lattice.cu: a thread block per run for site percolation
 cudaError_t launch_site_groups(const UfParams &p, bool given, bool span, cudaStream_t s);
 
 // nz_canonical.cu

@@ -1,8 +1,8 @@
 // nz_uf.cu -- permutations, reference rows and the union-find's dispatch.
 //
 // Bond percolation (percolate/hpc.py:249-307, bond_sample_states) is launched by
-// nz_ufg.cu, site percolation by nz_lattice.cu; both write the per-step records
-// that the consumers share.
+// nz_ufg.cu, site percolation by nz_lattice.cu, very many runs by nz_uft.cu; all
+// write the per-step records that the consumers share.
 #include <cstdint>
 
 #include "nz_common.cuh"
@@ -69,6 +69,7 @@ const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *no
 
 cudaError_t launch_uf_window(const UfParams &p, int perm_mode, bool span, cudaStream_t s) {
     const bool given = perm_mode != NZ_PERM_PHILOX;
+    if (run_per_thread(p)) return launch_uf_threads(p, given, span, s);
     return p.g.site ? launch_site_groups(p, given, span, s) : launch_uf_groups(p, given, span, s);
 }
 
