@@ -127,3 +127,15 @@ def test_edge_lists_with_a_thread_per_run(gpu, oracle, spanning, both):
         assert np.array_equal(host['m2'][:, r], ref['moments_u64'][:, 2])
         if spanning:
             assert np.array_equal(host['max_span'][:, r] >> 31, ref['span'])
+
+
+@pytest.mark.parametrize('kind,L,model', [
+    ('chain', 501, 'bond'), ('chain', 502, 'site'), ('chain', 503, 'bond'), ('chain', 504, 'site'),
+    ('grid', 23, 'bond'), ('grid', 25, 'site'), ('torus', 13, 'bond'), ('torus', 14, 'site')])
+def test_node_words_between_windows(gpu, kind, L, model):
+    """Places of runs at every multiple of 4 bytes, and copies that are no
+    multiple of 16: the windows' sums are those of one window."""
+    from pypercolate_gb300.ensemble import Ensemble
+    a, b = (_micro(Ensemble(kind, L, [0.4], model=model, window=w).run(301, key=2)) for w in (0, 101))
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
