@@ -77,8 +77,10 @@ struct Nodes;
 
 template <>
 struct Nodes<true, false> {
-    uint16_t *val;
-    uint8_t *flag;
+    // volatile: other threads of the block shorten paths meanwhile (any parent read
+    // is an ancestor), so no access may be repeated or kept (1 % of the time)
+    volatile uint16_t *val;
+    volatile uint8_t *flag;
     __device__ __forceinline__ uint32_t load(uint32_t x) const { return ((uint32_t)flag[x] << 24) | val[x]; }
     __device__ __forceinline__ void shorten(uint32_t x, uint32_t parent) const { val[x] = (uint16_t)parent; }
     __device__ __forceinline__ void link(uint32_t x, uint32_t parent) const {
@@ -506,7 +508,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
     typedef Nodes<SHARED, TORUS> NodesT;
     NodesT nd;
     if constexpr (SHARED) {
-        nd.val = reinterpret_cast<uint16_t *>(nodes);
+        nd.val = reinterpret_cast<volatile uint16_t *>(nodes);
         nd.flag = nodes + val_bytes(g.N);
         if constexpr (TORUS) nd.off = reinterpret_cast<int32_t *>(nodes + val_bytes(g.N) + flag_bytes(g.N));
     } else if constexpr (TORUS) {
@@ -562,7 +564,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
         corrupt = (st.flags & kFlagCorrupt) != 0;
         if (t < 2) sh.wrap[t] = (st.flags & (t == 0 ? kFlagWrapX : kFlagWrapY)) ? 0u : 0xffffffffu;
         if constexpr (SHARED) {
-            copy_words<W>(reinterpret_cast<uint32_t *>(nd.val), run.home, node_bytes<TORUS>(g.N) / 4u);
+            copy_words<W>(reinterpret_cast<uint32_t *>(nodes), run.home, node_bytes<TORUS>(g.N) / 4u);
         }
         if (t == 0) {
             Sums<NARROW> c;
@@ -1156,7 +1158,7 @@ __device__ __forceinline__ bool group_run(const GraphDev &g, const Run &run, Gro
         if (t == 0 && (!SITE || G != kNone)) nd.set_root(G, g_size, g_sides);
         __syncthreads();
         if constexpr (SHARED) {
-            copy_words<W>(run.home, reinterpret_cast<const uint32_t *>(nd.val), node_bytes<TORUS>(g.N) / 4u);
+            copy_words<W>(run.home, reinterpret_cast<const uint32_t *>(nodes), node_bytes<TORUS>(g.N) / 4u);
         }
     }
     const bool bad = __syncthreads_or(corrupt);
