@@ -139,3 +139,30 @@ def test_node_words_between_windows(gpu, kind, L, model):
     a, b = (_micro(Ensemble(kind, L, [0.4], model=model, window=w).run(301, key=2)) for w in (0, 101))
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize('M', [1, 2, 3, 100, 255, 256])
+@pytest.mark.parametrize('arrays', [False, True])
+def test_short_permutations_of_many_seeds(gpu, M, arrays):
+    """numpy's permutations of 32,768 seeds, a thread each, against those of
+    fewer, a block each, and against numpy's own."""
+    import torch
+    rng = np.random.default_rng(M)
+    runs, width = 32768, 3 if arrays else 1
+    words = rng.integers(0, 2 ** 32, (runs, width), dtype=np.uint32)
+    lens = rng.integers(1, width + 1, runs).astype(np.int32) if arrays else np.zeros(runs, np.int32)
+    d_words, d_lens = gpu.to_device(words), gpu.to_device(lens)
+
+    def draw(first, count):
+        out = torch.empty(count * M, dtype=torch.int32, device='cuda')
+        gpu.check(gpu.lib_handle().nz_permutations(
+            M, count, gpu.PERM_MT19937, 0, 0, gpu.ptr(d_words[4 * width * first:]), gpu.ptr(d_lens[4 * first:]), width,
+            gpu.ptr(out), gpu.stream_handle()), 'nz_permutations')
+        return out.view(count, M)
+
+    whole = draw(0, runs)
+    for first in (0, 20000):
+        assert torch.equal(whole[first:first + 12768], draw(first, 12768))
+    for r in (0, 1, runs - 1):
+        seed = words[r, :lens[r]].tolist() if arrays else int(words[r, 0])
+        assert np.array_equal(whole[r].cpu().numpy(), np.random.RandomState(seed).permutation(M))
