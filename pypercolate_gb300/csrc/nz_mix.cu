@@ -1,4 +1,4 @@
-// nz_mix.cu -- batched uneven ensembles in one persistent launch.
+// nz_mix.cu -- batched uneven ensembles: one launch per range of sizes.
 //
 // n_runs independent runs whose substrate is drawn per run: with probability
 // chain_share a spanning_1d_chain(l), l log-uniform in [chain_min, chain_max],
@@ -20,7 +20,9 @@
 //      a run per thread block (nz_group.cuh) with as many warps as fill the SMs
 //      with the blocks that fit there: node words in global memory above
 //      65,536, in shared memory below.  The blocks stay and claim runs with an
-//      atomic counter, the largest lattices first.
+//      atomic counter, the largest lattices first.  (Very many runs of lattices of
+//      at most 4,096 words with the fused reduction: mix_thread_kernel, a run per
+//      thread.)
 //      At F evenly spaced occupation checkpoints
 //      n_j = floor(j M / (F - 1)) each run either writes its exact
 //      statistics (records) or, with the fused reduction, adds them and
@@ -39,6 +41,7 @@
 #include "nz_common.cuh"
 #include "nz_group.cuh"
 #include "nz_internal.cuh"
+#include "nz_thread.cuh"
 #include "nz_wide.cuh"
 
 namespace nz {
@@ -73,6 +76,17 @@ __device__ __forceinline__ void class_graph(const MixDev &m, uint32_t cls, uint3
 // node words a run of class cls needs: grid_slots(L) (the tiled layout) or l
 __device__ __forceinline__ uint32_t class_slots(const MixDev &m, uint32_t cls) {
     return cls < m.n_grid ? grid_slots(m.grid_min + cls) : m.chain_min + (cls - m.n_grid);
+}
+
+// the rest of the GraphDev of class cls, whose L, N and M are set
+__device__ __forceinline__ void set_class_graph(const MixDev &m, uint32_t cls, uint32_t kind, GraphDev &g) {
+    g.kind = (int32_t)kind; g.site = 0; g.wrap = 0;
+    g.slots = class_slots(m, cls);
+    g.tile_cols = kind == NZ_GRAPH_GRID2D ? (g.L + 3u) >> 2 : 0u;
+    g.two_l_m1 = kind == NZ_GRAPH_GRID2D ? 2u * g.L - 1u : 1u;
+    g.row_edges = kind == NZ_GRAPH_GRID2D ? (g.L - 1u) * g.two_l_m1 : 0u;
+    g.inv_two_l_m1 = 1.0f / (float)g.two_l_m1;
+    g.eu = g.ev = nullptr; g.side = nullptr;
 }
 
 __global__ void mix_class_kernel(MixDev m, uint32_t *cls, uint32_t *counts) {
@@ -191,8 +205,8 @@ constexpr int kSqMax = 10, kSqM0 = 12, kSqM2 = 14, kSqM3 = 17, kSqM4 = 21;
 static_assert(kSqM4 + 6 == kMixCellWords, "cell layout");
 
 // Adds 32-bit limbs into the words of one cell.  When every active lane of
-// the warp adds into the same cell (runs of one lattice reach their
-// checkpoints together), the lanes' limbs are summed first (redux.sync on
+// the warp adds into the same cell (with a thread per run, neighbours in the queue
+// being runs of one lattice), the lanes' limbs are summed first (redux.sync on
 // 16-bit halves, so 32 lanes' sums fit 32 bits) and one lane issues the
 // atomic: 27 atomics per warp and checkpoint instead of up to 27 x 32.
 struct CellAdder {
@@ -342,13 +356,8 @@ __global__ void __launch_bounds__(32 * W, 24 / W) mix_group_kernel(MixLaunch p, 
         uint32_t kind, L, N, M;
         class_graph(p.m, cls, kind, L, N, M);
         if (threadIdx.x == 0) {
-            g.kind = (int32_t)kind; g.site = 0; g.wrap = 0; g.L = L; g.N = N; g.M = M;
-            g.slots = class_slots(p.m, cls);
-            g.tile_cols = kind == NZ_GRAPH_GRID2D ? (L + 3u) >> 2 : 0u;
-            g.two_l_m1 = kind == NZ_GRAPH_GRID2D ? 2u * L - 1u : 1u;
-            g.row_edges = kind == NZ_GRAPH_GRID2D ? (L - 1u) * g.two_l_m1 : 0u;
-            g.inv_two_l_m1 = 1.0f / (float)g.two_l_m1;
-            g.eu = g.ev = nullptr; g.side = nullptr;
+            g.L = L; g.N = N; g.M = M;
+            set_class_graph(p.m, cls, kind, g);
         }
         __syncthreads();
         run.id = id;
@@ -363,6 +372,75 @@ __global__ void __launch_bounds__(32 * W, 24 / W) mix_group_kernel(MixLaunch p, 
         const bool bad = group::group_run<W, SHARED, false, false>(g, run, sh, claims, smem + (size_t)claim_count * 4u, sink);
         if (bad && threadIdx.x == 0) atomicAdd(p.acc.errors, 1u);
         __syncthreads();
+    }
+}
+
+// The fused reduction of small lattices: a thread per run.  Runs of one lattice
+// are neighbours in the queue, so a warp's lanes mostly reach their checkpoints
+// together and add their limbs up before one of them adds to the cell (27 atomics
+// a warp and checkpoint).  Blocks of a run each would issue these per run.
+// `node`: this thread's slot, as many words as the segment's largest lattice has.
+template <int KIND>
+__device__ __forceinline__ void mix_thread_run(const MixDev &m, uint64_t key, uint32_t id, const GraphDev &g,
+                                               uint32_t *node, uint64_t *cells, uint32_t *errors) {
+    for (uint32_t j = 0; j < g.slots; ++j) {
+        uint32_t i = j;
+        if (KIND == NZ_GRAPH_GRID2D && kGridTiled) {
+            const uint32_t tile = j >> 3, w = j & 7u, tr = tile / g.tile_cols, tc = tile - tr * g.tile_cols;
+            const uint32_t row = 2u * tr + (w >> 2), col = 4u * tc + (w & 3u);
+            if (row >= g.L || col >= g.L) continue;  // a padding slot, never read
+            i = row * g.L + col;
+        }
+        node[j] = make_root(1u, node_sides<KIND>(g, i));
+    }
+    FeistelPerm fp;
+    fp.init(key, id, g.M);
+    thread::Tally t;
+    t.st.t2 = t.st.t3 = t.st.t4_lo = t.st.t0 = g.N;
+    t.st.t4_hi = 0;
+    t.st.max = 1;
+    t.st.flags = 0;
+    const uint32_t F = (uint32_t)m.F;
+    auto row_of = [&](uint32_t j) { return (uint32_t)(((uint64_t)j * g.M) / (F - 1u)); };
+    uint32_t j = 0, target = 0;
+    for (uint32_t n = 0; n <= g.M; ++n) {
+        if (n > 0) {
+            uint32_t u, v;
+            decode_edge_slots<KIND>(g, fp.at(n - 1u), u, v);
+            thread::link(node, u, v, node[u], node[v], true, t);
+        }
+        if (n != target) continue;
+        const RunState &st = t.st;
+        const uint64_t mx = st.max, mx2 = mx * mx, mx3 = mx2 * mx, mx4_lo = mx3 * mx;
+        const uint32_t m4_hi = (uint32_t)(st.t4_hi - __umul64hi(mx3, mx) - (st.t4_lo < mx4_lo ? 1u : 0u));
+        while (j < F && n == target) {  // several checkpoints share row n where F - 1 > M
+            mix_checkpoint(cells + (size_t)j * kMixCellWords, st.max, (st.flags & kFlagSpan) != 0, st.t0 - 1u,
+                           st.t2 - mx2, st.t3 - mx3, st.t4_lo - mx4_lo, m4_hi);
+            ++j;
+            if (j < F) target = row_of(j);
+        }
+    }
+    if (t.st.flags & kFlagCorrupt) atomicAdd(errors, 1u);
+}
+
+// (80 registers: 6 blocks on an SM)
+constexpr int kMixThreads = 128;
+__global__ void __launch_bounds__(kMixThreads, 6) mix_thread_kernel(MixLaunch p, int segment, uint32_t threads,
+                                                                    uint32_t slot_words) {
+    const uint32_t t = blockIdx.x * kMixThreads + threadIdx.x;
+    if (t >= threads) return;
+    const uint64_t key = *p.m.key_ptr;
+    const uint32_t end = p.begin[segment + 1];
+    uint32_t *node = p.nodes + (size_t)t * slot_words;
+    for (uint32_t pos = atomicAdd(p.head + segment, 1u); pos < end; pos = atomicAdd(p.head + segment, 1u)) {
+        const uint32_t id = p.queue[pos], cls = p.cls[id];
+        uint32_t kind;
+        GraphDev g;
+        class_graph(p.m, cls, kind, g.L, g.N, g.M);
+        set_class_graph(p.m, cls, kind, g);
+        uint64_t *cells = p.cells + (size_t)cls * (uint32_t)p.m.F * kMixCellWords;
+        if (kind == NZ_GRAPH_GRID2D) mix_thread_run<NZ_GRAPH_GRID2D>(p.m, key, id, g, node, cells, p.acc.errors);
+        else mix_thread_run<NZ_GRAPH_CHAIN1D>(p.m, key, id, g, node, cells, p.acc.errors);
     }
 }
 
@@ -488,6 +566,52 @@ static int launch_segment(const MixLaunch &p, int segment, uint32_t words, int p
                : NZ_ERR_CUDA;
 }
 
+// Node words that the slots of segment k's threads have, and their number: 6 blocks
+// to an SM, as far as the caller's slots reach.
+static uint32_t thread_words(const MixLaunch &p, int k) {
+    return (uint32_t)std::min<uint64_t>(segment_words(k - 1), p.home_words);
+}
+static uint32_t thread_count(const MixLaunch &p, int k) {
+    const uint64_t slots = (uint64_t)p.T * p.home_words / thread_words(p, k);
+    return (uint32_t)std::min<uint64_t>({152ull * 6 * kMixThreads, slots, (uint64_t)p.m.n_runs});
+}
+
+// Runs that segment k can expect, its lengths being log-uniform.
+static double expected_runs(const MixLaunch &p, int k) {
+    auto part = [](uint32_t lo, uint32_t hi, uint32_t a, uint32_t b) {  // lengths a .. b - 1 of lo .. hi
+        if (a >= b) return 0.0;
+        if (lo == hi) return 1.0;
+        return std::min(1.0, (log(b - 0.5) - log(a - 0.5)) / log((double)hi / lo));
+    };
+    uint32_t a = p.m.grid_min, b = p.m.grid_max + 1u;
+    while (a < b && grid_slots(a) <= segment_words(k)) ++a;
+    while (a < b && grid_slots(b - 1u) > segment_words(k - 1)) --b;
+    const double grids = part(p.m.grid_min, p.m.grid_max, a, b);
+    const double chains = part(p.m.chain_min, p.m.chain_max, std::max(p.m.chain_min, segment_words(k) + 1u),
+                               std::min(p.m.chain_max, segment_words(k - 1)) + 1u);
+    const double share = p.m.chain_share / 4294967296.0;
+    return p.m.n_runs * ((1.0 - share) * grids + share * chains);
+}
+
+// Is a thread per run the better one for the fused reduction of segment k (3 or 4)?
+// A thread's steps take some 2.9 us each, so the largest lattice's are the least time;
+// a block of a run adds all its checkpoints' limbs itself.  ms by blocks and by threads,
+// 256 checkpoints: 10^6 runs of grids 2-16 and chains 2-64 67 and 8.5, 10^5 7.5 and 3.4,
+// 10^4 1.6 and 3; of grids 8-31 and chains 64-1000 55 and 26, 5.5 and 6.9; 3 10^5 of grids
+// 33-64 and chains 2000-4096 171 and 83, 10^5 57 and 37, 3 10^4 17.6 and 27.
+static bool mix_threads(const MixLaunch &p, int k) {
+    const double runs = expected_runs(p, k);
+    return thread_count(p, k) >= std::min(runs, 65536.0) && runs >= (k == 4 ? 20000.0 + 100.0 * thread_words(p, k) : 50000.0);
+}
+
+static int launch_threads(const MixLaunch &p, int k, cudaStream_t s) {
+    const uint32_t threads = thread_count(p, k);
+    return launch_kernel(mix_thread_kernel, dim3((threads + kMixThreads - 1) / kMixThreads), kMixThreads, 0, 0, s, p, k, threads,
+                         thread_words(p, k)) == cudaSuccess
+               ? NZ_OK
+               : NZ_ERR_CUDA;
+}
+
 template <bool FUSED>
 static int launch_segments(const MixLaunch &p, cudaStream_t s) {
     const uint64_t most = std::max<uint64_t>(grid_slots(p.m.grid_max), p.m.chain_max);
@@ -500,6 +624,11 @@ static int launch_segments(const MixLaunch &p, cudaStream_t s) {
     if (used(0)) st = launch_segment<12, false, FUSED>(p, 0, (uint32_t)most, 2, s);
     if (st == NZ_OK && used(1)) st = launch_segment<24, true, FUSED>(p, 1, segment_words(0), 1, s);
     if (st == NZ_OK && used(2)) st = launch_segment<8, true, FUSED>(p, 2, segment_words(1), 3, s);
+    if constexpr (FUSED) {
+        if (st == NZ_OK && used(3)) st = mix_threads(p, 3) ? launch_threads(p, 3, s) : launch_segment<2, true, true>(p, 3, segment_words(2), 11, s);
+        if (st == NZ_OK && used(4)) st = mix_threads(p, 4) ? launch_threads(p, 4, s) : launch_segment<1, true, true>(p, 4, segment_words(3), 24, s);
+        return st;
+    }
     if (st == NZ_OK && used(3)) st = launch_segment<2, true, FUSED>(p, 3, segment_words(2), 11, s);
     if (st == NZ_OK && used(4)) st = launch_segment<1, true, FUSED>(p, 4, segment_words(3), 24, s);
     return st;

@@ -166,3 +166,24 @@ def test_short_permutations_of_many_seeds(gpu, M, arrays):
     for r in (0, 1, runs - 1):
         seed = words[r, :lens[r]].tolist() if arrays else int(words[r, 0])
         assert np.array_equal(whole[r].cpu().numpy(), np.random.RandomState(seed).permutation(M))
+
+
+@pytest.mark.parametrize('runs,grid,chain,share,checkpoints', [
+    (60000, (1, 16), (1, 64), 0.5, 256),           # more checkpoints than most have rows
+    (130000, (8, 31), (64, 1000), 0.5, 64),        # all lattices up to 1,024 node words
+    (60000, (33, 64), (2000, 4096), 0.1, 101),     # up to 4,096
+    (50001, (64, 64), (64, 64), 0.0, 1000),        # one lattice
+    (300000, (2, 90), (3, 9000), 0.4, 33)])        # some in blocks, some in threads
+def test_fused_uneven_runs_in_threads(gpu, runs, grid, chain, share, checkpoints):
+    """Every count, sum and M2 of the fused reduction of very many runs is that
+    of the records', and of the fused one with too few node slots for threads."""
+    from pypercolate_gb300.mix import MixEnsemble
+    out = []
+    for fused, threads in ((False, None), (True, None), (True, 8)):
+        m = MixEnsemble(runs, grid=grid, chain=chain, chain_share=share, checkpoints=checkpoints, fused=fused,
+                        threads=threads).run(77)
+        out.append(m.results())
+        del m
+    for other in out[1:]:
+        for k, v in out[0].items():
+            assert np.array_equal(v, other[k]), k
