@@ -33,7 +33,7 @@ namespace {
 using namespace thread;
 
 constexpr int kThreads = 128;
-constexpr uint32_t kTinyNodes = 200, kTinyTorus = 121;  // largest N in shared memory
+constexpr uint32_t kTinyNodes = 256, kTinyTorus = 121;  // largest N in shared memory
 
 // Where a run's rows go (n-major), in increasing order.
 struct Rows {
@@ -261,12 +261,13 @@ __global__ void __launch_bounds__(kThreads) torus_thread_kernel(UfParams p, bool
 // A thread's node words lie in shared memory, 16 bits each (root: bit 15, sides
 // 13..14, size; else the parent; word x of thread t at x * kThreads + t), on the
 // torus with the displacement from the parent as one integer dx 2^16 + dy.
-// All totals of N <= kTinyNodes nodes fit 32 bits (N^4 < 2^31).  Four rows of a
-// run are written at a time, in the tiles' 16-byte pieces.  10^6 runs of 8 x 8: 2.3 ms;
+// Totals are kept modulo 2^32, which all moments are below (sum' s^4 <= max s^3 (N -
+// s) < N^4 / 9).  Four rows of a run are written at a time, in the tiles' 16-byte
+// pieces.  10^6 runs of 8 x 8: 2.3 ms;
 // with node words in global memory 6.0, and 14.3 with rows written value by value,
 // a warp's 32 lanes in 32 lines.
 constexpr uint32_t kTinyRoot = 0x8000u;
-static_assert((uint64_t)kTinyNodes * kTinyNodes * kTinyNodes * kTinyNodes < 1ull << 31, "totals in 32 bits");
+static_assert((uint64_t)kTinyNodes * kTinyNodes * kTinyNodes * kTinyNodes / 9 < 1ull << 32, "moments in 32 bits");
 
 struct TinyRows {
     uint32_t ms[4][kThreads], m2[4][kThreads], m3[4][kThreads], m4[4][kThreads];
@@ -505,8 +506,9 @@ cudaError_t launch_kind(const UfParams &p, bool given, bool span, cudaStream_t s
 // Where a thread per run is the better one, each line where both take the same
 // time.  Union-find in ms, a group per run and a thread per run:
 //   ensembles, 10^6 runs: 8 x 8 7.6 and 2.3, 12 x 12 14.0 and 6.4, chains of 200
-//   10.5 and 3.6, sites of 8 x 8 8.2 and 1.3; 20,000 runs of 8 x 8 0.17 and 0.11, of
-//   chains of 200 0.24 each.  The torus needs three times the memory, so that only
+//   10.5 and 3.6, sites of 8 x 8 8.2 and 1.3, 5 10^5 of 16 x 16 8.7 and 4.1, sites 9.6 and
+//   4.6; 33,000 runs of 8 x 8 0.30 and 0.12, of 16 x 16 0.64 and 0.45; 20,000 of 8 x 8 0.17
+//   and 0.11, of chains of 200 0.24 each.  The torus needs three times the memory, so that only
 //   one block fits an SM beyond 121 nodes (10^6 / 2 runs of 11 x 11 6.5 and 3.0, 12 x
 //   12 8.4 and 10.4).
 //   n-major, bonds: 10^5 runs of 16 x 16 3.2 and 2.1, of 64 x 64 79 and 53, 50,000 of

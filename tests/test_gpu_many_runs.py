@@ -43,16 +43,16 @@ def test_sums_do_not_depend_on_the_slices(gpu, kind, L, model, wrap, runs):
 
 
 # the smallest, the largest and odd sizes of the lattices whose node words lie in
-# a block's shared memory with a thread per run (N <= 200, on the torus 121), and
+# a block's shared memory with a thread per run (N <= 256, on the torus 121), and
 # the first beyond
 @pytest.mark.parametrize('kind,L,model,wrap', [
     ('grid', 1, 'bond', 'either'), ('grid', 2, 'bond', 'either'), ('grid', 9, 'bond', 'either'),
-    ('grid', 14, 'bond', 'either'), ('grid', 15, 'bond', 'either'), ('chain', 1, 'bond', 'either'),
-    ('chain', 2, 'bond', 'either'), ('chain', 200, 'bond', 'either'), ('chain', 201, 'bond', 'either'),
+    ('grid', 16, 'bond', 'either'), ('grid', 17, 'bond', 'either'), ('chain', 1, 'bond', 'either'),
+    ('chain', 2, 'bond', 'either'), ('chain', 256, 'bond', 'either'), ('chain', 257, 'bond', 'either'),
     ('torus', 1, 'bond', 'either'), ('torus', 2, 'bond', 'x'), ('torus', 3, 'bond', 'both'),
     ('torus', 11, 'bond', 'y'), ('torus', 12, 'bond', 'both'), ('grid', 1, 'site', 'either'),
-    ('grid', 5, 'site', 'either'), ('grid', 14, 'site', 'either'), ('chain', 1, 'site', 'either'),
-    ('chain', 173, 'site', 'either'), ('torus', 1, 'site', 'either'), ('torus', 2, 'site', 'either'),
+    ('grid', 5, 'site', 'either'), ('grid', 16, 'site', 'either'), ('chain', 1, 'site', 'either'),
+    ('chain', 173, 'site', 'either'), ('chain', 256, 'site', 'either'), ('torus', 1, 'site', 'either'), ('torus', 2, 'site', 'either'),
     ('torus', 7, 'site', 'both'), ('torus', 11, 'site', 'x')])
 @pytest.mark.parametrize('window', [0, 37])
 def test_ensembles_with_a_thread_per_run(gpu, kind, L, model, wrap, window):
