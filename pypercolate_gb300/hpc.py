@@ -29,6 +29,7 @@ are bit-identical to the reference's for the same seed.  The keyword
 ``rng='philox'`` (swallowed by the reference's ``**kwargs``) selects the
 project's Philox-keyed permutation instead, with ``seed`` as the Philox key.
 """
+import copy
 import functools
 import os
 
@@ -86,9 +87,14 @@ def finalized_canonical_averages_dtype(spanning_cluster=True):
 
 
 @functools.lru_cache(maxsize=None)
-def _dtype(name, spanning):
-    """np.dtype of a row type (numpy parses the field strings on every use)."""
+def _parsed_dtype(name, spanning):
     return np.dtype(globals()[name + '_dtype'](spanning))
+
+
+def _dtype(name, spanning):
+    """np.dtype of a row type (numpy parses the field strings on every use).  A
+    copy each time: renaming a result's fields changes its dtype in place."""
+    return copy.copy(_parsed_dtype(name, spanning))
 
 
 # ---------------------------------------------------------------------------
