@@ -94,7 +94,7 @@ def _parsed_dtype(name, spanning):
 def _dtype(name, spanning):
     """np.dtype of a row type (numpy parses the field strings on every use).  A
     copy each time: renaming a result's fields changes its dtype in place."""
-    return copy.copy(_parsed_dtype(name, spanning))
+    return copy.copy(_parsed_dtype(name, bool(spanning)))
 
 
 # ---------------------------------------------------------------------------

@@ -15,3 +15,11 @@ def test_row_types_are_not_shared(name, spanning):
     assert rows.dtype == want
     rows.dtype.names = tuple('f%d' % i for i in range(len(want.names)))
     assert hpc._dtype(name, spanning).names == want.names
+
+
+@pytest.mark.parametrize('spanning', [np.array(True), np.array(False), [0], [], {'a': 1}, np.True_, 1, None])
+def test_row_types_of_any_truth_value(spanning):
+    """As the types' own functions take it: by its truth, hashable or not."""
+    from pypercolate_gb300 import hpc
+    for name in ROWS:
+        assert hpc._dtype(name, spanning) == np.dtype(getattr(hpc, name + '_dtype')(spanning))
