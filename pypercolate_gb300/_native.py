@@ -279,10 +279,12 @@ def ptr(t):
 
 
 def to_host(t, dtype, shape):
-    """Device byte buffer -> numpy array of the given dtype/shape."""
-    n = int(np.prod(shape)) * np.dtype(dtype).itemsize
-    raw = t[:n].cpu().numpy() if n else np.zeros(0, np.uint8)  # memory of its own
-    return raw.view(dtype).reshape(shape)
+    """Device byte buffer -> numpy array of the given dtype/shape, with memory of
+    its own that the copy goes into."""
+    out = np.empty(shape, dtype=dtype)
+    if out.nbytes:
+        torch_cuda().from_numpy(out.reshape(-1).view(np.uint8)).copy_(t[:out.nbytes])
+    return out
 
 
 def make_graph(kind, length=0, num_nodes=0, num_edges=0, edge_u=None, edge_v=None,
