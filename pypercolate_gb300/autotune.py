@@ -15,14 +15,18 @@ results may name.
 
 Each candidate runs the same workload, timed with CUDA events on the
 launching stream; the fastest wins.  Results are cached in a JSON file keyed
-by the GPU name and the workload, so later processes reuse the choice.
+by the GPU name, the kernels' sources and the workload, so later processes reuse
+the choice as long as it was made with their kernels.
 """
+import functools
+import hashlib
 import json
 import os
 
 import numpy as np
 
 from . import _native as nat
+from .build import CSRC
 
 DEFAULT_CACHE = os.path.join(os.path.expanduser('~'), '.cache', 'pypercolate_gb300',
                              'autotune.json')
@@ -39,9 +43,19 @@ def _candidates(nmax, free_bytes):
     return out or [(8192, 128, 0)]
 
 
+@functools.lru_cache(maxsize=None)
+def _kernels(path):
+    """Digest of the kernels' sources."""
+    digest = hashlib.sha256()
+    for name in sorted(os.listdir(path)):
+        with open(os.path.join(path, name), 'rb') as f:
+            digest.update(name.encode() + b'\0' + f.read() + b'\0')
+    return digest.hexdigest()[:16]
+
+
 def _key(spec_tuple):
     torch = nat.torch_cuda()
-    return '%s|%s' % (torch.cuda.get_device_name(), ','.join(map(str, spec_tuple)))
+    return '%s|%s|%s' % (torch.cuda.get_device_name(), _kernels(CSRC), ','.join(map(str, spec_tuple)))
 
 
 def tune_mix(n_runs, grid=(8, 512), chain=(1024, 65536), chain_share=0.5, checkpoints=256,
