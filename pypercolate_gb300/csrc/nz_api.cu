@@ -780,9 +780,10 @@ size_t mix_layout(Carver &c, const NzMixSpec &sp, int32_t n_runs, int32_t T, Mix
     L.queue = c.take<uint32_t>(n_runs);
     L.begin = c.take<uint32_t>(kMixSegments + 1);
     L.head = c.take<uint32_t>(kMixSegments);
-    L.nodes = c.take<uint32_t>((size_t)T * nmax);
-    L.home_words = nmax;
     L.fused = sp.reduction == NZ_MIX_REDUCE_FUSED;
+    L.home_words = nmax;
+    L.node_words = mix_node_words(nmax, n_runs, T);
+    L.nodes = c.take<uint32_t>(L.node_words);
     L.rec = MixRec{};
     L.cells = nullptr;
     if (L.fused) {
@@ -833,7 +834,6 @@ int nz_mix(const NzMixSpec *spec, const uint32_t *thr_grid, const uint32_t *thr_
     L.m.thr_grid = thr_grid;
     L.m.thr_chain = thr_chain;
     L.m.F = spec->checkpoints;
-    L.T = threads;
     L.acc.count = out->count;
     L.acc.span = out->span;
     L.acc.sum_lo = out->sum_lo;

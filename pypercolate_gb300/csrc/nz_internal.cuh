@@ -180,14 +180,16 @@ struct MixLaunch {
     MixDev m;
     uint32_t *cls, *counts, *order, *offsets, *cursor, *queue;
     uint32_t *begin, *head;  // [kMixSegments + 1], [kMixSegments]
-    uint32_t *nodes;         // [T][home_words]
-    uint64_t home_words;
-    int32_t T;
+    uint32_t *nodes;         // [node_words]
+    uint64_t node_words;
+    uint64_t home_words;     // of the largest lattice
     bool fused;       // NZ_MIX_REDUCE_FUSED: cells, else records + mix_reduce_kernel
     MixRec rec;       // [n_runs][F] per plane (records only)
     uint64_t *cells;  // [classes][F][kMixCellWords] (fused only)
     MixAccum acc;
 };
+// node words in global memory that launch_mix uses, of at most T slots of home_words
+uint64_t mix_node_words(uint64_t home_words, int32_t n_runs, int32_t T);
 int launch_mix(const MixLaunch &p, cudaStream_t s);
 
 }  // namespace nz

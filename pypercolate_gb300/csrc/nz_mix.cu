@@ -559,21 +559,35 @@ static int launch_segment(const MixLaunch &p, int segment, uint32_t words, int p
     const size_t smem = (size_t)claims * 4u + nodes;
     int blocks = 152 * per_sm;
     if (blocks > p.m.n_runs) blocks = p.m.n_runs;
-    if (!SHARED && blocks > p.T) blocks = p.T;  // one node array each
+    if (!SHARED) blocks = (int)std::min<uint64_t>(blocks, p.node_words / p.home_words);  // one node array each
     return launch_kernel(mix_group_kernel<W, SHARED, FUSED>, dim3(blocks), 32 * W, smem, group::most_shared<W, SHARED>(), s, p,
                          segment, claims, p.home_words) == cudaSuccess
                ? NZ_OK
                : NZ_ERR_CUDA;
 }
 
-// Node words that the slots of segment k's threads have, and their number: 6 blocks
-// to an SM, as far as the caller's slots reach.
+constexpr uint64_t kMostThreads = 152ull * 6 * kMixThreads;  // 6 blocks to an SM
+constexpr uint64_t kMostHomes = 152ull * 2;                   // blocks of the largest lattices
+constexpr int32_t kFewestThreads = 20000;                     // runs for which there are no threads below
+
+// A place for each resident run beyond shared memory, or a slot for each thread of
+// the fused reduction (a size for both reductions); the segments run one after
+// another.
+uint64_t mix_node_words(uint64_t home_words, int32_t n_runs, int32_t T) {
+    const uint64_t runs = (uint64_t)n_runs;
+    const uint64_t homes = home_words > segment_words(0) ? std::min(kMostHomes, runs) * home_words : 0;
+    const uint64_t threads =
+        n_runs >= kFewestThreads ? std::min(kMostThreads, runs) * std::min<uint64_t>(segment_words(2), home_words) : 0;
+    return std::min((uint64_t)T * home_words, std::max(homes, threads));
+}
+
+// Node words that the slots of segment k's threads have, and their number, as far as
+// the slots reach.
 static uint32_t thread_words(const MixLaunch &p, int k) {
     return (uint32_t)std::min<uint64_t>(segment_words(k - 1), p.home_words);
 }
 static uint32_t thread_count(const MixLaunch &p, int k) {
-    const uint64_t slots = (uint64_t)p.T * p.home_words / thread_words(p, k);
-    return (uint32_t)std::min<uint64_t>({152ull * 6 * kMixThreads, slots, (uint64_t)p.m.n_runs});
+    return (uint32_t)std::min<uint64_t>({kMostThreads, p.node_words / thread_words(p, k), (uint64_t)p.m.n_runs});
 }
 
 // Runs that segment k can expect, its lengths being log-uniform.
@@ -601,7 +615,7 @@ static double expected_runs(const MixLaunch &p, int k) {
 // 33-64 and chains 2000-4096 171 and 83, 10^5 57 and 37, 3 10^4 17.6 and 27.
 static bool mix_threads(const MixLaunch &p, int k) {
     const double runs = expected_runs(p, k);
-    return thread_count(p, k) >= std::min(runs, 65536.0) && runs >= (k == 4 ? 20000.0 + 100.0 * thread_words(p, k) : 50000.0);
+    return thread_count(p, k) >= std::min(runs, 65536.0) && runs >= (k == 4 ? kFewestThreads + 100.0 * thread_words(p, k) : 50000.0);
 }
 
 static int launch_threads(const MixLaunch &p, int k, cudaStream_t s) {
