@@ -2,16 +2,15 @@
 
 tune_mix       batched uneven ensembles (``nz_mix``): the reduction (per-run
                checkpoint records reduced by a second kernel, or fused into
-               the union-find as exact integer atomics) and the node slots of
-               the lattices too large for shared memory.
+               the union-find as exact integer atomics).
 tune_ensemble  one lattice per ensemble (``nz_ensemble_tuned``): the record
                window (rows reduced and convolved per pass: the reduction
                tiling over n), its schedule and the slices of runs of the
                canonical run reduction (its tiling over runs).
 
-Both also time arguments that the kernels no longer depend on (threads per
-CTA, probability tiles, node slots in shared memory), which callers and cached
-results may name.
+Arguments that the kernels do not depend on (threads per CTA, probability tiles,
+node slots in shared memory) are left at their defaults; a caller's candidates may
+name them.
 
 Each candidate runs the same workload, timed with CUDA events on the
 launching stream; the fastest wins.  Results are cached in a JSON file keyed
@@ -32,15 +31,8 @@ DEFAULT_CACHE = os.path.join(os.path.expanduser('~'), '.cache', 'pypercolate_gb3
                              'autotune.json')
 
 
-def _candidates(nmax, free_bytes):
-    """(node slots, threads per CTA, shared-memory words) to try."""
-    out = []
-    for threads, block, smem in ((49152, 128, 0), (65536, 128, 0), (98304, 128, 0),
-                                 (131072, 128, 0), (65536, 64, 0), (98304, 64, 0),
-                                 (65536, 128, 64), (98304, 128, 128)):
-        if 4 * nmax * threads <= 0.6 * free_bytes:
-            out.append((threads, block, smem))
-    return out or [(8192, 128, 0)]
+# (node slots, threads per CTA, shared-memory words): more slots than any launch uses
+_MIX_SHAPES = [(49152, 128, 0)]
 
 
 @functools.lru_cache(maxsize=None)
@@ -62,8 +54,9 @@ def tune_mix(n_runs, grid=(8, 512), chain=(1024, 65536), chain_share=0.5, checkp
              sample_runs=None, cache_path=DEFAULT_CACHE, candidates=None, key=7):
     """Best (threads, block, smem_words, fused) for this workload and the
     table of all timings: {'best': (...), 'table': [(threads, block, smem,
-    fused, G adds/s), ...]}.  The launch shapes are timed with the records
-    reduction; the fastest shape is then timed with the fused reduction too."""
+    fused, G adds/s), ...]}.  The launch shapes (one, unless `candidates` names
+    others) are timed with the records reduction; the fastest shape is then timed
+    with the fused reduction too."""
     from .mix import MixEnsemble
     torch = nat.torch_cuda()
     spec = ('mix2', n_runs, grid[0], grid[1], chain[0], chain[1], chain_share, checkpoints)
@@ -78,9 +71,7 @@ def tune_mix(n_runs, grid=(8, 512), chain=(1024, 65536), chain_share=0.5, checkp
         hit = cache[ck]
         return {'best': tuple(hit['best']), 'table': hit['table'], 'cached': True}
     sample = int(min(n_runs, sample_runs or n_runs))
-    nmax = max(grid[1] ** 2, chain[1])
-    free, _ = torch.cuda.mem_get_info()
-    cands = candidates or _candidates(nmax, free)
+    cands = candidates or _MIX_SHAPES
 
     def timed(threads, block, smem, fused):
         ens = MixEnsemble(sample, grid=grid, chain=chain, chain_share=chain_share,
@@ -120,15 +111,14 @@ def default_window(M, n_runs):
 
 
 def ensemble_candidates(M, n_runs):
-    """The library's defaults, then one launch-shape change at a time.
-    (uf_block, m2_tile and conv_tile have no effect: the library's kernels
-    choose their blocks by the sizes.)"""
+    """The library's defaults, then one launch-shape change at a time (of those
+    that have an effect: the library's kernels choose uf_block, m2_tile and
+    conv_tile by the sizes)."""
     w = default_window(M, n_runs)
     base = {'uf_block': 128, 'm2_tile': 8, 'conv_tile': 8, 'taper': 0,
             'reduce_slices': 64 if n_runs >= 65536 else 16, 'window': w}
     out = [dict(base)]
-    for key, vals in (('uf_block', (64, 32)), ('m2_tile', (16,)), ('conv_tile', (16,)), ('taper', (1,)),
-                      ('window', (min(M + 1, max(256, w // 2)), min(M + 1, (3 * w) // 2))),
+    for key, vals in (('taper', (1,)), ('window', (min(M + 1, max(256, w // 2)), min(M + 1, (3 * w) // 2))),
                       ('reduce_slices', (16 if base['reduce_slices'] != 16 else 64, 256))):
         for v in vals:
             c = dict(base)
