@@ -602,8 +602,7 @@ __global__ void __launch_bounds__(kConvRuns) conv_window_kernel(ConvParams p) {
             double *o = p.acc + ((size_t)r * p.P + pi) * 7;
             o[s] += acc[j];
             if (MAXSET) {
-                // (a p that is no number makes this no number too)
-                if (p.spanning) o[0] += fma(0.0, acc[j], acc0[j]);
+                if (p.spanning) o[0] += acc0[j];
                 o[3] += acc3[j];
             }
         }
