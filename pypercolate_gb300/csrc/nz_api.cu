@@ -151,7 +151,7 @@ int nz_microcanonical(const NzGraph *graph, int32_t spanning, int32_t n_runs, in
     micro_layout(c, g, n_runs, perm_mode, &nodes, &state, &flag, &mt_perms);
     if (!workspace || !c.ok()) return NZ_ERR_WORKSPACE;
     cudaStream_t s = as_stream(stream);
-    const uint32_t *init_flag = launch_init_runs(g, n_runs, nodes, state, flag, s);
+    const uint32_t *init_flag = launch_init_flag(g, flag, s);
     const uint32_t *perm_src = perms;
     int mode = perm_mode;
     if (perm_mode == NZ_PERM_MT19937) {
@@ -611,7 +611,6 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning, int32_t n_runs, ui
     {
         ProfScope prof(NZ_PROF_SETUP, s);
         if (cudaMemsetAsync(L.flag, 0, 4 * sizeof(uint32_t), s) != cudaSuccess) return NZ_ERR_CUDA;
-        launch_init_runs(g, n_runs, L.nodes, L.state, L.flag, s);
     }
 
     AuxGuard aux{aux_checkout()};

@@ -288,16 +288,6 @@ __device__ __forceinline__ void decode_edge_slots(const GraphDev &g, uint32_t e,
     }
 }
 
-// slot of node i (see decode_edge_slots)
-template <int KIND>
-__device__ __forceinline__ uint32_t node_slot(const GraphDev &g, uint32_t i) {
-    if (KIND == NZ_GRAPH_GRID2D && kGridTiled) {
-        const uint32_t r = i / g.L;
-        return grid_slot(g.tile_cols, r, i - r * g.L);
-    }
-    return i;
-}
-
 template <int KIND>
 __device__ __forceinline__ uint32_t node_sides(const GraphDev &g, uint32_t i) {
     if (KIND == NZ_GRAPH_GRID2D) {

@@ -45,10 +45,8 @@ struct UfParams {
 };
 
 // nz_uf.cu
-// sets up the runs as far as launch_uf_window does not do so itself; returns
-// UfParams::init_flag
-const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
-                                 uint32_t *flag_scratch, cudaStream_t s);
+// explicit edge lists: UfParams::init_flag, in the caller's word (other graphs: null)
+const uint32_t *launch_init_flag(const GraphDev &g, uint32_t *flag_scratch, cudaStream_t s);
 cudaError_t launch_uf_window(const UfParams &p, int perm_mode, bool span, cudaStream_t s);
 void launch_philox_perms(uint32_t M, int32_t n_runs, uint64_t key, uint64_t run0, uint32_t *out,
                          cudaStream_t s);

@@ -58,9 +58,7 @@ __global__ void pack_rows_kernel(NzRecords rec, int32_t run, uint32_t N, uint32_
 }
 
 // ------------------------------------------------------------ launchers
-const uint32_t *launch_init_runs(const GraphDev &g, int32_t n_runs, uint32_t *nodes, RunState *state,
-                                 uint32_t *flag_scratch, cudaStream_t s) {
-    // the union-find kernel initialises its runs itself
+const uint32_t *launch_init_flag(const GraphDev &g, uint32_t *flag_scratch, cudaStream_t s) {
     if (g.kind != NZ_GRAPH_EDGES) return nullptr;
     cudaMemsetAsync(flag_scratch, 0, sizeof(uint32_t), s);
     any_both_sides_kernel<<<(g.N + 255) / 256 < 1024 ? (g.N + 255) / 256 : 1024, 256, 0, s>>>(g, flag_scratch);

@@ -67,9 +67,6 @@ __device__ __forceinline__ double u256_to_f64(const U256 &a) {
     const double t64 = 18446744073709551616.0;
     return ((a.w[3] * t64 + (double)a.w[2]) * t64 + (double)a.w[1]) * t64 + (double)a.w[0];
 }
-__device__ __forceinline__ double u128_f64(u128 x) {
-    return fma((double)(uint64_t)(x >> 64), 18446744073709551616.0, (double)(uint64_t)x);
-}
 
 // running sum of 128-bit terms
 struct U192 {
