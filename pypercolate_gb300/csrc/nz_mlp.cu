@@ -82,10 +82,24 @@ constexpr uint32_t kGSbo = (kGK / 8) * tc::kCoreBytes;
 struct GemmSmem {
     __nv_bfloat16 a[2][kGM * kGK];
     __nv_bfloat16 b[2][kGN * kGK];
-    float part[kGThreads];
+    float2 part[kGThreads];
     float bias[kGN];
     uint64_t mbar[2];
     uint32_t tmem;
+};
+
+// A running FP32 sum and its rounding errors.
+struct ColSum {
+    float s = 0.0f, c = 0.0f;
+    __device__ __forceinline__ void add(float x) {
+        const float t = s + x, b = t - s;  // TwoSum
+        c += (s - (t - b)) + (x - b);
+        s = t;
+    }
+    __device__ __forceinline__ void add8(const float (&v)[8]) {
+        add(((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+    }
+    __device__ __forceinline__ float value() const { return s + c; }
 };
 
 __device__ uint32_t g_mlp_errors;  // tiles whose mbarrier waits gave up
@@ -156,7 +170,7 @@ __device__ __forceinline__ void load8(const T *src, int64_t s_row, int64_t s_k, 
 // store.  colsum: += this thread's values of row t % tile.
 template <int TILE, bool WIDE, bool COLSUM, class T>
 __device__ __forceinline__ void stage_operand(__nv_bfloat16 *dst, const T *src, int64_t s_row, int64_t s_k, int row0,
-                                              int rows, int tile, int k0, int K, float &colsum) {
+                                              int rows, int tile, int k0, int K, ColSum &colsum) {
     const bool k_fast = s_k == 1 && !COLSUM;
     // items: (row, group of 8 k).  K contiguous: 8 rows x 4 groups per warp
     // (128 contiguous bytes of each row); else 32 rows per warp
@@ -173,10 +187,7 @@ __device__ __forceinline__ void stage_operand(__nv_bfloat16 *dst, const T *src, 
     }
 #pragma unroll
     for (int q = 0; q < kItems; ++q) {
-        if (COLSUM) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) colsum += v[q][k];
-        }
+        if (COLSUM) colsum.add8(v[q]);
         if (at[q] >= 0)
             *reinterpret_cast<uint4 *>(dst + at[q]) =
                 make_uint4(pack_bf16(v[q][0], v[q][1]), pack_bf16(v[q][2], v[q][3]), pack_bf16(v[q][4], v[q][5]),
@@ -206,7 +217,12 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
     K = min(K - kb, k_split);
     float *C = out.C + blockIdx.z * out.slice;
     const float *A = in.A + (int64_t)kb * in.sak;
-    const uint32_t cols = ntile <= 32 ? 32u : 64u;  // TMEM: power of two >= 32
+    constexpr bool kSums = sizeof(T) == 4;  // FP32 B: the gradient of the pre-activations
+    // TMEM: a power of two >= 32.  The weight gradients (long sums over the batch, in
+    // FP32 that the tensor cores round toward zero) have two accumulators, of half a
+    // slice's chunks each: 16 slices are as accurate as 32 were (positive values,
+    // 8,192 samples: 2.6e-8 of the sum on average, 2.3e-7 with one accumulator)
+    const uint32_t acc_cols = ntile <= 32 ? 32u : 64u, cols = kSums ? 2u * acc_cols : acc_cols;
     start_next();
     // rows t % 128 of C; threads 128 .. 255 take columns 32 .. 63
     const int m = m0 + (t & 127), j0 = (t >> 7) * 32;
@@ -225,9 +241,8 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
     const uint32_t tmem = sh.tmem;
     wait_previous();
     if (t < ntile) sh.bias[t] = out.bias && n0 + t < N ? out.bias[n0 + t] : 0.0f;
-    const int nch = (K + kGK - 1) / kGK;
-    constexpr bool kSums = sizeof(T) == 4;  // FP32 B: the gradient of the pre-activations
-    float colsum = 0.0f, none = 0.0f;
+    const int nch = (K + kGK - 1) / kGK, half = kSums ? (nch + 1) / 2 : nch;  // chunks of the first accumulator
+    ColSum colsum, none;
     const bool sums = kSums && out.colsum && blockIdx.y == 0;
     const T *B = in.B + (int64_t)kb * in.sbk;
     auto stage = [&](int c, int buf) {
@@ -248,9 +263,9 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
 #pragma unroll
             for (int ks = 0; ks < kGK / 16; ++ks) {
                 const uint32_t o = (uint32_t)ks * 2 * tc::kCoreBytes;  // K = 16: two core matrices
-                mma_bf16(tmem, tc::smem_desc(a0 + o, tc::kCoreBytes, kGSbo),
+                mma_bf16(c < half ? tmem : tmem + acc_cols, tc::smem_desc(a0 + o, tc::kCoreBytes, kGSbo),
                          tc::smem_desc(b0 + o, tc::kCoreBytes, kGSbo), bf16_idesc(ntile),
-                         (c > 0 || ks > 0) ? 1u : 0u);
+                         ((c > 0 && c != half) || ks > 0) ? 1u : 0u);
             }
             tc::mma_commit(tc::smem_u32(&sh.mbar[buf]));
         }
@@ -262,7 +277,7 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
     }
     // MMAs complete in order: the last chunk issued covers them all
     if (c > 0 && !tc::mbar_wait(tc::smem_u32(&sh.mbar[(c - 1) & 1]), ((c - 1) >> 1) & 1)) bad = true;
-    sh.part[t] = colsum;
+    sh.part[t] = make_float2(colsum.s, colsum.c);
     tc::fence_before();
     const bool any_bad = __syncthreads_or(bad) || c < nch;
     tc::fence_after();
@@ -286,7 +301,15 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
             for (int j = 0; j < 32; ++j) v[j] = __int_as_float(0x7fc00000);
             if (t == 0) atomicAdd(&g_mlp_errors, 1u);
         } else {
-            tc::tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)j0, v);
+            const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)j0;
+            tc::tmem_ld32(at, v);
+            if constexpr (kSums) {
+                if (half < nch) {
+                    tc::tmem_ld32(at + acc_cols, z);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] += z[j];
+                }
+            }
         }
         if (m < M) {
             const bool store_z = out.Z && out.epi != Epi::kBack;
@@ -318,9 +341,12 @@ __global__ void __launch_bounds__(kGThreads) mlp_gemm_kernel(int M, int N, int K
     }
     // column sums: the threads that staged one column, in order
     if (sums && t < ntile && n0 + t < N) {
-        float x = 0.0f;
-        for (int q = t; q < kGThreads; q += ntile) x += sh.part[q];
-        out.colsum[blockIdx.z * out.slice + n0 + t] = any_bad ? __int_as_float(0x7fc00000) : x;
+        ColSum x;
+        for (int q = t; q < kGThreads; q += ntile) {
+            x.add(sh.part[q].x);
+            x.c += sh.part[q].y;
+        }
+        out.colsum[blockIdx.z * out.slice + n0 + t] = any_bad ? __int_as_float(0x7fc00000) : x.value();
     }
     tc::fence_before();
     __syncthreads();
@@ -336,10 +362,10 @@ __global__ void splitk_sum_kernel(const float *slices, int splits, int64_t strid
     start_next();
     wait_previous();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-        float acc = 0.0f;
+        ColSum acc;
 #pragma unroll 8
-        for (int z = 0; z < splits; ++z) acc += slices[z * stride + i];
-        out[i] = acc;
+        for (int z = 0; z < splits; ++z) acc.add(slices[z * stride + i]);
+        out[i] = acc.value();
     }
 }
 
