@@ -1145,13 +1145,13 @@ __device__ __forceinline__ void micro_accumulate(const MicroParams &p, const Mic
     p.acc.m2[idx] = ss;
 }
 
-// Slice blockIdx.y of the runs; with more than one slice its sums go to p.part.
-template <bool NARROW>
+// SLICED: slice blockIdx.y of the runs, whose sums go to p.part.
+template <bool NARROW, bool SLICED>
 __global__ void __launch_bounds__(32 * kMicroWarps, 2) micro_tiled_kernel(MicroParams p, int slice) {
     __shared__ MicroSums<NARROW> s_sum[32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t i = blockIdx.x * 32u + lane;
-    const int r0 = (int)blockIdx.y * slice, r1 = min(r0 + slice, p.n_runs);
+    const int r0 = SLICED ? (int)blockIdx.y * slice : 0, r1 = SLICED ? min(r0 + slice, p.n_runs) : p.n_runs;
     const NzRecords &rec = p.rec;
     MicroSums<NARROW> a = {};
     uint64_t q_max = 0, q_m0 = 0, s_m2 = 0;  // per thread: at most 2^20 runs' values < 2^42
@@ -1204,7 +1204,7 @@ __global__ void __launch_bounds__(32 * kMicroWarps, 2) micro_tiled_kernel(MicroP
     a.q_max = q_max;
     a.q_m0 = q_m0;
     micro_combine<NARROW>(a, s_sum);
-    if (gridDim.y == 1) {
+    if constexpr (!SLICED) {
         micro_accumulate<NARROW>(p, s_sum);
     } else if (warp == 0) {
         reinterpret_cast<MicroSums<NARROW> *>(p.part)[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 32 + lane] =
@@ -1236,8 +1236,12 @@ static void launch_micro_tiled(const MicroParams &p, uint32_t rows, cudaStream_t
     const int blocks = (int)((rows + 31) / 32);
     const int slices = std::max(1, std::min(kMicroBlocks / blocks, p.n_runs / kMicroSliceRuns));
     const int slice = (p.n_runs + slices - 1) / slices;
-    micro_tiled_kernel<NARROW><<<dim3(blocks, slices), 32 * kMicroWarps, 0, s>>>(p, slice);
-    if (slices > 1) micro_slices_kernel<NARROW><<<blocks, 32 * kMicroWarps, 0, s>>>(p, slices);
+    if (slices == 1) {
+        micro_tiled_kernel<NARROW, false><<<blocks, 32 * kMicroWarps, 0, s>>>(p, p.n_runs);
+        return;
+    }
+    micro_tiled_kernel<NARROW, true><<<dim3(blocks, slices), 32 * kMicroWarps, 0, s>>>(p, slice);
+    micro_slices_kernel<NARROW><<<blocks, 32 * kMicroWarps, 0, s>>>(p, slices);
 }
 
 size_t micro_part_bytes() { return sizeof(MicroSums<false>) * 32 * kMicroBlocks; }
