@@ -614,7 +614,7 @@ def main():
         torch.cuda.empty_cache()
 
     # batched uneven workload: 10^6 runs, 2D L log-uniform in [8, 512] and
-    # chains l log-uniform in [1024, 65536], 50/50, one persistent launch per
+    # chains l log-uniform in [1024, 65536], 50/50, one launch sequence per
     # ensemble replayed as a CUDA graph; reduction from the autotuner
     mix = None
     if args.mix_runs > 0:
@@ -688,8 +688,8 @@ def main():
                                   R, args.P, not args.no_micro),
                    'L': L, 'N': N, 'M': M, 'runs_per_step': R, 'P': args.P,
                    'precision': args.precision, 'l2_fetch_bytes': l2_fetch,
-                   'l2': 'inputs larger than L2 (%.1f GB of union-find state per step)'
-                         % (R * N * 4 / 1e9)},
+                   'l2': 'inputs larger than L2 (%.1f GB of records written and read per step)'
+                         % (R * (M + 1) * uf_bytes / 1e9)},
         'roofline': {'bound': 'instruction latency (node words in shared memory; HBM carries the records only)',
                      'achieved': achieved, 'peak': peak, 'unit': 'GB/s',
                      'frac': achieved / peak, 'traffic': UF_TRAFFIC_PER_ADD * adds_per_launch,

@@ -387,7 +387,7 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning,
                       double *acc_mean, double *acc_m2,
                       const NzMicroAccum *micro, void *stream);
 
-/* ---- batched uneven ensembles (one persistent launch) ------------------ */
+/* ---- batched uneven ensembles ------------------------------------------ */
 /* Run r draws its substrate from Philox-4x32-10 (key, counter r): a chain
  * with probability chain_share / 2^32, else a square lattice; the length L
  * (or l) is the largest grid_min + i (chain_min + i) with thr[i] <= u, u a
@@ -399,7 +399,7 @@ int nz_ensemble_tuned(const NzGraph *graph, int32_t spanning,
  * spanning counts (percolate/percolate.py:450-705 statistics at those n).
  * `reduction` picks how (identical results): NZ_MIX_REDUCE_RECORDS -- each
  * run writes its checkpoint statistics, a second kernel reduces them per
- * class; NZ_MIX_REDUCE_FUSED -- the union-find threads add each run's
+ * class; NZ_MIX_REDUCE_FUSED -- the union-find adds each run's
  * statistics and squares into its class's sums themselves (exact integer
  * atomics), and a per-cell kernel only forms the outputs.  The fused form
  * needs no per-run records and is faster where lattices have many runs each;
@@ -426,9 +426,10 @@ typedef struct NzMixAccum {
     uint32_t *errors;  /* [1] runs skipped by a failed internal check (0)    */
 } NzMixAccum;
 
-/* Workspace for n_runs runs with `threads` node slots in global memory, each
- * sized for the largest lattice of the spec (only lattices beyond 65,536 node
- * words use them, one per resident run).  Beside the node slots: per-run
+/* Workspace for n_runs runs with at most `threads` node slots in global memory,
+ * each sized for the largest lattice of the spec; no more of them than there are
+ * resident runs beyond 65,536 node words (304), or than 116,736 threads of 4,096
+ * words take (very many small runs, fused).  Beside the node words: per-run
  * checkpoint records (36 B per run and checkpoint) for NZ_MIX_REDUCE_RECORDS,
  * per-class sums (216 B per class and checkpoint) for NZ_MIX_REDUCE_FUSED. */
 size_t nz_mix_workspace_bytes(const NzMixSpec *spec, int32_t n_runs,
@@ -436,8 +437,8 @@ size_t nz_mix_workspace_bytes(const NzMixSpec *spec, int32_t n_runs,
 /* key_dev: device pointer to the Philox key (read by the kernels, so a
  * captured CUDA graph of this call can be replayed with another key).
  * threads: node slots (at most that many of the largest lattices run at a
- * time); block and smem_words are checked and have no effect: a thread block
- * takes a run, its size and memory chosen by the lattice's.
+ * time); block and smem_words are checked and have no effect: a thread block,
+ * or a thread, takes a run, by the lattice's size and the number of runs.
  * Output arrays are overwritten (not accumulated). */
 int nz_mix(const NzMixSpec *spec, const uint32_t *thr_grid,
            const uint32_t *thr_chain, const uint64_t *key_dev, int32_t n_runs,

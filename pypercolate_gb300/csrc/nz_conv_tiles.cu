@@ -17,8 +17,9 @@
 // and m4, 0.86 for m2.  Reading the rows of one run straight from global memory,
 // 16 bytes per thread and 128 bytes apart, kept the load pipe busy 80 % of the
 // time and took 0.48, 2.0 (m0, m3 and m4) and 0.92 ms; 16 probabilities per CTA
-// in two groups of threads 0.54, 0.27, 0.32 and 1.06.  What bounds it now: the
-// FP32 pipe for max and m2, the three CTAs that fit an SM for m3 and m4.
+// in two groups of threads 0.54, 0.27, 0.32 and 1.06.  What bounds it now (4,000 runs
+// at L = 64, profiled): the issue slots, 78 % used by m2 (FMA pipe 49 %), 62 % by max
+// (ALU pipe 51 %, FMA 25 %); 43 % by m3 and m4, of which three CTAs fit an SM.
 #include <cstdint>
 #include <type_traits>
 

@@ -43,9 +43,11 @@
 // nz_common.cuh in global memory, of which the resident blocks' ones stay
 // near L2's size.
 //
-// What bounds it: dependent integer instructions (about 700 warp instructions
-// per 32 bonds, each waiting 4 to 6 cycles for the one before), so warps per SM
-// are worth more than anything; memory is idle.
+// What bounds it: dependent integer instructions and barriers (some 750 warp
+// instructions per 32 bonds at L = 64, 1,000 at L = 256, a warp's next one 7 and 11
+// cycles after the last), so warps per SM are worth more than anything; memory is
+// idle.  Very many runs of small lattices, and n-major records of very many runs, are
+// nz_uft.cu's.
 #pragma once
 
 #include <cstdint>

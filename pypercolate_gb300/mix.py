@@ -1,5 +1,5 @@
-"""Batched uneven ensembles: thousands of runs of different lattices in one
-persistent launch (libnzgb300 ``nz_mix``).
+"""Batched uneven ensembles: thousands of runs of different lattices in one call
+(libnzgb300 ``nz_mix``), one launch per range of sizes.
 
 Each run r draws its substrate from Philox(key, r): a spanning_1d_chain(l)
 with probability ``chain_share``, else a spanning_2d_grid(L), the length
@@ -8,7 +8,7 @@ log-uniform in its range and rounded to the nearest integer
 ``checkpoints`` evenly spaced occupation numbers to exact sums and M2 of the
 microcanonical statistics (percolate/percolate.py:450-705 at those n).
 
-``fused=True`` reduces the runs inside the persistent union-find (each run
+``fused=True`` reduces the runs inside the union-find (each run
 adds its statistics and their squares into its lattice's exact sums by
 integer atomics) instead of writing per-run checkpoint records for a second
 kernel; the results are identical.
