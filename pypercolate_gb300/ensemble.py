@@ -56,7 +56,8 @@ class Ensemble:
     micro     also accumulate microcanonical run-reductions for every n
     window    rows per union-find launch (0: sized to ~32 GiB of records per window)
     tuning    launch shapes {'uf_block', 'm2_tile', 'reduce_slices', 'conv_tile', 'taper'}
-              (autotune.tune_ensemble picks them; None: the library's defaults)
+              (autotune.tune_ensemble picks them; None: the library's defaults);
+              reduce_slices and taper alone have an effect
     """
 
     def __init__(self, kind='grid', length=16, ps=None, spanning=True, precision='fp32',
