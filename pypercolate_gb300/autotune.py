@@ -32,7 +32,8 @@ DEFAULT_CACHE = os.path.join(os.path.expanduser('~'), '.cache', 'pypercolate_gb3
 
 
 # (node slots, threads per CTA, shared-memory words): more slots than any launch uses
-_MIX_SHAPES = [(49152, 128, 0)]
+# (116,736, by the threads of the fused reduction; the workspace holds no more)
+_MIX_SHAPES = [(131072, 128, 0)]
 
 
 @functools.lru_cache(maxsize=None)

@@ -35,3 +35,21 @@ def test_one_shape_of_uneven_batches():
     depends on them."""
     from pypercolate_gb300 import autotune as A
     assert len(A._MIX_SHAPES) == 1 and A._MIX_SHAPES[0][0] >= 304
+
+
+@pytest.mark.parametrize('grid,chain', [((2, 16), (2, 64)), ((8, 64), (64, 4096)), ((8, 512), (1024, 65536))])
+@pytest.mark.parametrize('fused', [False, True])
+def test_uneven_batches_are_tuned_with_all_node_words(grid, chain, fused):
+    """The shape that is timed takes no slot from a batch of very many small
+    lattices: as much memory as with a slot for every run."""
+    pytest.importorskip('torch')
+    from pypercolate_gb300 import _native as nat
+    from pypercolate_gb300 import autotune as A
+    from pypercolate_gb300 import build
+    build.build()
+    spec = nat.NzMixSpec()
+    spec.grid_min, spec.grid_max = grid
+    spec.chain_min, spec.chain_max = chain
+    spec.chain_share, spec.checkpoints, spec.reduction = 1 << 31, 256, int(fused)
+    size = nat.lib_handle().nz_mix_workspace_bytes
+    assert size(spec, 10 ** 6, A._MIX_SHAPES[0][0]) == size(spec, 10 ** 6, 10 ** 6)
