@@ -13,20 +13,25 @@ namespace nz {
 // Launches with `smem` bytes of dynamic shared memory.  How much a kernel may be
 // given is a property of the kernel, for all host threads of the context alike: it
 // is set to `most`, the most that any call gives it, and so never taken from under
-// another thread's launch.
+// another thread's launch.  A failure is the returned status alone: it is not left
+// as the context's last error, which the next call's checks, here or in the caller's
+// program, would take for their own.
 template <class... P, class... A>
 cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, size_t most, cudaStream_t s,
                           A... args) {
-    if (most > 40 * 1024) {  // (with the static shared memory, beyond what is given unasked)
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    if (most > 40 * 1024)  // (with the static shared memory, beyond what is given unasked)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
 }
 
 struct UfParams {

@@ -1,6 +1,11 @@
 """Sizes at which a launch's grid or a block's memory ends, on the GPU."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
+
+from pypercolate_gb300 import build
 
 pytestmark = pytest.mark.gpu
 
@@ -74,3 +79,23 @@ def test_threads_with_blocks_of_different_memory(gpu, what):
     for t in threads:
         t.join()
     assert not failed
+
+
+def test_a_launch_that_fails_leaves_no_error_behind(gpu, tmp_path):
+    """What a launch returns, for a block or a shared-memory limit that the host
+    refuses, is not found again by the next call's check."""
+    source = tmp_path / 'refused.cu'
+    source.write_text('''
+#include <cstdio>
+#include "nz_internal.cuh"
+__global__ void nothing() {}
+int main() {
+    const bool block = nz::launch_kernel(nothing, dim3(1), 4096, 0, 0, nullptr) != cudaSuccess;
+    const bool limit = nz::launch_kernel(nothing, dim3(1), 32, 0, 1 << 30, nullptr) != cudaSuccess;
+    printf("%d %d %d\\n", block, limit, (int)cudaPeekAtLastError());
+}
+''')
+    program = str(tmp_path / 'refused')
+    subprocess.run([build.nvcc(), *build.ARCH, '-std=c++17', '--expt-relaxed-constexpr', '-I', build.CSRC, '-I',
+                    os.path.join(os.path.dirname(build.HERE), 'include'), '-o', program, str(source)], check=True)
+    assert subprocess.run([program], check=True, capture_output=True, text=True).stdout.split() == ['1', '1', '0']
