@@ -99,7 +99,8 @@ struct ColSum {
     __device__ __forceinline__ void add8(const float (&v)[8]) {
         add(((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
     }
-    __device__ __forceinline__ float value() const { return s + c; }
+    // (of a sum with an infinity the errors are no numbers, and the sum is what it is)
+    __device__ __forceinline__ float value() const { return isfinite(c) ? s + c : s; }
 };
 
 __device__ uint32_t g_mlp_errors;  // tiles whose mbarrier waits gave up
