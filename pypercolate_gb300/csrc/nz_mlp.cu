@@ -71,7 +71,7 @@ static void launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t 
 // one 16-byte shared-memory store whose 8-lane phases cover 128 bytes; all loads
 // of a chunk, and of the epilogue, are issued before the first is used.  A
 // launch by itself, from cold caches, takes 10 to 17 us; one element at a time, with
-// two divisions each and 2-byte stores, it took 38.  A step of 22 launches takes 175
+// two divisions each and 2-byte stores, it took 38.  A step of 22 launches takes 176
 // us, 210 when each waits for the one before to drain.  64-column tiles put 64 CTAs on a batch of 4096.
 constexpr int kGM = 128;   // rows of C per CTA (TMEM lanes)
 constexpr int kGK = 64;    // K per staged chunk: 4 MMAs of K = 16
